@@ -15,6 +15,13 @@ enum DeviceError : int {
     kDevMbarrierTimeout = 1,   // a bounded mbarrier wait ran out
 };
 
+// The engine's error word lies in pinned host memory: a run that meets no error never touches it, so clearing it and
+// reading it back cost no device work.  (Plain store: there is one code.)
+__device__ __forceinline__ void record_error(int32_t *err, DeviceError code) {
+    *reinterpret_cast<volatile int32_t *>(err) = code;
+    __threadfence_system();
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

@@ -379,7 +379,7 @@ sddmm_dense_tile_kernel(const DenseArgs args, const __grid_constant__ CUtensorMa
                     if (j + 2 < static_cast<uint32_t>(my_jobs)) load_ids(j + 2, nxt0, nxt1);
                 }
             }
-            if (!ok) atomicCAS(args.err, kDevOk, kDevMbarrierTimeout);
+            if (!ok) record_error(args.err, kDevMbarrierTimeout);
         } else if (lane == 0) {
             bool ok = prod_ok;
             uint32_t jb = 0;  // jobs whose MMAs have been issued (phase of acc_free / acc_full)
@@ -405,7 +405,7 @@ sddmm_dense_tile_kernel(const DenseArgs args, const __grid_constant__ CUtensorMa
                 }
                 if (it + 1 < total && !issue_tma(it + 1)) { ok = false; break; }   // refill the operand buffer
             }
-            if (!ok) atomicCAS(args.err, kDevOk, kDevMbarrierTimeout);
+            if (!ok) record_error(args.err, kDevMbarrierTimeout);
         }
     } else {
         // ===================== epilogue warps =====================
@@ -523,7 +523,7 @@ sddmm_dense_tile_kernel(const DenseArgs args, const __grid_constant__ CUtensorMa
                 int got = 1;
                 if (lane == 0) {
                     got = (SPLIT3 ? mbar_wait_bounded(acc_full_of(jb & 1u), (jb >> 1) & 1u) : mbar_wait_bounded(acc_full, jb & 1u)) ? 1 : 0;
-                    if (!got) atomicCAS(args.err, kDevOk, kDevMbarrierTimeout);
+                    if (!got) record_error(args.err, kDevMbarrierTimeout);
                 }
                 __syncwarp();
                 ok = __shfl_sync(kFullMask, got, 0) != 0;

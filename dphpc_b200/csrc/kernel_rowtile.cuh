@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kRowTileWarps * 32, (CPL == 1) ? SDDMM_ROWTILE
             };
             if (wb < s_hi) request_window(wb);   // in flight while the A rows land
             if (!mbar_wait_bounded(&bar[b], (phases >> b) & 1u)) {
-                atomicCAS(args.err, kDevOk, kDevMbarrierTimeout);
+                record_error(args.err, kDevMbarrierTimeout);
                 // every thread of the CTA waits on the same phase, so all leave together -- after the copies
                 // already requested for the next stage have landed (bounded again)
                 cp_async_wait_all();
