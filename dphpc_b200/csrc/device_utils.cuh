@@ -191,4 +191,40 @@ __device__ __forceinline__ float group8_transpose_reduce(const float (&acc)[8], 
     return keep + __shfl_xor_sync(kFullMask, send, 1);
 }
 
+// ---- block-wide sums and scans (blocks of kPlanBlock threads) --------------------------------
+constexpr int kPlanBlock = 256;
+__device__ __forceinline__ int32_t warp_inclusive_scan(int32_t v, int lane) {
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int32_t t = __shfl_up_sync(kFullMask, v, off);
+        if (lane >= off) v += t;
+    }
+    return v;
+}
+// inclusive scan of one value per thread over a block of kPlanBlock threads; returns the thread's inclusive prefix,
+// *total = block sum
+__device__ __forceinline__ int32_t block_inclusive_scan(int32_t v, int32_t *total) {
+    __shared__ int32_t warp_sums[kPlanBlock / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int32_t inc = warp_inclusive_scan(v, lane);
+    if (lane == 31) warp_sums[w] = inc;
+    __syncthreads();
+    int32_t base = 0, tot = 0;
+#pragma unroll
+    for (int k = 0; k < kPlanBlock / 32; ++k) {
+        const int32_t t = warp_sums[k];
+        if (k < w) base += t;
+        tot += t;
+    }
+    __syncthreads();
+    *total = tot;
+    return inc + base;
+}
+// sum of one value per thread, to every thread
+__device__ __forceinline__ int32_t block_sum(int32_t v) {
+    int32_t total;
+    block_inclusive_scan(v, &total);
+    return total;
+}
+
 }  // namespace sddmm

@@ -27,6 +27,7 @@
 #include "kernel_rowtile.cuh"
 #include "kernel_spmm.cuh"
 #include "plan_kernels.cuh"
+#include "unit_plan.cuh"
 
 using namespace sddmm;
 
@@ -95,7 +96,8 @@ struct sddmm_b200_engine {
     float *d_sval = nullptr, *d_pval = nullptr;
     float *d_A32 = nullptr, *d_B32 = nullptr;
     __nv_bfloat16 *d_A16 = nullptr, *d_B16 = nullptr;
-    unsigned char *d_touched = nullptr;
+    uint32_t *d_touched = nullptr;      // one bit per column (with d_pc and d_rowstart in one piece that is cleared at once)
+    size_t plan_clear_bytes = 0;
     uint32_t *d_rowstart = nullptr;
     int2 *d_item_rows = nullptr;
     int32_t *d_coo_rows = nullptr;
@@ -137,11 +139,18 @@ struct sddmm_b200_engine {
 
     // row-segment path (short and power-law rows; column panels when B is much larger than L2)
     int2 *d_units = nullptr;
-    int32_t *d_unit_cols = nullptr;    // column panels: per-unit copies of column indices and S values, 8 slots of {column, value} per unit
-    float *d_unit_sval = nullptr;      // (the same array: the values are its odd words)
+    int32_t *d_unit_cols = nullptr;    // 8 column indices per unit
+    float *d_unit_sval = nullptr;      // column panels: 8 S values per unit
     bool seg_copies = false;           // ... in use by the current plan
-    int32_t *d_unit_off = nullptr;     // per (panel, row): units before it (scan of the counts)
+    int32_t *d_unit_off = nullptr;     // residual lists: per row, units before it (scan of the counts)
     int32_t *d_scan_tiles = nullptr;
+    // Operand rows as the row-segment kernels read them: rows of Ks elements, a multiple of 32 bytes.  Ks = K where K is
+    // one already (A, B themselves), else zero-padded copies.
+    int64_t Ks = 0;
+    float *d_Ap = nullptr, *d_Bp = nullptr;
+    bool d_Ap_wanted = false;
+    bool group_tried = false;          // a grouping was matched exactly and then dropped
+    bool copies_joined = false;        // the upload's copies and conversions are already ordered before the plan's read-back
     int64_t unit_cap = 0;
     int32_t panels = 1;                // column panels the unit list is ordered by
     int32_t panel_cols = 0;            // columns per panel
@@ -169,6 +178,7 @@ struct sddmm_b200_engine {
     int64_t spmm_k2 = 0;
     float *d_X = nullptr, *d_Y = nullptr;
     int2 *d_spmm_units = nullptr;
+    int32_t *d_spmm_cols = nullptr;
     cudaEvent_t ev_spmm0 = nullptr, ev_spmm1 = nullptr;
 
     // plan
@@ -301,6 +311,7 @@ double env_double(const char *name, double fallback) {
 // slice over the same unit list, each adding to P.val -- a slice of B is small enough for column panels to keep it in
 // L2, where the whole rows are not (knob "k_slices": 0 = never, 1 = whenever K allows).
 int choose_k_slices(const sddmm_b200_engine *e) {
+    if (e->K > 256) return static_cast<int>(e->Ks / 64);   // rows longer than the kernels' largest instantiation (Ks is a multiple of 64)
     if (e->mode == SDDMM_B200_BF16 || e->K < 128 || e->K % 64 != 0 || e->knob_k_slices == 0) return 1;
     const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20);
     if (e->knob_k_slices < 0 && static_cast<double>(e->N) * e->K * 4.0 <= 4.0 * l2) return 1;
@@ -318,7 +329,7 @@ int choose_k_slices(const sddmm_b200_engine *e) {
 bool long_rows_candidate(const sddmm_b200_engine *e) {
     if (e->knob_long_rows == 0) return false;
     const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20);
-    return static_cast<double>(e->N) * (e->seg_slices > 1 ? 64 : e->K) * static_cast<double>(elem_bytes(e)) > l2 &&
+    return static_cast<double>(e->N) * (e->seg_slices > 1 ? 64 : e->Ks) * static_cast<double>(elem_bytes(e)) > l2 &&
            e->nnz / std::max<int64_t>(1, 8 * e->M) < 2;
 }
 int choose_long_rows(const sddmm_b200_engine *e) {
@@ -331,14 +342,19 @@ int choose_panels(const sddmm_b200_engine *e) {
     if (e->knob_panels >= 1 && e->knob_panels <= 64) return static_cast<int>(e->knob_panels);
     if (long_rows_candidate(e)) {   // measured on the power-law configuration (B 333 MB): 4 panels 458 us, 6 446 us, 8 442-447 us
         const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20);
-        return static_cast<int>(std::max(2.0, std::min(8.0, std::ceil(static_cast<double>(e->N) * (e->seg_slices > 1 ? 64 : e->K) *
+        return static_cast<int>(std::max(2.0, std::min(8.0, std::ceil(static_cast<double>(e->N) * (e->seg_slices > 1 ? 64 : e->Ks) *
                                                                       static_cast<double>(elem_bytes(e)) / (0.5 * l2)))));
     }
     const double eb = static_cast<double>(elem_bytes(e));
-    const double b_bytes = static_cast<double>(e->N) * (e->seg_slices > 1 ? 64 : e->K) * eb;
+    const double b_bytes = static_cast<double>(e->N) * (e->seg_slices > 1 ? 64 : e->Ks) * eb;
     const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20);
     if (b_bytes <= l2) return 1;
-    if (e->mode == SDDMM_B200_BF16) return 1;   // measured: with bf16 storage the extra segments cost more than the saved DRAM reads
+    // bf16 storage, measured with 1.45 M rows of B: K = 64 (B 1.5 x L2) 590 / 618 / 634 us with 1 / 2 / 3 panels, K = 128 (3 x L2)
+    // 1809 / 1142 / 1092 / 1096 / 1150 us with 1 .. 5
+    if (e->mode == SDDMM_B200_BF16) {
+        if (b_bytes <= 2.0 * l2) return 1;
+        return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(static_cast<int64_t>(std::ceil(b_bytes / l2)), e->nnz / std::max<int64_t>(1, 8 * e->M)), 4)));
+    }
     // measured on B200 (126 MB of L2): panels of about 96 MB are as good as smaller ones, and a run shorter than a segment
     // wastes gather slots -- so at most one panel per 8 nonzeros of an average row, and never more than 4
     const double panel = e->knob_panel_mb > 0 ? e->knob_panel_mb * (1 << 20) : 0.75 * l2;
@@ -348,8 +364,28 @@ int choose_panels(const sddmm_b200_engine *e) {
 }
 
 // Lay out the arena for the current dimensions and point the views into it.
-int carve_arena(sddmm_b200_engine *e, bool coo, int n_items) {
+// Which inputs the row-segment kernels take (the scalar and the row-tile kernel are left with the rest): K below 8 that is
+// no multiple of 4 stays with the scalar kernel, a padded row would be several times the real one.
+bool seg_possible(const sddmm_b200_engine *e) {
+    if ((e->flags & SDDMM_B200_FLAG_NO_ROW_SEGMENTS) || e->knob_rowseg == 0 || e->M >= kUnitRowLimit) return false;
+    return e->K % 4 == 0 || e->K >= 8;
+}
+
+// Elements from one row to the next for the row-segment kernels.  Rows start on a 128-byte line (short rows: do not cross
+// one), so that a piece of a row is one line: with rows of 200 bytes back to back a piece touches two, and K = 50 takes
+// longer than K = 64 (64 against 46 us for 2.4 M nonzeros).
+int64_t padded_row(const sddmm_b200_engine *e) {
+    const int64_t line = e->mode == SDDMM_B200_BF16 ? 64 : 32, K = e->K;
+    if (K > 256) return (K + 63) / 64 * 64;
+    if (4 * K <= line) return line / 4;
+    if (2 * K <= line) return line / 2;
+    return (K + line - 1) / line * line;
+}
+
+int carve_arena(sddmm_b200_engine *e, bool coo, int n_items, bool allow_padding) {
     Carve c;
+    e->use_seg = seg_possible(e) && (allow_padding || (e->K % 8 == 0 && e->K <= 256));
+    e->Ks = e->use_seg ? padded_row(e) : e->K;
     const size_t nnz = static_cast<size_t>(e->nnz), M = static_cast<size_t>(e->M), N = static_cast<size_t>(e->N),
                  K = static_cast<size_t>(e->K);
     const size_t o_rp = c.take((M + 1) * 4);
@@ -359,13 +395,19 @@ int carve_arena(sddmm_b200_engine *e, bool coo, int n_items) {
     const size_t o_A = c.take(M * K * 4);
     const size_t o_B = c.take(N * K * 4);
     const bool bf = e->mode == SDDMM_B200_BF16;
-    const size_t o_A16 = bf ? c.take(M * K * 2) : 0;
-    const size_t o_B16 = bf ? c.take(N * K * 2) : 0;
-    const size_t o_touch = c.take(N);
+    const size_t Ks = static_cast<size_t>(e->Ks);
+    const size_t o_A16 = bf ? c.take(M * Ks * 2) : 0;
+    const size_t o_B16 = bf ? c.take(N * Ks * 2) : 0;
+    const bool padded = !bf && e->use_seg && (e->Ks != e->K);
+    e->d_Ap_wanted = padded;
+    const size_t o_Ap = padded ? c.take(M * Ks * 4) : 0;
+    const size_t o_Bp = padded ? c.take(N * Ks * 4) : 0;
+    const size_t o_pc = c.take(sizeof(PlanCounters));
+    const size_t o_touch = c.take((N / 32 + 1) * 4);
     const size_t o_rs = c.take((nnz / 32 + 2) * 4);
+    e->plan_clear_bytes = c.off - o_pc;
     const size_t o_items = c.take(static_cast<size_t>(std::max(n_items, 1)) * sizeof(int2));
     const size_t o_coo = coo ? c.take(nnz * 4 + 16) : 0;
-    const size_t o_pc = c.take(sizeof(PlanCounters));
     const size_t o_gok = c.take(M / 2 + 4);   // one byte per row group (groups of >= 2 rows, plus the leading partial group)
     // row-segment path: unit list (upper bound: one unit per 8 nonzeros plus one ragged unit per row and panel), scan scratch
     e->seg_slices = choose_k_slices(e);
@@ -380,10 +422,11 @@ int carve_arena(sddmm_b200_engine *e, bool coo, int n_items) {
     }
     e->unit_cap = static_cast<int64_t>(nnz / 8 + runs + 8);
     const size_t scan_n = M * static_cast<size_t>(e->panels);
-    const size_t o_units = c.take(static_cast<size_t>(e->unit_cap) * sizeof(int4));   // (row groups use 16-byte headers)
-    const size_t o_ucols = e->panels > 1 ? c.take(static_cast<size_t>(e->unit_cap) * 64) : 0;
-    const size_t o_uoff = c.take((scan_n + 1) * 4);
-    const size_t o_stile = c.take((scan_n / kScanTile + 2) * 4);
+    const size_t o_units = c.take(static_cast<size_t>(e->unit_cap + 8) * sizeof(int4));   // (row groups use 16-byte headers)
+    const size_t o_ucols = c.take(static_cast<size_t>(e->unit_cap + 8) * 32);
+    const size_t o_uval = e->panels > 1 ? c.take(static_cast<size_t>(e->unit_cap + 8) * 32) : 0;
+    const size_t o_uoff = c.take((M + 1) * 4);
+    const size_t o_stile = c.take((scan_n / kUnitTile + M / kScanTile + 2) * 4);
     // dense-tile path: only carved when the mode, K and the size of the 64x64 tile grid allow it
     e->tiles_per_row = static_cast<int32_t>((N + 63) / 64);
     e->tile_grid = static_cast<int64_t>((M + 63) / 64) * e->tiles_per_row;
@@ -426,8 +469,10 @@ int carve_arena(sddmm_b200_engine *e, bool coo, int n_items) {
     e->d_Ax = split ? reinterpret_cast<float *>(b + o_ax) : nullptr;
     e->d_Bx = split ? reinterpret_cast<float *>(b + o_bx) : nullptr;
     e->d_units = reinterpret_cast<int2 *>(b + o_units);
-    e->d_unit_cols = e->panels > 1 ? reinterpret_cast<int32_t *>(b + o_ucols) : nullptr;
-    e->d_unit_sval = e->panels > 1 ? reinterpret_cast<float *>(b + o_ucols) : nullptr;
+    e->d_unit_cols = reinterpret_cast<int32_t *>(b + o_ucols);
+    e->d_unit_sval = e->panels > 1 ? reinterpret_cast<float *>(b + o_uval) : nullptr;
+    e->d_Ap = padded ? reinterpret_cast<float *>(b + o_Ap) : nullptr;
+    e->d_Bp = padded ? reinterpret_cast<float *>(b + o_Bp) : nullptr;
     e->d_unit_off = reinterpret_cast<int32_t *>(b + o_uoff);
     e->d_scan_tiles = reinterpret_cast<int32_t *>(b + o_stile);
     e->d_rp = reinterpret_cast<int32_t *>(b + o_rp);
@@ -439,7 +484,7 @@ int carve_arena(sddmm_b200_engine *e, bool coo, int n_items) {
     e->d_B32 = reinterpret_cast<float *>(b + o_B);
     e->d_A16 = bf ? reinterpret_cast<__nv_bfloat16 *>(b + o_A16) : nullptr;
     e->d_B16 = bf ? reinterpret_cast<__nv_bfloat16 *>(b + o_B16) : nullptr;
-    e->d_touched = reinterpret_cast<unsigned char *>(b + o_touch);
+    e->d_touched = reinterpret_cast<uint32_t *>(b + o_touch);
     e->d_rowstart = reinterpret_cast<uint32_t *>(b + o_rs);
     e->d_item_rows = reinterpret_cast<int2 *>(b + o_items);
     e->d_coo_rows = coo ? reinterpret_cast<int32_t *>(b + o_coo) : nullptr;
@@ -471,10 +516,16 @@ int convert_storage(sddmm_b200_engine *e) {
         k_split_concat_tf32<<<grid_for(e->N * e->K, kBlock, cap), kBlock, 0, e->stream>>>(e->d_B32, e->d_Bx, e->N, static_cast<int32_t>(e->K), 0);
         CU_TRY(e, cudaGetLastError());
     }
+    const int32_t K = static_cast<int32_t>(e->K), Ks = static_cast<int32_t>(e->Ks);
+    if (e->d_Ap) {
+        k_pad_rows<<<grid_for(e->M * (Ks / 4), kBlock, cap), kBlock, 0, e->stream>>>(e->d_A32, e->d_Ap, e->M, K, Ks);
+        k_pad_rows<<<grid_for(e->N * (Ks / 4), kBlock, cap), kBlock, 0, e->stream>>>(e->d_B32, e->d_Bp, e->N, K, Ks);
+        CU_TRY(e, cudaGetLastError());
+    }
     if (e->mode != SDDMM_B200_BF16) return SDDMM_B200_OK;
     // (the fp32 copies keep the rounded values: the dense-tile kernel reads them through its tensor maps)
-    k_f32_to_bf16<<<grid_for(e->M * e->K, kBlock, cap), kBlock, 0, e->stream>>>(e->d_A32, e->d_A16, e->M * e->K);
-    k_f32_to_bf16<<<grid_for(e->N * e->K, kBlock, cap), kBlock, 0, e->stream>>>(e->d_B32, e->d_B16, e->N * e->K);
+    k_f32_to_bf16<<<grid_for(e->M * (Ks / 4), kBlock, cap), kBlock, 0, e->stream>>>(e->d_A32, e->d_A16, e->M, K, Ks);
+    k_f32_to_bf16<<<grid_for(e->N * (Ks / 4), kBlock, cap), kBlock, 0, e->stream>>>(e->d_B32, e->d_B16, e->N, K, Ks);
     CU_TRY(e, cudaGetLastError());
     return SDDMM_B200_OK;
 }
@@ -673,131 +724,140 @@ RowGroupFn pick_rowgroup(int rows, int cpl) {
 }
 
 using RowSegGroupFn = void (*)(const RowSegGroupArgs);
-RowSegGroupFn pick_rowseg_group(int rows, int cpl) {
-    if (cpl == 1) return rows == 2 ? sddmm_rowseg_group_kernel<1, 2> : rows == 3 ? sddmm_rowseg_group_kernel<1, 3> : sddmm_rowseg_group_kernel<1, 4>;
-    return rows == 2 ? sddmm_rowseg_group_kernel<2, 2> : rows == 3 ? sddmm_rowseg_group_kernel<2, 3> : sddmm_rowseg_group_kernel<2, 4>;
+template <int CPL>
+RowSegGroupFn pick_rowseg_group_rows(int rows) {
+    return rows == 2 ? sddmm_rowseg_group_kernel<CPL, 2> : rows == 3 ? sddmm_rowseg_group_kernel<CPL, 3> : sddmm_rowseg_group_kernel<CPL, 4>;
+}
+// rows of 32 or 64 elements (nullptr: no instantiation)
+RowSegGroupFn pick_rowseg_group(const sddmm_b200_engine *e, int rows) {
+    return e->Ks == 32 ? pick_rowseg_group_rows<1>(rows) : e->Ks == 64 ? pick_rowseg_group_rows<2>(rows) : nullptr;
+}
+
+using RowSegFn = void (*)(const RowSegArgs);
+
+template <bool COPIES>
+RowSegFn pick_rowseg(int pieces) {
+    switch (pieces) {
+        case 1: return sddmm_rowseg_kernel<1, COPIES, false>;
+        case 2: return sddmm_rowseg_kernel<2, COPIES, false>;
+        case 3: return sddmm_rowseg_kernel<3, COPIES, false>;
+        case 4: return sddmm_rowseg_kernel<4, COPIES, false>;
+        case 5: return sddmm_rowseg_kernel<5, COPIES, false>;
+        case 6: return sddmm_rowseg_kernel<6, COPIES, false>;
+        case 7: return sddmm_rowseg_kernel<7, COPIES, false>;
+        default: return sddmm_rowseg_kernel<8, COPIES, false>;
+    }
+}
+template <bool COPIES>
+RowSegFn pick_rowseg_bf16(int64_t Ks) {
+    if (Ks <= 32) return sddmm_rowseg_bf16_kernel<1, 16, 8, 3, COPIES>;
+    if (Ks <= 64) return sddmm_rowseg_bf16_kernel<1, 32, 8, 2, COPIES>;
+    if (Ks <= 128) return sddmm_rowseg_bf16_kernel<2, 32, 4, 2, COPIES>;
+    if (Ks <= 192) return sddmm_rowseg_bf16_kernel<3, 32, 4, 1, COPIES>;
+    return sddmm_rowseg_bf16_kernel<4, 32, 2, 1, COPIES>;
+}
+// The row-segment kernel instantiation for this engine's storage and K (`copies`: S values from the per-unit copies).
+RowSegFn seg_function(const sddmm_b200_engine *e, bool copies) {
+    if (e->mode == SDDMM_B200_BF16) return copies ? pick_rowseg_bf16<true>(e->Ks) : pick_rowseg_bf16<false>(e->Ks);
+    if (e->seg_slices > 1) return copies ? sddmm_rowseg_kernel<2, true, true> : sddmm_rowseg_kernel<2, false, true>;   // a 64-column slice
+    const int pieces = static_cast<int>((e->Ks + 31) / 32);
+    return copies ? pick_rowseg<true>(pieces) : pick_rowseg<false>(pieces);
+}
+// persistent grid of a streaming kernel over `n_units` units, `per_step` of them per warp step
+int seg_grid(sddmm_b200_engine *e, const void *fn, int warps, int per_step, int64_t n_units, int32_t *grid) {
+    int occ = 0;
+    CU_TRY(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, warps * 32, 0));
+    if (occ < 1) return fail(e, SDDMM_B200_ERR_CUDA, "row-segment kernel does not fit on an SM");
+    const int64_t steps = (n_units + per_step - 1) / per_step;
+    *grid = static_cast<int32_t>(std::min<int64_t>((steps + warps - 1) / warps, static_cast<int64_t>(e->sm_count) * occ));
+    return SDDMM_B200_OK;
+}
+
+bool group_possible(const sddmm_b200_engine *e) {
+    if (e->mode == SDDMM_B200_BF16 || (e->flags & SDDMM_B200_FLAG_NO_ROW_GROUPS) || e->M < 4) return false;
+    return e->knob_group_units != 0 && e->use_seg ? pick_rowseg_group(e, 2) != nullptr : (e->K == 32 || e->K == 64);
+}
+// candidates: G = 2, 3, 4 rows per group, first full group starting at row 0 .. G-1 (counters slot = G(G-1)/2 - 1 + first)
+int group_slot(int G, int first) { return G * (G - 1) / 2 - 1 + first; }
+int group_sample(const sddmm_b200_engine *e) { return e->M > 65536 ? 16 : 1; }   // large inputs: G and `first` are chosen on a 1-in-16 sample of the groups
+int enqueue_group_sample(sddmm_b200_engine *e) {
+    const int every = group_sample(e);
+    const dim3 grid(grid_for((e->M / 2 / every + 2) * 32, kBlock, e->sm_count * 2), 9);
+    k_group_match<<<grid, kBlock, 0, e->stream>>>(e->d_rp, e->d_col, static_cast<int32_t>(e->M), static_cast<int32_t>(e->nnz), 0, 0, every, nullptr,
+                                                  e->d_pc->group_cover, e->d_pc->group_count);
+    CU_TRY(e, cudaGetLastError());
+    return SDDMM_B200_OK;
 }
 
 // Row groups: groups of 2, 3 or 4 consecutive rows with one column list (first full group at row 0 .. G-1) share each gather of B.
-// The path is taken (for the whole matrix) when it removes at least 30 % of the gathers; fp32 storage, K = 32 or 64.
+// The path is taken (for the whole matrix) when it removes at least 30 % of the gathers; fp32 storage, K <= 256.
+// base_pc: counters that include enqueue_group_sample's.
 int build_rowgroup_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
-    const bool eligible = e->mode != SDDMM_B200_BF16 && !(e->flags & SDDMM_B200_FLAG_NO_ROW_GROUPS) && (e->K == 32 || e->K == 64) &&
-                          e->M >= 4 && base_pc.max_row_nnz <= 8192;
-    if (!eligible) return SDDMM_B200_OK;
+    if (!group_possible(e) || base_pc.max_row_nnz > 8192) return SDDMM_B200_OK;
     cudaStream_t s = e->stream;
-    const int cap = e->sm_count * 8;
-    // candidates: G = 2, 3, 4 rows per group, first full group starting at row 0 .. G-1 (9 counting passes, counters slot = G(G-1)/2 - 1 + first)
-    auto slot = [](int G, int first) { return G * (G - 1) / 2 - 1 + first; };
-    auto groups_of = [&](int G, int first) { return static_cast<int32_t>(1 + (e->M - first + G - 1) / G); };
-    const int every = e->M > 65536 ? 16 : 1;   // large inputs: choose G and `first` on a 1-in-16 sample of the groups
-    for (int G = 2; G <= 4; ++G)
-        for (int first = 0; first < G; ++first)
-            k_group_match<<<grid_for(static_cast<int64_t>(groups_of(G, first) / every + 1) * 32, kBlock, cap), kBlock, 0, s>>>(
-                e->d_rp, e->d_col, static_cast<int32_t>(e->M), G, first, groups_of(G, first), every, nullptr,
-                &e->d_pc->group_cover[slot(G, first)], &e->d_pc->group_count[slot(G, first)]);
-    CU_TRY(e, cudaGetLastError());
-    PlanCounters pc;
-    if (int rc = read_counters(e, &pc)) return rc;
+    const int every = group_sample(e);
+    const int32_t M = static_cast<int32_t>(e->M), nnz = static_cast<int32_t>(e->nnz);
     int best = 0, best_first = 0;
     double best_saved = 0.0;
     for (int G = 2; G <= 4; ++G)
         for (int first = 0; first < G; ++first) {
-            const double saved = static_cast<double>(pc.group_cover[slot(G, first)]) * every * (1.0 - 1.0 / G);   // gathers of B that disappear (estimate)
+            const double saved = static_cast<double>(base_pc.group_cover[group_slot(G, first)]) * every * (1.0 - 1.0 / G);   // gathers of B that disappear (estimate)
             if (saved > best_saved) { best_saved = saved; best = G; best_first = first; }
         }
     if (best == 0 || best_saved < 0.3 * static_cast<double>(e->nnz)) return SDDMM_B200_OK;
-    const int32_t n_groups = groups_of(best, best_first);
-    const int bs = slot(best, best_first);
+    const int32_t n_groups = group_count(M, best, best_first);
+    const int bs = group_slot(best, best_first);
+    const bool units = e->knob_group_units != 0 && e->use_seg;
+    e->group_tried = true;
+    // exact match of the chosen grouping, and -- speculating that the sample was right -- the unit list over it
     CU_TRY(e, cudaMemsetAsync(&e->d_pc->group_cover[bs], 0, sizeof(unsigned long long), s));
     CU_TRY(e, cudaMemsetAsync(&e->d_pc->group_count[bs], 0, sizeof(int), s));
-    k_group_match<<<grid_for(static_cast<int64_t>(n_groups) * 32, kBlock, cap), kBlock, 0, s>>>(
-        e->d_rp, e->d_col, static_cast<int32_t>(e->M), best, best_first, n_groups, 1, e->d_group_ok, &e->d_pc->group_cover[bs],
-        &e->d_pc->group_count[bs]);
+    k_group_match<<<grid_for(static_cast<int64_t>(n_groups) * 32, kBlock, e->sm_count * 8), kBlock, 0, s>>>(
+        e->d_rp, e->d_col, M, nnz, best, best_first, 1, e->d_group_ok, &e->d_pc->group_cover[bs], &e->d_pc->group_count[bs]);
+    if (units) {
+        const RunsOfGroups runs{e->d_rp, e->d_col, M, nnz, best, best_first, e->d_group_ok};
+        const int tiles = static_cast<int>((e->M + kUnitTile - 1) / kUnitTile);
+        CU_TRY(e, cudaMemsetAsync(&e->d_pc->units, 0, sizeof(unsigned long long), s));
+        k_unit_sums<<<tiles, kUnitBlock, 0, s>>>(runs, e->M, e->d_scan_tiles, e->d_pc);
+        k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, e->M, e->d_scan_tiles, e->unit_cap, e->d_pc, reinterpret_cast<int4 *>(e->d_units), e->d_unit_cols);
+    }
     CU_TRY(e, cudaGetLastError());
-    if (int rc = read_counters(e, &pc)) return rc;   // exact counts of the chosen grouping
+    PlanCounters pc;
+    if (int rc = read_counters(e, &pc)) return rc;
     if (static_cast<double>(pc.group_cover[bs]) * (1.0 - 1.0 / best) < 0.3 * static_cast<double>(e->nnz)) return SDDMM_B200_OK;   // the sample overestimated
-    RowGroupFn fn = pick_rowgroup(best, static_cast<int>(e->K / 32));
-    int occ = 0;
-    CU_TRY(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kRowGroupWarps * 32, 0));
-    if (occ < 1) return fail(e, SDDMM_B200_ERR_CUDA, "row-group kernel does not fit on an SM");
+    sddmm_b200_plan_info &p = e->plan;
+    if (units) {
+        if (pc.units == 0 || pc.units > static_cast<unsigned long long>(std::min<int64_t>(e->unit_cap, kUnitLimit)))
+            return fail(e, SDDMM_B200_ERR_CUDA, "row-group plan: %llu units for a list of %lld", pc.units, (long long)e->unit_cap);
+        e->n_units = static_cast<int32_t>(pc.units);
+        if (int rc = seg_grid(e, reinterpret_cast<const void *>(pick_rowseg_group(e, best)), kRowSegWarps, 4, e->n_units, &p.rowgroup_grid)) return rc;
+        p.rowseg_units = e->n_units;
+        p.rowseg_panels = 1;
+    } else {
+        RowGroupFn fn = pick_rowgroup(best, static_cast<int>(e->K / 32));
+        int occ = 0;
+        CU_TRY(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kRowGroupWarps * 32, 0));
+        if (occ < 1) return fail(e, SDDMM_B200_ERR_CUDA, "row-group kernel does not fit on an SM");
+        p.rowgroup_grid = std::min((n_groups + kRowGroupWarps - 1) / kRowGroupWarps, e->sm_count * occ);
+    }
     e->rg_rows = best;
     e->rg_first = best_first;
     e->rg_groups = n_groups;
-    sddmm_b200_plan_info &p = e->plan;
+    e->rg_units = units;
     p.rowgroup_nnz = static_cast<int64_t>(pc.group_cover[bs]);
     p.rowgroup_groups = pc.group_count[bs];
     p.rowgroup_rows = best;
-    p.rowgroup_grid = std::min((n_groups + kRowGroupWarps - 1) / kRowGroupWarps, e->sm_count * occ);
-    // Shared segments: the group's column list cut into units of 8 columns that serve all G rows (row-segment group kernel).
-    e->rg_units = e->knob_group_units != 0 && e->M < kUnitRowLimit;
-    if (e->rg_units) {
-        const int32_t M = static_cast<int32_t>(e->M);
-        const int n_tiles = static_cast<int>((e->M + kScanTile - 1) / kScanTile);
-        const int capb = e->sm_count * 32;
-        k_group_unit_count<<<grid_for(e->M, kBlock, capb), kBlock, 0, s>>>(e->d_rp, M, best, best_first, e->d_group_ok, e->d_unit_off);
-        k_scan_tile_sums<<<n_tiles, kScanBlock, 0, s>>>(e->d_unit_off, e->M, e->d_scan_tiles);
-        k_scan_sums<<<1, kScanBlock, 0, s>>>(e->d_scan_tiles, n_tiles, &e->d_pc->units);
-        k_scan_apply<<<n_tiles, kScanBlock, 0, s>>>(e->d_unit_off, e->M, e->d_scan_tiles);
-        k_group_unit_fill<<<grid_for(e->M * 32, kBlock, capb), kBlock, 0, s>>>(e->d_rp, M, best, best_first, e->d_group_ok, e->d_unit_off,
-                                                                               reinterpret_cast<int4 *>(e->d_units));
-        CU_TRY(e, cudaGetLastError());
-        if (int rc = read_counters(e, &pc)) return rc;
-        if (pc.units == 0 || pc.units > static_cast<unsigned long long>(e->unit_cap))
-            return fail(e, SDDMM_B200_ERR_CUDA, "row-group plan: %llu units for a list of %lld", pc.units, (long long)e->unit_cap);
-        e->n_units = static_cast<int32_t>(pc.units);
-        int occ2 = 0;
-        CU_TRY(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, pick_rowseg_group(best, static_cast<int>(e->K / 32)), kRowSegWarps * 32, 0));
-        if (occ2 < 1) return fail(e, SDDMM_B200_ERR_CUDA, "row-segment group kernel does not fit on an SM");
-        const int64_t n_quads = (static_cast<int64_t>(e->n_units) + 3) / 4;
-        p.rowseg_units = e->n_units;
-        p.rowseg_panels = 1;
-        p.rowgroup_grid = static_cast<int32_t>(std::min<int64_t>((n_quads + kRowSegWarps - 1) / kRowSegWarps, static_cast<int64_t>(e->sm_count) * occ2));
-    }
     p.rowtile_nnz = 0;
     p.rowtile_items = 0;
     p.n_kernels = 1;
     return SDDMM_B200_OK;
 }
 
-template <typename ET>
-using RowSegFn = void (*)(const RowSegArgs);
-
-template <typename ET, bool HINT>
-RowSegFn<ET> pick_rowseg_hint(int cpl, bool exact) {
-    switch (cpl) {
-        case 1: return exact ? sddmm_rowseg_kernel<1, true, ET, HINT> : sddmm_rowseg_kernel<1, false, ET, HINT>;
-        case 2: return exact ? sddmm_rowseg_kernel<2, true, ET, HINT> : sddmm_rowseg_kernel<2, false, ET, HINT>;
-        case 4: return exact ? sddmm_rowseg_kernel<4, true, ET, HINT> : sddmm_rowseg_kernel<4, false, ET, HINT>;
-        case 8: return exact ? sddmm_rowseg_kernel<8, true, ET, HINT> : sddmm_rowseg_kernel<8, false, ET, HINT>;
-        default: return nullptr;
-    }
-}
-template <typename ET>
-RowSegFn<ET> pick_rowseg(int cpl, bool exact, bool hint = false) {
-    return hint ? pick_rowseg_hint<ET, true>(cpl, exact) : pick_rowseg_hint<ET, false>(cpl, exact);
-}
-
-// The row-segment kernel instantiation for this engine's storage and K.  bf16 storage with K >= 64 reads 16-byte chunks
-// (8 elements: 8 lanes cover a 128-byte piece in one request), otherwise chunks of 4 elements.
-bool seg_wide_bf16(const sddmm_b200_engine *e) { return e->mode == SDDMM_B200_BF16 && e->K >= 64; }
-const void *seg_function(const sddmm_b200_engine *e, bool hint) {
-    if (seg_wide_bf16(e)) {
-        const int cpl = round_up_cpl((e->K + 1) / 2);   // chunks of 8: K / 64 lanes-rounds
-        return reinterpret_cast<const void *>(pick_rowseg<Bf16x8>(cpl, e->K == 64 * cpl, hint));
-    }
-    if (e->seg_slices > 1)   // a 64-column slice of fp32 rows
-        return hint ? reinterpret_cast<const void *>(sddmm_rowseg_kernel<2, true, float, true, true>)
-                    : reinterpret_cast<const void *>(sddmm_rowseg_kernel<2, true, float, false, true>);
-    const bool exact = e->K == 32 * e->cpl;
-    return e->mode == SDDMM_B200_BF16 ? reinterpret_cast<const void *>(pick_rowseg<__nv_bfloat16>(e->cpl, exact, hint))
-                                      : reinterpret_cast<const void *>(pick_rowseg<float>(e->cpl, exact, hint));
-}
-
 // What the dense tiles left, as row segments: the uncovered runs of every row cut into units, so that the residual
 // kernel touches only those nonzeros (a kernel that walks all work items and skips the covered nonzeros costs as much as
 // the whole matrix when the tiles leave a little in every item).
 int build_residual_units(sddmm_b200_engine *e) {
-    if ((e->flags & SDDMM_B200_FLAG_NO_ROW_SEGMENTS) || e->knob_rowseg == 0 || e->M >= kUnitRowLimit) return SDDMM_B200_OK;
+    if (!e->use_seg) return SDDMM_B200_OK;
     const int32_t M = static_cast<int32_t>(e->M);
     const int n_tiles = static_cast<int>((e->M + kScanTile - 1) / kScanTile);
     const int cap = e->sm_count * 32;
@@ -810,107 +870,116 @@ int build_residual_units(sddmm_b200_engine *e) {
     PlanCounters pc;
     if (int rc = read_counters(e, &pc)) return rc;
     if (pc.units == 0 || pc.units > static_cast<unsigned long long>(e->unit_cap)) return SDDMM_B200_OK;   // (the row-tile kernel takes the residual)
-    k_residual_unit_fill<<<grid_for(e->M, kBlock, cap), kBlock, 0, s>>>(e->d_rp, M, e->d_covered, e->d_unit_off, e->d_units);
+    k_residual_unit_fill<<<grid_for(e->M, kBlock, cap), kBlock, 0, s>>>(e->d_rp, M, e->d_covered, e->d_unit_off, e->d_col, e->d_units, e->d_unit_cols);
+    k_unit_pad<<<1, 64, 0, s>>>(e->d_units, e->d_unit_cols, e->d_pc, e->unit_cap);
     CU_TRY(e, cudaGetLastError());
-    int occ = 0;
-    CU_TRY(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, seg_function(e, false), kRowSegWarps * 32, 0));
-    if (occ < 1) return SDDMM_B200_OK;
     e->n_units = static_cast<int32_t>(pc.units);
     e->seg_residual = true;
-    const int64_t n_quads = (static_cast<int64_t>(e->n_units) + 3) / 4;
     e->plan.rowseg_units = e->n_units;
     e->plan.rowseg_panels = 1;
     e->plan.rowseg_passes = e->seg_slices;
-    e->plan.rowseg_grid = static_cast<int32_t>(std::min<int64_t>((n_quads + kRowSegWarps - 1) / kRowSegWarps, static_cast<int64_t>(e->sm_count) * occ));
+    return seg_grid(e, reinterpret_cast<const void *>(seg_function(e, false)), kRowSegWarps, 8, e->n_units, &e->plan.rowseg_grid);
+}
+
+// Enqueue the unit list over the whole matrix with `panels` column panels (1: whole rows, whose tile sums k_row_stats has
+// left when have_sums).
+int enqueue_unit_list(sddmm_b200_engine *e, int32_t panels, bool have_sums) {
+    const int32_t M = static_cast<int32_t>(e->M), nnz = static_cast<int32_t>(e->nnz);
+    cudaStream_t s = e->stream;
+    const int64_t n = static_cast<int64_t>(panels) * M;
+    const int tiles = static_cast<int>((n + kUnitTile - 1) / kUnitTile);
+    if (!have_sums) CU_TRY(e, cudaMemsetAsync(&e->d_pc->units, 0, sizeof(unsigned long long), s));
+    if (panels > 1) {
+        const RunsOfPanels runs{e->d_rp, e->d_col, M, nnz, panels, e->panel_cols, e->long_rows};
+        k_unit_sums<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->d_pc);
+        k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->unit_cap, e->d_pc, e->d_units, e->d_unit_cols);
+    } else {
+        const RunsOfRows runs{e->d_rp, e->d_col, M, nnz};
+        if (!have_sums) k_unit_sums<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->d_pc);
+        k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->unit_cap, e->d_pc, e->d_units, e->d_unit_cols);
+    }
+    if (e->mode == SDDMM_B200_BF16) k_unit_pad<<<1, 64, 0, s>>>(e->d_units, e->d_unit_cols, e->d_pc, e->unit_cap);
+    CU_TRY(e, cudaGetLastError());
     return SDDMM_B200_OK;
 }
 
-// Row segments: the unit list (rows cut into segments of at most 8 nonzeros, panel-major when B is cut into column
-// panels) is counted, scanned and written on the device; the host only reads the total.  Taken unless the rows are
-// long on average (the A-row-tile kernel keeps the A chunk of a long row in registers over the whole row).
-int build_rowseg_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
-    const int seg_env = e->knob_rowseg < 0 ? -1 : static_cast<int>(e->knob_rowseg);   // 0 never, 1 whenever possible
-    e->use_seg = false;
+// Row segments over the whole matrix.  built: panels of the list that is already there (0: none), counted in pc.
+int build_rowseg_plan(sddmm_b200_engine *e, PlanCounters pc, int32_t built) {
     e->seg_copies = false;
     e->n_units = 0;
-    if ((e->flags & SDDMM_B200_FLAG_NO_ROW_SEGMENTS) || seg_env == 0 || e->M >= kUnitRowLimit) return SDDMM_B200_OK;
-    int32_t panels = base_pc.unsorted_cols ? 1 : e->panels;   // a panel run is a contiguous piece of a row only when its columns are sorted
+    if (!e->use_seg) return SDDMM_B200_OK;
+    int32_t panels = pc.unsorted_cols ? 1 : e->panels;   // a panel run is a contiguous piece of a row only when its columns are sorted
     if (panels == 1) e->long_rows = 0;
     if (e->long_rows > 0 && e->knob_long_rows < 0) {
         // panels for the long rows only pay when those rows hold a good share of the nonzeros
         unsigned long long in_long = 0;
         for (int b = 0; b < SDDMM_B200_HIST_BINS; ++b)
-            if (b >= 1 && (1ll << (b - 1)) >= e->long_rows) in_long += base_pc.hist_nnz[b];
+            if (b >= 1 && (1ll << (b - 1)) >= e->long_rows) in_long += pc.hist_nnz[b];
         if (5 * in_long < 2 * static_cast<unsigned long long>(e->nnz)) {   // < 40 %: every row whole, one pass
             e->long_rows = 0;
             panels = 1;
-            if (e->knob_k_slices < 0) e->seg_slices = 1;
+            if (e->knob_k_slices < 0 && e->K <= 256) e->seg_slices = 1;
         }
     }
-    const int32_t M = static_cast<int32_t>(e->M);
-    const int64_t n = static_cast<int64_t>(panels) * M;
-    const int n_tiles = static_cast<int>((n + kScanTile - 1) / kScanTile);
-    const int cap = e->sm_count * 32;
-    cudaStream_t s = e->stream;
-    k_unit_count<<<grid_for(n, kBlock, cap), kBlock, 0, s>>>(e->d_rp, e->d_col, M, panels, e->panel_cols, e->long_rows, e->d_unit_off);
-    k_scan_tile_sums<<<n_tiles, kScanBlock, 0, s>>>(e->d_unit_off, n, e->d_scan_tiles);
-    k_scan_sums<<<1, kScanBlock, 0, s>>>(e->d_scan_tiles, n_tiles, &e->d_pc->units);
-    k_scan_apply<<<n_tiles, kScanBlock, 0, s>>>(e->d_unit_off, n, e->d_scan_tiles);
-    e->seg_copies = panels > 1 && e->d_unit_cols != nullptr;
-    k_unit_fill<<<grid_for(n * 32, kBlock, cap), kBlock, 0, s>>>(e->d_rp, e->d_col, M, panels, e->panel_cols, e->long_rows, e->d_unit_off, e->d_units,
-                                                                  e->seg_copies ? e->d_unit_cols : nullptr);
-    CU_TRY(e, cudaGetLastError());
-    PlanCounters pc;
-    if (int rc = read_counters(e, &pc)) return rc;
-    if (pc.units == 0 || pc.units > static_cast<unsigned long long>(e->unit_cap) || pc.units >= (1ull << 31))
+    if (built != panels) {
+        if (int rc = enqueue_unit_list(e, panels, false)) return rc;
+        if (int rc = read_counters(e, &pc)) return rc;
+    }
+    e->seg_copies = panels > 1;
+    if (pc.units == 0 || pc.units > static_cast<unsigned long long>(std::min<int64_t>(e->unit_cap, kUnitLimit)))
         return fail(e, SDDMM_B200_ERR_CUDA, "row-segment plan: %llu units for a list of %lld", pc.units, (long long)e->unit_cap);
-    const void *fn = seg_function(e, false);
-    int occ = 0;
-    CU_TRY(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kRowSegWarps * 32, 0));
-    if (occ < 1) return fail(e, SDDMM_B200_ERR_CUDA, "row-segment kernel does not fit on an SM");
     e->n_units = static_cast<int32_t>(pc.units);
-    e->use_seg = true;
     sddmm_b200_plan_info &p = e->plan;
-    const int64_t n_quads = (static_cast<int64_t>(e->n_units) + 3) / 4;
     p.rowseg_nnz = e->nnz;
     p.rowseg_units = e->n_units;
     p.rowseg_panels = panels;
     p.rowseg_passes = e->seg_slices;
-    p.rowseg_grid = static_cast<int32_t>(std::min<int64_t>((n_quads + kRowSegWarps - 1) / kRowSegWarps, static_cast<int64_t>(e->sm_count) * occ));
     p.rowtile_nnz = 0;
     p.rowtile_items = 0;
     p.n_kernels = 1;
-    return SDDMM_B200_OK;
+    return seg_grid(e, reinterpret_cast<const void *>(seg_function(e, e->seg_copies)), kRowSegWarps, 8, e->n_units, &p.rowseg_grid);
 }
 
-int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items) {
+// Validation + statistics + plan.  join_copies: order the rest of the upload (copies on the side stream, conversions) before
+// the first read-back, so that one wait of the host covers both.
+int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies) {
     const int cap = e->sm_count * 8;
     cudaStream_t s = e->stream;
-    CU_TRY(e, cudaMemsetAsync(e->d_pc, 0, sizeof(PlanCounters), s));
-    CU_TRY(e, cudaMemsetAsync(e->d_touched, 0, static_cast<size_t>(e->N), s));
-    CU_TRY(e, cudaMemsetAsync(e->d_rowstart, 0, (static_cast<size_t>(e->nnz) / 32 + 2) * 4, s));
-    if (e->d_coo_rows) {
+    CU_TRY(e, cudaMemsetAsync(e->d_pc, 0, e->plan_clear_bytes, s));   // counters, distinct columns, row-start bits
+    e->n_dense = 0;
+    e->n_units = 0;
+    e->rg_rows = 0;
+    e->seg_copies = false;
+    e->group_tried = false;
+    e->copies_joined = false;
+    if (e->d_coo_rows)   // (rows out of order or out of range are counted, and every later kernel checks the bounds it gets from row_ptr)
         k_coo_to_row_ptr<<<grid_for(e->nnz + 1, kBlock, cap), kBlock, 0, s>>>(e->d_coo_rows, e->nnz, static_cast<int32_t>(e->M),
                                                                               e->coo_row_base, e->d_rp, e->d_pc);
-        // refuse to interpret a row_ptr built from unsorted rows
-        PlanCounters pc0;
-        if (int rc = read_counters(e, &pc0)) return rc;
-        if (pc0.bad_coo) return fail(e, SDDMM_B200_ERR_INDEX, "COO row indices must be sorted and inside [0, M)");
-    }
-    k_row_stats<<<grid_for(e->M, kBlock, 1 << 30), kBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, e->d_rowstart, e->d_pc);
-    CU_TRY(e, cudaGetLastError());
-    PlanCounters pc;
-    if (int rc = read_counters(e, &pc)) return rc;
-    if (pc.bad_row_ptr) return fail(e, SDDMM_B200_ERR_INDEX, "row_ptr must start at 0, end at nnz and be non-decreasing");
+    // What will most likely run is enqueued before anything is read back: the plain or panel-major unit list (not where
+    // tiles, or the row statistics, decide first) and the sample that looks for row groups.
+    const bool whole_rows = e->use_seg && !e->dense_possible && e->panels == 1;
+    const bool early_list = e->use_seg && !e->dense_possible && e->long_rows == 0 && e->nnz > 0;
+    k_row_stats<<<static_cast<int>((e->M + kUnitTile - 1) / kUnitTile), kUnitBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, e->d_rowstart,
+                                                                                            whole_rows ? e->d_scan_tiles : nullptr, e->d_pc);
     if (e->nnz > 0) {
         k_col_scan<<<grid_for(e->nnz, kBlock, cap), kBlock, 0, s>>>(e->d_col, e->nnz, static_cast<int32_t>(e->N), e->d_rowstart,
                                                                     e->d_touched, e->d_pc);
-        k_count_bytes<<<grid_for(e->N, kBlock, cap), kBlock, 0, s>>>(e->d_touched, e->N, &e->d_pc->cols_touched);
-        k_item_rows<<<grid_for(n_items, kBlock, 1 << 30), kBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, item_nnz, n_items,
-                                                                          e->d_item_rows);
         CU_TRY(e, cudaGetLastError());
+        if (group_possible(e))
+            if (int rc = enqueue_group_sample(e)) return rc;
+        if (early_list)
+            if (int rc = enqueue_unit_list(e, e->panels, whole_rows)) return rc;
     }
+    CU_TRY(e, cudaGetLastError());
+    if (join_copies && !e->dense_possible && e->panels == 1) {
+        CU_TRY(e, cudaStreamWaitEvent(s, e->ev_h2d, 0));
+        if (int rc = convert_storage(e)) return rc;
+        e->copies_joined = true;
+    }
+    PlanCounters pc;
     if (int rc = read_counters(e, &pc)) return rc;
+    if (pc.bad_coo) return fail(e, SDDMM_B200_ERR_INDEX, "COO row indices must be sorted and inside [0, M)");
+    if (pc.bad_row_ptr) return fail(e, SDDMM_B200_ERR_INDEX, "row_ptr must start at 0, end at nnz and be non-decreasing");
     if (pc.bad_col) return fail(e, SDDMM_B200_ERR_INDEX, "column index outside [0, N)");
 
     sddmm_b200_plan_info &p = e->plan;
@@ -928,8 +997,6 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items) {
     const size_t eb = elem_bytes(e);
     e->cpl = round_up_cpl(e->K);
     e->use_scalar = (e->K % 4 != 0) || e->cpl == 0 || static_cast<size_t>(e->K) * eb > kMaxStageBytes;
-    if (e->mode == SDDMM_B200_BF16 && (e->use_scalar || e->K % 8 != 0))
-        return fail(e, SDDMM_B200_ERR_UNSUPPORTED, "bf16 storage needs K %% 8 == 0 and K <= 256 (K = %lld)", (long long)e->K);
     p.rowtile_item_nnz = item_nnz;
     p.rowtile_block = kBlock;
     e->n_dense = 0;
@@ -939,7 +1006,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items) {
         return SDDMM_B200_OK;
     }
     e->seg_residual = false;
-    if (!e->use_scalar) {
+    if (e->dense_possible) {
         int st = build_dense_plan(e, pc, item_nnz, n_items);
         if (st) return st;
         if (e->n_dense > 0 && e->n_residual_items > 0) {
@@ -947,13 +1014,12 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items) {
             if (st) return st;
         }
     }
-    e->rg_rows = 0;
-    e->use_seg = false;
-    if (!e->use_scalar && e->n_dense == 0) {
+    if (e->n_dense == 0) {
         int st = build_rowgroup_plan(e, pc);
         if (st) return st;
         if (e->rg_rows) return SDDMM_B200_OK;
-        st = build_rowseg_plan(e, pc);
+        // (a grouping that was tried and dropped has used the list's memory)
+        st = build_rowseg_plan(e, pc, early_list && !e->group_tried ? (pc.unsorted_cols && e->panels > 1 ? 0 : e->panels) : 0);
         if (st) return st;
         if (e->use_seg) return SDDMM_B200_OK;
     }
@@ -971,6 +1037,9 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items) {
         p.n_kernels = 1 + dense_kernels;
         return SDDMM_B200_OK;
     }
+    if (!e->use_scalar)
+        k_item_rows<<<grid_for(n_items, kBlock, 1 << 30), kBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, item_nnz, n_items,
+                                                                          e->d_item_rows);
     if (e->use_scalar) {
         p.rowtile_rows_per_stage = 0;
         p.rowtile_smem_bytes = 0;
@@ -1042,16 +1111,21 @@ int upload_common(sddmm_b200_engine *e, int64_t M, int64_t N, int64_t K, int64_t
     e->M = M; e->N = N; e->K = K; e->nnz = nnz;
     const int item_nnz = choose_item_nnz(e);
     const int n_items = static_cast<int>((nnz + item_nnz - 1) / item_nnz);
-    int st = carve_arena(e, coo_rows != nullptr, n_items);
+    if (e->mode == SDDMM_B200_BF16 && (K % 8 != 0 || K > 256))
+        return fail(e, SDDMM_B200_ERR_UNSUPPORTED, "bf16 storage needs K %% 8 == 0 and K <= 256 (K = %lld)", (long long)K);
+    int st = carve_arena(e, coo_rows != nullptr, n_items, true);
+    if (st == SDDMM_B200_ERR_OOM && e->d_Ap_wanted) st = carve_arena(e, coo_rows != nullptr, n_items, false);   // without the padded copies of A and B
     if (st) return st;
     // The pattern goes first on the main stream and is planned there while S.val, A and B -- which the plan does not
     // read -- still cross the host link on the side stream.
     cudaStream_t s = e->stream, s2 = e->side_stream;
     if (e->h2d_after) CU_TRY(e, cudaStreamWaitEvent(s, e->h2d_after, 0));
     st = enqueue_copies(e, row_ptr, coo_rows, col_idx, s_val, A, B, kind);
-    if (!st) st = build_plan(e, item_nnz, n_items);
-    if (!st) st = cuda_status(e, cudaStreamWaitEvent(s, e->ev_h2d, 0));
-    if (!st) st = convert_storage(e);
+    if (!st) st = build_plan(e, item_nnz, n_items, kind == cudaMemcpyDeviceToDevice);
+    if (!st && !e->copies_joined) {
+        st = cuda_status(e, cudaStreamWaitEvent(s, e->ev_h2d, 0));
+        if (!st) st = convert_storage(e);
+    }
     if (!st) st = cuda_status(e, cudaStreamSynchronize(s));   // the caller's buffers are free again when this returns
     if (st) {   // nothing of a failed upload may still be reading the caller's buffers
         cudaStreamSynchronize(s2);
@@ -1079,37 +1153,36 @@ int mark_kernel(sddmm_b200_engine *e, const char *name, cudaStream_t st) {
     return SDDMM_B200_OK;
 }
 
+// the rows of A and B as the row-segment kernels read them
+const void *seg_rows_a(const sddmm_b200_engine *e) { return e->mode == SDDMM_B200_BF16 ? static_cast<const void *>(e->d_A16) : e->d_Ap ? e->d_Ap : e->d_A32; }
+const void *seg_rows_b(const sddmm_b200_engine *e) { return e->mode == SDDMM_B200_BF16 ? static_cast<const void *>(e->d_B16) : e->d_Bp ? e->d_Bp : e->d_B32; }
+
+// bytes of a row that hold elements, in whole 32-byte parts (bf16 rows of at most 32 elements: 16-byte parts)
+int32_t seg_row_bytes(const sddmm_b200_engine *e) {
+    const int64_t bytes = e->K * static_cast<int64_t>(elem_bytes(e)), part = e->mode == SDDMM_B200_BF16 && e->Ks <= 32 ? 16 : 32;
+    return static_cast<int32_t>((bytes + part - 1) / part * part);
+}
+
 // the row-segment kernel over the engine's unit list (the whole matrix, or what the dense tiles left)
 int launch_rowseg(sddmm_b200_engine *e, cudaStream_t stream, float *p_val) {
     const sddmm_b200_plan_info &p = e->plan;
     RowSegArgs g;
-    g.units = e->d_units; g.col_idx = e->d_col; g.s_val = e->d_sval; g.p_val = p_val;
-    g.n_units = e->n_units; g.K = static_cast<int32_t>(e->K);
-    // L2 is asked to keep the gathered B rows when they can stay: one column panel at a time
-    g.b_evict_last = p.rowseg_panels > 1 ? 1 : 0;
-    g.b_fraction = e->knob_b_fraction > 0 ? static_cast<float>(std::min(1.0, e->knob_b_fraction)) : 1.0f;
-    g.unit_cols = e->d_unit_cols; g.unit_sval = e->d_unit_sval;
-    if (!e->seg_copies) g.b_evict_last = 0;   // (the hinted instantiation reads the per-unit copies)
-    g.row_stride = 0;
-    g.accumulate = 0;
+    g.units = e->d_units; g.unit_cols = e->d_unit_cols; g.s_val = e->seg_copies ? e->d_unit_sval : e->d_sval; g.p_val = p_val;
+    g.A = seg_rows_a(e); g.B = seg_rows_b(e);
+    g.n_units = e->n_units;
+    g.row_stride = static_cast<uint32_t>(e->Ks * elem_bytes(e));
+    g.row_bytes = seg_row_bytes(e);
     if (int st = begin_kernel(e, stream)) return st;
-    if (e->mode == SDDMM_B200_BF16) {
-        g.A = e->d_A16; g.B = e->d_B16;
-    } else {
-        g.A = e->d_A32; g.B = e->d_B32;
-    }
-    const auto fn = reinterpret_cast<RowSegFn<float>>(const_cast<void *>(seg_function(e, g.b_evict_last != 0)));
     if (e->seg_slices > 1) {   // one launch per 64-column slice of K, in stream order: each adds to what the earlier ones wrote
-        g.K = 64;
-        g.row_stride = static_cast<uint32_t>(e->K * 4);
+        const RowSegFn first = e->seg_copies ? sddmm_rowseg_kernel<2, true, false> : sddmm_rowseg_kernel<2, false, false>;
+        g.row_bytes = 256;
         for (int sl = 0; sl < e->seg_slices; ++sl) {
-            g.A = e->d_A32 + 64 * sl;
-            g.B = e->d_B32 + 64 * sl;
-            g.accumulate = sl > 0 ? 1 : 0;
-            fn<<<p.rowseg_grid, kRowSegWarps * 32, 0, stream>>>(g);
+            (sl ? seg_function(e, e->seg_copies) : first)<<<p.rowseg_grid, kRowSegWarps * 32, 0, stream>>>(g);
+            g.A = static_cast<const float *>(g.A) + 64;
+            g.B = static_cast<const float *>(g.B) + 64;
         }
     } else {
-        fn<<<p.rowseg_grid, kRowSegWarps * 32, 0, stream>>>(g);
+        seg_function(e, e->seg_copies)<<<p.rowseg_grid, kRowSegWarps * 32, 0, stream>>>(g);
     }
     return mark_kernel(e, "sddmm_rowseg_kernel", stream);   // (the slices of one step count as one kernel in the timing table)
 }
@@ -1120,7 +1193,7 @@ int launch_all(sddmm_b200_engine *e, float *p_val) {
     e->kernels_launched = 0;
     if (e->nnz == 0) return SDDMM_B200_OK;
     int st = SDDMM_B200_OK;
-    if (e->use_scalar) {
+    if (e->use_scalar && !e->use_seg) {
         if ((st = begin_kernel(e, e->stream))) return st;
         sddmm_scalar_kernel<<<p.rowtile_grid, kBlock, 0, e->stream>>>(e->d_rp, e->d_col, e->d_sval, p_val, e->d_A32, e->d_B32,
                                                                       static_cast<int32_t>(e->M), static_cast<int32_t>(e->K), e->nnz);
@@ -1129,9 +1202,10 @@ int launch_all(sddmm_b200_engine *e, float *p_val) {
     if (e->rg_rows && e->rg_units) {
         RowSegGroupArgs g;
         g.ghdr = reinterpret_cast<const int4 *>(e->d_units); g.col_idx = e->d_col; g.s_val = e->d_sval; g.p_val = p_val;
-        g.A = e->d_A32; g.B = e->d_B32; g.n_units = e->n_units; g.K = static_cast<int32_t>(e->K);
+        g.A = static_cast<const float *>(seg_rows_a(e)); g.B = static_cast<const float *>(seg_rows_b(e));
+        g.n_units = e->n_units; g.K = static_cast<int32_t>(e->Ks);
         if ((st = begin_kernel(e, e->stream))) return st;
-        pick_rowseg_group(e->rg_rows, static_cast<int>(e->K / 32))<<<p.rowgroup_grid, kRowSegWarps * 32, 0, e->stream>>>(g);
+        pick_rowseg_group(e, e->rg_rows)<<<p.rowgroup_grid, kRowSegWarps * 32, 0, e->stream>>>(g);
         return mark_kernel(e, "sddmm_rowseg_group_kernel", e->stream);
     }
     if (e->rg_rows) {
@@ -1142,7 +1216,7 @@ int launch_all(sddmm_b200_engine *e, float *p_val) {
         pick_rowgroup(e->rg_rows, static_cast<int>(e->K / 32))<<<p.rowgroup_grid, kRowGroupWarps * 32, 0, e->stream>>>(g);
         return mark_kernel(e, "sddmm_rowgroup_kernel", e->stream);
     }
-    if (e->use_seg) return launch_rowseg(e, e->stream, p_val);
+    if (e->use_seg && e->n_dense == 0) return launch_rowseg(e, e->stream, p_val);
     // the two kernels write disjoint nonzeros: when both run, the row-tile kernel goes to the side stream
     static const bool no_side = std::getenv("SDDMM_B200_NO_SIDE_STREAM") != nullptr;   // tuning / debugging knob
     const bool both = e->n_dense > 0 && e->n_residual_items > 0 && !no_side;
@@ -1177,7 +1251,7 @@ int launch_all(sddmm_b200_engine *e, float *p_val) {
     a.item_ids = e->n_dense > 0 ? e->d_item_ids : nullptr;
     a.covered = e->n_dense > 0 ? e->d_covered : nullptr;
     a.err = e->h_err; a.nnz = e->nnz;
-    a.M = static_cast<int32_t>(e->M); a.K = static_cast<int32_t>(e->K);
+    a.M = static_cast<int32_t>(e->M); a.K = static_cast<int32_t>(e->K);   // (this kernel runs without row segments only: Ks = K)
     a.n_items = p.rowtile_items; a.item_nnz = p.rowtile_item_nnz; a.rows_per_stage = p.rowtile_rows_per_stage;
     if ((st = begin_kernel(e, rt_stream))) return st;
     if (e->mode == SDDMM_B200_BF16) {
@@ -1663,7 +1737,7 @@ int spmm_prepare(sddmm_b200_engine *e, int64_t K2) {
     Carve c;
     const size_t M = static_cast<size_t>(e->M), N = static_cast<size_t>(e->N), nnz = static_cast<size_t>(e->nnz);
     const size_t cap = nnz / 8 + std::min(M, nnz) + 8;
-    const size_t o_x = c.take(N * K2 * 4), o_y = c.take(M * K2 * 4), o_u = c.take(cap * sizeof(int2));
+    const size_t o_x = c.take(N * K2 * 4), o_y = c.take(M * K2 * 4), o_u = c.take(cap * sizeof(int2)), o_uc = c.take(cap * 32);
     const bool grow = c.off > e->spmm_arena.cap;
     if (grow) {
         if (e->spmm_arena.base) CU_TRY(e, cudaFree(e->spmm_arena.base));
@@ -1683,17 +1757,16 @@ int spmm_prepare(sddmm_b200_engine *e, int64_t K2) {
     e->d_X = reinterpret_cast<float *>(b + o_x);
     e->d_Y = reinterpret_cast<float *>(b + o_y);
     e->d_spmm_units = reinterpret_cast<int2 *>(b + o_u);
+    e->d_spmm_cols = reinterpret_cast<int32_t *>(b + o_uc);
     e->spmm_k2 = K2;
     if (e->spmm_units == 0 || moved) {   // plain row segments (one panel, no groups), counted / scanned / written on the device
         const int32_t Mi = static_cast<int32_t>(e->M);
-        const int n_tiles = static_cast<int>((e->M + kScanTile - 1) / kScanTile);
-        const int capb = e->sm_count * 32;
         cudaStream_t s = e->stream;
-        k_unit_count<<<grid_for(e->M, kBlock, capb), kBlock, 0, s>>>(e->d_rp, e->d_col, Mi, 1, 0, 0, e->d_unit_off);
-        k_scan_tile_sums<<<n_tiles, kScanBlock, 0, s>>>(e->d_unit_off, e->M, e->d_scan_tiles);
-        k_scan_sums<<<1, kScanBlock, 0, s>>>(e->d_scan_tiles, n_tiles, &e->d_pc->units);
-        k_scan_apply<<<n_tiles, kScanBlock, 0, s>>>(e->d_unit_off, e->M, e->d_scan_tiles);
-        k_unit_fill<<<grid_for(e->M * 32, kBlock, capb), kBlock, 0, s>>>(e->d_rp, e->d_col, Mi, 1, 0, 0, e->d_unit_off, e->d_spmm_units, nullptr);
+        const RunsOfRows runs{e->d_rp, e->d_col, Mi, static_cast<int32_t>(e->nnz)};
+        const int tiles = static_cast<int>((e->M + kUnitTile - 1) / kUnitTile);
+        CU_TRY(e, cudaMemsetAsync(&e->d_pc->units, 0, sizeof(unsigned long long), s));
+        k_unit_sums<<<tiles, kUnitBlock, 0, s>>>(runs, e->M, e->d_scan_tiles, e->d_pc);
+        k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, e->M, e->d_scan_tiles, static_cast<int64_t>(cap), e->d_pc, e->d_spmm_units, e->d_spmm_cols);
         CU_TRY(e, cudaGetLastError());
         PlanCounters pc;
         if (int rc = read_counters(e, &pc)) return rc;

@@ -46,14 +46,26 @@ __device__ __forceinline__ void group_rows(int32_t g, int32_t G, int32_t first, 
     r1 = g == 0 ? first : min(r0 + G, M);
 }
 
+// ... and how many groups there are
+__host__ __device__ __forceinline__ int32_t group_count(int32_t M, int32_t G, int32_t first) { return 1 + (M - first + G - 1) / G; }
+
 constexpr int kRowGroupWarps = 8;
 
 // Which groups of G rows share one column list.  One warp per group; only every `every`-th group is
 // looked at (every > 1: a sample, to choose G and `first` cheaply; group_ok is then not written).
 // cover += nonzeros inside matching groups; groups += matching groups.
-__global__ void k_group_match(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int32_t M, int32_t G, int32_t first,
-                              int32_t n_groups, int32_t every, uint8_t *__restrict__ group_ok, unsigned long long *__restrict__ cover,
-                              int *__restrict__ groups) {
+// G = 0: the nine candidates (G = 2, 3, 4; first full group at row 0 .. G-1), one per blockIdx.y, each counted in its slot
+// G (G - 1) / 2 - 1 + first.  (row_ptr and the columns may not have been validated yet: row bounds are checked here, columns are only compared.)
+__global__ void k_group_match(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int32_t M, int32_t nnz, int32_t G, int32_t first,
+                              int32_t every, uint8_t *__restrict__ group_ok, unsigned long long *__restrict__ cover, int *__restrict__ groups) {
+    if (G == 0) {
+        const int y = static_cast<int>(blockIdx.y);
+        G = y < 2 ? 2 : y < 5 ? 3 : 4;
+        first = y - (G * (G - 1) / 2 - 1);
+        cover += y;
+        groups += y;
+    }
+    const int32_t n_groups = group_count(M, G, first);
     const int lane = threadIdx.x & 31;
     const int64_t warp0 = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
     const int64_t n_warps = (gridDim.x * static_cast<int64_t>(blockDim.x)) >> 5;
@@ -65,10 +77,10 @@ __global__ void k_group_match(const int32_t *__restrict__ rp, const int32_t *__r
         if (ok) {
             const int32_t s0 = rp[r0];
             len = rp[r0 + 1] - s0;
-            ok = len > 0;
+            ok = len > 0 && s0 >= 0 && s0 <= nnz - len;
             for (int t = 1; t < G && ok; ++t) {
                 const int32_t st = rp[r0 + t];
-                ok = (rp[r0 + t + 1] - st) == len;
+                ok = (rp[r0 + t + 1] - st) == len && st >= 0 && st <= nnz - len;
                 if (ok) {
                     bool same = true;
                     for (int32_t j = lane; j < len; j += 32) same = same && (col[s0 + j] == col[st + j]);

@@ -1,28 +1,27 @@
-// Row-segment SDDMM kernel: the path for short and power-law rows.
+// Row-segment SDDMM kernels: the general path for short, long and power-law rows.
 //
-// Work decomposition (no atomics, exactly one writer per nonzero):
-//   * every row is cut into SEGMENTS of at most 8 consecutive nonzeros; the list of segments
-//     ("units": first CSR position, row, count) is built once per upload on the device, so the
-//     kernel itself searches nothing and stages nothing -- it is one streaming loop;
-//   * a warp step takes 4 consecutive units, one per 8-lane group.  Inside a group lane l loads
-//     column index l and S value l of the segment (one 32-byte access per group), the 8 column
-//     indices are exchanged with shuffles, every B row is read as one contiguous line by the
-//     group (lane = one 16-byte chunk; K > 32: more chunks per lane, 8 independent gathers per
-//     lane in flight), the lane's chunk of the ONE A row of the segment sits in registers, and
-//     the K-dot is reduced with the transposing shuffle tree that leaves nonzero l on lane l, so
-//     P.val is written by the lane that read S.val;
-//   * the unit two steps ahead and the column indices / S values one step ahead are requested
-//     before the current gathers are consumed.
+// Work decomposition (no atomics, exactly one writer per nonzero): every row is cut into SEGMENTS of at most 8
+// consecutive nonzeros.  The list of segments ("units": first CSR position, row, count) and a copy of each unit's 8
+// column indices are built once per upload on the device (unit_plan.cuh), so the kernels search nothing and stage
+// nothing -- they are one streaming loop, grid-stride, balanced whatever the row-length distribution.
 //
-// Column panels: when B is much larger than the L2 cache the unit list is built PANEL-MAJOR --
-// the columns are cut into P panels, a row contributes one run of segments per panel it touches,
-// and all segments of panel 0 come before those of panel 1 and so on.  All CTAs walk the list in
-// step, so the gathers of a panel find their B rows in L2 (the B loads carry an L2 evict_last
-// hint, the streams evict_first).  col_idx, S.val and P.val stay in CSR order: a run is a
-// contiguous piece of its row.
+// A warp step takes 8 consecutive units, one per group of 4 lanes.  A row of A or B is read in PIECES of 128 bytes: lane t
+// of a group holds bytes [32t, 32t + 32) of the piece in one 256-bit load, so one load instruction fetches the same piece
+// of 8 B rows (one per unit), and the A piece in registers serves the unit's 8 nonzeros.  The loop is ROLLING: as soon as
+// the B piece of slot i has been multiplied, its registers are given to the piece that slot needs next (the next piece of
+// the same units, or the first one of the next units), so a warp has 8 loads of 1 KB in flight all the time; unit headers
+// and column indices run one to two steps ahead, the A piece one stage ahead.  Every load is unconditional and in range (a
+// slot past a segment's end repeats its last nonzero, a group past the list's end the last unit); stores are predicated.
 //
-// A "chunk" is 4 consecutive K elements (8 for wide bf16 chunks).  CPL = chunks per lane, so K <= 8 * CPL chunks.
-// EXACT = (K == 8 * CPL chunks): no chunk-range predicates in the inner loop.
+// What bounds it: per nonzero one B row crosses from L2 to the SM (random 128-byte rows that hit L2: at most 153 G rows/s
+// measured, 64 bytes per clock and SM) and, where B does not fit L2, comes from HBM.  37.5 M nonzeros, K = 32, B in L2:
+// 294 us = 18.6 TB/s, against 347-365 us for a form with 16-byte chunks on groups of 8 lanes, which issues twice the loads
+// and four times the instructions per nonzero.
+//
+// Column panels: when B is much larger than the L2 cache the unit list is built PANEL-MAJOR -- the columns are cut into P
+// panels, a row contributes one run of segments per panel it touches, and all segments of panel 0 come before those of
+// panel 1 and so on.  All CTAs walk the list in step, so the gathers of a panel find most of their B rows in L2.  (L2
+// eviction hints on the gathers or on the streams make no difference: measured.)
 #pragma once
 
 #include "device_utils.cuh"
@@ -31,212 +30,290 @@ namespace sddmm {
 
 // unit.x = CSR position of the first nonzero of the segment; unit.y = row * 8 + (count - 1)
 constexpr int kUnitRowLimit = 1 << 28;   // rows the encoding can name
+constexpr int64_t kUnitLimit = (int64_t(1) << 31) - (int64_t(1) << 22);   // units a list may hold: step arithmetic stays in 32 bits
 
 struct RowSegArgs {
-    const int2 *units;        // n_units (> 0)
-    const int32_t *col_idx;   // nnz
-    const float *s_val;       // nnz
-    float *p_val;             // nnz
-    const void *A;            // M x K, element type ET
-    const void *B;            // N x K, element type ET
+    const int2 *units;         // n_units (> 0), padded to a multiple of 8 with copies of the last one
+    const int32_t *unit_cols;  // 8 column indices per unit (slots past the count repeat the last one)
+    const float *s_val;        // nnz values in CSR order, or (COPIES) 8 per unit in list order
+    float *p_val;              // nnz
+    const void *A;             // rows row_stride bytes apart, 32-byte aligned
+    const void *B;
     int32_t n_units;
-    int32_t K;
-    int32_t b_evict_last;     // B gathers ask L2 to keep their lines (column panels)
-    float b_fraction;         // share of the B lines the hint applies to (1 = all)
-    // column panels: copies of the units' column indices and S values, 8 slots of {column, value} per unit in list order
-    // (slots past the segment's end repeat its last nonzero): one 8-byte load per lane.  A panel run is a short piece of its
-    // row, so reading col_idx / S.val in place would touch one or two 32-byte sectors of a 128-byte line per unit; the
-    // copies are read front to back.  unit_sval is the same array (the values are its odd words).
-    const int32_t *unit_cols;
-    const float *unit_sval;
-    // K in slices (large K, B far larger than L2): the launch covers columns [k0, k0 + K) of rows that are row_stride bytes
-    // apart (A and B point at column k0; 0 = rows of exactly K elements) and, from the second slice on, adds to P.val
-    uint32_t row_stride;
-    int32_t accumulate;
+    uint32_t row_stride;       // bytes, a multiple of 32
+    int32_t row_bytes;         // bytes of a row that this launch covers (a multiple of 32)
 };
 
 constexpr int kRowSegWarps = 8;
-#ifndef SDDMM_ROWSEG_MINB1
-#define SDDMM_ROWSEG_MINB1 4   // resident CTAs per SM the compiler must allow for, K <= 32
-#endif
-#ifndef SDDMM_ROWSEG_MINBN
-#define SDDMM_ROWSEG_MINBN 2   // same, K > 32
-#endif
 
-// ---- L2 cache policy and loads that carry one (column panels) ------------------------------
-__device__ __forceinline__ uint64_t policy_evict_last(float fraction) {
-    uint64_t p;
-    asm("createpolicy.fractional.L2::evict_last.b64 %0, %1;" : "=l"(p) : "f"(fraction));
-    return p;
+// ---- 256-bit loads (32-byte aligned) and packed fp32 arithmetic ------------------------------------------------------
+// (volatile: the order in which the loads are written is the order of the rolling loop)
+struct Piece {
+    float2 v[4];
+};
+struct Cols8 {
+    int32_t v[8];
+};
+__device__ __forceinline__ Piece ld_piece(const unsigned char *p) {
+    Piece r;
+    asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(r.v[0].x), "=f"(r.v[0].y), "=f"(r.v[1].x), "=f"(r.v[1].y), "=f"(r.v[2].x), "=f"(r.v[2].y), "=f"(r.v[3].x),
+                   "=f"(r.v[3].y)
+                 : "l"(p));
+    return r;
 }
-// (read-only data and always-valid addresses: plain asm, the compiler may schedule these freely)
-__device__ __forceinline__ float4 ld_chunk_hint(const float4 *p, uint64_t pol) {
+__device__ __forceinline__ float4 ld_part(const unsigned char *p) {
     float4 v;
-    asm("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(pol));
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
     return v;
 }
-__device__ __forceinline__ uint2 ld_chunk_hint(const uint2 *p, uint64_t pol) {
-    uint2 v;
-    asm("ld.global.nc.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(v.x), "=r"(v.y) : "l"(p), "l"(pol));
-    return v;
+__device__ __forceinline__ Cols8 ld_cols(const int32_t *p) {
+    Cols8 r;
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
+                 : "l"(p));
+    return r;
 }
-__device__ __forceinline__ uint4 ld_chunk_hint(const uint4 *p, uint64_t pol) {
-    uint4 v;
-    asm("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(pol));
-    return v;
+// two IEEE fused multiply-adds in one instruction
+__device__ __forceinline__ float2 fma2(const float2 &a, const float2 &b, const float2 &c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<unsigned long long &>(d))
+        : "l"(reinterpret_cast<const unsigned long long &>(a)), "l"(reinterpret_cast<const unsigned long long &>(b)),
+          "l"(reinterpret_cast<const unsigned long long &>(c)));
+    return d;
 }
-
-// HINT: column panels -- the B gathers carry the L2 evict_last policy and column indices / S values come from the
-// per-unit copies (one instantiation with, one without: no branch per load).
-// SLICED: the launch covers a 64-column slice of longer rows (args.row_stride apart) and may add to P.val.
-// The add-to-P.val path (a predicated load of the old value at the top of a step, used by the final multiply-add) is
-// also compiled into the HINT instantiations although only slices switch it on: measured on the Poisson-rows
-// configuration with two column panels, K = 32, 575 -> 525 us per launch with it (the load is never issued; it changes
-// how the compiler groups the step's gathers into waits), while the instantiations without panels lose 6 % with it
-// (power-law rows 569 -> 604 us) and therefore do not carry it.
-template <int CPL, bool EXACT, typename ET, bool HINT, bool SLICED = false>
-__global__ void __launch_bounds__(kRowSegWarps * 32, (CPL == 1) ? SDDMM_ROWSEG_MINB1 : SDDMM_ROWSEG_MINBN) sddmm_rowseg_kernel(const RowSegArgs args) {
-    using chunk_t = typename ChunkOf<ET>::type;
-    using areg_t = typename ChunkOf<ET>::areg;
-    const int lane = threadIdx.x & 31;
-    const int gl = lane & 7;          // lane inside its 8-lane group = chunk of a 128-byte piece = nonzero of the segment
-    const int gbase = lane & 24;      // first lane of the group
-    const int grp = lane >> 3;        // which of the warp's 4 units
-    const int nchunks = EXACT ? 8 * CPL : (args.K / ChunkOf<ET>::elems);
-    const uint32_t row_bytes = SLICED ? args.row_stride : static_cast<uint32_t>(nchunks) * sizeof(chunk_t);   // distance between rows
-    constexpr bool kAccumulates = HINT || SLICED;
-    constexpr int QS = (CPL >= 2) ? 2 : 1;   // chunks gathered per nonzero per step
-    // chunks of this lane that exist (K < 32 * CPL: the lane's last chunks lie past the row and are read as chunk 0, times zero)
-    uint64_t pol_b = 0;
-    if (HINT) pol_b = policy_evict_last(args.b_fraction);
-
-    const int64_t n_quads = (static_cast<int64_t>(args.n_units) + 3) >> 2;
-    const int64_t n_warps = static_cast<int64_t>(gridDim.x) * kRowSegWarps;
-    int64_t q = static_cast<int64_t>(blockIdx.x) * kRowSegWarps + (threadIdx.x >> 5);
-    if (q >= n_quads) return;
-    const int last_unit = args.n_units - 1;
-
-    // per lane: byte offset of its chunk c inside a row, and whether the chunk exists
-    uint32_t ch_off[CPL];
-    float ch_on[CPL];
+__device__ __forceinline__ float dot_piece(const Piece &a, const Piece &b, float acc) {
+    float2 s = make_float2(acc, 0.f);
 #pragma unroll
-    for (int c = 0; c < CPL; ++c) {
-        const int ch = gl + 8 * c;
-        const bool on = EXACT || ch < nchunks;
-        ch_off[c] = static_cast<uint32_t>(on ? ch : 0) * sizeof(chunk_t);
-        ch_on[c] = on ? 1.f : 0.f;
-    }
-    const unsigned char *Ab = reinterpret_cast<const unsigned char *>(args.A);
-    const unsigned char *Bb = reinterpret_cast<const unsigned char *>(args.B);
+    for (int k = 0; k < 4; ++k) s = fma2(a.v[k], b.v[k], s);
+    return s.x + s.y;
+}
+// What the lanes past the end of a row's last piece read in place of A (one operand's zero is enough).  They are sent here
+// by their address: clearing the registers after the load would make every warp wait for it on the spot.
+__device__ __align__(32) const float g_zero_part[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+__device__ __forceinline__ const unsigned char *row_at(const unsigned char *base, int32_t row, uint32_t stride) {
+    return base + static_cast<uint64_t>(static_cast<uint32_t>(row)) * stride;
+}
 
-    // Every load below is unconditional and in range: a group past the end of the list repeats the last unit, a lane
-    // past the end of its segment repeats the segment's last nonzero; only the final store is predicated.
-    auto unit_index = [&](int64_t qq) -> int64_t { const int64_t u = 4 * qq + grp; return u < last_unit ? u : last_unit; };
-    auto load_unit = [&](int64_t qq) -> int2 { return __ldcs(args.units + unit_index(qq)); };
-    auto own_slot = [&](const int2 &u) -> int { return u.x + min(gl, u.y & 7); };
-    // column index / S value of this lane's nonzero of a unit, read in place (u: that unit's header)
-    auto own_col = [&](int64_t, const int2 &u) -> int { return __ldcs(args.col_idx + own_slot(u)); };
-    auto own_val = [&](int64_t, const int2 &u) -> float { return __ldcs(args.s_val + own_slot(u)); };
-
-    // (HINT: column index and S value of a slot lie side by side in the per-unit copies: one 8-byte load)
-    auto own_pair = [&](int64_t qq) -> int2 { return __ldcs(reinterpret_cast<const int2 *>(args.unit_cols) + 8 * unit_index(qq) + gl); };
-    int2 u_cur = load_unit(q);
-    int2 u_nxt = load_unit(q + n_warps);
-    int c_own;
-    float s_own;
-    if (HINT) {
-        const int2 cs = own_pair(q);
-        c_own = cs.x;
-        s_own = __int_as_float(cs.y);
-    } else {
-        c_own = own_col(q, u_cur);
-        s_own = own_val(q, u_cur);
+// Sum 8 per-lane values over the 4 lanes of a group: lane t ends up with the sums of slots t and t + 4.  (The additions of
+// a slot are the same ones whatever its position, so a nonzero's value does not depend on how its row was cut.)
+__device__ __forceinline__ float2 group4_transpose_reduce(const float (&a)[8], int t) {
+    float w[4];
+    const bool odd = (t & 1) != 0, high = (t & 2) != 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {   // w[i]: slot 2i + (t & 1)
+        const float send = odd ? a[2 * i] : a[2 * i + 1];
+        const float keep = odd ? a[2 * i + 1] : a[2 * i];
+        w[i] = keep + __shfl_xor_sync(kFullMask, send, 1);
     }
+    float2 r;
+    r.x = (high ? w[1] : w[0]) + __shfl_xor_sync(kFullMask, high ? w[0] : w[1], 2);
+    r.y = (high ? w[3] : w[2]) + __shfl_xor_sync(kFullMask, high ? w[2] : w[3], 2);
+    return r;
+}
+
+// fp32 rows of NP pieces (the last one may be partial: the lanes past its end multiply by zero).  COPIES: S values come from per-unit copies in list order (column panels: a run is a short piece of its row, whose
+// sectors two or more panel passes would read in turn).  ACC: add to P.val (later slices of K).
+// (All index arithmetic of the loop is 32-bit: with 64-bit selects the compiler splits the loop body and the rolling is
+// lost, 488 -> 574 us.  NP is a compile-time number for the same reason.)
+template <int NP, bool COPIES, bool ACC>
+__global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(const RowSegArgs args) {
+    const int lane = threadIdx.x & 31;
+    const int t = lane & 3;        // 32-byte part of a piece
+    const int grp = lane >> 2;     // which of the warp's 8 units
+    const int n_steps = (args.n_units + 7) >> 3;
+    const int n_warps = static_cast<int>(gridDim.x) * kRowSegWarps;
+    int b = static_cast<int>(blockIdx.x) * kRowSegWarps + (threadIdx.x >> 5);
+    if (b >= n_steps) return;
+    const int last_unit = args.n_units - 1;
+    const bool off = 128 * (NP - 1) + 32 * t >= args.row_bytes;   // this lane's part of the last piece lies past the row
+    const uint32_t stride = args.row_stride;
+    const unsigned char *At = static_cast<const unsigned char *>(args.A) + 32 * t;
+    const unsigned char *Bt = static_cast<const unsigned char *>(args.B) + 32 * t;
+    const int o_last = off ? args.row_bytes - 32 - 32 * t : 128 * (NP - 1);   // (such a lane reads the row's last 32 bytes)
+
+    auto unit_index = [&](int step) -> int { const int u = 8 * step + grp; return u < last_unit ? u : last_unit; };
+    auto load_unit = [&](int step) -> int2 { return __ldcs(args.units + unit_index(step)); };
+    auto load_cols = [&](int step) -> Cols8 { return ld_cols(args.unit_cols + 8 * static_cast<int64_t>(unit_index(step))); };
+    auto piece_offset = [&](int p) -> int { return p == NP - 1 ? o_last : 128 * p; };
+    auto load_a = [&](int row, int p) -> Piece {
+        const unsigned char *q = row_at(At + piece_offset(p), row, stride);
+        return ld_piece(p == NP - 1 && off ? reinterpret_cast<const unsigned char *>(g_zero_part) : q);
+    };
+
+    int2 un = load_unit(b), un_next = load_unit(b + n_warps);
+    Cols8 cols = load_cols(b);
+    Piece a = load_a(un.y >> 3, 0), bq[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) bq[i] = ld_piece(row_at(Bt + piece_offset(0), cols.v[i], stride));
+    Cols8 cols_next = load_cols(b + n_warps);
 
     while (true) {
-        const int row = u_cur.y >> 3;
-        const int j = u_cur.x + gl;
-        const bool valid = (gl <= (u_cur.y & 7)) && (4 * q + grp <= last_unit);
-        const float s = s_own;
-        float p_old = 0.f;   // (a later K slice: what the earlier slices left, requested before the gathers)
-        if (kAccumulates && args.accumulate && valid) p_old = __ldcs(args.p_val + j);
-
-        // ---- this lane's chunk(s) of the segment's A row ----
-        areg_t areg[CPL];
-        {
-            const unsigned char *arow = Ab + static_cast<uint64_t>(static_cast<uint32_t>(row)) * row_bytes;
-#pragma unroll
-            for (int c = 0; c < CPL; ++c) {
-                areg[c] = unpack_chunk(ldg_chunk(reinterpret_cast<const chunk_t *>(arow + ch_off[c])));
-                if (!EXACT) scale_chunk(areg[c], ch_on[c]);
-            }
-        }
-        // ---- the 8 column indices of the segment ----
-        const unsigned char *brow[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            brow[i] = Bb + static_cast<uint64_t>(static_cast<uint32_t>(__shfl_sync(kFullMask, c_own, gbase + i))) * row_bytes;
+        const int next = b + n_warps;
+        const int count = 8 * b + grp <= last_unit ? (un.y & 7) : -1;
+        // S values of the slots this lane will write (t and t + 4), requested before the gathers
+        const float *sv = COPIES ? args.s_val + 8 * static_cast<int64_t>(unit_index(b)) : args.s_val + un.x;
+        const float s0 = __ldcs(sv + (COPIES ? t : min(t, un.y & 7)));
+        const float s1 = __ldcs(sv + (COPIES ? t + 4 : min(t + 4, un.y & 7)));
+        float p0 = 0.f, p1 = 0.f;
+        if (ACC && t <= count) p0 = __ldcs(args.p_val + un.x + t);
+        if (ACC && t + 4 <= count) p1 = __ldcs(args.p_val + un.x + t + 4);
+        const int2 un_next2 = load_unit(next + n_warps);
+        const Cols8 cols_next2 = load_cols(next + n_warps);
 
         float acc[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-
-        // ---- gather B rows (first pass), then request what the next steps need, then multiply ----
-        chunk_t bq[8][QS];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int p = 0; p < NP; ++p) {
+            const bool last = p == NP - 1;
+            const int p_next = last ? 0 : p + 1;
+            const Piece a_next = load_a((last ? un_next.y : un.y) >> 3, p_next);
 #pragma unroll
-            for (int qq = 0; qq < QS; ++qq) {
-                const chunk_t *src = reinterpret_cast<const chunk_t *>(brow[i] + ch_off[qq]);
-                bq[i][qq] = HINT ? ld_chunk_hint(src, pol_b) : ldg_chunk(src);
+            for (int i = 0; i < 8; ++i) {
+                acc[i] = dot_piece(a, bq[i], acc[i]);
+                bq[i] = ld_piece(row_at(Bt + piece_offset(p_next), last ? cols_next.v[i] : cols.v[i], stride));
             }
-        const int64_t q_next = q + n_warps;
-        const int2 u_nxt2 = load_unit(q_next + n_warps);
-        if (HINT) {
-            const int2 cs = own_pair(q_next);
-            c_own = cs.x;
-            s_own = __int_as_float(cs.y);
-        } else {
-            c_own = own_col(q_next, u_nxt);
-            s_own = own_val(q_next, u_nxt);
+            a = a_next;
         }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int qq = 0; qq < QS; ++qq) acc[i] = dot_chunk(areg[qq], unpack_chunk(bq[i][qq]), acc[i]);
-        // more than QS chunks per lane: the remaining chunks of the same 8 rows
-#pragma unroll
-        for (int q0 = QS; q0 < CPL; q0 += QS) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int qq = 0; qq < QS; ++qq) {
-                    const chunk_t *src = reinterpret_cast<const chunk_t *>(brow[i] + ch_off[q0 + qq]);
-                    bq[i][qq] = HINT ? ld_chunk_hint(src, pol_b) : ldg_chunk(src);
-                }
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int qq = 0; qq < QS; ++qq) acc[i] = dot_chunk(areg[q0 + qq], unpack_chunk(bq[i][qq]), acc[i]);
-        }
-        const float dot = group8_transpose_reduce(acc, gl);   // lane gl: nonzero gl of the segment
-        if (valid) __stcs(args.p_val + j, kAccumulates ? fmaf(dot, s, p_old) : dot * s);
+        const float2 dot = group4_transpose_reduce(acc, t);
+        if (t <= count) __stcs(args.p_val + un.x + t, ACC ? fmaf(dot.x, s0, p0) : dot.x * s0);
+        if (t + 4 <= count) __stcs(args.p_val + un.x + t + 4, ACC ? fmaf(dot.y, s1, p1) : dot.y * s1);
 
-        q = q_next;
-        if (q >= n_quads) break;   // warp-uniform
-        u_cur = u_nxt;
-        u_nxt = u_nxt2;
+        if (next >= n_steps) break;   // warp-uniform
+        b = next;
+        un = un_next;
+        un_next = un_next2;
+        cols = cols_next;
+        cols_next = cols_next2;
     }
 }
 
-// ---- row groups: segments shared by NR consecutive rows with identical column lists ---------------
+// ---- bf16 storage ----------------------------------------------------------------------------------------------------
+// The products of a gathered bf16 row with its A row run on mma.sync (m16n8k16, fp32 accumulators): unpacking to fp32 and
+// multiplying costs two instructions per element and was what bounded this mode.  The 16 rows of the first operand are the
+// gathered B rows of the 8 slots of TWO units, the 8 columns of the second operand are the A rows of the warp step's 8
+// units; of the 16 x 8 products the 2 columns that belong to the two units are kept.  The order of the k elements is free
+// as long as both operands use the same one, so the fragments are exactly what a lane has loaded (LB contiguous bytes of
+// its row) and nothing is shuffled: lane (slot g, part t) of a step ends up with slot g of units 2t and 2t + 1.
+// 37.5 M nonzeros, B in L2: K = 32 / 64 / 128 299 / 403 / 601 us, against 375 / 512 / 912 us with unpack + FMA.  (Gathered
+// rows as the second operand, one unit per instruction, doubles the number of mma: 327 / 440 / 740 us.)
+template <int LB>
+struct Frag {
+    uint32_t r[LB / 4];
+};
+__device__ __forceinline__ void ld_frag(Frag<32> &f, const unsigned char *p) {
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(f.r[0]), "=r"(f.r[1]), "=r"(f.r[2]), "=r"(f.r[3]), "=r"(f.r[4]), "=r"(f.r[5]), "=r"(f.r[6]), "=r"(f.r[7])
+                 : "l"(p));
+}
+__device__ __forceinline__ void ld_frag(Frag<16> &f, const unsigned char *p) {
+    asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(f.r[0]), "=r"(f.r[1]), "=r"(f.r[2]), "=r"(f.r[3]) : "l"(p));
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// NP pieces of 4 * LB bytes per row (the last one may be partial), R units' rows in flight per warp
+template <int NP, int LB, int R, int MINB, bool COPIES>
+__global__ void __launch_bounds__(kRowSegWarps * 32, MINB) sddmm_rowseg_bf16_kernel(const RowSegArgs args) {
+    const int lane = threadIdx.x & 31;
+    const int t = lane & 3;        // LB-byte part of a piece
+    const int grp = lane >> 2;     // slot of a gathered row, unit of an A row
+    const int n_steps = (args.n_units + 7) >> 3;
+    const int n_warps = static_cast<int>(gridDim.x) * kRowSegWarps;
+    int b = static_cast<int>(blockIdx.x) * kRowSegWarps + (threadIdx.x >> 5);
+    if (b >= n_steps) return;
+    const int last_unit = args.n_units - 1, last_step = n_steps - 1;
+    const bool off = 4 * LB * (NP - 1) + LB * t >= args.row_bytes;   // this lane's part of the last piece lies past the row
+    const uint32_t stride = args.row_stride;
+    const unsigned char *At = static_cast<const unsigned char *>(args.A) + LB * t;
+    const unsigned char *Bt = static_cast<const unsigned char *>(args.B) + LB * t;
+    const int o_last = off ? args.row_bytes - LB - LB * t : 4 * LB * (NP - 1);   // (such a lane reads the row's last LB bytes)
+
+    struct Row {
+        Frag<LB> p[NP];
+    };
+    auto piece_offset = [&](int p) -> int { return p == NP - 1 ? o_last : 4 * LB * p; };
+    auto load_row = [&](Row &f, const unsigned char *base, int row) {
+        const unsigned char *q = row_at(base, row, stride);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) ld_frag(f.p[p], q + piece_offset(p));
+    };
+    auto load_a = [&](Row &f, int row) {
+        const unsigned char *q = row_at(At, row, stride);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) ld_frag(f.p[p], p == NP - 1 && off ? reinterpret_cast<const unsigned char *>(g_zero_part) : q + piece_offset(p));
+    };
+    auto load_code = [&](int step) -> int { return __ldcs(&args.units[8 * static_cast<int64_t>(min(step, last_step)) + grp].y); };
+    auto load_cols = [&](int step) -> Cols8 {   // slot grp of the step's 8 units
+        Cols8 c;
+        const int32_t *q = args.unit_cols + 64 * static_cast<int64_t>(min(step, last_step)) + grp;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) c.v[u] = __ldcs(q + 8 * u);
+        return c;
+    };
+
+    int code_next = load_code(b + n_warps);
+    Cols8 cols = load_cols(b);
+    Row a, bq[R];
+    load_a(a, load_code(b) >> 3);
+#pragma unroll
+    for (int u = 0; u < R; ++u) load_row(bq[u], Bt, cols.v[u]);
+
+    while (true) {
+        const int next = b + n_warps;
+        const int4 un = __ldcs(reinterpret_cast<const int4 *>(args.units + 8 * static_cast<int64_t>(b)) + t);   // units 2t, 2t + 1
+        const int c0 = 8 * b + 2 * t <= last_unit ? (un.y & 7) : -1, c1 = 8 * b + 2 * t + 1 <= last_unit ? (un.w & 7) : -1;
+        const float *sv = args.s_val + 64 * static_cast<int64_t>(b) + 16 * t + grp;
+        const float s0 = COPIES ? __ldcs(sv) : __ldcs(args.s_val + un.x + min(grp, un.y & 7));
+        const float s1 = COPIES ? __ldcs(sv + 8) : __ldcs(args.s_val + un.z + min(grp, un.w & 7));
+        const int code_next2 = load_code(next + n_warps);
+        const Cols8 cols_next = load_cols(next);
+        Row a_next;
+        load_a(a_next, code_next >> 3);
+        float r0 = 0.f, r1 = 0.f;
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+            float c[4] = {0.f, 0.f, 0.f, 0.f};
+            Row &x = bq[u % R], &y = bq[(u + 1) % R];
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+#pragma unroll
+                for (int k = 0; k < LB / 4; k += 2) mma_bf16(c, x.p[p].r[k], y.p[p].r[k], x.p[p].r[k + 1], y.p[p].r[k + 1], a.p[p].r[k], a.p[p].r[k + 1]);
+            load_row(x, Bt, u + R < 8 ? cols.v[(u + R) & 7] : cols_next.v[(u + R) & 7]);
+            load_row(y, Bt, u + 1 + R < 8 ? cols.v[(u + 1 + R) & 7] : cols_next.v[(u + 1 + R) & 7]);
+            if (u == 2 * t) {   // columns 2t (slots of unit u) and 2t + 1 (slots of unit u + 1)
+                r0 = c[0];
+                r1 = c[3];
+            }
+        }
+        if (grp <= c0) __stcs(args.p_val + un.x + grp, r0 * s0);
+        if (grp <= c1) __stcs(args.p_val + un.z + grp, r1 * s1);
+
+        if (next >= n_steps) break;   // warp-uniform
+        b = next;
+        code_next = code_next2;
+        cols = cols_next;
+        a = a_next;
+    }
+}
+
+// ---- row groups: segments shared by NR consecutive rows with identical column lists ---------------------------------
 // Block-structured matrices (several unknowns per mesh node) repeat one column list over the G rows of a block row.
 // A unit of such a group covers 8 columns of the shared list for all G rows: each B row is gathered ONCE and dotted
 // with G rows of A, so the traffic between L2 and the SM -- what bounds the gather -- drops by the factor G.
 //   ghdr[u]  .x = CSR position of the segment in the group's first row, .y = first row * 8 + (count - 1),
 //            .z = row length L (row t of the group holds the segment at .x + t * L: equal lengths, consecutive rows),
 //            .w = rows that share the unit (1 for rows outside matching groups, else G)
-// fp32 storage, K = 32 * CPL, CPL in {1, 2}; NR = G.
+// fp32 storage, rows of 32 * CPL elements (zero-padded where K is less), CPL in {1, 2}; NR = G.  The NR rows of A and
+// NR x 8 sums need the registers that the kernel above gives to 256-bit loads and to rolling: here a group is 8 lanes of
+// 16 bytes, 4 units per warp step.  Bound by the load/store unit and the shuffles: with every load an L1 hit it still takes
+// 289 of 302 us (36.8 M nonzeros in 3 x 3 blocks, K = 64).  Tried and no faster: the rolling loop with 16-byte parts (322 us)
+// and with 32-byte parts on 4 lanes (329-440 us: 12 to 16 warps do not cover the latency), packed fp32 arithmetic (332 us).
 struct RowSegGroupArgs {
     const int4 *ghdr;         // n_units (> 0)
     const int32_t *col_idx;   // nnz
@@ -335,242 +412,6 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, (CPL == 1) ? 3 : 2) sddmm_r
         if (q >= n_quads) break;   // warp-uniform
         u_cur = u_nxt;
         u_nxt = u_nxt2;
-    }
-}
-
-// rows of group g when groups of G rows start at row `first` (group 0 = the rows before it)
-__device__ __forceinline__ void unit_group_rows(int32_t g, int32_t G, int32_t first, int32_t M, int32_t &r0, int32_t &r1) {
-    r0 = g == 0 ? 0 : first + (g - 1) * G;
-    r1 = g == 0 ? first : min(r0 + G, M);
-}
-// one thread per row: units the row contributes -- the leader of a matching group speaks for its whole group
-__global__ void k_group_unit_count(const int32_t *__restrict__ rp, int32_t M, int32_t G, int32_t first, const uint8_t *__restrict__ group_ok,
-                                   int32_t *__restrict__ counts) {
-    for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < M; r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int32_t g = r < first ? 0 : 1 + static_cast<int32_t>((r - first) / G);
-        int32_t r0, r1;
-        unit_group_rows(g, G, first, M, r0, r1);
-        const int32_t len = rp[r + 1] - rp[r];
-        counts[r] = (group_ok[g] && r != r0) ? 0 : (len + 7) >> 3;
-    }
-}
-// one warp per row: write its units at the scanned offset
-__global__ void k_group_unit_fill(const int32_t *__restrict__ rp, int32_t M, int32_t G, int32_t first, const uint8_t *__restrict__ group_ok,
-                                  const int32_t *__restrict__ offsets, int4 *__restrict__ ghdr) {
-    const int lane = threadIdx.x & 31;
-    const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t r = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5; r < M; r += n_warps) {
-        const int32_t g = r < first ? 0 : 1 + static_cast<int32_t>((r - first) / G);
-        int32_t r0, r1;
-        unit_group_rows(g, G, first, M, r0, r1);
-        const bool matched = group_ok[g] != 0;
-        if (matched && r != r0) continue;
-        const int32_t s = rp[r], e = rp[r + 1];
-        const int32_t n_units = (e - s + 7) >> 3;
-        const int32_t off = offsets[r];
-        for (int32_t u = lane; u < n_units; u += 32) {
-            const int32_t start = s + 8 * u;
-            ghdr[off + u] = make_int4(start, static_cast<int32_t>(r) * 8 + (min(8, e - start) - 1), e - s, matched ? G : 1);
-        }
-    }
-}
-
-// ---- building the unit list (once per upload) -------------------------------------------
-// Run of row i inside column panel p: [s, e) in CSR positions.  One panel: the whole row.
-// Needs non-decreasing column indices inside a row when there is more than one panel.
-// long_rows > 0: only rows of at least that many nonzeros are cut into column panels (panels 0 .. panels-2, panel_cols
-// columns each); the shorter rows follow whole, as the last "panel" of the list -- a run of one or two nonzeros would
-// leave most of a segment's slots empty.
-__device__ __forceinline__ void panel_run(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int32_t i, int32_t p,
-                                          int32_t panels, int32_t panel_cols, int32_t long_rows, int32_t &s, int32_t &e) {
-    const int32_t a = rp[i], b = rp[i + 1];
-    if (panels == 1) {
-        s = a;
-        e = b;
-        return;
-    }
-    if (long_rows > 0) {
-        const bool is_long = b - a >= long_rows;
-        if (p == panels - 1) {           // the short rows, whole
-            s = a;
-            e = is_long ? a : b;
-            return;
-        }
-        if (!is_long) {
-            s = e = a;
-            return;
-        }
-        --panels;                        // the real column panels
-    }
-    auto lower = [&](int64_t c) {   // first position whose column is >= c
-        int32_t lo = a, hi = b;
-        while (lo < hi) {
-            const int32_t mid = (lo + hi) >> 1;
-            if (col[mid] < c) lo = mid + 1; else hi = mid;
-        }
-        return lo;
-    };
-    s = (p == 0) ? a : lower(static_cast<int64_t>(p) * panel_cols);
-    e = (p == panels - 1) ? b : lower(static_cast<int64_t>(p + 1) * panel_cols);
-}
-
-// one thread per (panel, row), panel-major: number of units of that run
-__global__ void k_unit_count(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int32_t M, int32_t panels,
-                             int32_t panel_cols, int32_t long_rows, int32_t *__restrict__ counts) {
-    const int64_t n = static_cast<int64_t>(panels) * M;
-    for (int64_t qi = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; qi < n;
-         qi += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int32_t p = static_cast<int32_t>(qi / M), i = static_cast<int32_t>(qi - static_cast<int64_t>(p) * M);
-        int32_t s, e;
-        panel_run(rp, col, i, p, panels, panel_cols, long_rows, s, e);
-        counts[qi] = (e - s + 7) >> 3;
-    }
-}
-
-// one warp per (panel, row): write its units at the scanned offset
-__global__ void k_unit_fill(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int32_t M, int32_t panels,
-                            int32_t panel_cols, int32_t long_rows, const int32_t *__restrict__ offsets, int2 *__restrict__ units,
-                            int32_t *__restrict__ ucols) {
-    const int lane = threadIdx.x & 31;
-    const int64_t n = static_cast<int64_t>(panels) * M;
-    const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t qi = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5; qi < n; qi += n_warps) {
-        const int32_t p = static_cast<int32_t>(qi / M), i = static_cast<int32_t>(qi - static_cast<int64_t>(p) * M);
-        int32_t s, e;
-        panel_run(rp, col, i, p, panels, panel_cols, long_rows, s, e);
-        const int32_t n_units = (e - s + 7) >> 3;
-        const int32_t off = offsets[qi];
-        for (int32_t u = lane; u < n_units; u += 32) {
-            const int32_t first = s + 8 * u;
-            const int32_t cnt = min(8, e - first);
-            units[off + u] = make_int2(first, i * 8 + (cnt - 1));
-        }
-        if (ucols)   // per-unit copies of the column indices (slots past the end of the run repeat its last column)
-            for (int32_t t = lane; t < 8 * n_units; t += 32) ucols[2 * (8 * static_cast<int64_t>(off) + t)] = col[min(s + t, e - 1)];
-    }
-}
-
-// per-unit copies of the S values (one thread per slot): refreshed whenever S.val changes
-__global__ void k_unit_values(const int2 *__restrict__ units, int32_t n_units, const float *__restrict__ s_val, float *__restrict__ usval) {   // usval: the {column, value} slots
-    for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < 8 * static_cast<int64_t>(n_units);
-         t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int2 u = units[t >> 3];
-        usval[2 * t + 1] = s_val[u.x + min(static_cast<int>(t & 7), u.y & 7)];
-    }
-}
-
-// ---- units over what the dense tiles left: runs of nonzeros whose bit in `covered` is clear -----------------------
-// first position in [j, b) whose bit equals `want`, or b
-__device__ __forceinline__ int32_t next_bit(const uint32_t *__restrict__ bits, int32_t j, int32_t b, bool want) {
-    while (j < b) {
-        uint32_t word = bits[j >> 5];
-        if (!want) word = ~word;
-        word >>= (j & 31);
-        if (word) return min(b, j + __ffs(word) - 1);
-        j = (j | 31) + 1;
-    }
-    return b;
-}
-// one thread per row: units of its uncovered runs
-__global__ void k_residual_unit_count(const int32_t *__restrict__ rp, int32_t M, const uint32_t *__restrict__ covered, int32_t *__restrict__ counts) {
-    for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < M; r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int32_t b = rp[r + 1];
-        int32_t n = 0;
-        for (int32_t j = next_bit(covered, rp[r], b, false); j < b;) {
-            const int32_t e = next_bit(covered, j, b, true);
-            n += (e - j + 7) >> 3;
-            j = next_bit(covered, e, b, false);
-        }
-        counts[r] = n;
-    }
-}
-__global__ void k_residual_unit_fill(const int32_t *__restrict__ rp, int32_t M, const uint32_t *__restrict__ covered,
-                                     const int32_t *__restrict__ offsets, int2 *__restrict__ units) {
-    for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < M; r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int32_t b = rp[r + 1];
-        int32_t off = offsets[r];
-        for (int32_t j = next_bit(covered, rp[r], b, false); j < b;) {
-            const int32_t e = next_bit(covered, j, b, true);
-            for (int32_t first = j; first < e; first += 8) units[off++] = make_int2(first, static_cast<int32_t>(r) * 8 + (min(8, e - first) - 1));
-            j = next_bit(covered, e, b, false);
-        }
-    }
-}
-
-// ---- exclusive scan of int32 counts (three small kernels) -----------------------------------
-constexpr int kScanBlock = 256;
-constexpr int kScanPerThread = 8;
-constexpr int kScanTile = kScanBlock * kScanPerThread;
-
-__device__ __forceinline__ int32_t warp_inclusive_scan(int32_t v, int lane) {
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int32_t t = __shfl_up_sync(kFullMask, v, off);
-        if (lane >= off) v += t;
-    }
-    return v;
-}
-// inclusive scan of one value per thread over a block of kScanBlock threads; returns the thread's inclusive prefix,
-// *total = block sum
-__device__ __forceinline__ int32_t block_inclusive_scan(int32_t v, int32_t *total) {
-    __shared__ int32_t warp_sums[kScanBlock / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int32_t inc = warp_inclusive_scan(v, lane);
-    if (lane == 31) warp_sums[w] = inc;
-    __syncthreads();
-    int32_t base = 0, tot = 0;
-#pragma unroll
-    for (int k = 0; k < kScanBlock / 32; ++k) {
-        const int32_t t = warp_sums[k];
-        if (k < w) base += t;
-        tot += t;
-    }
-    __syncthreads();
-    *total = tot;
-    return inc + base;
-}
-
-// pass 1: sum of every tile of kScanTile values
-__global__ void __launch_bounds__(kScanBlock) k_scan_tile_sums(const int32_t *__restrict__ v, int64_t n, int32_t *__restrict__ tile_sums) {
-    const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile + static_cast<int64_t>(threadIdx.x) * kScanPerThread;
-    int32_t local = 0;
-#pragma unroll
-    for (int k = 0; k < kScanPerThread; ++k)
-        if (base + k < n) local += v[base + k];
-    int32_t total;
-    block_inclusive_scan(local, &total);
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
-}
-// pass 2 (one block): exclusive scan of the tile sums in place; *grand_total = sum of everything
-__global__ void __launch_bounds__(kScanBlock) k_scan_sums(int32_t *__restrict__ tile_sums, int32_t n_tiles, unsigned long long *__restrict__ grand_total) {
-    int64_t carry = 0;
-    for (int32_t base = 0; base < n_tiles; base += kScanBlock) {
-        const int32_t idx = base + static_cast<int32_t>(threadIdx.x);
-        const int32_t v = idx < n_tiles ? tile_sums[idx] : 0;
-        int32_t total;
-        const int32_t inc = block_inclusive_scan(v, &total);
-        if (idx < n_tiles) tile_sums[idx] = static_cast<int32_t>(carry) + inc - v;
-        carry += total;
-    }
-    if (threadIdx.x == 0) *grand_total = static_cast<unsigned long long>(carry);
-}
-// pass 3: exclusive scan inside every tile plus the tile's offset, in place
-__global__ void __launch_bounds__(kScanBlock) k_scan_apply(int32_t *__restrict__ v, int64_t n, const int32_t *__restrict__ tile_offsets) {
-    const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile + static_cast<int64_t>(threadIdx.x) * kScanPerThread;
-    int32_t x[kScanPerThread];
-    int32_t local = 0;
-#pragma unroll
-    for (int k = 0; k < kScanPerThread; ++k) {
-        x[k] = (base + k < n) ? v[base + k] : 0;
-        local += x[k];
-    }
-    int32_t total;
-    const int32_t inc = block_inclusive_scan(local, &total);
-    int32_t run = tile_offsets[blockIdx.x] + inc - local;
-#pragma unroll
-    for (int k = 0; k < kScanPerThread; ++k) {
-        if (base + k < n) v[base + k] = run;
-        run += x[k];
     }
 }
 

@@ -41,9 +41,15 @@ __device__ __forceinline__ int len_bin(int len) {
     return b < SDDMM_B200_HIST_BINS ? b : SDDMM_B200_HIST_BINS - 1;
 }
 
-// one thread per row: monotonicity, histogram, max, nonempty count, row-start bits
-__global__ void k_row_stats(const int32_t *__restrict__ rp, int32_t M, int64_t nnz, uint32_t *__restrict__ row_start_bits,
-                            PlanCounters *__restrict__ pc) {
+// unit lists (unit_plan.cuh) are scanned in tiles of this many entries
+constexpr int kUnitBlock = kPlanBlock;
+constexpr int kUnitTile = 1024;                          // entries per tile (4 per thread)
+constexpr int kUnitPerThread = kUnitTile / kUnitBlock;
+
+// One tile of rows per block: monotonicity, histogram, max, nonempty count, row-start bits, and (tile_sums != nullptr) the
+// units of the tile when every row is one run -- pass 1 of the plain unit list.
+__global__ void __launch_bounds__(kUnitBlock) k_row_stats(const int32_t *__restrict__ rp, int32_t M, int64_t nnz, uint32_t *__restrict__ row_start_bits,
+                                                          int32_t *__restrict__ tile_sums, PlanCounters *__restrict__ pc) {
     __shared__ unsigned int sh[SDDMM_B200_HIST_BINS];
     __shared__ unsigned long long sh_nnz[SDDMM_B200_HIST_BINS];
     __shared__ unsigned int s_nonempty;
@@ -51,14 +57,18 @@ __global__ void k_row_stats(const int32_t *__restrict__ rp, int32_t M, int64_t n
     if (threadIdx.x < SDDMM_B200_HIST_BINS) { sh[threadIdx.x] = 0; sh_nnz[threadIdx.x] = 0; }
     if (threadIdx.x == 0) { s_nonempty = 0; s_max = 0; }
     __syncthreads();
-    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (i < M) {
+    int32_t units = 0;
+#pragma unroll
+    for (int k = 0; k < kUnitPerThread; ++k) {
+        const int64_t i = blockIdx.x * static_cast<int64_t>(kUnitTile) + k * kUnitBlock + threadIdx.x;
+        if (i >= M) break;
         const int a = rp[i], b = rp[i + 1];
         const int len = b - a;
         if (len < 0 || a < 0 || b > nnz) {
             pc->bad_row_ptr = 1;
         } else {
             atomicAdd(&sh[len_bin(len)], 1u);
+            units += (len + 7) >> 3;
             if (len > 0) {
                 atomicAdd(&sh_nnz[len_bin(len)], static_cast<unsigned long long>(len));
                 atomicAdd(&s_nonempty, 1u);
@@ -69,7 +79,11 @@ __global__ void k_row_stats(const int32_t *__restrict__ rp, int32_t M, int64_t n
         if (i == 0 && a != 0) pc->bad_row_ptr = 1;
         if (i == M - 1 && b != nnz) pc->bad_row_ptr = 1;
     }
-    __syncthreads();
+    const int32_t total = block_sum(units);   // (a block-wide barrier)
+    if (threadIdx.x == 0 && tile_sums) {
+        tile_sums[blockIdx.x] = total;
+        if (total) atomicAdd(&pc->units, static_cast<unsigned long long>(total));
+    }
     if (threadIdx.x < SDDMM_B200_HIST_BINS && sh[threadIdx.x]) {
         atomicAdd(&pc->hist[threadIdx.x], (unsigned long long)sh[threadIdx.x]);
         if (sh_nnz[threadIdx.x]) atomicAdd(&pc->hist_nnz[threadIdx.x], sh_nnz[threadIdx.x]);
@@ -80,9 +94,10 @@ __global__ void k_row_stats(const int32_t *__restrict__ rp, int32_t M, int64_t n
     }
 }
 
-// one thread per nonzero: column range, touched-column flags, in-row ordering
-__global__ void k_col_scan(const int32_t *__restrict__ col, int64_t nnz, int32_t N, const uint32_t *__restrict__ row_start_bits,
-                           unsigned char *__restrict__ touched, PlanCounters *__restrict__ pc) {
+// one thread per nonzero: column range, distinct columns (one bit each), in-row ordering
+__global__ void __launch_bounds__(kPlanBlock) k_col_scan(const int32_t *__restrict__ col, int64_t nnz, int32_t N, const uint32_t *__restrict__ row_start_bits,
+                           uint32_t *__restrict__ touched, PlanCounters *__restrict__ pc) {
+    int32_t fresh = 0;
     for (int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; j < nnz;
          j += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const int c = col[j];
@@ -90,7 +105,8 @@ __global__ void k_col_scan(const int32_t *__restrict__ col, int64_t nnz, int32_t
             pc->bad_col = 1;
             continue;
         }
-        if (!touched[c]) touched[c] = 1;
+        const uint32_t bit = 1u << (c & 31);
+        if (!(touched[c >> 5] & bit) && !(atomicOr(&touched[c >> 5], bit) & bit)) ++fresh;   // (a stale read only costs an atomic)
         const bool is_start = (row_start_bits[j >> 5] >> (j & 31)) & 1u;
         if (!is_start && j > 0) {
             const int prev = col[j - 1];
@@ -98,15 +114,8 @@ __global__ void k_col_scan(const int32_t *__restrict__ col, int64_t nnz, int32_t
             if (prev == c) pc->dup_cols = 1;
         }
     }
-}
-
-__global__ void k_count_bytes(const unsigned char *__restrict__ flags, int64_t n, unsigned long long *__restrict__ out) {
-    unsigned int local = 0;
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        local += flags[i] ? 1u : 0u;
-    for (int off = 16; off > 0; off >>= 1) local += __shfl_xor_sync(kFullMask, local, off);
-    if ((threadIdx.x & 31) == 0 && local) atomicAdd(out, (unsigned long long)local);
+    const int32_t total = block_sum(fresh);
+    if (threadIdx.x == 0 && total) atomicAdd(&pc->cols_touched, static_cast<unsigned long long>(total));
 }
 
 // COO (sorted by row) -> row_ptr.  Thread j owns the rows in (row[j-1], row[j]].  `base` is subtracted from every row index
@@ -413,13 +422,40 @@ __global__ void k_split_concat_tf32(const float *__restrict__ in, float *__restr
     }
 }
 
-// bf16 storage: out = bf16(in), and `in` keeps the rounded value (as fp32) for the tensor-core path
-__global__ void k_f32_to_bf16(float *__restrict__ in, __nv_bfloat16 *__restrict__ out, int64_t n) {
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const __nv_bfloat16 r = __float2bfloat16_rn(in[i]);
-        out[i] = r;
-        in[i] = __bfloat162float(r);
+// rows of K floats -> rows of Ks floats (a multiple of 8), zero-padded
+__global__ void k_pad_rows(const float *__restrict__ in, float *__restrict__ out, int64_t rows, int32_t K, int32_t Ks) {
+    const int32_t quads = Ks / 4;
+    const int64_t n = rows * quads;
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int64_t r = i / quads;
+        const int32_t k = 4 * static_cast<int32_t>(i - r * quads);
+        const float *src = in + r * K + k;
+        float4 v;
+        v.x = k < K ? src[0] : 0.f;
+        v.y = k + 1 < K ? src[1] : 0.f;
+        v.z = k + 2 < K ? src[2] : 0.f;
+        v.w = k + 3 < K ? src[3] : 0.f;
+        reinterpret_cast<float4 *>(out)[i] = v;
+    }
+}
+
+// bf16 storage: out = bf16(in) in rows of Ks >= K elements (zero-padded; K, Ks multiples of 4), and `in` keeps the rounded
+// value (as fp32) for the tensor-core path
+__global__ void k_f32_to_bf16(float *__restrict__ in, __nv_bfloat16 *__restrict__ out, int64_t rows, int32_t K, int32_t Ks) {
+    const int32_t quads = Ks / 4;
+    const int64_t n = rows * quads;
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int64_t r = i / quads;
+        const int32_t k = 4 * static_cast<int32_t>(i - r * quads);
+        uint2 packed = make_uint2(0u, 0u);
+        if (k < K) {
+            float4 *src = reinterpret_cast<float4 *>(in + r * K + k);
+            const float4 v = *src;
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+            packed = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+            *src = make_float4(__low2float(lo), __high2float(lo), __low2float(hi), __high2float(hi));
+        }
+        reinterpret_cast<uint2 *>(out)[i] = packed;
     }
 }
 

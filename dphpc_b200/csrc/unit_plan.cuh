@@ -1,0 +1,280 @@
+// Building the unit lists of the row-segment kernels (once per upload, all on the device).
+//
+// A list is made from ENTRIES, each a run of consecutive nonzeros of one row (a whole row; the part of a row inside a
+// column panel; the leader of a row group; nothing).  Two kernels: the first sums the units of every tile of entries, the
+// second scans inside its tile, adds the sums of the tiles before it, and writes headers and column indices with one
+// thread per slot -- balanced whatever the run lengths, and nothing but the list itself goes to memory.
+#pragma once
+
+#include "device_utils.cuh"
+#include "kernel_rowseg.cuh"
+#include "plan_kernels.cuh"
+
+namespace sddmm {
+
+// ---- entries -> runs.  (A row_ptr that has not been validated yet may be anything: runs outside [0, nnz) are empty.) ----
+struct RunsOfRows {   // one entry per row: the whole row
+    static constexpr bool kSorted = false;   // needs sorted columns
+    const int32_t *rp;
+    const int32_t *col;
+    int32_t M, nnz;
+    __device__ __forceinline__ int32_t row(int64_t q) const { return static_cast<int32_t>(q); }
+    __device__ __forceinline__ void run(int64_t q, int32_t &s, int32_t &e) const {
+        s = rp[q];
+        e = rp[q + 1];
+        if (s < 0 || e < s || e > nnz) s = e = 0;
+    }
+};
+// One entry per (panel, row), panel-major.  Needs non-decreasing column indices inside a row.
+// long_rows > 0: only rows of at least that many nonzeros are cut into column panels (panels 0 .. panels-2, panel_cols
+// columns each); the shorter rows follow whole, as the last "panel" of the list -- a run of one or two nonzeros would
+// leave most of a segment's slots empty.
+struct RunsOfPanels {
+    static constexpr bool kSorted = true;
+    const int32_t *rp;
+    const int32_t *col;
+    int32_t M, nnz, panels, panel_cols, long_rows;
+    __device__ __forceinline__ int32_t row(int64_t q) const { return static_cast<int32_t>(q % M); }
+    __device__ __forceinline__ void run(int64_t q, int32_t &s, int32_t &e) const {
+        const int32_t p = static_cast<int32_t>(q / M), i = static_cast<int32_t>(q - static_cast<int64_t>(p) * M);
+        const int32_t a = rp[i], b = rp[i + 1];
+        s = e = 0;
+        if (a < 0 || b < a || b > nnz) return;
+        int32_t cut = panels;
+        if (long_rows > 0) {
+            const bool is_long = b - a >= long_rows;
+            if (p == panels - 1) {           // the short rows, whole
+                s = a;
+                e = is_long ? a : b;
+                return;
+            }
+            if (!is_long) return;
+            cut = panels - 1;                // the real column panels
+        }
+        s = p == 0 ? a : lower_col(col, a, b, static_cast<int64_t>(p) * panel_cols);
+        e = p == cut - 1 ? b : lower_col(col, a, b, static_cast<int64_t>(p + 1) * panel_cols);
+        if (e < s) e = s;                    // (unsorted columns: the list will not be built)
+    }
+};
+// rows of group g when groups of G rows start at row `first` (group 0 = the rows before it)
+__device__ __forceinline__ void unit_group_rows(int32_t g, int32_t G, int32_t first, int32_t M, int32_t &r0, int32_t &r1) {
+    r0 = g == 0 ? 0 : first + (g - 1) * G;
+    r1 = g == 0 ? first : min(r0 + G, M);
+}
+struct RunsOfGroups {   // one entry per row: the leader of a matching group speaks for its whole group
+    static constexpr bool kSorted = false;
+    const int32_t *rp;
+    const int32_t *col;
+    int32_t M, nnz, G, first;
+    const uint8_t *group_ok;
+    __device__ __forceinline__ int32_t row(int64_t q) const { return static_cast<int32_t>(q); }
+    __device__ __forceinline__ bool matched(int32_t r, int32_t &leader) const {
+        const int32_t g = r < first ? 0 : 1 + (r - first) / G;
+        int32_t end;
+        unit_group_rows(g, G, first, M, leader, end);
+        return group_ok[g] != 0;
+    }
+    __device__ __forceinline__ void run(int64_t q, int32_t &s, int32_t &e) const {
+        const int32_t r = static_cast<int32_t>(q);
+        int32_t leader;
+        s = rp[r];
+        e = matched(r, leader) && r != leader ? s : rp[r + 1];
+    }
+};
+
+// pass 1: units of every tile; the grand total goes to pc->units
+template <typename Runs>
+__global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs runs, int64_t n, int32_t *__restrict__ tile_sums, PlanCounters *__restrict__ pc) {
+    const int64_t base = static_cast<int64_t>(blockIdx.x) * kUnitTile;
+    int32_t local = 0;
+#pragma unroll
+    for (int k = 0; k < kUnitPerThread; ++k) {
+        const int64_t q = base + k * kUnitBlock + threadIdx.x;
+        if (q < n) {
+            int32_t s, e;
+            runs.run(q, s, e);
+            local += (e - s + 7) >> 3;
+        }
+    }
+    const int32_t total = block_sum(local);
+    if (threadIdx.x == 0) {
+        tile_sums[blockIdx.x] = total;
+        if (total) atomicAdd(&pc->units, static_cast<unsigned long long>(total));
+    }
+}
+
+// pass 2: the units of a tile.  HDR = int2 (plain units) or int4 (row groups).
+template <typename Runs, typename HDR>
+__global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n, const int32_t *__restrict__ tile_sums, int64_t cap,
+                                                           const PlanCounters *__restrict__ pc, HDR *__restrict__ units,
+                                                           int32_t *__restrict__ unit_cols) {
+    // enqueued before the host has seen the counters: nothing is written for a pattern that it is about to refuse
+    if (pc->bad_row_ptr || pc->bad_coo || (Runs::kSorted && pc->unsorted_cols)) return;
+    __shared__ int32_t first_unit[kUnitTile + 1];   // of the tile's entries, relative to the tile
+    __shared__ int32_t start[kUnitTile], length[kUnitTile];
+    int64_t before = 0;
+    {
+        int32_t part = 0;
+        for (int i = threadIdx.x; i < static_cast<int>(blockIdx.x); i += kUnitBlock) part += tile_sums[i];
+        before = block_sum(part);
+    }
+    const int64_t base = static_cast<int64_t>(blockIdx.x) * kUnitTile;
+    int32_t cnt[kUnitPerThread], local = 0;
+#pragma unroll
+    for (int k = 0; k < kUnitPerThread; ++k) {
+        const int i = threadIdx.x * kUnitPerThread + k;
+        int32_t s = 0, e = 0;
+        if (base + i < n) runs.run(base + i, s, e);
+        start[i] = s;
+        length[i] = e - s;
+        cnt[k] = (e - s + 7) >> 3;
+        local += cnt[k];
+    }
+    int32_t total;
+    int32_t at = block_inclusive_scan(local, &total) - local;
+#pragma unroll
+    for (int k = 0; k < kUnitPerThread; ++k) {
+        first_unit[threadIdx.x * kUnitPerThread + k] = at;
+        at += cnt[k];
+    }
+    if (threadIdx.x == kUnitBlock - 1) first_unit[kUnitTile] = at;
+    __syncthreads();
+    if (before + total > cap) return;
+    const int slot = threadIdx.x & 7;
+    for (int32_t u = threadIdx.x >> 3; u < total; u += kUnitBlock / 8) {
+        int lo = 0, hi = kUnitTile;      // the entry that holds unit u: the last one that starts at or before it
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (first_unit[mid] <= u) lo = mid; else hi = mid;
+        }
+        const int32_t skip = 8 * (u - first_unit[lo]);
+        const int32_t first = start[lo] + skip, count = min(8, length[lo] - skip);
+        unit_cols[8 * (before + u) + slot] = runs.col[first + min(slot, count - 1)];
+        if (slot == 0) {
+            const int32_t row = runs.row(base + lo);
+            HDR h;
+            h.x = first;
+            h.y = row * 8 + (count - 1);
+            if constexpr (sizeof(HDR) == sizeof(int4)) {
+                int32_t leader;
+                h.z = length[lo];
+                h.w = runs.matched(row, leader) ? runs.G : 1;
+            }
+            units[before + u] = h;
+        }
+    }
+}
+
+// copies of the last unit up to a multiple of 8 (the bf16 kernel reads a step's 8 units as one block)
+__global__ void k_unit_pad(int2 *__restrict__ units, int32_t *__restrict__ unit_cols, const PlanCounters *__restrict__ pc, int64_t cap) {
+    const int64_t n = static_cast<int64_t>(pc->units);
+    if (n == 0 || n > cap) return;
+    const int64_t u = n + (threadIdx.x >> 3);
+    if (u >= ((n + 7) & ~int64_t(7))) return;
+    unit_cols[8 * u + (threadIdx.x & 7)] = unit_cols[8 * (n - 1) + (threadIdx.x & 7)];
+    if ((threadIdx.x & 7) == 0) units[u] = units[n - 1];
+}
+
+// per-unit copies of the S values (column panels), one thread per slot: refreshed whenever S.val changes
+__global__ void k_unit_values(const int2 *__restrict__ units, int32_t n_units, const float *__restrict__ s_val, float *__restrict__ usval) {
+    for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < 8 * static_cast<int64_t>(n_units);
+         t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int2 u = units[t >> 3];
+        usval[t] = s_val[u.x + min(static_cast<int>(t & 7), u.y & 7)];
+    }
+}
+
+// ---- units over what the dense tiles left: runs of nonzeros whose bit in `covered` is clear -----------------------
+// first position in [j, b) whose bit equals `want`, or b
+__device__ __forceinline__ int32_t next_bit(const uint32_t *__restrict__ bits, int32_t j, int32_t b, bool want) {
+    while (j < b) {
+        uint32_t word = bits[j >> 5];
+        if (!want) word = ~word;
+        word >>= (j & 31);
+        if (word) return min(b, j + __ffs(word) - 1);
+        j = (j | 31) + 1;
+    }
+    return b;
+}
+// one thread per row: units of its uncovered runs
+__global__ void k_residual_unit_count(const int32_t *__restrict__ rp, int32_t M, const uint32_t *__restrict__ covered, int32_t *__restrict__ counts) {
+    for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < M; r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int32_t b = rp[r + 1];
+        int32_t n = 0;
+        for (int32_t j = next_bit(covered, rp[r], b, false); j < b;) {
+            const int32_t e = next_bit(covered, j, b, true);
+            n += (e - j + 7) >> 3;
+            j = next_bit(covered, e, b, false);
+        }
+        counts[r] = n;
+    }
+}
+__global__ void k_residual_unit_fill(const int32_t *__restrict__ rp, int32_t M, const uint32_t *__restrict__ covered,
+                                     const int32_t *__restrict__ offsets, const int32_t *__restrict__ col, int2 *__restrict__ units,
+                                     int32_t *__restrict__ unit_cols) {
+    for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < M; r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+        const int32_t b = rp[r + 1];
+        int32_t off = offsets[r];
+        for (int32_t j = next_bit(covered, rp[r], b, false); j < b;) {
+            const int32_t e = next_bit(covered, j, b, true);
+            for (int32_t first = j; first < e; first += 8, ++off) {
+                const int32_t count = min(8, e - first);
+                units[off] = make_int2(first, static_cast<int32_t>(r) * 8 + (count - 1));
+#pragma unroll
+                for (int i = 0; i < 8; ++i) unit_cols[8 * static_cast<int64_t>(off) + i] = col[first + min(i, count - 1)];
+            }
+            j = next_bit(covered, e, b, false);
+        }
+    }
+}
+
+// ---- exclusive scan of int32 counts (three small kernels) -----------------------------------
+constexpr int kScanBlock = 256;
+constexpr int kScanPerThread = 8;
+constexpr int kScanTile = kScanBlock * kScanPerThread;
+
+// pass 1: sum of every tile of kScanTile values
+__global__ void __launch_bounds__(kScanBlock) k_scan_tile_sums(const int32_t *__restrict__ v, int64_t n, int32_t *__restrict__ tile_sums) {
+    const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile + static_cast<int64_t>(threadIdx.x) * kScanPerThread;
+    int32_t local = 0;
+#pragma unroll
+    for (int k = 0; k < kScanPerThread; ++k)
+        if (base + k < n) local += v[base + k];
+    int32_t total;
+    block_inclusive_scan(local, &total);
+    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
+}
+// pass 2 (one block): exclusive scan of the tile sums in place; *grand_total = sum of everything
+__global__ void __launch_bounds__(kScanBlock) k_scan_sums(int32_t *__restrict__ tile_sums, int32_t n_tiles, unsigned long long *__restrict__ grand_total) {
+    int64_t carry = 0;
+    for (int32_t base = 0; base < n_tiles; base += kScanBlock) {
+        const int32_t idx = base + static_cast<int32_t>(threadIdx.x);
+        const int32_t v = idx < n_tiles ? tile_sums[idx] : 0;
+        int32_t total;
+        const int32_t inc = block_inclusive_scan(v, &total);
+        if (idx < n_tiles) tile_sums[idx] = static_cast<int32_t>(carry) + inc - v;
+        carry += total;
+    }
+    if (threadIdx.x == 0) *grand_total = static_cast<unsigned long long>(carry);
+}
+// pass 3: exclusive scan inside every tile plus the tile's offset, in place
+__global__ void __launch_bounds__(kScanBlock) k_scan_apply(int32_t *__restrict__ v, int64_t n, const int32_t *__restrict__ tile_offsets) {
+    const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile + static_cast<int64_t>(threadIdx.x) * kScanPerThread;
+    int32_t x[kScanPerThread];
+    int32_t local = 0;
+#pragma unroll
+    for (int k = 0; k < kScanPerThread; ++k) {
+        x[k] = (base + k < n) ? v[base + k] : 0;
+        local += x[k];
+    }
+    int32_t total;
+    const int32_t inc = block_inclusive_scan(local, &total);
+    int32_t run = tile_offsets[blockIdx.x] + inc - local;
+#pragma unroll
+    for (int k = 0; k < kScanPerThread; ++k) {
+        if (base + k < n) v[base + k] = run;
+        run += x[k];
+    }
+}
+
+}  // namespace sddmm
