@@ -180,6 +180,10 @@ struct sddmm_b200_engine {
     int2 *d_spmm_units = nullptr;
     int32_t *d_spmm_cols = nullptr;
     cudaEvent_t ev_spmm0 = nullptr, ev_spmm1 = nullptr;
+    // Y goes back to the host in up to kSpmmChunks row ranges, each as soon as its part of the kernel is done
+    static constexpr int kSpmmChunks = 8;
+    cudaEvent_t ev_chunk[kSpmmChunks] = {};
+    int32_t spmm_cut[kSpmmChunks + 1] = {};   // units before row M * c / kSpmmChunks
 
     // plan
     sddmm_b200_plan_info plan;
@@ -426,7 +430,7 @@ int carve_arena(sddmm_b200_engine *e, bool coo, int n_items, bool allow_padding)
     const size_t o_ucols = c.take(static_cast<size_t>(e->unit_cap + 8) * 32);
     const size_t o_uval = e->panels > 1 ? c.take(static_cast<size_t>(e->unit_cap + 8) * 32) : 0;
     const size_t o_uoff = c.take((M + 1) * 4);
-    const size_t o_stile = c.take((scan_n / kUnitTile + M / kScanTile + 2) * 4);
+    const size_t o_stile = c.take((static_cast<size_t>(std::max(unit_tiles(static_cast<int64_t>(scan_n)), unit_tiles(e->M))) + M / kScanTile + 2) * 4);
     // dense-tile path: only carved when the mode, K and the size of the 64x64 tile grid allow it
     e->tiles_per_row = static_cast<int32_t>((N + 63) / 64);
     e->tile_grid = static_cast<int64_t>((M + 63) / 64) * e->tiles_per_row;
@@ -779,7 +783,8 @@ bool group_possible(const sddmm_b200_engine *e) {
 }
 // candidates: G = 2, 3, 4 rows per group, first full group starting at row 0 .. G-1 (counters slot = G(G-1)/2 - 1 + first)
 int group_slot(int G, int first) { return G * (G - 1) / 2 - 1 + first; }
-int group_sample(const sddmm_b200_engine *e) { return e->M > 65536 ? 16 : 1; }   // large inputs: G and `first` are chosen on a 1-in-16 sample of the groups
+// G and `first` are chosen on a sample of the groups (about 8 000 rows' worth, at most 1 in 16 of them); the chosen grouping is then matched exactly
+int group_sample(const sddmm_b200_engine *e) { return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(16, e->M / 8192))); }
 int enqueue_group_sample(sddmm_b200_engine *e) {
     const int every = group_sample(e);
     const dim3 grid(grid_for((e->M / 2 / every + 2) * 32, kBlock, e->sm_count * 2), 9);
@@ -816,7 +821,7 @@ int build_rowgroup_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
         e->d_rp, e->d_col, M, nnz, best, best_first, 1, e->d_group_ok, &e->d_pc->group_cover[bs], &e->d_pc->group_count[bs]);
     if (units) {
         const RunsOfGroups runs{e->d_rp, e->d_col, M, nnz, best, best_first, e->d_group_ok};
-        const int tiles = static_cast<int>((e->M + kUnitTile - 1) / kUnitTile);
+        const int tiles = unit_tiles(e->M);
         CU_TRY(e, cudaMemsetAsync(&e->d_pc->units, 0, sizeof(unsigned long long), s));
         k_unit_sums<<<tiles, kUnitBlock, 0, s>>>(runs, e->M, e->d_scan_tiles, e->d_pc);
         k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, e->M, e->d_scan_tiles, e->unit_cap, e->d_pc, reinterpret_cast<int4 *>(e->d_units), e->d_unit_cols);
@@ -887,7 +892,7 @@ int enqueue_unit_list(sddmm_b200_engine *e, int32_t panels, bool have_sums) {
     const int32_t M = static_cast<int32_t>(e->M), nnz = static_cast<int32_t>(e->nnz);
     cudaStream_t s = e->stream;
     const int64_t n = static_cast<int64_t>(panels) * M;
-    const int tiles = static_cast<int>((n + kUnitTile - 1) / kUnitTile);
+    const int tiles = unit_tiles(n);
     if (!have_sums) CU_TRY(e, cudaMemsetAsync(&e->d_pc->units, 0, sizeof(unsigned long long), s));
     if (panels > 1) {
         const RunsOfPanels runs{e->d_rp, e->d_col, M, nnz, panels, e->panel_cols, e->long_rows};
@@ -959,7 +964,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     // tiles, or the row statistics, decide first) and the sample that looks for row groups.
     const bool whole_rows = e->use_seg && !e->dense_possible && e->panels == 1;
     const bool early_list = e->use_seg && !e->dense_possible && e->long_rows == 0 && e->nnz > 0;
-    k_row_stats<<<static_cast<int>((e->M + kUnitTile - 1) / kUnitTile), kUnitBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, e->d_rowstart,
+    k_row_stats<<<unit_tiles(e->M), kUnitBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, e->d_rowstart,
                                                                                             whole_rows ? e->d_scan_tiles : nullptr, e->d_pc);
     if (e->nnz > 0) {
         k_col_scan<<<grid_for(e->nnz, kBlock, cap), kBlock, 0, s>>>(e->d_col, e->nnz, static_cast<int32_t>(e->N), e->d_rowstart,
@@ -1346,6 +1351,7 @@ int sddmm_b200_create(sddmm_b200_engine **out, int device, int mode, uint32_t fl
         ok = ok && cudaEventCreate(&e->ev_begin[i]) == cudaSuccess && cudaEventCreate(&e->ev_end[i]) == cudaSuccess;
     ok = ok && cudaEventCreate(&e->ev_run0) == cudaSuccess && cudaEventCreate(&e->ev_run1) == cudaSuccess;
     ok = ok && cudaEventCreate(&e->ev_spmm0) == cudaSuccess && cudaEventCreate(&e->ev_spmm1) == cudaSuccess;
+    for (cudaEvent_t &ev : e->ev_chunk) ok = ok && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&e->ev_stage, cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming) == cudaSuccess;
@@ -1379,6 +1385,8 @@ int sddmm_b200_destroy(sddmm_b200_engine *e) {
         if (e->ev_stage) cudaEventDestroy(e->ev_stage);
         if (e->ev_spmm0) cudaEventDestroy(e->ev_spmm0);
         if (e->ev_spmm1) cudaEventDestroy(e->ev_spmm1);
+        for (cudaEvent_t ev : e->ev_chunk)
+            if (ev) cudaEventDestroy(ev);
         if (e->h_err) cudaFreeHost(e->h_err);
         if (e->h_pc) cudaFreeHost(e->h_pc);
         for (int i = 0; i < sddmm_b200_engine::kMaxKernels; ++i) {
@@ -1763,15 +1771,19 @@ int spmm_prepare(sddmm_b200_engine *e, int64_t K2) {
         const int32_t Mi = static_cast<int32_t>(e->M);
         cudaStream_t s = e->stream;
         const RunsOfRows runs{e->d_rp, e->d_col, Mi, static_cast<int32_t>(e->nnz)};
-        const int tiles = static_cast<int>((e->M + kUnitTile - 1) / kUnitTile);
+        const int tiles = unit_tiles(e->M);
         CU_TRY(e, cudaMemsetAsync(&e->d_pc->units, 0, sizeof(unsigned long long), s));
         k_unit_sums<<<tiles, kUnitBlock, 0, s>>>(runs, e->M, e->d_scan_tiles, e->d_pc);
         k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, e->M, e->d_scan_tiles, static_cast<int64_t>(cap), e->d_pc, e->d_spmm_units, e->d_spmm_cols);
+        k_unit_cuts<<<1, 32, 0, s>>>(e->d_spmm_units, Mi, sddmm_b200_engine::kSpmmChunks, e->d_pc);
         CU_TRY(e, cudaGetLastError());
         PlanCounters pc;
         if (int rc = read_counters(e, &pc)) return rc;
         if (pc.units == 0 || pc.units > cap) return fail(e, SDDMM_B200_ERR_CUDA, "consumer plan: %llu units for a list of %zu", pc.units, cap);
         e->spmm_units = static_cast<int32_t>(pc.units);
+        for (int c = 1; c < sddmm_b200_engine::kSpmmChunks; ++c) e->spmm_cut[c] = pc.unit_cut[c];
+        e->spmm_cut[0] = 0;
+        e->spmm_cut[sddmm_b200_engine::kSpmmChunks] = e->spmm_units;
     }
     return SDDMM_B200_OK;
 }
@@ -1796,20 +1808,37 @@ int sddmm_b200_spmm(sddmm_b200_engine *e, int64_t K2, const float *X, float *Y) 
     if (X) CU_TRY(e, cudaMemcpyAsync(e->d_X, X, static_cast<size_t>(e->N) * K2 * 4, cudaMemcpyHostToDevice, s));
     CU_TRY(e, cudaEventRecord(e->ev_spmm0, s));
     CU_TRY(e, cudaMemsetAsync(e->d_Y, 0, ybytes, s));
-    SpmmArgs a;
-    a.units = e->d_spmm_units; a.col_idx = e->d_col; a.p_val = e->d_pval; a.X = X ? e->d_X : e->d_B32; a.Y = e->d_Y;
-    a.n_units = e->spmm_units; a.K2 = static_cast<int32_t>(K2);
     const int cpl = round_up_cpl(K2);
     SpmmFn fn = pick_spmm(cpl, K2 == 32 * cpl);
     int occ = 0;
     CU_TRY(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kSpmmWarps * 32, 0));
     if (occ < 1) return fail(e, SDDMM_B200_ERR_CUDA, "consumer kernel does not fit on an SM");
-    const int64_t n_quads = (static_cast<int64_t>(e->spmm_units) + 3) / 4;
-    const int grid = static_cast<int>(std::min<int64_t>((n_quads + kSpmmWarps - 1) / kSpmmWarps, static_cast<int64_t>(e->sm_count) * occ));
-    fn<<<grid, kSpmmWarps * 32, 0, s>>>(a);
-    CU_TRY(e, cudaGetLastError());
+    // Row ranges of about 4 MB of Y: while a range crosses the link the next one is computed (the copy of all of Y after the
+    // whole kernel: 100 003 rows, K2 = 64, 103 us of kernel before 465 us of copy).
+    constexpr int kMost = sddmm_b200_engine::kSpmmChunks;
+    const int chunks = ybytes >= (size_t(32) << 20) ? 8 : ybytes >= (size_t(16) << 20) ? 4 : ybytes >= (size_t(8) << 20) ? 2 : 1;
+    int64_t row[kMost + 1];
+    for (int c = 0; c <= chunks; ++c) row[c] = e->M * (c * (kMost / chunks)) / kMost;
+    for (int c = 0; c < chunks; ++c) {
+        const int32_t u0 = e->spmm_cut[c * (kMost / chunks)], u1 = e->spmm_cut[(c + 1) * (kMost / chunks)];
+        if (u1 > u0) {
+            SpmmArgs a;
+            a.units = e->d_spmm_units + u0; a.col_idx = e->d_col; a.p_val = e->d_pval; a.X = X ? e->d_X : e->d_B32; a.Y = e->d_Y;
+            a.n_units = u1 - u0; a.K2 = static_cast<int32_t>(K2);
+            const int64_t n_quads = (static_cast<int64_t>(a.n_units) + 3) / 4;
+            const int grid = static_cast<int>(std::min<int64_t>((n_quads + kSpmmWarps - 1) / kSpmmWarps, static_cast<int64_t>(e->sm_count) * occ));
+            fn<<<grid, kSpmmWarps * 32, 0, s>>>(a);
+            CU_TRY(e, cudaGetLastError());
+        }
+        CU_TRY(e, cudaEventRecord(e->ev_chunk[c], s));
+    }
     CU_TRY(e, cudaEventRecord(e->ev_spmm1, s));
-    CU_TRY(e, cudaMemcpyAsync(Y, e->d_Y, ybytes, cudaMemcpyDeviceToHost, s));
+    for (int c = 0; c < chunks; ++c) {
+        CU_TRY(e, cudaStreamWaitEvent(e->side_stream, e->ev_chunk[c], 0));
+        const size_t at = static_cast<size_t>(row[c]) * K2, n = static_cast<size_t>(row[c + 1] - row[c]) * K2;
+        if (n) CU_TRY(e, e->stager2.download(Y + at, e->d_Y + at, n * 4, e->side_stream));
+    }
+    CU_TRY(e, cudaStreamSynchronize(e->side_stream));
     return sddmm_b200_sync(e);
 }
 

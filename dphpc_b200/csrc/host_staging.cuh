@@ -2,7 +2,7 @@
 //
 // The driver stages such a copy through its own pinned buffer on one thread, which on this class of host moves about
 // 10 GB/s -- a fifth of what the link carries from pinned memory.  Here the staging is done by a small pool of host
-// threads: a copy is cut into 8 MiB pieces, the pool memcpy()s piece c+1 into one of two pinned ring buffers while the DMA
+// threads: a copy is cut into 4 MiB pieces, the pool memcpy()s piece c+1 into one of three pinned ring buffers while the DMA
 // engine moves piece c, and the other way round for downloads.  Pinned or registered host memory and device memory take
 // the direct cudaMemcpyAsync path.  Like a pageable cudaMemcpyAsync, a staged call returns when the caller's buffer is
 // free again (uploads) or filled (downloads).
@@ -15,6 +15,7 @@
 #include <emmintrin.h>
 #endif
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <cstdlib>
 #include <cstdint>
@@ -26,7 +27,9 @@
 
 namespace sddmm {
 
-// a fixed pool of host threads that runs "slice k of n" jobs; the caller takes part
+// A fixed pool of host threads that runs "slice k of n" jobs; the caller takes part.  A staged copy hands over a piece every
+// hundred microseconds, so the threads look for the next job for a while before they go to sleep, and a slice is taken
+// with one compare-and-swap on {job, slices, next slice}.
 class HostPool {
 public:
     static HostPool &instance() {
@@ -36,26 +39,25 @@ public:
     int width() const { return static_cast<int>(workers_.size()) + 1; }
     // fn(k) for k in [0, n), spread over the pool; returns when all are done
     void run(int n, const std::function<void(int)> &fn) {
-        if (n <= 1 || workers_.empty()) {
+        if (n <= 1 || n > kMaxSlices || workers_.empty()) {
             for (int k = 0; k < n; ++k) fn(k);
             return;
         }
         std::lock_guard<std::mutex> one_at_a_time(run_mu_);   // callers on different host threads (one per device) take turns
-        std::unique_lock<std::mutex> lock(mu_);
-        job_ = &fn;
-        next_ = 0;
-        total_ = n;
-        pending_ = n;
-        ++generation_;
-        cv_.notify_all();
-        lock.unlock();
-        work();   // the caller helps
-        lock.lock();
-        done_.wait(lock, [&] { return pending_ == 0; });
-        job_ = nullptr;
+        job_ = &fn;                                           // (nobody holds a slice of the previous job any more: pending_ was 0)
+        pending_.store(n, std::memory_order_relaxed);
+        const uint64_t job = (ticket_.load(std::memory_order_relaxed) >> 32) + 1;
+        ticket_.store(job << 32 | static_cast<uint64_t>(n) << 16, std::memory_order_seq_cst);
+        if (sleepers_.load(std::memory_order_seq_cst) > 0) {
+            std::lock_guard<std::mutex> lock(mu_);
+            cv_.notify_all();
+        }
+        while (take()) {}   // the caller helps
+        while (pending_.load(std::memory_order_acquire) != 0) relax();
     }
 
 private:
+    static constexpr int kMaxSlices = 0xFFFF;
     HostPool() {
         unsigned hw = std::thread::hardware_concurrency();
         unsigned want = std::min(hw ? hw / 2 : 2u, 8u);
@@ -69,46 +71,54 @@ private:
     ~HostPool() {
         {
             std::lock_guard<std::mutex> lock(mu_);
-            stop_ = true;
-            ++generation_;
+            stop_.store(true);
         }
         cv_.notify_all();
         for (std::thread &t : workers_) t.join();
     }
-    void work() {
-        while (true) {
-            int k;
-            const std::function<void(int)> *fn;
-            {
-                std::lock_guard<std::mutex> lock(mu_);
-                if (!job_ || next_ >= total_) return;
-                k = next_++;
-                fn = job_;
-            }
-            (*fn)(k);
-            std::lock_guard<std::mutex> lock(mu_);
-            if (--pending_ == 0) done_.notify_all();
-        }
+    static void relax() {
+#if defined(__SSE2__)
+        _mm_pause();
+#else
+        std::this_thread::yield();
+#endif
+    }
+    static bool open(uint64_t t) { return (t & 0xFFFF) < ((t >> 16) & 0xFFFF); }
+    // run one slice of the current job, if one is left
+    bool take() {
+        uint64_t t = ticket_.load(std::memory_order_acquire);
+        do {
+            if (!open(t)) return false;
+        } while (!ticket_.compare_exchange_weak(t, t + 1, std::memory_order_acq_rel, std::memory_order_acquire));
+        (*job_)(static_cast<int>(t & 0xFFFF));   // (the job cannot end before this slice has been counted off)
+        pending_.fetch_sub(1, std::memory_order_acq_rel);
+        return true;
     }
     void loop() {
-        unsigned long long seen = 0;
-        while (true) {
-            {
-                std::unique_lock<std::mutex> lock(mu_);
-                cv_.wait(lock, [&] { return generation_ != seen; });
-                seen = generation_;
-                if (stop_) return;
+        while (!stop_.load(std::memory_order_relaxed)) {
+            while (take()) {}
+            const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(200);
+            bool found = false;
+            while (!found && std::chrono::steady_clock::now() < until) {
+                for (int i = 0; i < 64 && !found; ++i) {
+                    relax();
+                    found = open(ticket_.load(std::memory_order_acquire));
+                }
             }
-            work();
+            if (found) continue;
+            std::unique_lock<std::mutex> lock(mu_);
+            sleepers_.fetch_add(1, std::memory_order_seq_cst);
+            cv_.wait(lock, [&] { return stop_.load() || open(ticket_.load(std::memory_order_seq_cst)); });
+            sleepers_.fetch_sub(1, std::memory_order_seq_cst);
         }
     }
     std::vector<std::thread> workers_;
     std::mutex mu_, run_mu_;
-    std::condition_variable cv_, done_;
+    std::condition_variable cv_;
     const std::function<void(int)> *job_ = nullptr;
-    int next_ = 0, total_ = 0, pending_ = 0;
-    unsigned long long generation_ = 0;
-    bool stop_ = false;
+    std::atomic<uint64_t> ticket_{0};   // job << 32 | slices << 16 | next slice
+    std::atomic<int> pending_{0}, sleepers_{0};
+    std::atomic<bool> stop_{false};
 };
 
 // memcpy whose stores bypass the cache (x86): the destination is a pinned staging buffer that the DMA engine reads next,
@@ -142,7 +152,7 @@ inline void stream_copy(void *dst, const void *src, size_t bytes) {
 
 inline void parallel_memcpy(void *dst, const void *src, size_t bytes, bool stream_stores = false) {
     HostPool &pool = HostPool::instance();
-    const int parts = static_cast<int>(std::min<size_t>(pool.width(), std::max<size_t>(1, bytes >> 20)));   // >= 1 MiB per slice
+    const int parts = static_cast<int>(std::min<size_t>(pool.width(), std::max<size_t>(1, bytes >> 17)));   // >= 128 KiB per slice
     if (parts <= 1) {
         if (stream_stores) stream_copy(dst, src, bytes); else std::memcpy(dst, src, bytes);
         return;
@@ -157,27 +167,27 @@ inline void parallel_memcpy(void *dst, const void *src, size_t bytes, bool strea
     });
 }
 
-// two pinned buffers of one engine, used alternately
+// a ring of pinned buffers of one engine
 struct HostStager {
-    // bytes per piece (= size of each pinned buffer); SDDMM_B200_STAGE_MB overrides the 8 MiB default (1 .. 256).
-    // Measured on a 16-core host with 8 pool threads, 678 MB up: 8 MiB 19-21 ms, 16 MiB 22-23 ms, 32 MiB 23-25 ms,
-    // 4 MiB and 2 MiB 43-75 ms (the per-piece hand-over dominates); 12 or 16 threads are no faster and at times far slower.
+    // bytes per piece (= size of each pinned buffer); SDDMM_B200_STAGE_MB overrides the 4 MiB default (1 .. 256).
     const size_t kPiece = [] {
-        size_t mb = 8;
+        size_t mb = 4;
         if (const char *env = std::getenv("SDDMM_B200_STAGE_MB")) {
             const int v = std::atoi(env);
             if (v >= 1 && v <= 256) mb = static_cast<size_t>(v);
         }
         return mb << 20;
     }();
-    static constexpr size_t kMinStaged = size_t(4) << 20;   // smaller copies are left to the driver
-    char *buf[2] = {nullptr, nullptr};
-    cudaEvent_t ev[2] = {nullptr, nullptr};
-    bool busy[2] = {false, false};
+    static constexpr size_t kMinStaged = size_t(512) << 10;   // smaller copies are left to the driver
+    static constexpr int kRing = 3;
+    char *buf[kRing] = {};
+    cudaEvent_t ev[kRing] = {};
+    bool busy[kRing] = {};
+    int next = 0;   // buffer the next piece takes
 
     bool ready() {
         if (buf[0]) return true;
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < kRing; ++i) {
             if (cudaHostAlloc(reinterpret_cast<void **>(&buf[i]), kPiece, cudaHostAllocDefault) != cudaSuccess ||
                 cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming) != cudaSuccess) {
                 cudaGetLastError();
@@ -188,7 +198,7 @@ struct HostStager {
         return true;
     }
     void release() {
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < kRing; ++i) {
             if (ev[i]) cudaEventDestroy(ev[i]);
             if (buf[i]) cudaFreeHost(buf[i]);
             ev[i] = nullptr;
@@ -208,9 +218,10 @@ struct HostStager {
     // host -> device on `stream`; the caller's buffer is free when this returns if it was staged
     cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t stream) {
         if (bytes < kMinStaged || !pageable(src) || !ready()) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream);
-        int b = 0;
-        for (size_t off = 0; off < bytes; off += kPiece, b ^= 1) {
+        for (size_t off = 0; off < bytes; off += kPiece) {
             const size_t len = std::min(kPiece, bytes - off);
+            const int b = next;
+            next = (next + 1) % kRing;
             if (busy[b]) {
                 const cudaError_t st = cudaEventSynchronize(ev[b]);
                 if (st != cudaSuccess) return st;
@@ -226,7 +237,7 @@ struct HostStager {
     // device -> host on `stream`; returns when the caller's buffer is filled (the stream has drained up to the copy)
     cudaError_t download(void *dst, const void *src, size_t bytes, cudaStream_t stream) {
         if (bytes < kMinStaged || !pageable(dst) || !ready()) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream);
-        for (int b = 0; b < 2; ++b)
+        for (int b = 0; b < kRing; ++b)
             if (busy[b]) {
                 const cudaError_t st = cudaEventSynchronize(ev[b]);
                 if (st != cudaSuccess) return st;
@@ -235,18 +246,18 @@ struct HostStager {
         const size_t pieces = (bytes + kPiece - 1) / kPiece;
         auto enqueue = [&](size_t c) -> cudaError_t {
             const size_t off = c * kPiece, len = std::min(kPiece, bytes - off);
-            cudaError_t st = cudaMemcpyAsync(buf[c & 1], static_cast<const char *>(src) + off, len, cudaMemcpyDeviceToHost, stream);
-            if (st == cudaSuccess) st = cudaEventRecord(ev[c & 1], stream);
+            cudaError_t st = cudaMemcpyAsync(buf[c % kRing], static_cast<const char *>(src) + off, len, cudaMemcpyDeviceToHost, stream);
+            if (st == cudaSuccess) st = cudaEventRecord(ev[c % kRing], stream);
             return st;
         };
-        cudaError_t st = enqueue(0);
+        cudaError_t st = cudaSuccess;
+        for (size_t c = 0; c < kRing - 1 && c < pieces && st == cudaSuccess; ++c) st = enqueue(c);
         for (size_t c = 0; c < pieces && st == cudaSuccess; ++c) {
-            st = cudaEventSynchronize(ev[c & 1]);          // piece c has landed in its pinned buffer
+            st = cudaEventSynchronize(ev[c % kRing]);                           // piece c has landed in its pinned buffer
             if (st != cudaSuccess) break;
-            if (c + 1 < pieces) st = enqueue(c + 1);       // the next piece crosses the link while this one is copied out
+            if (c + kRing - 1 < pieces) st = enqueue(c + kRing - 1);            // later pieces cross the link while this one is copied out
             const size_t off = c * kPiece, len = std::min(kPiece, bytes - off);
-            parallel_memcpy(static_cast<char *>(dst) + off, buf[c & 1], len);
-            if (st != cudaSuccess) break;
+            parallel_memcpy(static_cast<char *>(dst) + off, buf[c % kRing], len);
         }
         return st;
     }

@@ -30,6 +30,7 @@ struct PlanCounters {
     int rowgroups;
     int group_count[9];                  // matching row groups, same slots
     int residual_items;
+    int unit_cut[8];                     // consumer: units before each of 8 equal row ranges
     unsigned long long units;            // row segments of the row-segment path
     unsigned long long window_nnz;       // nonzeros inside the selected 64x64 windows (summed per window)
     int n_anchors;                       // candidate origins of the arbitrary-offset tile detection
@@ -43,8 +44,11 @@ __device__ __forceinline__ int len_bin(int len) {
 
 // unit lists (unit_plan.cuh) are scanned in tiles of this many entries
 constexpr int kUnitBlock = kPlanBlock;
-constexpr int kUnitTile = 1024;                          // entries per tile (4 per thread)
-constexpr int kUnitPerThread = kUnitTile / kUnitBlock;
+constexpr int kUnitTileMax = 1024;
+// Entries per tile: small tiles for short lists, so that every SM has several blocks to build (200 000 rows: 113 us in 196
+// blocks of 1024 entries), larger ones for long lists, because a block adds up the sums of all tiles before its own.
+__host__ __device__ __forceinline__ int unit_tile(int64_t n) { return n > (1 << 20) ? kUnitTileMax : n > (1 << 18) ? 256 : 128; }
+inline int unit_tiles(int64_t n) { return static_cast<int>((n + unit_tile(n) - 1) / unit_tile(n)); }
 
 // One tile of rows per block: monotonicity, histogram, max, nonempty count, row-start bits, and (tile_sums != nullptr) the
 // units of the tile when every row is one run -- pass 1 of the plain unit list.
@@ -52,32 +56,38 @@ __global__ void __launch_bounds__(kUnitBlock) k_row_stats(const int32_t *__restr
                                                           int32_t *__restrict__ tile_sums, PlanCounters *__restrict__ pc) {
     __shared__ unsigned int sh[SDDMM_B200_HIST_BINS];
     __shared__ unsigned long long sh_nnz[SDDMM_B200_HIST_BINS];
-    __shared__ unsigned int s_nonempty;
     __shared__ int s_max;
     if (threadIdx.x < SDDMM_B200_HIST_BINS) { sh[threadIdx.x] = 0; sh_nnz[threadIdx.x] = 0; }
-    if (threadIdx.x == 0) { s_nonempty = 0; s_max = 0; }
+    if (threadIdx.x == 0) s_max = 0;
     __syncthreads();
     int32_t units = 0;
-#pragma unroll
-    for (int k = 0; k < kUnitPerThread; ++k) {
-        const int64_t i = blockIdx.x * static_cast<int64_t>(kUnitTile) + k * kUnitBlock + threadIdx.x;
-        if (i >= M) break;
-        const int a = rp[i], b = rp[i + 1];
-        const int len = b - a;
-        if (len < 0 || a < 0 || b > nnz) {
-            pc->bad_row_ptr = 1;
-        } else {
-            atomicAdd(&sh[len_bin(len)], 1u);
-            units += (len + 7) >> 3;
-            if (len > 0) {
-                atomicAdd(&sh_nnz[len_bin(len)], static_cast<unsigned long long>(len));
-                atomicAdd(&s_nonempty, 1u);
-                atomicMax(&s_max, len);
-                atomicOr(&row_start_bits[a >> 5], 1u << (a & 31));
+    const int tile = unit_tile(M);
+    for (int k = threadIdx.x; k < (tile + 31) / 32 * 32; k += kUnitBlock) {   // (whole warps)
+        const int64_t i = blockIdx.x * static_cast<int64_t>(tile) + k;
+        int len = -1;                                // no row, or one that is refused
+        if (i < M && k < tile) {
+            const int a = rp[i], b = rp[i + 1];
+            if (b < a || a < 0 || b > nnz || (i == 0 && a != 0) || (i == M - 1 && b != nnz)) {
+                pc->bad_row_ptr = 1;
+            } else {
+                len = b - a;
+                units += (len + 7) >> 3;
+                if (len > 0) atomicOr(&row_start_bits[a >> 5], 1u << (a & 31));
             }
         }
-        if (i == 0 && a != 0) pc->bad_row_ptr = 1;
-        if (i == M - 1 && b != nnz) pc->bad_row_ptr = 1;
+        // the rows of a warp share few length bins: one shared-memory update per bin and warp
+        const unsigned live = __ballot_sync(kFullMask, len >= 0);
+        if (len >= 0) {
+            const int bin = len_bin(len);
+            const unsigned same = __match_any_sync(live, bin);
+            const unsigned lo = __reduce_add_sync(same, static_cast<unsigned>(len) & 0xffffu), hi = __reduce_add_sync(same, static_cast<unsigned>(len) >> 16);
+            const int longest = __reduce_max_sync(same, len);
+            if ((threadIdx.x & 31) == __ffs(same) - 1) {
+                atomicAdd(&sh[bin], __popc(same));
+                atomicAdd(&sh_nnz[bin], (static_cast<unsigned long long>(hi) << 16) + lo);
+                atomicMax(&s_max, longest);
+            }
+        }
     }
     const int32_t total = block_sum(units);   // (a block-wide barrier)
     if (threadIdx.x == 0 && tile_sums) {
@@ -89,31 +99,51 @@ __global__ void __launch_bounds__(kUnitBlock) k_row_stats(const int32_t *__restr
         if (sh_nnz[threadIdx.x]) atomicAdd(&pc->hist_nnz[threadIdx.x], sh_nnz[threadIdx.x]);
     }
     if (threadIdx.x == 0) {
-        if (s_nonempty) atomicAdd(&pc->rows_nonempty, (unsigned long long)s_nonempty);
+        unsigned int nonempty = 0;
+        for (int k = 1; k < SDDMM_B200_HIST_BINS; ++k) nonempty += sh[k];
+        if (nonempty) atomicAdd(&pc->rows_nonempty, static_cast<unsigned long long>(nonempty));
         if (s_max) atomicMax(&pc->max_row_nnz, s_max);
     }
 }
 
-// one thread per nonzero: column range, distinct columns (one bit each), in-row ordering
+// four nonzeros per thread: column range, distinct columns (one bit each), in-row ordering.  col is 16-byte aligned.
 __global__ void __launch_bounds__(kPlanBlock) k_col_scan(const int32_t *__restrict__ col, int64_t nnz, int32_t N, const uint32_t *__restrict__ row_start_bits,
-                           uint32_t *__restrict__ touched, PlanCounters *__restrict__ pc) {
+                                                         uint32_t *__restrict__ touched, PlanCounters *__restrict__ pc) {
     int32_t fresh = 0;
-    for (int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; j < nnz;
-         j += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int c = col[j];
-        if (c < 0 || c >= N) {
-            pc->bad_col = 1;
-            continue;
+    bool bad = false, unsorted = false, dup = false;
+    const int64_t stride = 4 * static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t j = 4 * (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x); j < nnz; j += stride) {
+        int c[5];
+        const int n = static_cast<int>(min(static_cast<int64_t>(4), nnz - j));
+        c[0] = j > 0 ? col[j - 1] : 0;
+        if (n == 4) {
+            const int4 q = *reinterpret_cast<const int4 *>(col + j);
+            c[1] = q.x; c[2] = q.y; c[3] = q.z; c[4] = q.w;
+        } else {
+            for (int k = 0; k < 4; ++k) c[k + 1] = col[j + min(k, n - 1)];
         }
-        const uint32_t bit = 1u << (c & 31);
-        if (!(touched[c >> 5] & bit) && !(atomicOr(&touched[c >> 5], bit) & bit)) ++fresh;   // (a stale read only costs an atomic)
-        const bool is_start = (row_start_bits[j >> 5] >> (j & 31)) & 1u;
-        if (!is_start && j > 0) {
-            const int prev = col[j - 1];
-            if (prev > c) pc->unsorted_cols = 1;
-            if (prev == c) pc->dup_cols = 1;
+        const uint32_t starts = row_start_bits[j >> 5] >> (j & 31);   // (j is a multiple of 4: the four bits lie in one word)
+        uint32_t word[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool in = c[k + 1] >= 0 && c[k + 1] < N;
+            bad |= !in;
+            // past L1: a block that keeps reading an old word would repeat the update for every nonzero of the column
+            word[k] = in ? __ldcg(&touched[c[k + 1] >> 5]) : ~0u;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t bit = 1u << (c[k + 1] & 31);
+            if (!(word[k] & bit) && !(atomicOr(&touched[c[k + 1] >> 5], bit) & bit)) ++fresh;
+            if (k < n && !((starts >> k) & 1u) && (j > 0 || k > 0)) {
+                unsorted |= c[k] > c[k + 1];
+                dup |= c[k] == c[k + 1];
+            }
         }
     }
+    if (bad) pc->bad_col = 1;
+    if (unsorted) pc->unsorted_cols = 1;
+    if (dup) pc->dup_cols = 1;
     const int32_t total = block_sum(fresh);
     if (threadIdx.x == 0 && total) atomicAdd(&pc->cols_touched, static_cast<unsigned long long>(total));
 }

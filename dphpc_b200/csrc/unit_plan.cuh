@@ -85,17 +85,15 @@ struct RunsOfGroups {   // one entry per row: the leader of a matching group spe
 // pass 1: units of every tile; the grand total goes to pc->units
 template <typename Runs>
 __global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs runs, int64_t n, int32_t *__restrict__ tile_sums, PlanCounters *__restrict__ pc) {
-    const int64_t base = static_cast<int64_t>(blockIdx.x) * kUnitTile;
+    const int tile = unit_tile(n);
+    const int64_t base = static_cast<int64_t>(blockIdx.x) * tile;
     int32_t local = 0;
-#pragma unroll
-    for (int k = 0; k < kUnitPerThread; ++k) {
-        const int64_t q = base + k * kUnitBlock + threadIdx.x;
-        if (q < n) {
+    for (int k = threadIdx.x; k < tile; k += kUnitBlock)
+        if (base + k < n) {
             int32_t s, e;
-            runs.run(q, s, e);
+            runs.run(base + k, s, e);
             local += (e - s + 7) >> 3;
         }
-    }
     const int32_t total = block_sum(local);
     if (threadIdx.x == 0) {
         tile_sums[blockIdx.x] = total;
@@ -110,19 +108,24 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n,
                                                            int32_t *__restrict__ unit_cols) {
     // enqueued before the host has seen the counters: nothing is written for a pattern that it is about to refuse
     if (pc->bad_row_ptr || pc->bad_coo || (Runs::kSorted && pc->unsorted_cols)) return;
-    __shared__ int32_t first_unit[kUnitTile + 1];   // of the tile's entries, relative to the tile
-    __shared__ int32_t start[kUnitTile], length[kUnitTile];
+    constexpr int kPerThread = kUnitTileMax / kUnitBlock;
+    __shared__ int32_t first_unit[kUnitTileMax + 1];   // of the tile's entries, relative to the tile
+    __shared__ int32_t start[kUnitTileMax], length[kUnitTileMax];
+    const int tile = unit_tile(n);
     int64_t before = 0;
     {
         int32_t part = 0;
         for (int i = threadIdx.x; i < static_cast<int>(blockIdx.x); i += kUnitBlock) part += tile_sums[i];
         before = block_sum(part);
     }
-    const int64_t base = static_cast<int64_t>(blockIdx.x) * kUnitTile;
-    int32_t cnt[kUnitPerThread], local = 0;
+    const int64_t base = static_cast<int64_t>(blockIdx.x) * tile;
+    const int per_thread = (tile + kUnitBlock - 1) / kUnitBlock;
+    int32_t cnt[kPerThread], local = 0;
 #pragma unroll
-    for (int k = 0; k < kUnitPerThread; ++k) {
-        const int i = threadIdx.x * kUnitPerThread + k;
+    for (int k = 0; k < kPerThread; ++k) {
+        cnt[k] = 0;
+        const int i = threadIdx.x * per_thread + k;
+        if (k >= per_thread || i >= tile) continue;
         int32_t s = 0, e = 0;
         if (base + i < n) runs.run(base + i, s, e);
         start[i] = s;
@@ -133,16 +136,16 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n,
     int32_t total;
     int32_t at = block_inclusive_scan(local, &total) - local;
 #pragma unroll
-    for (int k = 0; k < kUnitPerThread; ++k) {
-        first_unit[threadIdx.x * kUnitPerThread + k] = at;
+    for (int k = 0; k < kPerThread; ++k) {
+        const int i = threadIdx.x * per_thread + k;
+        if (k < per_thread && i < tile) first_unit[i] = at;
         at += cnt[k];
     }
-    if (threadIdx.x == kUnitBlock - 1) first_unit[kUnitTile] = at;
     __syncthreads();
     if (before + total > cap) return;
     const int slot = threadIdx.x & 7;
     for (int32_t u = threadIdx.x >> 3; u < total; u += kUnitBlock / 8) {
-        int lo = 0, hi = kUnitTile;      // the entry that holds unit u: the last one that starts at or before it
+        int lo = 0, hi = tile;           // the entry that holds unit u: the last one that starts at or before it
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
             if (first_unit[mid] <= u) lo = mid; else hi = mid;
@@ -163,6 +166,18 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n,
             units[before + u] = h;
         }
     }
+}
+
+// units before row M * c / parts, c < parts <= 8, of a list in row order
+__global__ void k_unit_cuts(const int2 *__restrict__ units, int32_t M, int32_t parts, PlanCounters *__restrict__ pc) {
+    if (static_cast<int>(threadIdx.x) >= parts) return;
+    const int32_t row = static_cast<int32_t>(static_cast<int64_t>(M) * threadIdx.x / parts);
+    int64_t lo = 0, hi = static_cast<int64_t>(pc->units);
+    while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if ((units[mid].y >> 3) < row) lo = mid + 1; else hi = mid;
+    }
+    pc->unit_cut[threadIdx.x] = static_cast<int>(lo);
 }
 
 // copies of the last unit up to a multiple of 8 (the bf16 kernel reads a step's 8 units as one block)
