@@ -967,8 +967,15 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     k_row_stats<<<unit_tiles(e->M), kUnitBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, e->d_rowstart,
                                                                                             whole_rows ? e->d_scan_tiles : nullptr, e->d_pc);
     if (e->nnz > 0) {
-        k_col_scan<<<grid_for(e->nnz, kBlock, cap), kBlock, 0, s>>>(e->d_col, e->nnz, static_cast<int32_t>(e->N), e->d_rowstart,
-                                                                    e->d_touched, e->d_pc);
+        const size_t bitmap = (static_cast<size_t>(e->N) + 31) / 32 * 4;
+        const int scan_blocks = grid_for(e->nnz, 4 * kColScanThreads, e->sm_count * 2);
+        if (bitmap <= kColScanLocalBytes) {
+            if (ensure_dynamic_smem_limit(reinterpret_cast<const void *>(k_col_scan<true>), e->device, kColScanLocalBytes))
+                return fail(e, SDDMM_B200_ERR_CUDA, "column scan: cannot raise the dynamic shared memory limit");
+            k_col_scan<true><<<std::min(scan_blocks, e->sm_count), kColScanThreads, bitmap, s>>>(e->d_col, e->nnz, static_cast<int32_t>(e->N), e->d_rowstart, e->d_touched, e->d_pc);
+        } else {
+            k_col_scan<false><<<scan_blocks, kColScanThreads, 0, s>>>(e->d_col, e->nnz, static_cast<int32_t>(e->N), e->d_rowstart, e->d_touched, e->d_pc);
+        }
         CU_TRY(e, cudaGetLastError());
         if (group_possible(e))
             if (int rc = enqueue_group_sample(e)) return rc;

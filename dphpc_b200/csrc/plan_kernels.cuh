@@ -106,13 +106,25 @@ __global__ void __launch_bounds__(kUnitBlock) k_row_stats(const int32_t *__restr
     }
 }
 
-// four nonzeros per thread: column range, distinct columns (one bit each), in-row ordering.  col is 16-byte aligned.
-__global__ void __launch_bounds__(kPlanBlock) k_col_scan(const int32_t *__restrict__ col, int64_t nnz, int32_t N, const uint32_t *__restrict__ row_start_bits,
-                                                         uint32_t *__restrict__ touched, PlanCounters *__restrict__ pc) {
+// Four nonzeros per thread: column range, distinct columns (one bit each), in-row ordering.  col is 16-byte aligned.
+// LOCAL: the bits are collected per block in shared memory (columns up to kColScanLocalBytes * 8) and merged once at the
+// end -- on the global bitmap every block that has not seen a bit yet updates it, and the updates of a popular word queue up
+// (5.2 M nonzeros over 200 000 columns: 18 us, against 51 us with cached reads of the global bitmap and 102 us past L1).
+constexpr int kColScanThreads = 1024;
+constexpr int kColScanLocalBytes = 200 * 1024;
+template <bool LOCAL>
+__global__ void __launch_bounds__(kColScanThreads) k_col_scan(const int32_t *__restrict__ col, int64_t nnz, int32_t N, const uint32_t *__restrict__ row_start_bits,
+                                                              uint32_t *__restrict__ touched, PlanCounters *__restrict__ pc) {
+    extern __shared__ uint32_t seen[];
+    const int words = static_cast<int>((static_cast<int64_t>(N) + 31) / 32);
+    if (LOCAL) {
+        for (int w = threadIdx.x; w < words; w += kColScanThreads) seen[w] = 0u;
+        __syncthreads();
+    }
     int32_t fresh = 0;
     bool bad = false, unsorted = false, dup = false;
-    const int64_t stride = 4 * static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t j = 4 * (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x); j < nnz; j += stride) {
+    const int64_t stride = 4 * static_cast<int64_t>(gridDim.x) * kColScanThreads;
+    for (int64_t j = 4 * (blockIdx.x * static_cast<int64_t>(kColScanThreads) + threadIdx.x); j < nnz; j += stride) {
         int c[5];
         const int n = static_cast<int>(min(static_cast<int64_t>(4), nnz - j));
         c[0] = j > 0 ? col[j - 1] : 0;
@@ -123,18 +135,18 @@ __global__ void __launch_bounds__(kPlanBlock) k_col_scan(const int32_t *__restri
             for (int k = 0; k < 4; ++k) c[k + 1] = col[j + min(k, n - 1)];
         }
         const uint32_t starts = row_start_bits[j >> 5] >> (j & 31);   // (j is a multiple of 4: the four bits lie in one word)
-        uint32_t word[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const bool in = c[k + 1] >= 0 && c[k + 1] < N;
-            bad |= !in;
-            // past L1: a block that keeps reading an old word would repeat the update for every nonzero of the column
-            word[k] = in ? __ldcg(&touched[c[k + 1] >> 5]) : ~0u;
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t bit = 1u << (c[k + 1] & 31);
-            if (!(word[k] & bit) && !(atomicOr(&touched[c[k + 1] >> 5], bit) & bit)) ++fresh;
+            if (c[k + 1] < 0 || c[k + 1] >= N) {
+                bad = true;
+            } else {
+                uint32_t *word = (LOCAL ? seen : touched) + (c[k + 1] >> 5);
+                const uint32_t bit = 1u << (c[k + 1] & 31);
+                if (!(*word & bit)) {   // (a stale read only costs an update)
+                    if (LOCAL) atomicOr(word, bit);
+                    else if (!(atomicOr(word, bit) & bit)) ++fresh;
+                }
+            }
             if (k < n && !((starts >> k) & 1u) && (j > 0 || k > 0)) {
                 unsorted |= c[k] > c[k + 1];
                 dup |= c[k] == c[k + 1];
@@ -144,8 +156,15 @@ __global__ void __launch_bounds__(kPlanBlock) k_col_scan(const int32_t *__restri
     if (bad) pc->bad_col = 1;
     if (unsorted) pc->unsorted_cols = 1;
     if (dup) pc->dup_cols = 1;
-    const int32_t total = block_sum(fresh);
-    if (threadIdx.x == 0 && total) atomicAdd(&pc->cols_touched, static_cast<unsigned long long>(total));
+    if (LOCAL) {
+        __syncthreads();
+        for (int w = threadIdx.x; w < words; w += kColScanThreads)
+            if (seen[w]) fresh += __popc(seen[w] & ~atomicOr(&touched[w], seen[w]));
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        fresh += __shfl_xor_sync(kFullMask, fresh, o);
+    }
+    if ((threadIdx.x & 31) == 0 && fresh) atomicAdd(&pc->cols_touched, static_cast<unsigned long long>(fresh));
 }
 
 // COO (sorted by row) -> row_ptr.  Thread j owns the rows in (row[j-1], row[j]].  `base` is subtracted from every row index

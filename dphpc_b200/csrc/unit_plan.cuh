@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n,
     // enqueued before the host has seen the counters: nothing is written for a pattern that it is about to refuse
     if (pc->bad_row_ptr || pc->bad_coo || (Runs::kSorted && pc->unsorted_cols)) return;
     constexpr int kPerThread = kUnitTileMax / kUnitBlock;
-    __shared__ int32_t first_unit[kUnitTileMax + 1];   // of the tile's entries, relative to the tile
+    __shared__ int32_t first_unit[kUnitTileMax];   // of the tile's entries, relative to the tile
     __shared__ int32_t start[kUnitTileMax], length[kUnitTileMax];
     const int tile = unit_tile(n);
     int64_t before = 0;
@@ -143,27 +143,43 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n,
     }
     __syncthreads();
     if (before + total > cap) return;
+    // four units at a time: the searches, then the loads, then the stores of all four are in flight together
+    constexpr int kBatch = 4, kGroups = kUnitBlock / 8;
     const int slot = threadIdx.x & 7;
-    for (int32_t u = threadIdx.x >> 3; u < total; u += kUnitBlock / 8) {
-        int lo = 0, hi = tile;           // the entry that holds unit u: the last one that starts at or before it
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (first_unit[mid] <= u) lo = mid; else hi = mid;
+    for (int32_t u0 = threadIdx.x >> 3; u0 < total; u0 += kBatch * kGroups) {
+        int32_t u[kBatch], entry[kBatch], first[kBatch], count[kBatch], c[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            u[k] = min(u0 + k * kGroups, total - 1);
+            entry[k] = 0;
         }
-        const int32_t skip = 8 * (u - first_unit[lo]);
-        const int32_t first = start[lo] + skip, count = min(8, length[lo] - skip);
-        unit_cols[8 * (before + u) + slot] = runs.col[first + min(slot, count - 1)];
-        if (slot == 0) {
-            const int32_t row = runs.row(base + lo);
-            HDR h;
-            h.x = first;
-            h.y = row * 8 + (count - 1);
-            if constexpr (sizeof(HDR) == sizeof(int4)) {
-                int32_t leader;
-                h.z = length[lo];
-                h.w = runs.matched(row, leader) ? runs.G : 1;
+        for (int half = tile >> 1; half > 0; half >>= 1)   // the entry that holds unit u: the last one that starts at or before it (tile: a power of two)
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k)
+                if (first_unit[entry[k] + half] <= u[k]) entry[k] += half;
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            const int32_t skip = 8 * (u[k] - first_unit[entry[k]]);
+            first[k] = start[entry[k]] + skip;
+            count[k] = min(8, length[entry[k]] - skip);
+            c[k] = runs.col[first[k] + min(slot, count[k] - 1)];
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            if (u0 + k * kGroups >= total) break;
+            unit_cols[8 * (before + u[k]) + slot] = c[k];
+            if (slot == 0) {
+                const int32_t row = runs.row(base + entry[k]);
+                HDR h;
+                h.x = first[k];
+                h.y = row * 8 + (count[k] - 1);
+                if constexpr (sizeof(HDR) == sizeof(int4)) {
+                    int32_t leader;
+                    h.z = length[entry[k]];
+                    h.w = runs.matched(row, leader) ? runs.G : 1;
+                }
+                units[before + u[k]] = h;
             }
-            units[before + u] = h;
         }
     }
 }
