@@ -255,9 +255,24 @@ __device__ __forceinline__ int32_t lower_col(const int32_t *__restrict__ col, in
     return lo;
 }
 
+// ... the same by a whole warp: 32 probes per step, so a row of 1 000 nonzeros takes two dependent loads instead of ten
+__device__ __forceinline__ int32_t warp_lower_col(const int32_t *__restrict__ col, int32_t lo, int32_t hi, int64_t c) {
+    const int lane = threadIdx.x & 31;
+    while (hi - lo > 32) {
+        const int32_t step = (hi - lo) / 33 + 1;                 // probes at lo + step * (lane + 1) - 1: 33 pieces of at most `step`
+        const int64_t at = lo + static_cast<int64_t>(step) * (lane + 1) - 1;
+        const bool below = at < hi && col[at] < c;
+        const int n = __popc(__ballot_sync(kFullMask, below));   // probes below c come first
+        const int64_t end = lo + static_cast<int64_t>(step) * (n + 1) - 1;
+        lo += step * n;
+        hi = static_cast<int32_t>(min(static_cast<int64_t>(hi), end));
+    }
+    return lo + __popc(__ballot_sync(kFullMask, lo + lane < hi && col[lo + lane] < c));
+}
+
 // ---- dense 64x64 windows at ARBITRARY offsets ("randomly placed blocks") ---------------------------------------------
 // Step 1, one warp per row: nonzero j is a CANDIDATE when at least `half` nonzeros of its row lie in the 64 columns
-// that start at its own column.  One bit per nonzero.
+// that start at its own column.  One bit per nonzero; a warp takes the 32 nonzeros of one word at a time.
 __global__ void k_window_candidates(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int32_t M, int32_t half,
                                     uint32_t *__restrict__ cand) {
     const int lane = threadIdx.x & 31;
@@ -265,10 +280,12 @@ __global__ void k_window_candidates(const int32_t *__restrict__ rp, const int32_
     for (int64_t r = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5; r < M; r += n_warps) {
         const int32_t a = rp[r], b = rp[r + 1];
         if (b - a < half) continue;
-        for (int32_t j = a + lane; j < b; j += 32) {
-            if (j + half > b) continue;
+        for (int32_t j0 = a & ~31; j0 < b; j0 += 32) {
+            const int32_t j = j0 + lane;
             // `half` nonzeros from j on fit into 64 columns <=> the (half-1)-th successor is closer than 64 columns
-            if (col[j + half - 1] - col[j] < 64) atomicOr(&cand[j >> 5], 1u << (j & 31));
+            const bool is = j >= a && j + half <= b && col[j + half - 1] - col[j] < 64;
+            const uint32_t word = __ballot_sync(kFullMask, is);
+            if (lane == 0 && word) atomicOr(&cand[j0 >> 5], word);   // (the first and the last word are shared with other rows)
         }
     }
 }
@@ -280,12 +297,41 @@ __device__ __forceinline__ int32_t window_count(const int32_t *__restrict__ rp, 
     return lower_col(col, lo, min(b, lo + 64), static_cast<int64_t>(c) + 64) - lo;
 }
 
-// Step 2, one thread per row: the row's candidates are cut greedily, left to right, into 64-column windows (a window
+// Does the pattern hold 64x64 blocks at all?  One thread per sampled nonzero: it counts when `half` nonzeros of its row fit
+// into the 64 columns from its own on AND the row 32 above or the row 32 below -- one of the two crosses the same block --
+// has a sixth of the 64 columns around it.  Long rows alone (power-law patterns) fulfil the first, not the second.
+__global__ void k_block_sample(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int32_t M, int64_t nnz, int32_t half, int32_t samples,
+                               PlanCounters *__restrict__ pc) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    bool hit = false;
+    if (t < samples) {
+        // evenly spaced, plus a part of the step that differs from sample to sample
+        const int64_t step = max(static_cast<int64_t>(1), nnz / samples);
+        const int64_t at = static_cast<int64_t>(t) * nnz / samples + static_cast<int64_t>((static_cast<uint32_t>(t) * 2654435761u) % static_cast<uint64_t>(step));
+        const int32_t j = static_cast<int32_t>(min(at, nnz - 1));
+        if (j + half <= nnz && static_cast<uint32_t>(col[j + half - 1] - col[j]) < 64u) {
+            int32_t lo = 0, hi = M;   // the row that holds j
+            while (hi - lo > 1) {
+                const int32_t mid = lo + (hi - lo) / 2;
+                if (rp[mid] <= j) lo = mid; else hi = mid;
+            }
+            const int32_t c = col[j] - 31;
+            auto crossed = [&](int32_t r) -> bool { return r >= 0 && r < M && window_count(rp, col, r, c) >= 11; };
+            hit = j + half <= rp[lo + 1] && (crossed(lo - 32) || crossed(lo + 32));
+        }
+    }
+    const unsigned all = __ballot_sync(kFullMask, hit);
+    if ((threadIdx.x & 31) == 0 && all) atomicAdd(&pc->block_samples, __popc(all));
+}
+
+// Step 2, one warp per row: the row's candidates are cut greedily, left to right, into 64-column windows (a window
 // starts at the first candidate at or after the end of the previous one), so every window of a row is visited once.  A
 // window whose row above is NOT dense in the same columns is the top edge of a block and anchors a tile there -- and
-// further tiles every 64 rows below it for as long as those rows stay dense in the same columns.
+// further tiles every 64 rows below it for as long as those rows stay dense in the same columns.  The cutting is serial,
+// two loads per window; the windows are judged 32 at a time, one per lane.
 __global__ void k_window_anchors(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int32_t M, int32_t half,
                                  const uint32_t *__restrict__ cand, int2 *__restrict__ anchors, int32_t cap, int *__restrict__ n_anchors) {
+    const int lane = threadIdx.x & 31;
     // first candidate position in [j, b), or b
     auto next_cand = [&](int32_t j, int32_t b) -> int32_t {
         while (j < b) {
@@ -295,20 +341,28 @@ __global__ void k_window_anchors(const int32_t *__restrict__ rp, const int32_t *
         }
         return b;
     };
-    for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < M; r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+    for (int64_t r = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5; r < M; r += n_warps) {
         const int32_t a = rp[r], b = rp[r + 1];
         if (b - a < half) continue;
-        for (int32_t w = next_cand(a, b); w < b;) {
-            const int32_t c = col[w];
-            const bool top = (r == 0) || window_count(rp, col, static_cast<int32_t>(r) - 1, c) < half;
-            if (top) {
+        int32_t w = next_cand(a, b);
+        while (w < b) {
+            int32_t mine = -1;   // first column of this lane's window
+            for (int k = 0; k < 32 && w < b; ++k) {
+                const int32_t c0 = w + lane < b ? col[w + lane] : INT32_MAX, c1 = w + 32 + lane < b ? col[w + 32 + lane] : INT32_MAX;
+                const int32_t c = __shfl_sync(kFullMask, c0, 0);
+                if (lane == k) mine = c;
+                const int inside = __popc(__ballot_sync(kFullMask, c0 - c < 64)) + __popc(__ballot_sync(kFullMask, c1 - c < 64));
+                w = next_cand(w + inside, b);
+            }
+            if (mine >= 0 && (r == 0 || window_count(rp, col, static_cast<int32_t>(r) - 1, mine) < half)) {
                 for (int32_t rr = static_cast<int32_t>(r); rr < M; rr += 64) {
-                    if (rr != r && window_count(rp, col, rr, c) < half) break;
+                    if (rr != r && window_count(rp, col, rr, mine) < half) break;
                     const int slot = atomicAdd(n_anchors, 1);
-                    if (slot < cap) anchors[slot] = make_int2(rr, c);
+                    if (slot < cap) anchors[slot] = make_int2(rr, mine);
                 }
             }
-            w = next_cand(lower_col(col, w, b, static_cast<int64_t>(c) + 64), b);
+            __syncwarp();
         }
     }
 }
