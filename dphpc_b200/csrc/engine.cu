@@ -581,6 +581,18 @@ int build_dense_plan(sddmm_b200_engine *e, const PlanCounters &base_pc, int item
     e->n_dense = 0;
     e->n_residual_items = n_items;
     if (!e->dense_possible || base_pc.unsorted_cols || base_pc.dup_cols || base_pc.max_row_nnz < 32) return SDDMM_B200_OK;
+    // Looking for tiles takes several passes over the pattern, so a cheap look comes first, in two steps: the column scan has
+    // counted the nonzeros that start a half-full 64-column window of their row (none of every fourth one: no tile), then
+    // sampled windows are compared with the rows 32 above and below; any that shows is enough.
+    if (e->knob_offset_tiles <= 0) {
+        if (base_pc.window_hint == 0) return SDDMM_B200_OK;
+        const int samples = static_cast<int>(std::min<int64_t>(e->nnz, 16384));
+        k_block_sample<<<grid_for(samples, kBlock, 1 << 30), kBlock, 0, e->stream>>>(e->d_rp, e->d_col, static_cast<int32_t>(e->M), e->nnz, 32, samples, e->d_pc);
+        CU_TRY(e, cudaGetLastError());
+        PlanCounters seen;
+        if (int rc = read_counters(e, &seen)) return rc;
+        if (seen.block_samples == 0) return SDDMM_B200_OK;
+    }
     const int cap = e->sm_count * 8;
     cudaStream_t s = e->stream;
     const int32_t M = static_cast<int32_t>(e->M);
@@ -645,10 +657,10 @@ int build_dense_plan(sddmm_b200_engine *e, const PlanCounters &base_pc, int item
         uint32_t *owner = offsets_used ? reinterpret_cast<uint32_t *>(e->d_pval) : nullptr;
         if (owner) {
             CU_TRY(e, cudaMemsetAsync(owner, 0xFF, static_cast<size_t>(e->nnz) * 4, s));
-            k_tile_propose<<<grid_for(static_cast<int64_t>(n_dense) * 64, kBlock, 1 << 30), kBlock, 0, s>>>(e->d_rp, e->d_col, M, e->dense_origin,
+            k_tile_propose<<<grid_for(static_cast<int64_t>(n_dense) * 64 * 32, kBlock, 1 << 30), kBlock, 0, s>>>(e->d_rp, e->d_col, M, e->dense_origin,
                                                                                                              n_dense, owner);
         }
-        k_tile_rows<DenseTileDesc><<<grid_for(static_cast<int64_t>(n_dense) * 64, kBlock, 1 << 30), kBlock, 0, s>>>(
+        k_tile_rows<DenseTileDesc><<<grid_for(static_cast<int64_t>(n_dense) * 64 * 32, kBlock, 1 << 30), kBlock, 0, s>>>(
             e->d_rp, e->d_col, M, e->dense_origin, n_dense, e->d_dense_descs, e->d_covered, item_nnz, e->d_item_covered, e->d_anchor_counts,
             e->d_pc, owner);
         return cuda_status(e, cudaGetLastError());
@@ -867,7 +879,7 @@ int build_residual_units(sddmm_b200_engine *e) {
     const int n_tiles = static_cast<int>((e->M + kScanTile - 1) / kScanTile);
     const int cap = e->sm_count * 32;
     cudaStream_t s = e->stream;
-    k_residual_unit_count<<<grid_for(e->M, kBlock, cap), kBlock, 0, s>>>(e->d_rp, M, e->d_covered, e->d_unit_off);
+    k_residual_unit_count<<<grid_for(e->M * 32, kBlock, cap), kBlock, 0, s>>>(e->d_rp, M, e->d_covered, e->d_unit_off);
     k_scan_tile_sums<<<n_tiles, kScanBlock, 0, s>>>(e->d_unit_off, e->M, e->d_scan_tiles);
     k_scan_sums<<<1, kScanBlock, 0, s>>>(e->d_scan_tiles, n_tiles, &e->d_pc->units);
     k_scan_apply<<<n_tiles, kScanBlock, 0, s>>>(e->d_unit_off, e->M, e->d_scan_tiles);
@@ -875,7 +887,7 @@ int build_residual_units(sddmm_b200_engine *e) {
     PlanCounters pc;
     if (int rc = read_counters(e, &pc)) return rc;
     if (pc.units == 0 || pc.units > static_cast<unsigned long long>(e->unit_cap)) return SDDMM_B200_OK;   // (the row-tile kernel takes the residual)
-    k_residual_unit_fill<<<grid_for(e->M, kBlock, cap), kBlock, 0, s>>>(e->d_rp, M, e->d_covered, e->d_unit_off, e->d_col, e->d_units, e->d_unit_cols);
+    k_residual_unit_fill<<<grid_for(e->M * 32, kBlock, cap), kBlock, 0, s>>>(e->d_rp, M, e->d_covered, e->d_unit_off, e->d_col, e->d_units, e->d_unit_cols);
     k_unit_pad<<<1, 64, 0, s>>>(e->d_units, e->d_unit_cols, e->d_pc, e->unit_cap);
     CU_TRY(e, cudaGetLastError());
     e->n_units = static_cast<int32_t>(pc.units);

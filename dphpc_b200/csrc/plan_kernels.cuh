@@ -33,6 +33,8 @@ struct PlanCounters {
     int unit_cut[8];                     // consumer: units before each of 8 equal row ranges
     unsigned long long units;            // row segments of the row-segment path
     unsigned long long window_nnz;       // nonzeros inside the selected 64x64 windows (summed per window)
+    unsigned long long window_hint;      // nonzeros (estimate from every fourth one) whose 31st successor lies less than 64 columns ahead
+    int block_samples;                   // sampled nonzeros that lie in what looks like a 64x64 block
     int n_anchors;                       // candidate origins of the arbitrary-offset tile detection
 };
 
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(kColScanThreads) k_col_scan(const int32_t *__r
         for (int w = threadIdx.x; w < words; w += kColScanThreads) seen[w] = 0u;
         __syncthreads();
     }
-    int32_t fresh = 0;
+    int32_t fresh = 0, dense = 0;
     bool bad = false, unsorted = false, dup = false;
     const int64_t stride = 4 * static_cast<int64_t>(gridDim.x) * kColScanThreads;
     for (int64_t j = 4 * (blockIdx.x * static_cast<int64_t>(kColScanThreads) + threadIdx.x); j < nnz; j += stride) {
@@ -134,6 +136,7 @@ __global__ void __launch_bounds__(kColScanThreads) k_col_scan(const int32_t *__r
         } else {
             for (int k = 0; k < 4; ++k) c[k + 1] = col[j + min(k, n - 1)];
         }
+        if (j + 31 < nnz && static_cast<uint32_t>(col[j + 31] - c[1]) < 64u) dense += 4;   // (across a row boundary by chance only)
         const uint32_t starts = row_start_bits[j >> 5] >> (j & 31);   // (j is a multiple of 4: the four bits lie in one word)
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -163,8 +166,10 @@ __global__ void __launch_bounds__(kColScanThreads) k_col_scan(const int32_t *__r
     }
     for (int o = 16; o > 0; o >>= 1) {
         fresh += __shfl_xor_sync(kFullMask, fresh, o);
+        dense += __shfl_xor_sync(kFullMask, dense, o);
     }
     if ((threadIdx.x & 31) == 0 && fresh) atomicAdd(&pc->cols_touched, static_cast<unsigned long long>(fresh));
+    if ((threadIdx.x & 31) == 0 && dense) atomicAdd(&pc->window_hint, static_cast<unsigned long long>(dense));
 }
 
 // COO (sorted by row) -> row_ptr.  Thread j owns the rows in (row[j-1], row[j]].  `base` is subtracted from every row index
@@ -394,94 +399,81 @@ __global__ void k_anchor_select(const int2 *__restrict__ anchors, const int32_t 
 // key, not by a race -- every (tile, row) proposes (row offset << 6 | column offset) for each of its nonzeros, the
 // smallest key wins (two tiles that hold the same nonzero differ in their origin, hence in the key), so the same matrix
 // always gets the same owners and the same tiles survive k_tile_keep.  owner: one word per nonzero, preset to ~0.
+// One warp per (tile, row).
 __global__ void k_tile_propose(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int32_t M, const int2 *__restrict__ origins,
                                int32_t n_dense, uint32_t *__restrict__ owner) {
-    const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    const int64_t g = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
     if (g >= static_cast<int64_t>(n_dense) * 64) return;
-    const int t = static_cast<int>(g >> 6), r = static_cast<int>(g & 63);
-    const int2 o = origins[t];
+    const int lane = threadIdx.x & 31, r = static_cast<int>(g & 63);
+    const int2 o = origins[g >> 6];
     const int row = o.x + r;
     if (row >= M) return;
-    const int end = rp[row + 1];
-    for (int j = lower_col(col, rp[row], end, o.y); j < end; ++j) {
-        const int c = col[j] - o.y;
-        if (c >= 64) break;
-        atomicMin(&owner[j], (static_cast<uint32_t>(r) << 6) | static_cast<uint32_t>(c));
+    const int end = rp[row + 1], start = warp_lower_col(col, rp[row], end, o.y);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int j = start + lane + 32 * h;
+        const int c = j < end ? col[j] - o.y : 64;
+        if (c < 64) atomicMin(&owner[j], (static_cast<uint32_t>(r) << 6) | static_cast<uint32_t>(c));
     }
 }
 
-// one thread per (dense tile, row): first CSR position of the row inside the tile's column range, presence mask of its 64
-// columns, and the OWN mask -- the nonzeros this tile computes.  Tiles on the 64-grid never overlap (owner == nullptr: a
-// nonzero is claimed in the `covered` bitmap and every claim succeeds); overlapping tiles own what k_tile_propose gave
-// them.  Owned nonzeros are credited to their work items.
+// One warp per (dense tile, row): first CSR position of the row inside the tile's column range, presence mask of its 64
+// columns, and the OWN mask -- the nonzeros this tile computes: all of them for tiles on the 64-grid, which never overlap
+// (owner == nullptr), else what k_tile_propose gave them.  Owned nonzeros are marked in `covered` and credited to their
+// work items.
 template <typename Desc>
 __global__ void k_tile_rows(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int32_t M, const int2 *__restrict__ origins,
                             int32_t n_dense, Desc *__restrict__ descs, uint32_t *__restrict__ covered, int32_t item_nnz,
                             int32_t *__restrict__ item_covered, int32_t *__restrict__ tile_owned, PlanCounters *__restrict__ pc,
                             const uint32_t *__restrict__ owner) {
-    const int64_t g = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (g >= static_cast<int64_t>(n_dense) * 64) return;
-    const int t = static_cast<int>(g >> 6), r = static_cast<int>(g & 63);
-    const int2 o = origins[t];
-    const int row = o.x + r;
-    const int c0 = o.y;
-    int start = 0;
-    unsigned long long mask = 0ull, own = 0ull;
-    if (row < M) {
-        const int end = rp[row + 1];
-        start = lower_col(col, rp[row], end, c0);
-        int n = 0;
-        for (int j = start; j < end; ++j) {
-            const int c = col[j] - c0;
-            if (c >= 64) break;
-            mask |= 1ull << c;
-            ++n;
-        }
-        // bit k of `got` = nonzero start + k is ours: by its key (overlapping tiles), else by claiming [start, start + n)
-        // in the bitmap word by word
-        unsigned long long got = 0ull;
-        if (owner) {
-            for (int k = 0; k < n; ++k)
-                if (owner[start + k] == ((static_cast<uint32_t>(r) << 6) | static_cast<uint32_t>(col[start + k] - c0))) got |= 1ull << k;
-        }
-        for (int j = start; j < start + n;) {
-            const int w = j >> 5, first = j & 31;
-            const int take = min(32 - first, start + n - j);
-            uint32_t bits = (take == 32 ? 0xffffffffu : ((1u << take) - 1u)) << first;
-            if (owner) {
-                bits &= static_cast<uint32_t>(got >> (j - start)) << first;   // mark what is ours as covered
-                if (bits) atomicOr(&covered[w], bits);
-            } else {
-                const uint32_t old = atomicOr(&covered[w], bits);
-                got |= static_cast<unsigned long long>((bits & ~old) >> first) << (j - start);
+    __shared__ int block_owned;
+    if (threadIdx.x == 0) block_owned = 0;
+    __syncthreads();
+    const int64_t g = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (g < static_cast<int64_t>(n_dense) * 64) {
+        const int t = static_cast<int>(g >> 6), r = static_cast<int>(g & 63);
+        const int2 o = origins[t];
+        const int row = o.x + r;
+        int start = 0, owned = 0;
+        uint32_t mask[2] = {0u, 0u}, own[2] = {0u, 0u};   // low and high word
+        if (row < M) {
+            const int end = rp[row + 1];
+            start = warp_lower_col(col, rp[row], end, o.y);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int j = start + lane + 32 * h;
+                const int c = j < end ? col[j] - o.y : 64;
+                const bool in = c < 64;
+                const bool got = in && (!owner || owner[j] == ((static_cast<uint32_t>(r) << 6) | static_cast<uint32_t>(c)));
+                const uint32_t bit = 1u << (c & 31);
+                mask[0] |= __reduce_or_sync(kFullMask, in && c < 32 ? bit : 0u);
+                mask[1] |= __reduce_or_sync(kFullMask, in && c >= 32 ? bit : 0u);
+                own[0] |= __reduce_or_sync(kFullMask, got && c < 32 ? bit : 0u);
+                own[1] |= __reduce_or_sync(kFullMask, got && c >= 32 ? bit : 0u);
+                const unsigned live = __ballot_sync(kFullMask, got);
+                owned += __popc(live);
+                if (got) {
+                    const unsigned word_peers = __match_any_sync(live, j >> 5);
+                    const unsigned bits = __reduce_or_sync(word_peers, 1u << (j & 31));
+                    if (lane == __ffs(word_peers) - 1) atomicOr(&covered[j >> 5], bits);
+                    const unsigned item_peers = __match_any_sync(live, j / item_nnz);
+                    if (lane == __ffs(item_peers) - 1) atomicAdd(&item_covered[j / item_nnz], __popc(item_peers));
+                }
             }
-            j += take;
         }
-        // rank k of the run -> its column bit
-        int k = 0, owned = 0;
-        for (unsigned long long m = mask; m; m &= m - 1, ++k)
-            if ((got >> k) & 1ull) {
-                own |= m & (~m + 1);
-                ++owned;
+        if (lane == 0) {
+            descs[t].start[r] = start;
+            descs[t].mask[r] = (static_cast<unsigned long long>(mask[1]) << 32) | mask[0];
+            descs[t].own[r] = (static_cast<unsigned long long>(own[1]) << 32) | own[0];
+            if (owned) {
+                atomicAdd(&tile_owned[t], owned);
+                atomicAdd(&block_owned, owned);
             }
-        if (owned) {
-            atomicAdd(&pc->dense_nnz, static_cast<unsigned long long>(owned));
-            atomicAdd(&tile_owned[t], owned);
-        }
-        // credit the owned nonzeros to the work items they lie in
-        for (int kk = 0; kk < n;) {
-            const int j = start + kk;
-            const int item = j / item_nnz;
-            const int take = min(n - kk, (item + 1) * item_nnz - j);
-            const unsigned long long seg = (take == 64 ? ~0ull : ((1ull << take) - 1ull)) << kk;
-            const int c = __popcll(got & seg);
-            if (c) atomicAdd(&item_covered[item], c);
-            kk += take;
         }
     }
-    descs[t].start[r] = start;
-    descs[t].mask[r] = mask;
-    descs[t].own[r] = own;
+    __syncthreads();
+    if (threadIdx.x == 0 && block_owned) atomicAdd(&pc->dense_nnz, static_cast<unsigned long long>(block_owned));
 }
 
 // Overlapping windows: a tile that ended up owning too few nonzeros (most of its window went to its neighbours) is not

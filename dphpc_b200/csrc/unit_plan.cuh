@@ -216,45 +216,66 @@ __global__ void k_unit_values(const int2 *__restrict__ units, int32_t n_units, c
 }
 
 // ---- units over what the dense tiles left: runs of nonzeros whose bit in `covered` is clear -----------------------
-// first position in [j, b) whose bit equals `want`, or b
-__device__ __forceinline__ int32_t next_bit(const uint32_t *__restrict__ bits, int32_t j, int32_t b, bool want) {
-    while (j < b) {
-        uint32_t word = bits[j >> 5];
-        if (!want) word = ~word;
-        word >>= (j & 31);
-        if (word) return min(b, j + __ffs(word) - 1);
-        j = (j | 31) + 1;
-    }
-    return b;
+// One warp per row, one word of the bitmap per lane; a run ends at the end of its word, so that words are independent.
+__device__ __forceinline__ uint32_t uncovered_bits(const uint32_t *__restrict__ covered, int32_t word, int32_t a, int32_t b) {
+    const int64_t first = 32 * static_cast<int64_t>(word);
+    uint32_t bits = ~covered[word];
+    if (first < a) bits &= ~0u << (a - first);
+    if (first + 32 > b) bits &= ~0u >> (first + 32 - b);
+    return bits;
 }
-// one thread per row: units of its uncovered runs
+// the next run of set bits: its start and length, taken out of `bits` (!= 0)
+__device__ __forceinline__ int take_run(uint32_t &bits, int &start) {
+    start = __ffs(bits) - 1;
+    const uint32_t rest = ~(bits >> start);
+    const int len = rest ? __ffs(rest) - 1 : 32;   // (rest = 0 only for a full word)
+    bits = start + len >= 32 ? 0u : bits & (~0u << (start + len));
+    return min(len, 32 - start);
+}
+__device__ __forceinline__ int run_units(uint32_t bits) {
+    int n = 0, start;
+    while (bits) n += (take_run(bits, start) + 7) >> 3;
+    return n;
+}
 __global__ void k_residual_unit_count(const int32_t *__restrict__ rp, int32_t M, const uint32_t *__restrict__ covered, int32_t *__restrict__ counts) {
-    for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < M; r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int32_t b = rp[r + 1];
-        int32_t n = 0;
-        for (int32_t j = next_bit(covered, rp[r], b, false); j < b;) {
-            const int32_t e = next_bit(covered, j, b, true);
-            n += (e - j + 7) >> 3;
-            j = next_bit(covered, e, b, false);
-        }
-        counts[r] = n;
+    const int lane = threadIdx.x & 31;
+    const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+    for (int64_t r = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5; r < M; r += n_warps) {
+        const int32_t a = rp[r], b = rp[r + 1];
+        int n = 0;
+        if (b > a)
+            for (int32_t w = (a >> 5) + lane; w <= (b - 1) >> 5; w += 32) n += run_units(uncovered_bits(covered, w, a, b));
+        n = static_cast<int>(__reduce_add_sync(kFullMask, static_cast<unsigned>(n)));
+        if (lane == 0) counts[r] = n;
     }
 }
 __global__ void k_residual_unit_fill(const int32_t *__restrict__ rp, int32_t M, const uint32_t *__restrict__ covered,
                                      const int32_t *__restrict__ offsets, const int32_t *__restrict__ col, int2 *__restrict__ units,
                                      int32_t *__restrict__ unit_cols) {
-    for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < M; r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int32_t b = rp[r + 1];
+    const int lane = threadIdx.x & 31;
+    const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+    for (int64_t r = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5; r < M; r += n_warps) {
+        const int32_t a = rp[r], b = rp[r + 1];
+        if (b <= a) continue;
         int32_t off = offsets[r];
-        for (int32_t j = next_bit(covered, rp[r], b, false); j < b;) {
-            const int32_t e = next_bit(covered, j, b, true);
-            for (int32_t first = j; first < e; first += 8, ++off) {
-                const int32_t count = min(8, e - first);
-                units[off] = make_int2(first, static_cast<int32_t>(r) * 8 + (count - 1));
+        const int32_t last = (b - 1) >> 5;
+        for (int32_t w0 = a >> 5; w0 <= last; w0 += 32) {
+            const int32_t w = w0 + lane;
+            uint32_t bits = w <= last ? uncovered_bits(covered, w, a, b) : 0u;
+            const int n = run_units(bits);
+            const int32_t before = warp_inclusive_scan(n, lane);
+            int32_t at = off + before - n;
+            int start;
+            while (bits) {
+                const int len = take_run(bits, start);
+                for (int skip = 0; skip < len; skip += 8, ++at) {
+                    const int32_t first = 32 * w + start + skip, count = min(8, len - skip);
+                    units[at] = make_int2(first, static_cast<int32_t>(r) * 8 + (count - 1));
 #pragma unroll
-                for (int i = 0; i < 8; ++i) unit_cols[8 * static_cast<int64_t>(off) + i] = col[first + min(i, count - 1)];
+                    for (int i = 0; i < 8; ++i) unit_cols[8 * static_cast<int64_t>(at) + i] = col[first + min(i, count - 1)];
+                }
             }
-            j = next_bit(covered, e, b, false);
+            off += __shfl_sync(kFullMask, before, 31);
         }
     }
 }
