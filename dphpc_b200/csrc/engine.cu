@@ -21,6 +21,7 @@
 
 #include "../../include/sddmm_b200.h"
 #include "host_staging.cuh"
+#include "kernel_dense_fma.cuh"
 #include "kernel_dense_tile.cuh"
 #include "kernel_rowgroup.cuh"
 #include "kernel_rowseg.cuh"
@@ -36,6 +37,7 @@ namespace {
 constexpr size_t kAlign = 256;
 constexpr int kBlock = 256;
 constexpr int kMaxStageBytes = 32 * 1024;  // A rows per stage buffer (a CTA holds two)
+constexpr int kTileHintShare = 64;         // fp32 mode: one nonzero in this many has to look as if it started a row of a tile
 constexpr int kDenseMinCount = 2048;       // a 64x64 tile is "dense" from half full
 
 struct Arena {
@@ -117,6 +119,7 @@ struct sddmm_b200_engine {
     const int2 *dense_origin = nullptr;
     bool dense_own = false;             // the tiles in use may overlap: the kernel looks at their own masks
     int seg_slices = 1;                 // row-segment path: K is taken in this many slices of 64 columns, one launch each
+    bool dense_fma = false;             // the tiles are computed in fp32 FMA instead of on the tensor cores
     bool dense_split3 = false;          // fp32-grade mode: operands through three slots, accumulator parked a tile at a time
     uint32_t *d_covered = nullptr;      // one bit per nonzero: owned by a dense tile
     uint32_t *d_cand = nullptr;         // one bit per nonzero: starts a half-full 64-column window of its row
@@ -438,7 +441,9 @@ int carve_arena(sddmm_b200_engine *e, bool coo, int n_items, bool allow_padding)
     // upload, every bf16 value is exactly a tf32 value (8 against 11 significand bits), so the tile products are exactly the
     // bf16-input / fp32-accumulate ones.
     const bool tc_mode = e->mode == SDDMM_B200_TF32 || e->mode == SDDMM_B200_FP32_TC || e->mode == SDDMM_B200_BF16;
-    e->dense_possible = tc_mode && !(e->flags & SDDMM_B200_FLAG_NO_DENSE_TILES) && K % 32 == 0 && K <= 256 && nnz >= kDenseMinCount;
+    // fp32 mode: the same tiles in plain fp32 arithmetic (unless the row-segment path is asked for or switched off)
+    const bool fma_mode = e->mode == SDDMM_B200_FP32 && e->use_seg && e->knob_rowseg != 1;
+    e->dense_possible = (tc_mode || fma_mode) && !(e->flags & SDDMM_B200_FLAG_NO_DENSE_TILES) && K % 32 == 0 && K <= 256 && nnz >= kDenseMinCount;
     e->aligned_possible = e->dense_possible && e->tile_grid <= (int64_t(1) << 22);
     // (tiles at arbitrary offsets may overlap, so there can be more of them than nnz / 2048; what does not fit is dropped)
     e->dense_cap = e->dense_possible ? static_cast<int32_t>(2 * (e->nnz / kDenseMinCount) + 16) : 0;
@@ -577,21 +582,26 @@ const void *dense_function(bool own, bool split3) {
     return own ? reinterpret_cast<const void *>(sddmm_dense_tile_kernel<true, false>) : reinterpret_cast<const void *>(sddmm_dense_tile_kernel<false, false>);
 }
 
+using DenseFmaFn = void (*)(const DenseFmaArgs);
+DenseFmaFn dense_fma_function(bool own) { return own ? sddmm_dense_tile_fma_kernel<true> : sddmm_dense_tile_fma_kernel<false>; }
+
 int build_dense_plan(sddmm_b200_engine *e, const PlanCounters &base_pc, int item_nnz, int n_items) {
     e->n_dense = 0;
     e->n_residual_items = n_items;
     if (!e->dense_possible || base_pc.unsorted_cols || base_pc.dup_cols || base_pc.max_row_nnz < 32) return SDDMM_B200_OK;
     // Looking for tiles takes several passes over the pattern, so a cheap look comes first, in two steps: the column scan has
     // counted the nonzeros that start a half-full 64-column window of their row (none of every fourth one: no tile), then
-    // sampled windows are compared with the rows 32 above and below; any that shows is enough.
+    // sampled windows are compared with the rows 32 above and below.  The tensor-core modes take any tile that shows; the
+    // fp32 mode, whose tiles gain less, wants about a tenth of the nonzeros in them (a quarter of a block's start a window).
+    const bool fp32 = e->mode == SDDMM_B200_FP32;
     if (e->knob_offset_tiles <= 0) {
-        if (base_pc.window_hint == 0) return SDDMM_B200_OK;
+        if (base_pc.window_hint == 0 || (fp32 && base_pc.window_hint * kTileHintShare < static_cast<unsigned long long>(e->nnz))) return SDDMM_B200_OK;
         const int samples = static_cast<int>(std::min<int64_t>(e->nnz, 16384));
         k_block_sample<<<grid_for(samples, kBlock, 1 << 30), kBlock, 0, e->stream>>>(e->d_rp, e->d_col, static_cast<int32_t>(e->M), e->nnz, 32, samples, e->d_pc);
         CU_TRY(e, cudaGetLastError());
         PlanCounters seen;
         if (int rc = read_counters(e, &seen)) return rc;
-        if (seen.block_samples == 0) return SDDMM_B200_OK;
+        if (seen.block_samples == 0 || (fp32 && static_cast<int64_t>(seen.block_samples) * kTileHintShare < samples)) return SDDMM_B200_OK;
     }
     const int cap = e->sm_count * 8;
     cudaStream_t s = e->stream;
@@ -687,13 +697,27 @@ int build_dense_plan(sddmm_b200_engine *e, const PlanCounters &base_pc, int item
                                                                           e->d_pc);
     CU_TRY(e, cudaGetLastError());
     if (int rc = read_counters(e, &pc)) return rc;
+    e->dense_own = offsets_used;   // tiles off the grid may overlap
+    sddmm_b200_plan_info &p = e->plan;
+    p.dense_tiles = n_dense;
+    p.dense_nnz = static_cast<int64_t>(pc.dense_nnz);
+    p.dense_tile_rows = p.dense_tile_cols = kDenseTile;
+    e->n_residual_items = pc.residual_items;
+    e->dense_fma = fp32;   // (the tensor-core modes are faster on theirs at every K: 50 and 59 us against 73 at K = 32)
+    if (e->dense_fma) {
+        int occ = 0;
+        CU_TRY(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, dense_fma_function(e->dense_own), kFmaThreads, 0));
+        if (occ < 1) return fail(e, SDDMM_B200_ERR_CUDA, "dense-tile FMA kernel does not fit on an SM");
+        e->n_dense = n_dense;
+        p.dense_block = kFmaThreads;
+        p.dense_grid = std::min(n_dense, e->sm_count * occ);
+        return SDDMM_B200_OK;
+    }
     const bool split = e->mode == SDDMM_B200_FP32_TC;
     const int64_t kx = split ? 3 * e->K : e->K;
     int st = make_operand_map(e, &e->map_a, split ? e->d_Ax : e->d_A32, e->M, kx);
     if (!st) st = make_operand_map(e, &e->map_b, split ? e->d_Bx : e->d_B32, e->N, kx);
     if (st) return st;
-    const bool own_masks = offsets_used;   // tiles off the grid may overlap
-    e->dense_own = own_masks;
     // fp32-grade mode, K >= 64: the three-slot operand scheme (measured on the 64 x 64-block configuration, K = 64 / 128:
     // 74 / 114 us against 93 / 160 us with one A block + one B block; K = 32: 63-66 us either way, the shared-memory data
     // pipe that the epilogue and the operand reads share is the limit there).  Knob "dense_split3": 0 = never, 1 = always.
@@ -704,11 +728,6 @@ int build_dense_plan(sddmm_b200_engine *e, const PlanCounters &base_pc, int item
         return fail(e, SDDMM_B200_ERR_CUDA, "dense-tile kernel: cannot raise the dynamic shared memory limit");
     CU_TRY(e, cudaFuncSetAttribute(dense_fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     e->n_dense = n_dense;
-    e->n_residual_items = pc.residual_items;
-    sddmm_b200_plan_info &p = e->plan;
-    p.dense_tiles = n_dense;
-    p.dense_nnz = static_cast<int64_t>(pc.dense_nnz);
-    p.dense_tile_rows = p.dense_tile_cols = kDenseTile;
     p.dense_block = kDenseThreads;
     p.dense_smem_bytes = static_cast<int32_t>(dense_smem);
     // Resident CTAs per SM, from the kernel's own resources (the runtime's occupancy query answers 1 for this kernel):
@@ -900,20 +919,22 @@ int build_residual_units(sddmm_b200_engine *e) {
 
 // Enqueue the unit list over the whole matrix with `panels` column panels (1: whole rows, whose tile sums k_row_stats has
 // left when have_sums).
-int enqueue_unit_list(sddmm_b200_engine *e, int32_t panels, bool have_sums) {
+int enqueue_unit_list(sddmm_b200_engine *e, int32_t panels, bool have_sums, bool unless_tiles = false) {
     const int32_t M = static_cast<int32_t>(e->M), nnz = static_cast<int32_t>(e->nnz);
     cudaStream_t s = e->stream;
     const int64_t n = static_cast<int64_t>(panels) * M;
     const int tiles = unit_tiles(n);
+    // (fp32 mode: tiles will most likely be looked for, and found, when the column scan's count is high enough -- no list then)
+    const unsigned long long skip = unless_tiles ? (static_cast<unsigned long long>(e->nnz) + kTileHintShare - 1) / kTileHintShare : ~0ull;
     if (!have_sums) CU_TRY(e, cudaMemsetAsync(&e->d_pc->units, 0, sizeof(unsigned long long), s));
     if (panels > 1) {
         const RunsOfPanels runs{e->d_rp, e->d_col, M, nnz, panels, e->panel_cols, e->long_rows};
         k_unit_sums<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->d_pc);
-        k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->unit_cap, e->d_pc, e->d_units, e->d_unit_cols);
+        k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->unit_cap, e->d_pc, e->d_units, e->d_unit_cols, skip);
     } else {
         const RunsOfRows runs{e->d_rp, e->d_col, M, nnz};
         if (!have_sums) k_unit_sums<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->d_pc);
-        k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->unit_cap, e->d_pc, e->d_units, e->d_unit_cols);
+        k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->unit_cap, e->d_pc, e->d_units, e->d_unit_cols, skip);
     }
     if (e->mode == SDDMM_B200_BF16) k_unit_pad<<<1, 64, 0, s>>>(e->d_units, e->d_unit_cols, e->d_pc, e->unit_cap);
     CU_TRY(e, cudaGetLastError());
@@ -974,8 +995,9 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
                                                                               e->coo_row_base, e->d_rp, e->d_pc);
     // What will most likely run is enqueued before anything is read back: the plain or panel-major unit list (not where
     // tiles, or the row statistics, decide first) and the sample that looks for row groups.
-    const bool whole_rows = e->use_seg && !e->dense_possible && e->panels == 1;
-    const bool early_list = e->use_seg && !e->dense_possible && e->long_rows == 0 && e->nnz > 0;
+    const bool tiles_first = e->dense_possible && e->mode != SDDMM_B200_FP32;   // (fp32 mode: tiles are the exception)
+    const bool whole_rows = e->use_seg && !tiles_first && e->panels == 1;
+    bool early_list = e->use_seg && !tiles_first && e->long_rows == 0 && e->nnz > 0;
     k_row_stats<<<unit_tiles(e->M), kUnitBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, e->d_rowstart,
                                                                                             whole_rows ? e->d_scan_tiles : nullptr, e->d_pc);
     if (e->nnz > 0) {
@@ -992,10 +1014,10 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         if (group_possible(e))
             if (int rc = enqueue_group_sample(e)) return rc;
         if (early_list)
-            if (int rc = enqueue_unit_list(e, e->panels, whole_rows)) return rc;
+            if (int rc = enqueue_unit_list(e, e->panels, whole_rows, e->dense_possible && e->knob_offset_tiles <= 0)) return rc;
     }
     CU_TRY(e, cudaGetLastError());
-    if (join_copies && !e->dense_possible && e->panels == 1) {
+    if (join_copies && !tiles_first && e->panels == 1) {
         CU_TRY(e, cudaStreamWaitEvent(s, e->ev_h2d, 0));
         if (int rc = convert_storage(e)) return rc;
         e->copies_joined = true;
@@ -1004,6 +1026,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     if (int rc = read_counters(e, &pc)) return rc;
     if (pc.bad_coo) return fail(e, SDDMM_B200_ERR_INDEX, "COO row indices must be sorted and inside [0, M)");
     if (pc.bad_row_ptr) return fail(e, SDDMM_B200_ERR_INDEX, "row_ptr must start at 0, end at nnz and be non-decreasing");
+    if (e->dense_possible && e->knob_offset_tiles <= 0 && pc.window_hint * kTileHintShare >= static_cast<unsigned long long>(e->nnz)) early_list = false;   // (it was left out)
     if (pc.bad_col) return fail(e, SDDMM_B200_ERR_INDEX, "column index outside [0, N)");
 
     sddmm_b200_plan_info &p = e->plan;
@@ -1249,7 +1272,15 @@ int launch_all(sddmm_b200_engine *e, float *p_val) {
         CU_TRY(e, cudaEventRecord(e->ev_fork, e->stream));
         CU_TRY(e, cudaStreamWaitEvent(e->side_stream, e->ev_fork, 0));
     }
-    if (e->n_dense > 0) {
+    if (e->n_dense > 0 && e->dense_fma) {
+        DenseFmaArgs d;
+        d.origins = e->dense_origin; d.descs = e->d_dense_descs; d.s_val = e->d_sval; d.p_val = p_val; d.A = e->d_A32; d.B = e->d_B32;
+        d.n_tiles = e->n_dense; d.M = static_cast<int32_t>(e->M); d.N = static_cast<int32_t>(e->N); d.K = static_cast<int32_t>(e->K);
+        if ((st = begin_kernel(e, e->stream))) return st;
+        dense_fma_function(e->dense_own)<<<p.dense_grid, kFmaThreads, 0, e->stream>>>(d);
+        if ((st = mark_kernel(e, "sddmm_dense_tile_fma_kernel", e->stream))) return st;
+        if (e->n_residual_items == 0) return SDDMM_B200_OK;
+    } else if (e->n_dense > 0) {
         DenseArgs d;
         d.origins = e->dense_origin; d.descs = e->d_dense_descs; d.s_val = e->d_sval; d.p_val = p_val; d.err = e->h_err;
         d.n_tiles = e->n_dense;

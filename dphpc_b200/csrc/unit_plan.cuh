@@ -105,8 +105,10 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs runs, int64_t n, 
 template <typename Runs, typename HDR>
 __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n, const int32_t *__restrict__ tile_sums, int64_t cap,
                                                            const PlanCounters *__restrict__ pc, HDR *__restrict__ units,
-                                                           int32_t *__restrict__ unit_cols) {
-    // enqueued before the host has seen the counters: nothing is written for a pattern that it is about to refuse
+                                                           int32_t *__restrict__ unit_cols, unsigned long long skip_hint = ~0ull) {
+    // enqueued before the host has seen the counters: nothing is written for a pattern that it is about to refuse, or for one
+    // that will be computed otherwise
+    if (pc->window_hint >= skip_hint) return;
     if (pc->bad_row_ptr || pc->bad_coo || (Runs::kSorted && pc->unsorted_cols)) return;
     constexpr int kPerThread = kUnitTileMax / kUnitBlock;
     __shared__ int32_t first_unit[kUnitTileMax];   // of the tile's entries, relative to the tile

@@ -836,3 +836,51 @@ def test_full_size_chunked_call_on_power_law_rows(engines, oracle):
     d.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,blocks", [(64, 64, 32, [(0, 0)]), (70, 131, 64, [(0, 64), (6, 0)]), (400, 300, 96, [(10, 20), (40, 50), (336, 236)]),
+                                          (1000, 1003, 256, [(0, 0), (64, 64), (936, 939), (500, 1)])])
+def test_dense_tiles_in_fp32_arithmetic(oracle, M, N, K, blocks):
+    """fp32 mode computes half-full 64x64 windows tile by tile: one tile alone, tiles at the last row and column, tiles that
+    overlap, several chunks of K, and what the tiles leave as row segments -- every nonzero once, within the fp32 bar."""
+    rng = np.random.default_rng(M + K)
+    dense = rng.random((M, N)) < (0.002 if len(blocks) > 1 else 0.0)
+    for r0, c0 in blocks:
+        dense[r0:r0 + 64, c0:c0 + 64] |= rng.random((min(64, M - r0), min(64, N - c0))) < 0.75
+    rows, cols = np.nonzero(dense)
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=M))]).astype(np.int32)
+    sv = rng.uniform(-1, 1, cols.size).astype(np.float32)
+    A, B = rng.uniform(-1, 1, (M, K)).astype(np.float32), rng.uniform(-1, 1, (N, K)).astype(np.float32)
+    with Engine(0, "fp32") as e:
+        e.set_knob("offset_tiles", 1)
+        p = check(e, "fp32", oracle, M, N, K, rp, cols.astype(np.int32), sv, A, B, what=f"fp32 tiles {M}x{N} K={K}")
+        plan = e.plan()
+        assert plan["dense_tiles"] >= 1 and plan["dense_nnz"] + plan["rowseg_nnz"] == cols.size
+        assert e.kernel_times()[0][0] == "sddmm_dense_tile_fma_kernel"
+        for _ in range(12):   # the later runs replay a captured one
+            e.run()
+            assert np.array_equal(e.download(), p)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode,K", [("fp32", k) for k in (8, 9, 33, 50, 64, 65, 130, 192, 224, 255, 256, 257, 300)] + [("bf16", k) for k in (8, 16, 24, 40, 72, 128, 136, 200, 256)])
+@pytest.mark.parametrize("panels", [1, 3])
+def test_row_segments_at_every_row_length_in_bytes(oracle, mode, K, panels):
+    """Rows that end inside a 128-byte piece, rows of every number of pieces, K beyond the longest instantiation (slices of a
+    padded row); 1 to 17 nonzeros per row; fewer units than a warp step and many."""
+    rng = np.random.default_rng(K)
+    for M, N in ((3, 40), (517, 700)):
+        lens = rng.integers(0, 18, M)
+        lens[0] = 17
+        rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+        ci = np.concatenate([np.sort(rng.choice(N, n, replace=False)) for n in lens]).astype(np.int32)
+        sv = rng.uniform(-1, 1, ci.size).astype(np.float32)
+        A, B = rng.uniform(-1, 1, (M, K)).astype(np.float32), rng.uniform(-1, 1, (N, K)).astype(np.float32)
+        with Engine(0, mode) as e:
+            e.set_knob("panels", panels)
+            check(e, mode, oracle, M, N, K, rp, ci, sv, A, B, what=f"{mode} K={K} {panels} panels {M}x{N}")
+            assert [n for n, _ in e.kernel_times()] == ["sddmm_rowseg_kernel"] and e.plan()["rowseg_nnz"] == ci.size
+            e.update_dense(A=2 * A)   # (the padded copies follow)
+            e.run()
+            p2 = e.download()
+        want = oracle.sddmm_csr(M, K, rp, ci, sv, 2 * A, B)
+        oracle_lib.assert_values_close(p2, want, oracle_lib.abs_dot_bound(oracle.coo_rows(M, rp), ci, sv, 2 * A, B), TOL[mode], f"{mode} K={K} update")
