@@ -1,0 +1,99 @@
+// Device buffers that outlive one engine.
+//
+// cudaMalloc and cudaFree go through the driver and, on a host that is shared, wait for whoever else is in there: measured
+// 0.4 to 20 ms a call, now and then 100 ms and more, where planning and computing a problem of 5 M nonzeros takes 0.25 ms.
+// A program that makes an engine per problem pays that per problem.  So an engine's buffers go to a pool when it is
+// destroyed (or outgrows them) and the next engine on that device takes them from there.
+//   * bounded: at most kBytes per device; what does not fit is freed at once;
+//   * given back: with the last engine of a device, and whenever an allocation fails;
+//   * safe: a buffer enters the pool only after the device has drained, as it would be freed; one mutex guards the lists.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <map>
+#include <mutex>
+#include <vector>
+
+namespace sddmm {
+
+class DevicePool {
+public:
+    static constexpr size_t kBytes = size_t(2) << 30;   // pooled per device: 1 % of the memory of a B200
+    static DevicePool &instance() {
+        static DevicePool *pool = new DevicePool();   // (never destroyed: engines of static storage may end after it would be)
+        return *pool;
+    }
+    void add_user(int device) {
+        std::lock_guard<std::mutex> lock(mu_);
+        ++devices_[device].users;
+    }
+    // `device` is current
+    void remove_user(int device) {
+        std::lock_guard<std::mutex> lock(mu_);
+        Device &d = devices_[device];
+        if (--d.users == 0) drop(d);
+    }
+    // A buffer of at least `bytes` on the current device: *cap is its size.  nullptr: out of memory.
+    void *take(int device, size_t bytes, size_t *cap) {
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            Device &d = devices_[device];
+            int best = -1;
+            for (int i = 0; i < static_cast<int>(d.free.size()); ++i)   // the smallest that fits, at most twice the size asked for
+                if (d.free[i].cap >= bytes && d.free[i].cap / 2 <= bytes && (best < 0 || d.free[i].cap < d.free[best].cap)) best = i;
+            if (best >= 0) {
+                const Block b = d.free[best];
+                d.free.erase(d.free.begin() + best);
+                d.pooled -= b.cap;
+                *cap = b.cap;
+                return b.p;
+            }
+        }
+        void *p = nullptr;
+        for (int attempt = 0; attempt < 2; ++attempt) {
+            if (cudaMalloc(&p, bytes) == cudaSuccess) {
+                *cap = bytes;
+                return p;
+            }
+            cudaGetLastError();
+            std::lock_guard<std::mutex> lock(mu_);
+            drop(devices_[device]);
+        }
+        return nullptr;
+    }
+    // `device` is current, nothing uses the buffer any more
+    void put(int device, void *p, size_t cap) {
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            Device &d = devices_[device];
+            if (d.users > 0 && d.pooled + cap <= kBytes) {
+                d.free.push_back(Block{p, cap});
+                d.pooled += cap;
+                return;
+            }
+        }
+        cudaFree(p);
+    }
+
+private:
+    struct Block {
+        void *p;
+        size_t cap;
+    };
+    struct Device {
+        int users = 0;
+        size_t pooled = 0;
+        std::vector<Block> free;
+    };
+    static void drop(Device &d) {
+        for (const Block &b : d.free) cudaFree(b.p);
+        d.free.clear();
+        d.pooled = 0;
+    }
+    std::mutex mu_;
+    std::map<int, Device> devices_;
+};
+
+}  // namespace sddmm

@@ -3,7 +3,7 @@
 // One engine = one CUDA device, one stream, one device arena that is reused
 // across uploads.  upload_*() copies the operands, validates the pattern on the
 // device, builds the row-length histogram and the kernel plan; run() enqueues
-// the kernels (from the second run of a plan on as one CUDA graph); download()
+// the kernels (of a plan that is run often as one CUDA graph); download()
 // copies P.val back.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "../../include/sddmm_b200.h"
+#include "device_pool.cuh"
 #include "host_staging.cuh"
 #include "kernel_dense_fma.cuh"
 #include "kernel_dense_tile.cuh"
@@ -71,7 +72,8 @@ struct sddmm_b200_engine {
     // 12 us as a kernel launch, 14.3 us as either between two timing events and 28.7 us with the error word cleared and
     // copied back around them (what every run did before).
     cudaGraphExec_t graph = nullptr;
-    int runs_of_plan = 0;          // runs since the last upload (or change of a knob): the second one builds the graph
+    static constexpr int kGraphAfter = 8;   // building one costs 90 us, replaying it saves about 12 us a run
+    int runs_of_plan = 0;          // runs since the last upload (or change of a knob)
     bool run_timing = false;       // last_run_ms has been called: run() records the event pair
     bool last_run_timed_whole = false;
     // chunked host-to-host calls (pipeline.cuh): copies of consecutive row chunks are chained through these
@@ -181,7 +183,6 @@ struct sddmm_b200_engine {
     int64_t spmm_k2 = 0;
     float *d_X = nullptr, *d_Y = nullptr;
     int2 *d_spmm_units = nullptr;
-    int32_t *d_spmm_cols = nullptr;
     cudaEvent_t ev_spmm0 = nullptr, ev_spmm1 = nullptr;
     // Y goes back to the host in up to kSpmmChunks row ranges, each as soon as its part of the kernel is done
     static constexpr int kSpmmChunks = 8;
@@ -242,23 +243,22 @@ int grid_for(int64_t n, int block, int cap) {
     return static_cast<int>(g);
 }
 
-int ensure_arena(sddmm_b200_engine *e, size_t bytes) {
-    if (bytes <= e->arena.cap) return SDDMM_B200_OK;
-    if (e->arena.base) {
-        CU_TRY(e, cudaFree(e->arena.base));
-        e->arena.base = nullptr;
-        e->arena.cap = 0;
+int grow_arena(sddmm_b200_engine *e, Arena &arena, size_t bytes, const char *what) {
+    if (bytes <= arena.cap) return SDDMM_B200_OK;
+    if (arena.base) {
+        CU_TRY(e, cudaDeviceSynchronize());   // (what cudaFree would do: a caller's own stream may still be reading P)
+        DevicePool::instance().put(e->device, arena.base, arena.cap);
+        arena.base = nullptr;
+        arena.cap = 0;
     }
-    void *p = nullptr;
-    cudaError_t st = cudaMalloc(&p, bytes);
-    if (st != cudaSuccess) {
-        cudaGetLastError();
-        return fail(e, SDDMM_B200_ERR_OOM, "device arena of %zu bytes: %s", bytes, cudaGetErrorString(st));
-    }
-    e->arena.base = static_cast<char *>(p);
-    e->arena.cap = bytes;
+    size_t cap = 0;
+    void *p = DevicePool::instance().take(e->device, bytes, &cap);
+    if (!p) return fail(e, SDDMM_B200_ERR_OOM, "%s of %zu bytes: out of memory", what, bytes);
+    arena.base = static_cast<char *>(p);
+    arena.cap = cap;
     return SDDMM_B200_OK;
 }
+int ensure_arena(sddmm_b200_engine *e, size_t bytes) { return grow_arena(e, e->arena, bytes, "device arena"); }
 
 // Upper bound of the row-tile kernel's dynamic shared memory: two buffers of kMaxStageBytes of A rows plus a row_ptr
 // slice of at most kMaxStageBytes / 16 + 1 entries (the shortest staged row is 16 bytes).
@@ -1324,13 +1324,13 @@ int launch_all(sddmm_b200_engine *e, float *p_val) {
     return SDDMM_B200_OK;
 }
 
-// One run's kernels on the main stream.  The first run of a plan launches them one by one (an upload per run pays for no
-// graph); the second captures them, and the graph is replayed from then on.
+// One run's kernels on the main stream.  The first runs of a plan launch them one by one (an upload per run pays for no
+// graph); a later one captures them, and the graph is replayed from then on.
 int enqueue_run(sddmm_b200_engine *e) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     CU_TRY(e, cudaStreamIsCapturing(e->stream, &capturing));
     if (e->kernel_timing || e->nnz == 0 || capturing != cudaStreamCaptureStatusNone) return launch_all(e, e->d_pval);
-    if (!e->graph && ++e->runs_of_plan >= 2) {
+    if (!e->graph && ++e->runs_of_plan > sddmm_b200_engine::kGraphAfter) {
         cudaGraph_t g = nullptr;
         CU_TRY(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
         const int st = launch_all(e, e->d_pval);
@@ -1394,6 +1394,7 @@ int sddmm_b200_create(sddmm_b200_engine **out, int device, int mode, uint32_t fl
     e->knob_k_slices = env_double("SDDMM_B200_K_SLICES", -1);
     e->knob_long_rows = env_double("SDDMM_B200_LONG_ROWS", -1);
     DeviceGuard g(device);
+    DevicePool::instance().add_user(device);
     bool ok = g.ok;
     ok = ok && cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&e->side_stream, cudaStreamNonBlocking) == cudaSuccess;
@@ -1427,8 +1428,10 @@ int sddmm_b200_destroy(sddmm_b200_engine *e) {
         if (e->stream) cudaStreamSynchronize(e->stream);
         if (e->side_stream) cudaStreamSynchronize(e->side_stream);
         drop_graph(e);
-        if (e->arena.base) cudaFree(e->arena.base);
-        if (e->spmm_arena.base) cudaFree(e->spmm_arena.base);
+        cudaDeviceSynchronize();   // (what cudaFree would do: a caller's own stream may still be reading P)
+        DevicePool::instance().put(e->device, e->arena.base, e->arena.cap);
+        DevicePool::instance().put(e->device, e->spmm_arena.base, e->spmm_arena.cap);
+        DevicePool::instance().remove_user(e->device);
         e->stager.release();
         e->stager2.release();
         if (e->b_stage) cudaFree(e->b_stage);
@@ -1790,51 +1793,47 @@ SpmmFn pick_spmm(int cpl, bool exact) {
     }
 }
 
-// X, Y and the consumer's unit list live in their own buffer (grown on demand, kept across calls)
-int spmm_prepare(sddmm_b200_engine *e, int64_t K2) {
+// X (unless it is B), Y and the consumer's unit list live in their own buffer (grown on demand, kept across calls).  Where
+// the run itself works on whole rows its list is the consumer's too.
+int spmm_prepare(sddmm_b200_engine *e, int64_t K2, bool own_x) {
     Carve c;
     const size_t M = static_cast<size_t>(e->M), N = static_cast<size_t>(e->N), nnz = static_cast<size_t>(e->nnz);
     const size_t cap = nnz / 8 + std::min(M, nnz) + 8;
-    const size_t o_x = c.take(N * K2 * 4), o_y = c.take(M * K2 * 4), o_u = c.take(cap * sizeof(int2)), o_uc = c.take(cap * 32);
-    const bool grow = c.off > e->spmm_arena.cap;
-    if (grow) {
-        if (e->spmm_arena.base) CU_TRY(e, cudaFree(e->spmm_arena.base));
-        e->spmm_arena.base = nullptr;
-        e->spmm_arena.cap = 0;
-        void *p = nullptr;
-        if (cudaMalloc(&p, c.off) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(e, SDDMM_B200_ERR_OOM, "consumer buffers of %zu bytes", c.off);
-        }
-        e->spmm_arena.base = static_cast<char *>(p);
-        e->spmm_arena.cap = c.off;
-        e->spmm_units = 0;
-    }
+    const bool shared = e->use_seg && e->n_dense == 0 && !e->rg_rows && e->plan.rowseg_panels == 1 && e->n_units > 0;
+    const size_t o_u = shared ? 0 : c.take(cap * sizeof(int2)), o_y = c.take(M * K2 * 4), o_x = own_x ? c.take(N * K2 * 4) : 0;
+    const char *old = e->spmm_arena.base;
+    if (int rc = grow_arena(e, e->spmm_arena, c.off, "consumer buffers")) return rc;
     char *b = e->spmm_arena.base;
-    const bool moved = e->d_spmm_units != reinterpret_cast<int2 *>(b + o_u);
-    e->d_X = reinterpret_cast<float *>(b + o_x);
+    e->d_X = own_x ? reinterpret_cast<float *>(b + o_x) : nullptr;
     e->d_Y = reinterpret_cast<float *>(b + o_y);
-    e->d_spmm_units = reinterpret_cast<int2 *>(b + o_u);
-    e->d_spmm_cols = reinterpret_cast<int32_t *>(b + o_uc);
+    e->d_spmm_units = shared ? e->d_units : reinterpret_cast<int2 *>(b + o_u);
     e->spmm_k2 = K2;
-    if (e->spmm_units == 0 || moved) {   // plain row segments (one panel, no groups), counted / scanned / written on the device
+    if (b != old && !shared) e->spmm_units = 0;
+    if (e->spmm_units == 0 && shared) {
+        k_unit_cuts<<<1, 32, 0, e->stream>>>(e->d_units, static_cast<int32_t>(e->M), sddmm_b200_engine::kSpmmChunks, e->n_units, e->d_pc);
+        CU_TRY(e, cudaGetLastError());
+        PlanCounters pc;
+        if (int rc = read_counters(e, &pc)) return rc;
+        e->spmm_units = e->n_units;
+        for (int k = 1; k < sddmm_b200_engine::kSpmmChunks; ++k) e->spmm_cut[k] = pc.unit_cut[k];
+    } else if (e->spmm_units == 0) {   // plain row segments (one panel, no groups), counted / scanned / written on the device
         const int32_t Mi = static_cast<int32_t>(e->M);
         cudaStream_t s = e->stream;
         const RunsOfRows runs{e->d_rp, e->d_col, Mi, static_cast<int32_t>(e->nnz)};
         const int tiles = unit_tiles(e->M);
         CU_TRY(e, cudaMemsetAsync(&e->d_pc->units, 0, sizeof(unsigned long long), s));
         k_unit_sums<<<tiles, kUnitBlock, 0, s>>>(runs, e->M, e->d_scan_tiles, e->d_pc);
-        k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, e->M, e->d_scan_tiles, static_cast<int64_t>(cap), e->d_pc, e->d_spmm_units, e->d_spmm_cols);
-        k_unit_cuts<<<1, 32, 0, s>>>(e->d_spmm_units, Mi, sddmm_b200_engine::kSpmmChunks, e->d_pc);
+        k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, e->M, e->d_scan_tiles, static_cast<int64_t>(cap), e->d_pc, e->d_spmm_units, nullptr);
+        k_unit_cuts<<<1, 32, 0, s>>>(e->d_spmm_units, Mi, sddmm_b200_engine::kSpmmChunks, -1, e->d_pc);
         CU_TRY(e, cudaGetLastError());
         PlanCounters pc;
         if (int rc = read_counters(e, &pc)) return rc;
         if (pc.units == 0 || pc.units > cap) return fail(e, SDDMM_B200_ERR_CUDA, "consumer plan: %llu units for a list of %zu", pc.units, cap);
         e->spmm_units = static_cast<int32_t>(pc.units);
         for (int c = 1; c < sddmm_b200_engine::kSpmmChunks; ++c) e->spmm_cut[c] = pc.unit_cut[c];
-        e->spmm_cut[0] = 0;
-        e->spmm_cut[sddmm_b200_engine::kSpmmChunks] = e->spmm_units;
     }
+    e->spmm_cut[0] = 0;
+    e->spmm_cut[sddmm_b200_engine::kSpmmChunks] = e->spmm_units;
     return SDDMM_B200_OK;
 }
 }  // namespace
@@ -1853,7 +1852,7 @@ int sddmm_b200_spmm(sddmm_b200_engine *e, int64_t K2, const float *X, float *Y) 
         std::memset(Y, 0, ybytes);
         return sddmm_b200_sync(e);
     }
-    int st = spmm_prepare(e, K2);   // (uses the plan scratch of the main arena: nothing of the run still needs it)
+    int st = spmm_prepare(e, K2, X != nullptr);   // (uses the plan scratch of the main arena: nothing of the run still needs it)
     if (st) return st;
     if (X) CU_TRY(e, cudaMemcpyAsync(e->d_X, X, static_cast<size_t>(e->N) * K2 * 4, cudaMemcpyHostToDevice, s));
     CU_TRY(e, cudaEventRecord(e->ev_spmm0, s));

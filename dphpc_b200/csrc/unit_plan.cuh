@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n,
 #pragma unroll
         for (int k = 0; k < kBatch; ++k) {
             if (u0 + k * kGroups >= total) break;
-            unit_cols[8 * (before + u[k]) + slot] = c[k];
+            if (unit_cols) unit_cols[8 * (before + u[k]) + slot] = c[k];
             if (slot == 0) {
                 const int32_t row = runs.row(base + entry[k]);
                 HDR h;
@@ -187,10 +187,11 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n,
 }
 
 // units before row M * c / parts, c < parts <= 8, of a list in row order
-__global__ void k_unit_cuts(const int2 *__restrict__ units, int32_t M, int32_t parts, PlanCounters *__restrict__ pc) {
+// (n_units < 0: as many as pc->units says)
+__global__ void k_unit_cuts(const int2 *__restrict__ units, int32_t M, int32_t parts, int32_t n_units, PlanCounters *__restrict__ pc) {
     if (static_cast<int>(threadIdx.x) >= parts) return;
     const int32_t row = static_cast<int32_t>(static_cast<int64_t>(M) * threadIdx.x / parts);
-    int64_t lo = 0, hi = static_cast<int64_t>(pc->units);
+    int64_t lo = 0, hi = n_units >= 0 ? n_units : static_cast<int64_t>(pc->units);
     while (lo < hi) {
         const int64_t mid = (lo + hi) >> 1;
         if ((units[mid].y >> 3) < row) lo = mid + 1; else hi = mid;
