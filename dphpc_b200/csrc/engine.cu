@@ -314,18 +314,20 @@ double env_double(const char *name, double fallback) {
 // Column panels of the row-segment path.  B is cut into panels when it is much larger than the L2 cache, so that the
 // gathers of one panel hit in L2; every panel pass reads the A rows it touches again and shortens the runs a row
 // contributes (a run of fewer than ~6 nonzeros leaves most of a segment's 8 slots empty), which bounds the count.
-// Large K, fp32 storage, B far larger than L2: K is taken in slices of 64 columns, one launch of the K = 64 kernel per
+// Large K, fp32 storage, B larger than L2: K is taken in slices of 64 columns, one launch of the K = 64 kernel per
 // slice over the same unit list, each adding to P.val -- a slice of B is small enough for column panels to keep it in
 // L2, where the whole rows are not (knob "k_slices": 0 = never, 1 = whenever K allows).
 int choose_k_slices(const sddmm_b200_engine *e) {
     if (e->K > 256) return static_cast<int>(e->Ks / 64);   // rows longer than the kernels' largest instantiation (Ks is a multiple of 64)
-    if (e->mode == SDDMM_B200_BF16 || e->K < 128 || e->K % 64 != 0 || e->knob_k_slices == 0) return 1;
+    if (e->mode == SDDMM_B200_BF16 || e->Ks < 128 || e->Ks % 64 != 0 || e->knob_k_slices == 0) return 1;
     const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20);
-    if (e->knob_k_slices < 0 && static_cast<double>(e->N) * e->K * 4.0 <= 4.0 * l2) return 1;
+    // measured, whole / in slices, with B 1 / 1.3 / 1.4 / 2.7 times L2: K = 128 371 / 342, K = 192 438 / 355, K = 128 395 / 394 and 997 / 889 us;
+    // with B 0.5 times L2, K = 256: 725 / 751
+    if (e->knob_k_slices < 0 && static_cast<double>(e->N) * e->Ks * 4.0 <= 0.9 * l2) return 1;
     // slices pay through the column panels they make room for; rows too short for panels are better off read whole
     // (power-law rows, mean length 14, K = 128: 2.04 ms whole against 2.12 ms in slices) -- unless the long rows get panels
     if (e->knob_k_slices < 0 && e->nnz / std::max<int64_t>(1, 8 * e->M) < 2 && e->knob_long_rows == 0) return 1;
-    return static_cast<int>(e->K / 64);
+    return static_cast<int>(e->Ks / 64);
 }
 
 // Rows too short for column panels on average, but B far larger than L2 (power-law row lengths: a few percent of the rows
@@ -362,11 +364,15 @@ int choose_panels(const sddmm_b200_engine *e) {
         if (b_bytes <= 2.0 * l2) return 1;
         return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(static_cast<int64_t>(std::ceil(b_bytes / l2)), e->nnz / std::max<int64_t>(1, 8 * e->M)), 4)));
     }
-    // measured on B200 (126 MB of L2): panels of about 96 MB are as good as smaller ones, and a run shorter than a segment
-    // wastes gather slots -- so at most one panel per 8 nonzeros of an average row, and never more than 4
-    const double panel = e->knob_panel_mb > 0 ? e->knob_panel_mb * (1 << 20) : 0.75 * l2;
+    // measured on B200 (126 MB of L2): a run shorter than a segment wastes gather slots, so panels of about 96 MB for rows of one
+    // piece (B 186 MB: 2 / 3 panels 507 / 514 us), 80 MB for longer rows, where a slot's waste weighs less against its row
+    // (K = 64, B 179 MB: 428 / 414 us, B 372 MB: 3 / 4 panels 1138 / 1116); at most one panel per 6 nonzeros of an average row
+    // (rows of at least 16), and never more than 4 (5: 3 % slower)
+    const bool one_piece = (e->seg_slices > 1 ? 64 : e->Ks) <= 32;
+    const double panel = e->knob_panel_mb > 0 ? e->knob_panel_mb * (1 << 20) : (one_piece ? 0.75 : 0.6) * l2;
     int64_t p = static_cast<int64_t>((b_bytes + panel - 1) / panel);
-    p = std::min<int64_t>(p, e->nnz / std::max<int64_t>(1, 8 * e->M));
+    if (e->nnz < 16 * e->M) p = 1;
+    p = std::min<int64_t>(p, e->nnz / std::max<int64_t>(1, 6 * e->M));
     return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(p, 4)));
 }
 
@@ -796,6 +802,12 @@ RowSegFn seg_function(const sddmm_b200_engine *e, bool copies) {
     if (e->mode == SDDMM_B200_BF16) return copies ? pick_rowseg_bf16<true>(e->Ks) : pick_rowseg_bf16<false>(e->Ks);
     if (e->seg_slices > 1) return copies ? sddmm_rowseg_kernel<2, true, true> : sddmm_rowseg_kernel<2, false, true>;   // a 64-column slice
     const int pieces = static_cast<int>((e->Ks + 31) / 32);
+    // whole rows of a B that does not fit L2, without panels (rows too short for them): the order that DRAM likes
+    if (!copies && static_cast<double>(e->N) * e->Ks * 4.0 > e->l2_bytes) {
+        if (pieces == 4) return sddmm_rowseg_wide_kernel<4>;
+        if (pieces == 6) return sddmm_rowseg_wide_kernel<6>;
+        if (pieces == 8) return sddmm_rowseg_wide_kernel<8>;
+    }
     return copies ? pick_rowseg<true>(pieces) : pick_rowseg<false>(pieces);
 }
 // persistent grid of a streaming kernel over `n_units` units, `per_step` of them per warp step

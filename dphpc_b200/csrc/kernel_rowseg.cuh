@@ -67,6 +67,16 @@ __device__ __forceinline__ float4 ld_part(const unsigned char *p) {
     asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
     return v;
 }
+// ... that has L2 fetch the whole 256-byte block it lies in: the first of two pieces of a row that are wanted one after the other
+__device__ __forceinline__ Piece ld_piece_of_two(const unsigned char *p) {
+    Piece r;
+    asm volatile("ld.global.nc.L2::256B.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(r.v[0].x), "=f"(r.v[0].y), "=f"(r.v[1].x), "=f"(r.v[1].y), "=f"(r.v[2].x), "=f"(r.v[2].y), "=f"(r.v[3].x),
+                   "=f"(r.v[3].y)
+                 : "l"(p));
+    return r;
+}
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ Cols8 ld_cols(const int32_t *p) {
     Cols8 r;
     asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -112,6 +122,12 @@ __device__ __forceinline__ float2 group4_transpose_reduce(const float (&a)[8], i
     r.y = (high ? w[3] : w[2]) + __shfl_xor_sync(kFullMask, high ? w[2] : w[3], 2);
     return r;
 }
+
+// How many stages before its load a piece of A is asked into L2.  A row of A is used by one or two units and comes from HBM,
+// whose latency under load is longer than a stage: 9 M nonzeros, B in L2, K = 256: 880 us without, 725 with (K = 64 185 -> 168,
+// K = 128 351 -> 325).  The best distances, measured, are 1, 3 and 2 for up to 2, 4 and more pieces; a prefetch of the whole row
+// two steps ahead takes too much of L2 (K = 256 950 us).
+__host__ __device__ constexpr int a_prefetch_stages(int pieces) { return pieces <= 2 ? 1 : pieces <= 4 ? 3 : 2; }
 
 // fp32 rows of NP pieces (the last one may be partial: the lanes past its end multiply by zero).  COPIES: S values come from per-unit copies in list order (column panels: a run is a short piece of its row, whose
 // sectors two or more panel passes would read in turn).  ACC: add to P.val (later slices of K).
@@ -170,10 +186,14 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
             const bool last = p == NP - 1;
             const int p_next = last ? 0 : p + 1;
             const Piece a_next = load_a((last ? un_next.y : un.y) >> 3, p_next);
+            constexpr int kAhead = a_prefetch_stages(NP);
+            const int pf = p + 1 + kAhead;   // ... and the A piece kAhead stages after that one, to L2
+            if (t == 0) prefetch_l2(row_at(static_cast<const unsigned char *>(args.A) + 128 * (pf % NP), (pf < NP ? un.y : pf < 2 * NP ? un_next.y : un_next2.y) >> 3, stride));
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 acc[i] = dot_piece(a, bq[i], acc[i]);
-                bq[i] = ld_piece(row_at(Bt + piece_offset(p_next), last ? cols_next.v[i] : cols.v[i], stride));
+                const unsigned char *q = row_at(Bt + piece_offset(p_next), last ? cols_next.v[i] : cols.v[i], stride);
+                bq[i] = NP > 1 && p_next % 2 == 0 ? ld_piece_of_two(q) : ld_piece(q);
             }
             a = a_next;
         }
@@ -187,6 +207,88 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
         un_next = un_next2;
         cols = cols_next;
         cols_next = cols_next2;
+    }
+}
+
+// The same for whole rows (NP even, at least 4) of a B that does not fit L2 and is gathered without column panels: DRAM is the
+// bound, and it likes few rows open at a time.  The stages go through all pieces of 4 slots, two pieces of 128 bytes at a
+// time, before the other 4: half the rows in flight, twice the bytes of each.  9 M nonzeros in rows of 13, B 358 / 717 MB:
+// K = 128 697 -> 638 us, K = 256 1581 -> 1559; with B in L2 the order above is faster (K = 128 385 against 414).
+template <int NP>
+__global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_wide_kernel(const RowSegArgs args) {
+    const int lane = threadIdx.x & 31;
+    const int t = lane & 3;
+    const int grp = lane >> 2;
+    const int n_steps = (args.n_units + 7) >> 3;
+    const int n_warps = static_cast<int>(gridDim.x) * kRowSegWarps;
+    int b = static_cast<int>(blockIdx.x) * kRowSegWarps + (threadIdx.x >> 5);
+    if (b >= n_steps) return;
+    const int last_unit = args.n_units - 1;
+    const bool off = 128 * (NP - 1) + 32 * t >= args.row_bytes;   // this lane's part of the last piece lies past the row
+    const uint32_t stride = args.row_stride;
+    const unsigned char *At = static_cast<const unsigned char *>(args.A) + 32 * t;
+    const unsigned char *Bt = static_cast<const unsigned char *>(args.B) + 32 * t;
+    const int o_last = off ? args.row_bytes - 32 - 32 * t : 128 * (NP - 1);
+    constexpr int kPairs = NP / 2;
+
+    auto unit_index = [&](int step) -> int { const int u = 8 * step + grp; return u < last_unit ? u : last_unit; };
+    auto load_unit = [&](int step) -> int2 { return __ldcs(args.units + unit_index(step)); };
+    auto load_cols = [&](int step) -> Cols8 { return ld_cols(args.unit_cols + 8 * static_cast<int64_t>(unit_index(step))); };
+    auto piece_offset = [&](int p) -> int { return p == NP - 1 ? o_last : 128 * p; };
+    auto load_a = [&](Piece (&a)[2], int row, int q) {
+        const unsigned char *r = row_at(At, row, stride);
+        a[0] = ld_piece(r + piece_offset(2 * q));
+        a[1] = ld_piece(2 * q + 1 == NP - 1 && off ? reinterpret_cast<const unsigned char *>(g_zero_part) : r + piece_offset(2 * q + 1));
+    };
+    auto load_b = [&](Piece (&x)[2], int col, int q) {
+        const unsigned char *r = row_at(Bt, col, stride);
+        x[0] = ld_piece(r + piece_offset(2 * q));
+        x[1] = ld_piece(r + piece_offset(2 * q + 1));
+    };
+
+    int2 un = load_unit(b), un_next = load_unit(b + n_warps);
+    Cols8 cols = load_cols(b);
+    Piece a[2], bq[4][2];
+    load_a(a, un.y >> 3, 0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) load_b(bq[i], cols.v[i], 0);
+
+    while (true) {
+        const int next = b + n_warps;
+        const int count = 8 * b + grp <= last_unit ? (un.y & 7) : -1;
+        const float *sv = args.s_val + un.x;
+        const float s0 = __ldcs(sv + min(t, un.y & 7));
+        const float s1 = __ldcs(sv + min(t + 4, un.y & 7));
+        const int2 un_next2 = load_unit(next + n_warps);
+        const Cols8 cols_next = load_cols(next);
+        float acc[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int q = 0; q < kPairs; ++q) {
+                const bool last = q == kPairs - 1, end = last && h == 1;
+                const int q_next = last ? 0 : q + 1;
+                Piece a_next[2];
+                load_a(a_next, (end ? un_next.y : un.y) >> 3, q_next);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    acc[4 * h + i] = dot_piece(a[1], bq[i][1], dot_piece(a[0], bq[i][0], acc[4 * h + i]));
+                    load_b(bq[i], end ? cols_next.v[i] : last ? cols.v[4 + i] : cols.v[4 * h + i], q_next);
+                }
+                a[0] = a_next[0];
+                a[1] = a_next[1];
+            }
+        const float2 dot = group4_transpose_reduce(acc, t);
+        if (t <= count) __stcs(args.p_val + un.x + t, dot.x * s0);
+        if (t + 4 <= count) __stcs(args.p_val + un.x + t + 4, dot.y * s1);
+
+        if (next >= n_steps) break;   // warp-uniform
+        b = next;
+        un = un_next;
+        un_next = un_next2;
+        cols = cols_next;
     }
 }
 

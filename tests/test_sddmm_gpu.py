@@ -884,3 +884,25 @@ def test_row_segments_at_every_row_length_in_bytes(oracle, mode, K, panels):
             p2 = e.download()
         want = oracle.sddmm_csr(M, K, rp, ci, sv, 2 * A, B)
         oracle_lib.assert_values_close(p2, want, oracle_lib.abs_dot_bound(oracle.coo_rows(M, rp), ci, sv, 2 * A, B), TOL[mode], f"{mode} K={K} update")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K,nnz_per_row", [(128, 9), (100, 9), (192, 12), (256, 7), (256, 17)])
+def test_rows_of_a_b_larger_than_the_cache(oracle, K, nnz_per_row):
+    """B larger than L2 and long rows of it: whole rows (short rows of S) in the order that keeps few of them in flight, the last
+    piece of a row partial (K = 100), and slices of K; two runs bit for bit."""
+    rng = np.random.default_rng(K + nnz_per_row)
+    N = (140 << 20) // (4 * K) + 7
+    M = 3001
+    lens = rng.integers(1, 2 * nnz_per_row, M)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = np.concatenate([np.unique(rng.integers(0, N, 2 * n))[:n] for n in lens]).astype(np.int32)
+    sv = rng.uniform(-1, 1, ci.size).astype(np.float32)
+    A, B = rng.uniform(-1, 1, (M, K)).astype(np.float32), rng.uniform(-1, 1, (N, K)).astype(np.float32)
+    for slices in (0, 1):
+        with Engine(0, "fp32") as e:
+            e.set_knob("k_slices", slices)
+            e.set_knob("long_rows", 0)
+            p = check(e, "fp32", oracle, M, N, K, rp, ci, sv, A, B, what=f"large B K={K} slices {slices}")
+            e.run()
+            assert np.array_equal(e.download(), p)
