@@ -120,7 +120,8 @@ struct sddmm_b200_engine {
     int2 *d_dense_origin2 = nullptr;    // ... (arbitrary-offset detection); `dense_origin` points at the list in use
     const int2 *dense_origin = nullptr;
     bool dense_own = false;             // the tiles in use may overlap: the kernel looks at their own masks
-    int seg_slices = 1;                 // row-segment path: K is taken in this many slices of 64 columns, one launch each
+    int seg_slices = 1;                 // row-segment path: K is taken in this many slices of slice_cols columns, one launch each
+    int slice_cols = 64;                // 64 or 128
     bool dense_fma = false;             // the tiles are computed in fp32 FMA instead of on the tensor cores
     bool dense_split3 = false;          // fp32-grade mode: operands through three slots, accumulator parked a tile at a time
     uint32_t *d_covered = nullptr;      // one bit per nonzero: owned by a dense tile
@@ -157,9 +158,10 @@ struct sddmm_b200_engine {
     bool group_tried = false;          // a grouping was matched exactly and then dropped
     bool copies_joined = false;        // the upload's copies and conversions are already ordered before the plan's read-back
     int64_t unit_cap = 0;
-    int32_t panels = 1;                // column panels the unit list is ordered by
-    int32_t panel_cols = 0;            // columns per panel
-    int32_t long_rows = 0;             // > 0: only rows of at least this many nonzeros are cut into panels, the others follow whole (as one more "panel")
+    int32_t panels_plain = 1;          // column panels when every row is cut
+    int32_t panels_long = 1, long_threshold = 0;   // ... when only rows of at least long_threshold (> 0) nonzeros are; the row statistics choose
+    int32_t panel_cols = 0;            // columns per panel of the list in use
+    int32_t long_rows = 0;             // > 0: the list in use cuts only rows of at least this many nonzeros, the others follow whole (as one more "panel")
     int32_t n_units = 0;
     bool use_seg = false;
     bool seg_residual = false;         // the row-segment kernel computes what the dense tiles left (units over the uncovered runs)
@@ -311,53 +313,63 @@ double env_double(const char *name, double fallback) {
     return v ? std::atof(v) : fallback;
 }
 
-// Column panels of the row-segment path.  B is cut into panels when it is much larger than the L2 cache, so that the
-// gathers of one panel hit in L2; every panel pass reads the A rows it touches again and shortens the runs a row
-// contributes (a run of fewer than ~6 nonzeros leaves most of a segment's 8 slots empty), which bounds the count.
-// Large K, fp32 storage, B larger than L2: K is taken in slices of 64 columns, one launch of the K = 64 kernel per
-// slice over the same unit list, each adding to P.val -- a slice of B is small enough for column panels to keep it in
-// L2, where the whole rows are not (knob "k_slices": 0 = never, 1 = whenever K allows).
-int choose_k_slices(const sddmm_b200_engine *e) {
-    if (e->K > 256) return static_cast<int>(e->Ks / 64);   // rows longer than the kernels' largest instantiation (Ks is a multiple of 64)
-    if (e->mode == SDDMM_B200_BF16 || e->Ks < 128 || e->Ks % 64 != 0 || e->knob_k_slices == 0) return 1;
-    const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20);
-    // measured, whole / in slices, with B 1 / 1.3 / 1.4 / 2.7 times L2: K = 128 371 / 342, K = 192 438 / 355, K = 128 395 / 394 and 997 / 889 us;
-    // with B 0.5 times L2, K = 256: 725 / 751
-    if (e->knob_k_slices < 0 && static_cast<double>(e->N) * e->Ks * 4.0 <= 0.9 * l2) return 1;
-    // slices pay through the column panels they make room for; rows too short for panels are better off read whole
-    // (power-law rows, mean length 14, K = 128: 2.04 ms whole against 2.12 ms in slices) -- unless the long rows get panels
-    if (e->knob_k_slices < 0 && e->nnz / std::max<int64_t>(1, 8 * e->M) < 2 && e->knob_long_rows == 0) return 1;
-    return static_cast<int>(e->Ks / 64);
+// Large K, fp32 storage: K is taken in slices, one launch per slice over the same unit list, each adding to P.val, where that
+// makes a slice of B fit L2 (or leaves column panels room) when the whole rows do not.  Measured, whole / in slices of 64, with
+// B 1 / 1.3 / 1.4 / 2.7 times L2: K = 128 371 / 342, K = 192 438 / 355, K = 128 395 / 394 and 997 / 889 us; with B 0.5 times
+// L2, K = 256: 725 / 751.  Slices of 128 where K allows two of them: K = 256, B 1.4 / 2.7 / 5.5 times L2, whole / 64 / 128
+// columns 925 / 1232 / 798, 518 / 493 / 420, 2378 / 2157 / 1987 us, and also with B in L2 when A is streamed (731 / 777 / 684).
+// Knob "k_slices": 0 = never, 1 = slices of 64 whenever K allows, 128 = of 128.
+void choose_k_slices(sddmm_b200_engine *e) {
+    e->slice_cols = e->Ks % 128 == 0 && (e->knob_k_slices >= 128 || (e->knob_k_slices != 1 && e->Ks >= 256)) ? 128 : 64;
+    e->seg_slices = 1;
+    const int slices = static_cast<int>(e->Ks / e->slice_cols);
+    if (e->K > 256) {   // rows longer than the kernels' largest instantiation (Ks is a multiple of 64)
+        e->seg_slices = slices;
+        return;
+    }
+    if (e->mode == SDDMM_B200_BF16 || e->Ks < 128 || e->Ks % 64 != 0 || e->knob_k_slices == 0) return;
+    const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20), row = static_cast<double>(e->Ks) * 4.0;
+    const bool pays = static_cast<double>(e->N) * row > 0.9 * l2 || (e->slice_cols == 128 && static_cast<double>(e->M) * row > 2.0 * l2);
+    if (e->knob_k_slices < 0 && !pays) return;
+    // (rows too short for panels, and none wanted for the long ones: whole rows)
+    if (e->knob_k_slices < 0 && e->nnz < 16 * e->M && e->knob_long_rows == 0) return;
+    e->seg_slices = slices;
 }
 
-// Rows too short for column panels on average, but B far larger than L2 (power-law row lengths: a few percent of the rows
-// hold most of the nonzeros): column panels for the rows of at least `long_rows` nonzeros only, the shorter rows follow
-// whole as one more entry of the panel-major list.  Returns the candidate threshold (0: not a candidate); e->panels is
-// then the number of real panels.  The plan confirms it once the row-length statistics are known (build_rowseg_plan).
-// Knob "long_rows": 0 = never, T >= 1 = threshold T with the panels the "panels" knob or the rule below gives.
-bool long_rows_candidate(const sddmm_b200_engine *e) {
-    if (e->knob_long_rows == 0) return false;
+// Column panels of the row-segment path.  B is cut into panels when it is larger than the L2 cache, so that the gathers of
+// one panel hit in L2; every panel pass reads the A rows it touches again and shortens the runs a row contributes, which
+// bounds the count.  Two forms; the plan takes the second where the row statistics say so (build_rowseg_plan):
+//   * plain: every row is cut;
+//   * long rows: only the rows of at least `long_threshold` nonzeros are cut, the shorter ones follow whole as one more entry
+//     of the panel-major list.  In power-law patterns a few percent of the rows hold most of the nonzeros and the many
+//     short ones would fall into runs of one or two: 20 M nonzeros, 1 M rows, K = 64 532 us plain, 396 us; 35 M, 1.5 M rows,
+//     K = 32 480 / 370 us; 36 M, 2.6 M rows, K = 32 561 us without panels, 447 us.
+// Knob "long_rows": 0 = never, T >= 1 = threshold T with the panels that the "panels" knob or the rule gives.
+double gathered_bytes(const sddmm_b200_engine *e, int64_t cols) { return static_cast<double>(e->N) * static_cast<double>(cols) * static_cast<double>(elem_bytes(e)); }
+
+// (K = 128: where the long rows get panels the rows are taken whole, 565 us against 586 in two slices)
+bool long_rows_whole(const sddmm_b200_engine *e) { return e->seg_slices > 1 && e->Ks == 128 && e->knob_k_slices < 0; }
+
+void choose_long_rows(sddmm_b200_engine *e) {
+    e->long_threshold = 0;
+    e->panels_long = 1;
+    if (e->knob_long_rows == 0) return;
     const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20);
-    return static_cast<double>(e->N) * (e->seg_slices > 1 ? 64 : e->Ks) * static_cast<double>(elem_bytes(e)) > l2 &&
-           e->nnz / std::max<int64_t>(1, 8 * e->M) < 2;
-}
-int choose_long_rows(const sddmm_b200_engine *e) {
-    if (e->knob_long_rows >= 1) return e->panels > 1 ? static_cast<int>(e->knob_long_rows) : 0;
-    if (!long_rows_candidate(e) || e->panels < 2) return 0;
-    return e->panels <= 4 ? 64 : 128;    // runs of 16 nonzeros or more on average (powers of two: the histogram's bins)
+    const double b = gathered_bytes(e, e->seg_slices > 1 && !long_rows_whole(e) ? e->slice_cols : e->Ks);
+    if (b <= l2 && !(e->knob_long_rows >= 1 && e->knob_panels >= 2)) return;
+    // B 333 MB, K = 32: 4 panels 458 us, 6 446 us, 8 442-447 us
+    e->panels_long = e->knob_panels >= 1 ? static_cast<int>(std::min(64.0, e->knob_panels)) : static_cast<int>(std::max(2.0, std::min(8.0, std::ceil(b / (0.5 * l2)))));
+    if (e->panels_long < 2) return;
+    // runs of 16 nonzeros or more on average (powers of two: the histogram's bins)
+    e->long_threshold = e->knob_long_rows >= 1 ? static_cast<int>(e->knob_long_rows) : e->panels_long <= 4 ? 64 : 128;
 }
 
 int choose_panels(const sddmm_b200_engine *e) {
     if (e->knob_panels >= 1 && e->knob_panels <= 64) return static_cast<int>(e->knob_panels);
-    if (long_rows_candidate(e)) {   // measured on the power-law configuration (B 333 MB): 4 panels 458 us, 6 446 us, 8 442-447 us
-        const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20);
-        return static_cast<int>(std::max(2.0, std::min(8.0, std::ceil(static_cast<double>(e->N) * (e->seg_slices > 1 ? 64 : e->Ks) *
-                                                                      static_cast<double>(elem_bytes(e)) / (0.5 * l2)))));
-    }
-    const double eb = static_cast<double>(elem_bytes(e));
-    const double b_bytes = static_cast<double>(e->N) * (e->seg_slices > 1 ? 64 : e->Ks) * eb;
+    const int64_t cols = e->seg_slices > 1 ? e->slice_cols : e->Ks;
+    const double b_bytes = gathered_bytes(e, cols);
     const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20);
-    if (b_bytes <= l2) return 1;
+    if (b_bytes <= l2 || e->nnz < 16 * e->M) return 1;   // (rows too short on average)
     // bf16 storage, measured with 1.45 M rows of B: K = 64 (B 1.5 x L2) 590 / 618 / 634 us with 1 / 2 / 3 panels, K = 128 (3 x L2)
     // 1809 / 1142 / 1092 / 1096 / 1150 us with 1 .. 5
     if (e->mode == SDDMM_B200_BF16) {
@@ -366,13 +378,10 @@ int choose_panels(const sddmm_b200_engine *e) {
     }
     // measured on B200 (126 MB of L2): a run shorter than a segment wastes gather slots, so panels of about 96 MB for rows of one
     // piece (B 186 MB: 2 / 3 panels 507 / 514 us), 80 MB for longer rows, where a slot's waste weighs less against its row
-    // (K = 64, B 179 MB: 428 / 414 us, B 372 MB: 3 / 4 panels 1138 / 1116); at most one panel per 6 nonzeros of an average row
-    // (rows of at least 16), and never more than 4 (5: 3 % slower)
-    const bool one_piece = (e->seg_slices > 1 ? 64 : e->Ks) <= 32;
-    const double panel = e->knob_panel_mb > 0 ? e->knob_panel_mb * (1 << 20) : (one_piece ? 0.75 : 0.6) * l2;
-    int64_t p = static_cast<int64_t>((b_bytes + panel - 1) / panel);
-    if (e->nnz < 16 * e->M) p = 1;
-    p = std::min<int64_t>(p, e->nnz / std::max<int64_t>(1, 6 * e->M));
+    // (K = 64, B 179 MB: 428 / 414 us, B 372 MB: 3 / 4 panels 1138 / 1116); at most one panel per 6 nonzeros of an average row,
+    // and never more than 4 (5: 3 % slower)
+    const double panel = e->knob_panel_mb > 0 ? e->knob_panel_mb * (1 << 20) : (cols <= 32 ? 0.75 : 0.6) * l2;
+    const int64_t p = std::min<int64_t>(static_cast<int64_t>((b_bytes + panel - 1) / panel), e->nnz / std::max<int64_t>(1, 6 * e->M));
     return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(p, 4)));
 }
 
@@ -423,23 +432,22 @@ int carve_arena(sddmm_b200_engine *e, bool coo, int n_items, bool allow_padding)
     const size_t o_coo = coo ? c.take(nnz * 4 + 16) : 0;
     const size_t o_gok = c.take(M / 2 + 4);   // one byte per row group (groups of >= 2 rows, plus the leading partial group)
     // row-segment path: unit list (upper bound: one unit per 8 nonzeros plus one ragged unit per row and panel), scan scratch
-    e->seg_slices = choose_k_slices(e);
-    e->panels = choose_panels(e);
-    e->long_rows = choose_long_rows(e);              // > 0: e->panels column panels for the long rows (still to be confirmed by the row statistics)
-    e->panel_cols = static_cast<int32_t>((N + e->panels - 1) / e->panels);
-    size_t runs = std::min(M * static_cast<size_t>(e->panels), nnz);
-    if (e->long_rows > 0) {
-        // a run per short row, and per panel for at most nnz / long_rows long rows
-        runs = std::min(M + std::min(nnz / static_cast<size_t>(e->long_rows), M) * static_cast<size_t>(e->panels), nnz);
-        e->panels += 1;                              // the short rows, whole, as the last entry of the list
+    choose_k_slices(e);
+    choose_long_rows(e);
+    e->panels_plain = choose_panels(e);
+    size_t runs = std::min(M * static_cast<size_t>(e->panels_plain), nnz);
+    size_t entries = M * static_cast<size_t>(e->panels_plain);
+    if (e->long_threshold > 0) {   // a run per short row, and per panel for at most nnz / long_threshold long rows
+        runs = std::max(runs, std::min(M + std::min(nnz / static_cast<size_t>(e->long_threshold), M) * static_cast<size_t>(e->panels_long), nnz));
+        entries = std::max(entries, M * static_cast<size_t>(e->panels_long + 1));
     }
+    const bool any_panels = e->panels_plain > 1 || e->long_threshold > 0;
     e->unit_cap = static_cast<int64_t>(nnz / 8 + runs + 8);
-    const size_t scan_n = M * static_cast<size_t>(e->panels);
     const size_t o_units = c.take(static_cast<size_t>(e->unit_cap + 8) * sizeof(int4));   // (row groups use 16-byte headers)
     const size_t o_ucols = c.take(static_cast<size_t>(e->unit_cap + 8) * 32);
-    const size_t o_uval = e->panels > 1 ? c.take(static_cast<size_t>(e->unit_cap + 8) * 32) : 0;
+    const size_t o_uval = any_panels ? c.take(static_cast<size_t>(e->unit_cap + 8) * 32) : 0;
     const size_t o_uoff = c.take((M + 1) * 4);
-    const size_t o_stile = c.take((static_cast<size_t>(std::max(unit_tiles(static_cast<int64_t>(scan_n)), unit_tiles(e->M))) + M / kScanTile + 2) * 4);
+    const size_t o_stile = c.take((static_cast<size_t>(std::max(unit_tiles(static_cast<int64_t>(entries)), unit_tiles(e->M))) + M / kScanTile + 2) * 4);
     // dense-tile path: only carved when the mode, K and the size of the 64x64 tile grid allow it
     e->tiles_per_row = static_cast<int32_t>((N + 63) / 64);
     e->tile_grid = static_cast<int64_t>((M + 63) / 64) * e->tiles_per_row;
@@ -485,7 +493,7 @@ int carve_arena(sddmm_b200_engine *e, bool coo, int n_items, bool allow_padding)
     e->d_Bx = split ? reinterpret_cast<float *>(b + o_bx) : nullptr;
     e->d_units = reinterpret_cast<int2 *>(b + o_units);
     e->d_unit_cols = reinterpret_cast<int32_t *>(b + o_ucols);
-    e->d_unit_sval = e->panels > 1 ? reinterpret_cast<float *>(b + o_uval) : nullptr;
+    e->d_unit_sval = any_panels ? reinterpret_cast<float *>(b + o_uval) : nullptr;
     e->d_Ap = padded ? reinterpret_cast<float *>(b + o_Ap) : nullptr;
     e->d_Bp = padded ? reinterpret_cast<float *>(b + o_Bp) : nullptr;
     e->d_unit_off = reinterpret_cast<int32_t *>(b + o_uoff);
@@ -797,16 +805,26 @@ RowSegFn pick_rowseg_bf16(int64_t Ks) {
     if (Ks <= 192) return sddmm_rowseg_bf16_kernel<3, 32, 4, 1, COPIES>;
     return sddmm_rowseg_bf16_kernel<4, 32, 2, 1, COPIES>;
 }
+// a slice of K (`add`: to what the earlier slices have written)
+RowSegFn pick_rowseg_slice(const sddmm_b200_engine *e, bool copies, bool add) {
+    if (e->slice_cols == 128) {
+        if (!copies && static_cast<double>(e->N) * 512.0 > e->l2_bytes) return add ? sddmm_rowseg_wide_kernel<4, true> : sddmm_rowseg_wide_kernel<4, false>;
+        if (add) return copies ? sddmm_rowseg_kernel<4, true, true> : sddmm_rowseg_kernel<4, false, true>;
+        return copies ? sddmm_rowseg_kernel<4, true, false> : sddmm_rowseg_kernel<4, false, false>;
+    }
+    if (add) return copies ? sddmm_rowseg_kernel<2, true, true> : sddmm_rowseg_kernel<2, false, true>;
+    return copies ? sddmm_rowseg_kernel<2, true, false> : sddmm_rowseg_kernel<2, false, false>;
+}
 // The row-segment kernel instantiation for this engine's storage and K (`copies`: S values from the per-unit copies).
 RowSegFn seg_function(const sddmm_b200_engine *e, bool copies) {
     if (e->mode == SDDMM_B200_BF16) return copies ? pick_rowseg_bf16<true>(e->Ks) : pick_rowseg_bf16<false>(e->Ks);
-    if (e->seg_slices > 1) return copies ? sddmm_rowseg_kernel<2, true, true> : sddmm_rowseg_kernel<2, false, true>;   // a 64-column slice
+    if (e->seg_slices > 1) return pick_rowseg_slice(e, copies, true);
     const int pieces = static_cast<int>((e->Ks + 31) / 32);
     // whole rows of a B that does not fit L2, without panels (rows too short for them): the order that DRAM likes
     if (!copies && static_cast<double>(e->N) * e->Ks * 4.0 > e->l2_bytes) {
-        if (pieces == 4) return sddmm_rowseg_wide_kernel<4>;
-        if (pieces == 6) return sddmm_rowseg_wide_kernel<6>;
-        if (pieces == 8) return sddmm_rowseg_wide_kernel<8>;
+        if (pieces == 4) return sddmm_rowseg_wide_kernel<4, false>;
+        if (pieces == 6) return sddmm_rowseg_wide_kernel<6, false>;
+        if (pieces == 8) return sddmm_rowseg_wide_kernel<8, false>;
     }
     return copies ? pick_rowseg<true>(pieces) : pick_rowseg<false>(pieces);
 }
@@ -954,24 +972,28 @@ int enqueue_unit_list(sddmm_b200_engine *e, int32_t panels, bool have_sums, bool
 }
 
 // Row segments over the whole matrix.  built: panels of the list that is already there (0: none), counted in pc.
-int build_rowseg_plan(sddmm_b200_engine *e, PlanCounters pc, int32_t built) {
+int build_rowseg_plan(sddmm_b200_engine *e, PlanCounters pc, bool built) {
     e->seg_copies = false;
     e->n_units = 0;
     if (!e->use_seg) return SDDMM_B200_OK;
-    int32_t panels = pc.unsorted_cols ? 1 : e->panels;   // a panel run is a contiguous piece of a row only when its columns are sorted
-    if (panels == 1) e->long_rows = 0;
-    if (e->long_rows > 0 && e->knob_long_rows < 0) {
-        // panels for the long rows only pay when those rows hold a good share of the nonzeros
+    // (a panel run is a contiguous piece of a row only when its columns are sorted)
+    bool use_long = e->long_threshold > 0 && !pc.unsorted_cols;
+    if (use_long && e->knob_long_rows < 0) {   // panels for the long rows only pay when those rows hold a good share of the nonzeros
         unsigned long long in_long = 0;
-        for (int b = 0; b < SDDMM_B200_HIST_BINS; ++b)
-            if (b >= 1 && (1ll << (b - 1)) >= e->long_rows) in_long += pc.hist_nnz[b];
-        if (5 * in_long < 2 * static_cast<unsigned long long>(e->nnz)) {   // < 40 %: every row whole, one pass
-            e->long_rows = 0;
-            panels = 1;
-            if (e->knob_k_slices < 0 && e->K <= 256) e->seg_slices = 1;
-        }
+        for (int b = 1; b < SDDMM_B200_HIST_BINS; ++b)
+            if ((1ll << (b - 1)) >= e->long_threshold) in_long += pc.hist_nnz[b];
+        use_long = 5 * in_long >= 2 * static_cast<unsigned long long>(e->nnz);   // 40 %
     }
-    if (built != panels) {
+    const int32_t cut = pc.unsorted_cols ? 1 : use_long ? e->panels_long : e->panels_plain;
+    const int32_t panels = use_long ? cut + 1 : cut;   // (the short rows, whole, are the last entry of the list)
+    e->long_rows = use_long ? e->long_threshold : 0;
+    e->panel_cols = static_cast<int32_t>((e->N + cut - 1) / cut);
+    if (e->knob_k_slices < 0 && e->K <= 256) {
+        if (use_long && long_rows_whole(e)) e->seg_slices = 1;
+        // slices of 64 that do not fit L2 and get no panels either: whole rows
+        if (!use_long && panels == 1 && e->slice_cols == 64 && e->nnz < 16 * e->M && gathered_bytes(e, 64) > e->l2_bytes) e->seg_slices = 1;
+    }
+    if (!built || panels > 1) {
         if (int rc = enqueue_unit_list(e, panels, false)) return rc;
         if (int rc = read_counters(e, &pc)) return rc;
     }
@@ -1008,8 +1030,9 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     // What will most likely run is enqueued before anything is read back: the plain or panel-major unit list (not where
     // tiles, or the row statistics, decide first) and the sample that looks for row groups.
     const bool tiles_first = e->dense_possible && e->mode != SDDMM_B200_FP32;   // (fp32 mode: tiles are the exception)
-    const bool whole_rows = e->use_seg && !tiles_first && e->panels == 1;
-    bool early_list = e->use_seg && !tiles_first && e->long_rows == 0 && e->nnz > 0;
+    const bool no_panels = e->panels_plain == 1 && e->long_threshold == 0;   // (else the row statistics decide first)
+    const bool whole_rows = e->use_seg && !tiles_first && no_panels;
+    bool early_list = whole_rows && e->nnz > 0;
     k_row_stats<<<unit_tiles(e->M), kUnitBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, e->d_rowstart,
                                                                                             whole_rows ? e->d_scan_tiles : nullptr, e->d_pc);
     if (e->nnz > 0) {
@@ -1026,10 +1049,10 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         if (group_possible(e))
             if (int rc = enqueue_group_sample(e)) return rc;
         if (early_list)
-            if (int rc = enqueue_unit_list(e, e->panels, whole_rows, e->dense_possible && e->knob_offset_tiles <= 0)) return rc;
+            if (int rc = enqueue_unit_list(e, 1, true, e->dense_possible && e->knob_offset_tiles <= 0)) return rc;
     }
     CU_TRY(e, cudaGetLastError());
-    if (join_copies && !tiles_first && e->panels == 1) {
+    if (join_copies && !tiles_first && no_panels) {
         CU_TRY(e, cudaStreamWaitEvent(s, e->ev_h2d, 0));
         if (int rc = convert_storage(e)) return rc;
         e->copies_joined = true;
@@ -1078,7 +1101,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         if (st) return st;
         if (e->rg_rows) return SDDMM_B200_OK;
         // (a grouping that was tried and dropped has used the list's memory)
-        st = build_rowseg_plan(e, pc, early_list && !e->group_tried ? (pc.unsorted_cols && e->panels > 1 ? 0 : e->panels) : 0);
+        st = build_rowseg_plan(e, pc, early_list && !e->group_tried);
         if (st) return st;
         if (e->use_seg) return SDDMM_B200_OK;
     }
@@ -1232,13 +1255,12 @@ int launch_rowseg(sddmm_b200_engine *e, cudaStream_t stream, float *p_val) {
     g.row_stride = static_cast<uint32_t>(e->Ks * elem_bytes(e));
     g.row_bytes = seg_row_bytes(e);
     if (int st = begin_kernel(e, stream)) return st;
-    if (e->seg_slices > 1) {   // one launch per 64-column slice of K, in stream order: each adds to what the earlier ones wrote
-        const RowSegFn first = e->seg_copies ? sddmm_rowseg_kernel<2, true, false> : sddmm_rowseg_kernel<2, false, false>;
-        g.row_bytes = 256;
+    if (e->seg_slices > 1) {   // one launch per slice of K, in stream order: each adds to what the earlier ones wrote
+        g.row_bytes = 4 * e->slice_cols;
         for (int sl = 0; sl < e->seg_slices; ++sl) {
-            (sl ? seg_function(e, e->seg_copies) : first)<<<p.rowseg_grid, kRowSegWarps * 32, 0, stream>>>(g);
-            g.A = static_cast<const float *>(g.A) + 64;
-            g.B = static_cast<const float *>(g.B) + 64;
+            pick_rowseg_slice(e, e->seg_copies, sl > 0)<<<p.rowseg_grid, kRowSegWarps * 32, 0, stream>>>(g);
+            g.A = static_cast<const float *>(g.A) + e->slice_cols;
+            g.B = static_cast<const float *>(g.B) + e->slice_cols;
         }
     } else {
         seg_function(e, e->seg_copies)<<<p.rowseg_grid, kRowSegWarps * 32, 0, stream>>>(g);

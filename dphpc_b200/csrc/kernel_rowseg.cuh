@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
 // bound, and it likes few rows open at a time.  The stages go through all pieces of 4 slots, two pieces of 128 bytes at a
 // time, before the other 4: half the rows in flight, twice the bytes of each.  9 M nonzeros in rows of 13, B 358 / 717 MB:
 // K = 128 697 -> 638 us, K = 256 1581 -> 1559; with B in L2 the order above is faster (K = 128 385 against 414).
-template <int NP>
+template <int NP, bool ACC>
 __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_wide_kernel(const RowSegArgs args) {
     const int lane = threadIdx.x & 31;
     const int t = lane & 3;
@@ -259,6 +259,9 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_wide_kernel
         const float *sv = args.s_val + un.x;
         const float s0 = __ldcs(sv + min(t, un.y & 7));
         const float s1 = __ldcs(sv + min(t + 4, un.y & 7));
+        float p0 = 0.f, p1 = 0.f;
+        if (ACC && t <= count) p0 = __ldcs(args.p_val + un.x + t);
+        if (ACC && t + 4 <= count) p1 = __ldcs(args.p_val + un.x + t + 4);
         const int2 un_next2 = load_unit(next + n_warps);
         const Cols8 cols_next = load_cols(next);
         float acc[8];
@@ -281,8 +284,8 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_wide_kernel
                 a[1] = a_next[1];
             }
         const float2 dot = group4_transpose_reduce(acc, t);
-        if (t <= count) __stcs(args.p_val + un.x + t, dot.x * s0);
-        if (t + 4 <= count) __stcs(args.p_val + un.x + t + 4, dot.y * s1);
+        if (t <= count) __stcs(args.p_val + un.x + t, ACC ? fmaf(dot.x, s0, p0) : dot.x * s0);
+        if (t + 4 <= count) __stcs(args.p_val + un.x + t + 4, ACC ? fmaf(dot.y, s1, p1) : dot.y * s1);
 
         if (next >= n_steps) break;   // warp-uniform
         b = next;

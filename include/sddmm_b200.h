@@ -182,11 +182,12 @@ int sddmm_b200_get_plan(sddmm_b200_engine *e, sddmm_b200_plan_info *info);
  *   "b_fraction"    with column panels the gathers of B carry an L2 evict_last hint: share of the lines it applies to, (0, 1]
  *   "group_units"   0: rows with identical column lists run the warp-per-group kernel instead of shared segments
  *   "offset_tiles"  0: dense tiles only on the 64-grid, 1: always also look for half-full 64x64 windows at arbitrary offsets
- *   "k_slices"      fp32 storage, K >= 128 and a multiple of 64: 1 = take K in slices of 64 columns (one launch each over the same
- *                   segment list, adding to P.val; default when B is about as large as the L2 or larger), 0 = never
- *   "long_rows"     rows too short for column panels on average but B far larger than L2: column panels for the rows of at
- *                   least this many nonzeros only, the shorter rows follow whole (default: 64 or 128, chosen with the number
- *                   of panels, when such rows hold at least 40 % of the nonzeros); 0 = never
+ *   "k_slices"      fp32 storage: 1 = take K (K >= 128 and a multiple of 64) in slices of 64 columns, 128 = of 128 columns (K a multiple of
+ *                   128), one launch each over the same segment list, adding to P.val (default, by K and size, when B is about as
+ *                   large as the L2 or larger), 0 = never
+ *   "long_rows"     B larger than L2: column panels for the rows of at least this many nonzeros only, the shorter rows follow
+ *                   whole (default: 64 or 128, chosen with the number of panels, when such rows hold at least 40 % of the
+ *                   nonzeros); 0 = never
  *   "dense_split3"  fp32-grade mode on dense tiles: 1 = operands through three shared-memory slots and two accumulators in
  *                   tensor memory (default for K >= 64), 0 = one A block + one B block like the other modes */
 int sddmm_b200_set_knob(sddmm_b200_engine *e, const char *name, double value);
