@@ -1429,6 +1429,7 @@ int sddmm_b200_create(sddmm_b200_engine **out, int device, int mode, uint32_t fl
     e->knob_long_rows = env_double("SDDMM_B200_LONG_ROWS", -1);
     DeviceGuard g(device);
     DevicePool::instance().add_user(device);
+    PinnedPool::instance().add_user();
     bool ok = g.ok;
     ok = ok && cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&e->side_stream, cudaStreamNonBlocking) == cudaSuccess;
@@ -1468,6 +1469,7 @@ int sddmm_b200_destroy(sddmm_b200_engine *e) {
         DevicePool::instance().remove_user(e->device);
         e->stager.release();
         e->stager2.release();
+        PinnedPool::instance().remove_user();
         if (e->b_stage) cudaFree(e->b_stage);
         if (e->ev_stage) cudaEventDestroy(e->ev_stage);
         if (e->ev_spmm0) cudaEventDestroy(e->ev_spmm0);
@@ -1734,9 +1736,7 @@ int sddmm_b200_stage_b(sddmm_b200_engine **engines, int n, int64_t N, int64_t K,
         if (!g.ok) return fail(e, SDDMM_B200_ERR_COMM, "device %d cannot be selected", e->device);
         e->b_stage_n = e->b_stage_k = 0;
         if (e->b_stage_cap < bytes) {
-            e->stager.release();
-        e->stager2.release();
-        if (e->b_stage) cudaFree(e->b_stage);
+            if (e->b_stage) cudaFree(e->b_stage);
             e->b_stage = nullptr;
             e->b_stage_cap = 0;
             void *p = nullptr;

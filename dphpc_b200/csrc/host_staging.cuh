@@ -167,6 +167,60 @@ inline void parallel_memcpy(void *dst, const void *src, size_t bytes, bool strea
     });
 }
 
+// Pinned buffers outlive the engine that asked for them (allocating one takes 0.3 ms at best and tens of ms on a busy host):
+// at most kMost are kept, and the last engine gives them all back.  A buffer is returned only when its copies have finished.
+class PinnedPool {
+public:
+    static constexpr size_t kMost = 12;   // two rings of two engines
+    static PinnedPool &instance() {
+        static PinnedPool *pool = new PinnedPool();   // (never destroyed: engines of static storage may end after it would be)
+        return *pool;
+    }
+    void add_user() {
+        std::lock_guard<std::mutex> lock(mu_);
+        ++users_;
+    }
+    void remove_user() {
+        std::lock_guard<std::mutex> lock(mu_);
+        if (--users_ > 0) return;
+        for (char *p : free_) cudaFreeHost(p);
+        free_.clear();
+    }
+    char *take(size_t bytes) {
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            if (bytes == size_ && !free_.empty()) {
+                char *p = free_.back();
+                free_.pop_back();
+                return p;
+            }
+        }
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return static_cast<char *>(p);
+    }
+    void put(char *p, size_t bytes) {
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            if (free_.empty()) size_ = bytes;   // (one size at a time: that of the last ring)
+            if (users_ > 0 && bytes == size_ && free_.size() < kMost) {
+                free_.push_back(p);
+                return;
+            }
+        }
+        cudaFreeHost(p);
+    }
+
+private:
+    std::mutex mu_;
+    std::vector<char *> free_;
+    size_t size_ = 0;
+    int users_ = 0;
+};
+
 // a ring of pinned buffers of one engine
 struct HostStager {
     // bytes per piece (= size of each pinned buffer); SDDMM_B200_STAGE_MB overrides the 4 MiB default (1 .. 256).
@@ -183,24 +237,33 @@ struct HostStager {
     char *buf[kRing] = {};
     cudaEvent_t ev[kRing] = {};
     bool busy[kRing] = {};
-    int next = 0;   // buffer the next piece takes
+    int last = kRing - 1;   // buffer the last piece took
 
-    bool ready() {
-        if (buf[0]) return true;
-        for (int i = 0; i < kRing; ++i) {
-            if (cudaHostAlloc(reinterpret_cast<void **>(&buf[i]), kPiece, cudaHostAllocDefault) != cudaSuccess ||
-                cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming) != cudaSuccess) {
-                cudaGetLastError();
-                release();
-                return false;
-            }
+    // buffer b of the ring, allocated when it is first used
+    bool ready(int b) {
+        if (!buf[b]) buf[b] = PinnedPool::instance().take(kPiece);
+        if (!ev[b] && cudaEventCreateWithFlags(&ev[b], cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            ev[b] = nullptr;
         }
-        return true;
+        return buf[b] && ev[b];
+    }
+    // the buffer for the next piece: one whose copy has finished if the ring has one (an engine of small copies then pins one
+    // buffer, not three: pinning 4 MiB costs 1 to 3 ms), else the next of the ring
+    int idle() {
+        for (int i = 0; i < kRing; ++i) {
+            const int b = (last + i) % kRing;
+            if (busy[b] && cudaEventQuery(ev[b]) == cudaSuccess) busy[b] = false;
+            if (buf[b] && !busy[b]) return last = b;
+        }
+        cudaGetLastError();   // (cudaErrorNotReady)
+        return last = (last + 1) % kRing;
     }
     void release() {
         for (int i = 0; i < kRing; ++i) {
+            if (ev[i]) cudaEventSynchronize(ev[i]);
             if (ev[i]) cudaEventDestroy(ev[i]);
-            if (buf[i]) cudaFreeHost(buf[i]);
+            if (buf[i]) PinnedPool::instance().put(buf[i], kPiece);
             ev[i] = nullptr;
             buf[i] = nullptr;
             busy[i] = false;
@@ -217,11 +280,11 @@ struct HostStager {
 
     // host -> device on `stream`; the caller's buffer is free when this returns if it was staged
     cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t stream) {
-        if (bytes < kMinStaged || !pageable(src) || !ready()) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream);
+        if (bytes < kMinStaged || !pageable(src)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream);
         for (size_t off = 0; off < bytes; off += kPiece) {
             const size_t len = std::min(kPiece, bytes - off);
-            const int b = next;
-            next = (next + 1) % kRing;
+            const int b = idle();
+            if (!ready(b)) return cudaMemcpyAsync(static_cast<char *>(dst) + off, static_cast<const char *>(src) + off, bytes - off, cudaMemcpyHostToDevice, stream);
             if (busy[b]) {
                 const cudaError_t st = cudaEventSynchronize(ev[b]);
                 if (st != cudaSuccess) return st;
@@ -236,14 +299,16 @@ struct HostStager {
     }
     // device -> host on `stream`; returns when the caller's buffer is filled (the stream has drained up to the copy)
     cudaError_t download(void *dst, const void *src, size_t bytes, cudaStream_t stream) {
-        if (bytes < kMinStaged || !pageable(dst) || !ready()) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream);
+        const size_t pieces = (bytes + kPiece - 1) / kPiece;
+        bool staged = bytes >= kMinStaged && pageable(dst);
+        for (int b = 0; staged && b < kRing && static_cast<size_t>(b) < pieces; ++b) staged = ready(b);
+        if (!staged) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream);
         for (int b = 0; b < kRing; ++b)
             if (busy[b]) {
                 const cudaError_t st = cudaEventSynchronize(ev[b]);
                 if (st != cudaSuccess) return st;
                 busy[b] = false;
             }
-        const size_t pieces = (bytes + kPiece - 1) / kPiece;
         auto enqueue = [&](size_t c) -> cudaError_t {
             const size_t off = c * kPiece, len = std::min(kPiece, bytes - off);
             cudaError_t st = cudaMemcpyAsync(buf[c % kRing], static_cast<const char *>(src) + off, len, cudaMemcpyDeviceToHost, stream);

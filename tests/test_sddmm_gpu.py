@@ -906,3 +906,19 @@ def test_rows_of_a_b_larger_than_the_cache(oracle, K, nnz_per_row):
             p = check(e, "fp32", oracle, M, N, K, rp, ci, sv, A, B, what=f"large B K={K} slices {slices}")
             e.run()
             assert np.array_equal(e.download(), p)
+
+
+@pytest.mark.parametrize("nnz", [(1 << 17) - 1, 1 << 17, (1 << 20) - 1, 1 << 20, (1 << 20) + 1, 3 * (1 << 20) + 5])
+def test_staged_host_copies_at_the_edges_of_a_piece(oracle, nnz):
+    """Pageable buffers go through pinned pieces of 4 MiB from 512 KiB on; the pieces pass from one engine to the next."""
+    M, N, K = 1024, nnz // 1024 + 7, 4
+    rng = np.random.default_rng(nnz)
+    rp = (np.arange(M + 1, dtype=np.int64) * nnz // M).astype(np.int32)
+    ci = np.concatenate([np.arange(b - a) for a, b in zip(rp[:-1], rp[1:])]).astype(np.int32)
+    sv = rng.uniform(-1, 1, nnz).astype(np.float32)
+    A, B = rng.uniform(-1, 1, (M, K)).astype(np.float32), rng.uniform(-1, 1, (N, K)).astype(np.float32)
+    for _ in range(2):
+        with Engine(0, "fp32") as e1, Engine(0, "fp32") as e2:
+            p1 = check(e1, "fp32", oracle, M, N, K, rp, ci, sv, A, B, what=f"nnz={nnz}")
+            p2 = check(e2, "fp32", oracle, M, N, K, rp, ci, 2 * sv, A, B, what=f"nnz={nnz}, second engine")
+            assert np.array_equal(2 * p1, p2)
