@@ -369,23 +369,33 @@ int choose_panels(const sddmm_b200_engine *e) {
     const int64_t cols = e->seg_slices > 1 ? e->slice_cols : e->Ks;
     const double b_bytes = gathered_bytes(e, cols);
     const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20);
-    if (b_bytes <= l2 || e->nnz < 16 * e->M) return 1;   // (rows too short on average)
+    const double mean = static_cast<double>(e->nnz) / std::max<double>(1.0, static_cast<double>(e->M));
+    const bool bf = e->mode == SDDMM_B200_BF16;
+    // Rows too short on average.  The longer a row of B, the more a gather that misses L2 costs against a half-empty segment.  Poisson
+    // rows, without / with 2 panels: K = 32, B 186 MB, mean 11 / 13 / 15: 282 / 290, 324 / 320, 368 / 353 us; K = 64, B 371 MB, mean
+    // 9 / 11 / 13 / 15: 524 / 537, 619 / 607, 723 / 685, 839 / 768; K = 96, B 346 MB, mean 10 / 13: 601 / 538, 779 / 655.
+    if (b_bytes <= l2 || mean < (bf ? 16.0 : cols <= 32 ? 13.0 : cols <= 64 ? 11.0 : 9.0)) return 1;
+    // Slices of 128 columns: panels that fit L2 one by one, if an average row has 3 nonzeros for each, or none.  Sustained, B 205 MB,
+    // mean 10, 1 / 2 panels: 577 / 527 us; 358 MB, 9.6, 1 / 2 / 3: 1158 / 1174 / 1122; 461 MB, 9.5: 1549 / 1659 / 1640, 12, 1 / 2 / 3 / 4:
+    // 2006 / 1999 / 1905 / 1859.
+    if (cols == 128 && e->seg_slices > 1 && mean < 16.0) {
+        const double need = std::ceil(b_bytes / l2);
+        return 3.0 * need > mean || need > 4.0 ? 1 : static_cast<int>(need);
+    }
     // bf16 storage, measured with 1.45 M rows of B: K = 64 (B 1.5 x L2) 590 / 618 / 634 us with 1 / 2 / 3 panels, K = 128 (3 x L2)
     // 1809 / 1142 / 1092 / 1096 / 1150 us with 1 .. 5
-    if (e->mode == SDDMM_B200_BF16) {
+    if (bf) {
         if (b_bytes <= 2.0 * l2) return 1;
         return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(static_cast<int64_t>(std::ceil(b_bytes / l2)), e->nnz / std::max<int64_t>(1, 8 * e->M)), 4)));
     }
     // measured on B200 (126 MB of L2): a run shorter than a segment wastes gather slots, so panels of about 96 MB for rows of one
     // piece (B 186 MB: 2 / 3 panels 507 / 514 us), 80 MB for longer rows, where a slot's waste weighs less against its row
-    // (K = 64, B 179 MB: 428 / 414 us, B 372 MB: 3 / 4 panels 1138 / 1116); at most one panel per 6 nonzeros of an average row,
+    // (K = 64, B 179 MB: 428 / 414 us, B 372 MB: 3 / 4 panels 1138 / 1116); at most 2, or one per 6 nonzeros of an average row,
     // and never more than 4 (5: 3 % slower)
     const double panel = e->knob_panel_mb > 0 ? e->knob_panel_mb * (1 << 20) : (cols <= 32 ? 0.75 : 0.6) * l2;
-    const int64_t p = std::min<int64_t>(static_cast<int64_t>((b_bytes + panel - 1) / panel), e->nnz / std::max<int64_t>(1, 6 * e->M));
-    return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(p, 4)));
+    return static_cast<int>(std::min(std::ceil(b_bytes / panel), std::min(4.0, std::max(2.0, std::floor(mean / 6.0)))));
 }
 
-// Lay out the arena for the current dimensions and point the views into it.
 // Which inputs the row-segment kernels take (the scalar and the row-tile kernel are left with the rest): K below 8 that is
 // no multiple of 4 stays with the scalar kernel, a padded row would be several times the real one.
 bool seg_possible(const sddmm_b200_engine *e) {
@@ -404,6 +414,7 @@ int64_t padded_row(const sddmm_b200_engine *e) {
     return (K + line - 1) / line * line;
 }
 
+// Lay out the arena for the current dimensions and point the views into it.
 int carve_arena(sddmm_b200_engine *e, bool coo, int n_items, bool allow_padding) {
     Carve c;
     e->use_seg = seg_possible(e) && (allow_padding || (e->K % 8 == 0 && e->K <= 256));
@@ -812,6 +823,7 @@ RowSegFn pick_rowseg_slice(const sddmm_b200_engine *e, bool copies, bool add) {
         if (add) return copies ? sddmm_rowseg_kernel<4, true, true> : sddmm_rowseg_kernel<4, false, true>;
         return copies ? sddmm_rowseg_kernel<4, true, false> : sddmm_rowseg_kernel<4, false, false>;
     }
+    if (!copies && static_cast<double>(e->N) * 256.0 > e->l2_bytes) return add ? sddmm_rowseg_wide_kernel<2, true> : sddmm_rowseg_wide_kernel<2, false>;
     if (add) return copies ? sddmm_rowseg_kernel<2, true, true> : sddmm_rowseg_kernel<2, false, true>;
     return copies ? sddmm_rowseg_kernel<2, true, false> : sddmm_rowseg_kernel<2, false, false>;
 }
@@ -822,6 +834,7 @@ RowSegFn seg_function(const sddmm_b200_engine *e, bool copies) {
     const int pieces = static_cast<int>((e->Ks + 31) / 32);
     // whole rows of a B that does not fit L2, without panels (rows too short for them): the order that DRAM likes
     if (!copies && static_cast<double>(e->N) * e->Ks * 4.0 > e->l2_bytes) {
+        if (pieces == 2) return sddmm_rowseg_wide_kernel<2, false>;
         if (pieces == 4) return sddmm_rowseg_wide_kernel<4, false>;
         if (pieces == 6) return sddmm_rowseg_wide_kernel<6, false>;
         if (pieces == 8) return sddmm_rowseg_wide_kernel<8, false>;
@@ -833,6 +846,7 @@ int seg_grid(sddmm_b200_engine *e, const void *fn, int warps, int per_step, int6
     int occ = 0;
     CU_TRY(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, warps * 32, 0));
     if (occ < 1) return fail(e, SDDMM_B200_ERR_CUDA, "row-segment kernel does not fit on an SM");
+    if (const char *v = std::getenv("SEGOCC")) occ = std::min(occ, std::atoi(v));
     const int64_t steps = (n_units + per_step - 1) / per_step;
     *grid = static_cast<int32_t>(std::min<int64_t>((steps + warps - 1) / warps, static_cast<int64_t>(e->sm_count) * occ));
     return SDDMM_B200_OK;
@@ -984,7 +998,17 @@ int build_rowseg_plan(sddmm_b200_engine *e, PlanCounters pc, bool built) {
             if ((1ll << (b - 1)) >= e->long_threshold) in_long += pc.hist_nnz[b];
         use_long = 5 * in_long >= 2 * static_cast<unsigned long long>(e->nnz);   // 40 %
     }
-    const int32_t cut = pc.unsorted_cols ? 1 : use_long ? e->panels_long : e->panels_plain;
+    int32_t plain = e->panels_plain;
+    if (plain > 1 && e->nnz < 16 * e->M && e->knob_panels < 1) {
+        // a mean that barely pays for panels has to be that of most rows, not of a few long ones: 60 % of them of 8 nonzeros or more
+        unsigned long long rows = 0, of_8 = 0;
+        for (int b = 1; b < SDDMM_B200_HIST_BINS; ++b) {
+            rows += pc.hist[b];
+            if (b >= 4) of_8 += pc.hist[b];
+        }
+        if (10 * of_8 < 6 * rows) plain = 1;
+    }
+    const int32_t cut = pc.unsorted_cols ? 1 : use_long ? e->panels_long : plain;
     const int32_t panels = use_long ? cut + 1 : cut;   // (the short rows, whole, are the last entry of the list)
     e->long_rows = use_long ? e->long_threshold : 0;
     e->panel_cols = static_cast<int32_t>((e->N + cut - 1) / cut);

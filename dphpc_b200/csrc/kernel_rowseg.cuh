@@ -210,10 +210,10 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
     }
 }
 
-// The same for whole rows (NP even, at least 4) of a B that does not fit L2 and is gathered without column panels: DRAM is the
+// The same for whole rows (NP even) of a B that does not fit L2 and is gathered without column panels: DRAM is the
 // bound, and it likes few rows open at a time.  The stages go through all pieces of 4 slots, two pieces of 128 bytes at a
 // time, before the other 4: half the rows in flight, twice the bytes of each.  9 M nonzeros in rows of 13, B 358 / 717 MB:
-// K = 128 697 -> 638 us, K = 256 1581 -> 1559; with B in L2 the order above is faster (K = 128 385 against 414).
+// K = 128 697 -> 638 us, K = 256 1581 -> 1559; 13 M nonzeros in rows of 9, B 373 MB: K = 64 558 -> 524; with B in L2 the order above is faster (K = 128 385 against 414).
 template <int NP, bool ACC>
 __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_wide_kernel(const RowSegArgs args) {
     const int lane = threadIdx.x & 31;

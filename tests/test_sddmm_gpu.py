@@ -922,3 +922,21 @@ def test_staged_host_copies_at_the_edges_of_a_piece(oracle, nnz):
             p1 = check(e1, "fp32", oracle, M, N, K, rp, ci, sv, A, B, what=f"nnz={nnz}")
             p2 = check(e2, "fp32", oracle, M, N, K, rp, ci, 2 * sv, A, B, what=f"nnz={nnz}, second engine")
             assert np.array_equal(2 * p1, p2)
+
+
+@pytest.mark.parametrize("K,nnz_per_row,panels", [(50, 9, 1), (64, 9, 1), (64, 13, 2), (96, 10, 2), (128, 13, 2), (256, 10, 2), (300, 9, 1)])
+def test_column_panels_of_short_rows(oracle, K, nnz_per_row, panels):
+    """B (a slice of it, where K is sliced) just larger than L2 and rows around the length from which column panels pay."""
+    rng = np.random.default_rng(K * nnz_per_row)
+    N = (136 << 20) // (4 * (128 if K == 256 else 64 if K in (50, 128, 300) else K)) + 7
+    M = 2003
+    lens = np.concatenate([np.full(M // 2, nnz_per_row), rng.integers(8, 2 * nnz_per_row - 7, M - M // 2)])
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = np.concatenate([np.unique(rng.integers(0, N, 2 * n + 8))[:n] for n in lens]).astype(np.int32)
+    sv = rng.uniform(-1, 1, ci.size).astype(np.float32)
+    A, B = rng.uniform(-1, 1, (M, K)).astype(np.float32), rng.random((N, K), np.float32) - np.float32(0.5)
+    with Engine(0, "fp32") as e:
+        check(e, "fp32", oracle, M, N, K, rp, ci, sv, A, B, what=f"K={K} rows of {nnz_per_row}")
+        assert e.plan()["rowseg_panels"] == panels
+        e.set_knob("panels", 3 - panels)   # the other form
+        check(e, "fp32", oracle, M, N, K, rp, ci, sv, A, B, what=f"K={K} rows of {nnz_per_row}, {3 - panels} panels")
