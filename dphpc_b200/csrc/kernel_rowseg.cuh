@@ -62,11 +62,6 @@ __device__ __forceinline__ Piece ld_piece(const unsigned char *p) {
                  : "l"(p));
     return r;
 }
-__device__ __forceinline__ float4 ld_part(const unsigned char *p) {
-    float4 v;
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
-}
 // ... that has L2 fetch the whole 256-byte block it lies in: the first of two pieces of a row that are wanted one after the other
 __device__ __forceinline__ Piece ld_piece_of_two(const unsigned char *p) {
     Piece r;
