@@ -377,10 +377,12 @@ int choose_panels(const sddmm_b200_engine *e) {
     if (b_bytes <= l2 || mean < (bf ? 16.0 : cols <= 32 ? 13.0 : cols <= 64 ? 11.0 : 9.0)) return 1;
     // Slices of 128 columns: panels that fit L2 one by one, if an average row has 3 nonzeros for each, or none.  Sustained, B 205 MB,
     // mean 10, 1 / 2 panels: 577 / 527 us; 358 MB, 9.6, 1 / 2 / 3: 1158 / 1174 / 1122; 461 MB, 9.5: 1549 / 1659 / 1640, 12, 1 / 2 / 3 / 4:
-    // 2006 / 1999 / 1905 / 1859.
-    if (cols == 128 && e->seg_slices > 1 && mean < 16.0) {
+    // 2006 / 1999 / 1905 / 1859; longer rows, 358 MB, 30, 3 / 4 / 5: 2390 / 2086 / 2084; 512 MB, 20, 4 / 5 / 6: 2836 / 2651 / 2834; 744 MB,
+    // 26, 4 / 5 / 6 / 7: 6027 / 5815 / 5538 / 5347.
+    if (cols == 128 && e->seg_slices > 1 && !bf) {
         const double need = std::ceil(b_bytes / l2);
-        return 3.0 * need > mean || need > 4.0 ? 1 : static_cast<int>(need);
+        if (mean < 16.0) return 3.0 * need > mean || need > 4.0 ? 1 : static_cast<int>(need);
+        return static_cast<int>(std::min(8.0, std::min(std::ceil(b_bytes / (0.8 * l2)), std::floor(mean / 3.5))));
     }
     // bf16 storage, measured with 1.45 M rows of B: K = 64 (B 1.5 x L2) 590 / 618 / 634 us with 1 / 2 / 3 panels, K = 128 (3 x L2)
     // 1809 / 1142 / 1092 / 1096 / 1150 us with 1 .. 5

@@ -62,6 +62,17 @@ __device__ __forceinline__ Piece ld_piece(const unsigned char *p) {
                  : "l"(p));
     return r;
 }
+// ... of A: used by one or two units, then not again before the rest of A has passed through, so it is the first to leave L2 and
+// B's rows stay.  20 M nonzeros in rows of 20, B 128 / 256 MB in panels: K = 32 271 -> 256 us, K = 64 567 -> 525; 37.5 M, rows of 26,
+// K = 32 511 -> 500, bf16 K = 128 1135 -> 1096.  (evict_last on the gathers of B adds nothing.)
+__device__ __forceinline__ Piece ld_piece_first(const unsigned char *p) {
+    Piece r;
+    asm volatile("ld.global.nc.L2::evict_first.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(r.v[0].x), "=f"(r.v[0].y), "=f"(r.v[1].x), "=f"(r.v[1].y), "=f"(r.v[2].x), "=f"(r.v[2].y), "=f"(r.v[3].x),
+                   "=f"(r.v[3].y)
+                 : "l"(p));
+    return r;
+}
 // ... that has L2 fetch the whole 256-byte block it lies in: the first of two pieces of a row that are wanted one after the other
 __device__ __forceinline__ Piece ld_piece_of_two(const unsigned char *p) {
     Piece r;
@@ -150,7 +161,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
     auto piece_offset = [&](int p) -> int { return p == NP - 1 ? o_last : 128 * p; };
     auto load_a = [&](int row, int p) -> Piece {
         const unsigned char *q = row_at(At + piece_offset(p), row, stride);
-        return ld_piece(p == NP - 1 && off ? reinterpret_cast<const unsigned char *>(g_zero_part) : q);
+        return ld_piece_first(p == NP - 1 && off ? reinterpret_cast<const unsigned char *>(g_zero_part) : q);
     };
 
     int2 un = load_unit(b), un_next = load_unit(b + n_warps);
@@ -232,8 +243,8 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_wide_kernel
     auto piece_offset = [&](int p) -> int { return p == NP - 1 ? o_last : 128 * p; };
     auto load_a = [&](Piece (&a)[2], int row, int q) {
         const unsigned char *r = row_at(At, row, stride);
-        a[0] = ld_piece(r + piece_offset(2 * q));
-        a[1] = ld_piece(2 * q + 1 == NP - 1 && off ? reinterpret_cast<const unsigned char *>(g_zero_part) : r + piece_offset(2 * q + 1));
+        a[0] = ld_piece_first(r + piece_offset(2 * q));
+        a[1] = ld_piece_first(2 * q + 1 == NP - 1 && off ? reinterpret_cast<const unsigned char *>(g_zero_part) : r + piece_offset(2 * q + 1));
     };
     auto load_b = [&](Piece (&x)[2], int col, int q) {
         const unsigned char *r = row_at(Bt, col, stride);
@@ -311,6 +322,13 @@ __device__ __forceinline__ void ld_frag(Frag<32> &f, const unsigned char *p) {
 __device__ __forceinline__ void ld_frag(Frag<16> &f, const unsigned char *p) {
     asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(f.r[0]), "=r"(f.r[1]), "=r"(f.r[2]), "=r"(f.r[3]) : "l"(p));
 }
+// (A, as above; the 16-byte form has no such qualifier)
+__device__ __forceinline__ void ld_frag_first(Frag<32> &f, const unsigned char *p) {
+    asm volatile("ld.global.nc.L2::evict_first.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(f.r[0]), "=r"(f.r[1]), "=r"(f.r[2]), "=r"(f.r[3]), "=r"(f.r[4]), "=r"(f.r[5]), "=r"(f.r[6]), "=r"(f.r[7])
+                 : "l"(p));
+}
+__device__ __forceinline__ void ld_frag_first(Frag<16> &f, const unsigned char *p) { ld_frag(f, p); }
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -346,7 +364,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, MINB) sddmm_rowseg_bf16_ker
     auto load_a = [&](Row &f, int row) {
         const unsigned char *q = row_at(At, row, stride);
 #pragma unroll
-        for (int p = 0; p < NP; ++p) ld_frag(f.p[p], p == NP - 1 && off ? reinterpret_cast<const unsigned char *>(g_zero_part) : q + piece_offset(p));
+        for (int p = 0; p < NP; ++p) ld_frag_first(f.p[p], p == NP - 1 && off ? reinterpret_cast<const unsigned char *>(g_zero_part) : q + piece_offset(p));
     };
     auto load_code = [&](int step) -> int { return __ldcs(&args.units[8 * static_cast<int64_t>(min(step, last_step)) + grp].y); };
     auto load_cols = [&](int step) -> Cols8 {   // slot grp of the step's 8 units
