@@ -155,6 +155,7 @@ struct sddmm_b200_engine {
     int64_t Ks = 0;
     float *d_Ap = nullptr, *d_Bp = nullptr;
     bool d_Ap_wanted = false;
+    bool slice_major = false;   // ... slice of K after slice of K, each of rows of slice_cols elements
     bool group_tried = false;          // a grouping was matched exactly and then dropped
     bool copies_joined = false;        // the upload's copies and conversions are already ordered before the plan's read-back
     int64_t unit_cap = 0;
@@ -313,6 +314,17 @@ double env_double(const char *name, double fallback) {
     return v ? std::atof(v) : fallback;
 }
 
+double gathered_bytes(const sddmm_b200_engine *e, int64_t cols) { return static_cast<double>(e->N) * static_cast<double>(cols) * static_cast<double>(elem_bytes(e)); }
+
+// K = 256 from B = 5 x L2 on, rows long enough for panels: slices of 64 that are stored one after the other, as matrices of 64 columns
+// of their own; side by side in rows of 1 KB the same slices take half as long again.  Sustained, B 0.7 / 1.0 / 1.5 GB, rows of 30 / 20 /
+// 26: slices of 128 side by side 2086 / 2651 / 5310 us, 64 side by side in the kernel before 2419 / 2852 / 5428, 64 one after the other
+// 1941 / 2360 / 4700 (of 128: 5360).  The re-ordered copies are made with every upload of A and B and cost about a fifth of a run.
+bool slices_apart(const sddmm_b200_engine *e) {
+    return e->mode != SDDMM_B200_BF16 && e->use_seg && e->knob_k_slices < 0 && e->Ks == 256 && e->nnz >= 16 * e->M &&
+           gathered_bytes(e, e->Ks) > 5.0 * (e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20));
+}
+
 // Large K, fp32 storage: K is taken in slices, one launch per slice over the same unit list, each adding to P.val, where that
 // makes a slice of B fit L2 (or leaves column panels room) when the whole rows do not.  Measured, whole / in slices of 64, with
 // B 1 / 1.3 / 1.4 / 2.7 times L2: K = 128 371 / 342, K = 192 438 / 355, K = 128 395 / 394 and 997 / 889 us; with B 0.5 times
@@ -320,6 +332,11 @@ double env_double(const char *name, double fallback) {
 // columns 925 / 1232 / 798, 518 / 493 / 420, 2378 / 2157 / 1987 us, and also with B in L2 when A is streamed (731 / 777 / 684).
 // Knob "k_slices": 0 = never, 1 = slices of 64 whenever K allows, 128 = of 128.
 void choose_k_slices(sddmm_b200_engine *e) {
+    if (e->slice_major) {
+        e->slice_cols = 64;
+        e->seg_slices = 4;
+        return;
+    }
     e->slice_cols = e->Ks % 128 == 0 && (e->knob_k_slices >= 128 || (e->knob_k_slices != 1 && e->Ks >= 256)) ? 128 : 64;
     e->seg_slices = 1;
     const int slices = static_cast<int>(e->Ks / e->slice_cols);
@@ -345,8 +362,6 @@ void choose_k_slices(sddmm_b200_engine *e) {
 //     short ones would fall into runs of one or two: 20 M nonzeros, 1 M rows, K = 64 532 us plain, 396 us; 35 M, 1.5 M rows,
 //     K = 32 480 / 370 us; 36 M, 2.6 M rows, K = 32 561 us without panels, 447 us.
 // Knob "long_rows": 0 = never, T >= 1 = threshold T with the panels that the "panels" knob or the rule gives.
-double gathered_bytes(const sddmm_b200_engine *e, int64_t cols) { return static_cast<double>(e->N) * static_cast<double>(cols) * static_cast<double>(elem_bytes(e)); }
-
 // (K = 128: where the long rows get panels the rows are taken whole, 565 us against 586 in two slices)
 bool long_rows_whole(const sddmm_b200_engine *e) { return e->seg_slices > 1 && e->Ks == 128 && e->knob_k_slices < 0; }
 
@@ -433,7 +448,9 @@ int carve_arena(sddmm_b200_engine *e, bool coo, int n_items, bool allow_padding)
     const size_t Ks = static_cast<size_t>(e->Ks);
     const size_t o_A16 = bf ? c.take(M * Ks * 2) : 0;
     const size_t o_B16 = bf ? c.take(N * Ks * 2) : 0;
-    const bool padded = !bf && e->use_seg && (e->Ks != e->K);
+    e->slice_major = allow_padding && slices_apart(e);
+    choose_k_slices(e);
+    const bool padded = !bf && e->use_seg && (e->Ks != e->K || e->slice_major);
     e->d_Ap_wanted = padded;
     const size_t o_Ap = padded ? c.take(M * Ks * 4) : 0;
     const size_t o_Bp = padded ? c.take(N * Ks * 4) : 0;
@@ -445,7 +462,6 @@ int carve_arena(sddmm_b200_engine *e, bool coo, int n_items, bool allow_padding)
     const size_t o_coo = coo ? c.take(nnz * 4 + 16) : 0;
     const size_t o_gok = c.take(M / 2 + 4);   // one byte per row group (groups of >= 2 rows, plus the leading partial group)
     // row-segment path: unit list (upper bound: one unit per 8 nonzeros plus one ragged unit per row and panel), scan scratch
-    choose_k_slices(e);
     choose_long_rows(e);
     e->panels_plain = choose_panels(e);
     size_t runs = std::min(M * static_cast<size_t>(e->panels_plain), nnz);
@@ -554,8 +570,8 @@ int convert_storage(sddmm_b200_engine *e) {
     }
     const int32_t K = static_cast<int32_t>(e->K), Ks = static_cast<int32_t>(e->Ks);
     if (e->d_Ap) {
-        k_pad_rows<<<grid_for(e->M * (Ks / 4), kBlock, cap), kBlock, 0, e->stream>>>(e->d_A32, e->d_Ap, e->M, K, Ks);
-        k_pad_rows<<<grid_for(e->N * (Ks / 4), kBlock, cap), kBlock, 0, e->stream>>>(e->d_B32, e->d_Bp, e->N, K, Ks);
+        k_pad_rows<<<grid_for(e->M * (Ks / 4), kBlock, cap), kBlock, 0, e->stream>>>(e->d_A32, e->d_Ap, e->M, K, Ks, e->slice_major ? e->slice_cols : Ks);
+        k_pad_rows<<<grid_for(e->N * (Ks / 4), kBlock, cap), kBlock, 0, e->stream>>>(e->d_B32, e->d_Bp, e->N, K, Ks, e->slice_major ? e->slice_cols : Ks);
         CU_TRY(e, cudaGetLastError());
     }
     if (e->mode != SDDMM_B200_BF16) return SDDMM_B200_OK;
@@ -1283,10 +1299,11 @@ int launch_rowseg(sddmm_b200_engine *e, cudaStream_t stream, float *p_val) {
     if (int st = begin_kernel(e, stream)) return st;
     if (e->seg_slices > 1) {   // one launch per slice of K, in stream order: each adds to what the earlier ones wrote
         g.row_bytes = 4 * e->slice_cols;
+        if (e->slice_major) g.row_stride = 4 * e->slice_cols;
         for (int sl = 0; sl < e->seg_slices; ++sl) {
             pick_rowseg_slice(e, e->seg_copies, sl > 0)<<<p.rowseg_grid, kRowSegWarps * 32, 0, stream>>>(g);
-            g.A = static_cast<const float *>(g.A) + e->slice_cols;
-            g.B = static_cast<const float *>(g.B) + e->slice_cols;
+            g.A = static_cast<const float *>(g.A) + e->slice_cols * (e->slice_major ? e->M : 1);
+            g.B = static_cast<const float *>(g.B) + e->slice_cols * (e->slice_major ? e->N : 1);
         }
     } else {
         seg_function(e, e->seg_copies)<<<p.rowseg_grid, kRowSegWarps * 32, 0, stream>>>(g);

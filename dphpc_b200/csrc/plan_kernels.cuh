@@ -517,8 +517,9 @@ __global__ void k_split_concat_tf32(const float *__restrict__ in, float *__restr
     }
 }
 
-// rows of K floats -> rows of Ks floats (a multiple of 8), zero-padded
-__global__ void k_pad_rows(const float *__restrict__ in, float *__restrict__ out, int64_t rows, int32_t K, int32_t Ks) {
+// rows of K floats -> rows of Ks floats (a multiple of 8), zero-padded; slice < Ks: slices of that many columns, all rows of one
+// before the next
+__global__ void k_pad_rows(const float *__restrict__ in, float *__restrict__ out, int64_t rows, int32_t K, int32_t Ks, int32_t slice) {
     const int32_t quads = Ks / 4;
     const int64_t n = rows * quads;
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -530,7 +531,8 @@ __global__ void k_pad_rows(const float *__restrict__ in, float *__restrict__ out
         v.y = k + 1 < K ? src[1] : 0.f;
         v.z = k + 2 < K ? src[2] : 0.f;
         v.w = k + 3 < K ? src[3] : 0.f;
-        reinterpret_cast<float4 *>(out)[i] = v;
+        const int32_t part = k / slice;
+        *reinterpret_cast<float4 *>(out + (part * rows + r) * slice + (k - part * slice)) = v;
     }
 }
 

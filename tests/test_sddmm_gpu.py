@@ -940,3 +940,23 @@ def test_column_panels_of_short_rows(oracle, K, nnz_per_row, panels):
         assert e.plan()["rowseg_panels"] == panels
         e.set_knob("panels", 3 - panels)   # the other form
         check(e, "fp32", oracle, M, N, K, rp, ci, sv, A, B, what=f"K={K} rows of {nnz_per_row}, {3 - panels} panels")
+
+
+@pytest.mark.parametrize("K", [250, 256])
+def test_slices_of_k_stored_one_after_the_other(oracle, K):
+    """B of more than five times L2 and rows that get panels; new values of A and B follow into the re-ordered copies."""
+    rng = np.random.default_rng(K)
+    M, N, n = 601, (640 << 20) // 1024 + 20001, 17
+    rp = (n * np.arange(M + 1)).astype(np.int32)
+    ci = np.concatenate([np.unique(rng.integers(0, N, 2 * n))[:n] for _ in range(M)]).astype(np.int32)
+    sv = rng.uniform(-1, 1, ci.size).astype(np.float32)
+    A, B = rng.uniform(-1, 1, (M, K)).astype(np.float32), rng.random((N, K), np.float32) - np.float32(0.5)
+    with Engine(0, "fp32") as e:
+        p = check(e, "fp32", oracle, M, N, K, rp, ci, sv, A, B, what=f"K={K}")
+        assert e.plan()["rowseg_passes"] == 4 and e.plan()["rowseg_panels"] == 2
+        e.update_dense(2 * A, B)
+        e.run()
+        assert np.array_equal(e.download(), 2 * p)
+        e.set_knob("k_slices", 128)
+        check(e, "fp32", oracle, M, N, K, rp, ci, sv, A, B, what=f"K={K} in slices of 128 side by side")
+        assert e.plan()["rowseg_passes"] == 2
