@@ -849,13 +849,19 @@ RowGroupFn pick_rowgroup(int rows, int cpl) {
 }
 
 using RowSegGroupFn = void (*)(const RowSegGroupArgs);
-template <int CPL>
+template <int LPR>
 RowSegGroupFn pick_rowseg_group_rows(int rows) {
-    return rows == 2 ? sddmm_rowseg_group_kernel<CPL, 2> : rows == 3 ? sddmm_rowseg_group_kernel<CPL, 3> : sddmm_rowseg_group_kernel<CPL, 4>;
+    return rows == 2 ? sddmm_rowseg_group_kernel<LPR, 2> : rows == 3 ? sddmm_rowseg_group_kernel<LPR, 3> : sddmm_rowseg_group_kernel<LPR, 4>;
 }
-// rows of 32 or 64 elements (nullptr: no instantiation)
+// rows of 32, 64, 128 or 256 elements (nullptr: no instantiation)
 RowSegGroupFn pick_rowseg_group(const sddmm_b200_engine *e, int rows) {
-    return e->Ks == 32 ? pick_rowseg_group_rows<1>(rows) : e->Ks == 64 ? pick_rowseg_group_rows<2>(rows) : nullptr;
+    switch (e->Ks) {
+        case 32: return pick_rowseg_group_rows<4>(rows);
+        case 64: return pick_rowseg_group_rows<8>(rows);
+        case 128: return pick_rowseg_group_rows<16>(rows);
+        case 256: return pick_rowseg_group_rows<32>(rows);
+        default: return nullptr;
+    }
 }
 
 using RowSegFn = void (*)(const RowSegArgs);
@@ -1005,7 +1011,7 @@ int build_rowgroup_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
         if (pc.units == 0 || pc.units > static_cast<unsigned long long>(std::min<int64_t>(e->unit_cap, kUnitLimit)))
             return fail(e, SDDMM_B200_ERR_CUDA, "row-group plan: %llu units for a list of %lld", pc.units, (long long)e->unit_cap);
         e->n_units = static_cast<int32_t>(pc.units);
-        if (int rc = seg_grid(e, reinterpret_cast<const void *>(pick_rowseg_group(e, best)), kRowSegWarps, 4, e->n_units, &p.rowgroup_grid)) return rc;
+        if (int rc = seg_grid(e, reinterpret_cast<const void *>(pick_rowseg_group(e, best)), kRowSegWarps, group_step_units(static_cast<int>(e->Ks / 8)), e->n_units, &p.rowgroup_grid)) return rc;
         p.rowseg_units = e->n_units;
         p.rowseg_panels = 1;
     } else {
@@ -1014,6 +1020,10 @@ int build_rowgroup_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
         CU_TRY(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kRowGroupWarps * 32, 0));
         if (occ < 1) return fail(e, SDDMM_B200_ERR_CUDA, "row-group kernel does not fit on an SM");
         p.rowgroup_grid = std::min((n_groups + kRowGroupWarps - 1) / kRowGroupWarps, e->sm_count * occ);
+    }
+    if (units && e->slice_major) {   // (whole rows here)
+        e->slice_major = false;
+        if (e->Ks == e->K) e->d_Ap = e->d_Bp = nullptr;
     }
     e->rg_rows = best;
     e->rg_first = best_first;
@@ -1437,9 +1447,9 @@ int launch_all(sddmm_b200_engine *e, float *p_val, cudaGraph_t graph = nullptr) 
     }
     if (e->rg_rows && e->rg_units) {
         RowSegGroupArgs g;
-        g.ghdr = reinterpret_cast<const int4 *>(e->d_units); g.col_idx = e->d_col; g.s_val = e->d_sval; g.p_val = p_val;
+        g.ghdr = reinterpret_cast<const int4 *>(e->d_units); g.unit_cols = e->d_unit_cols; g.s_val = e->d_sval; g.p_val = p_val;
         g.A = static_cast<const float *>(seg_rows_a(e)); g.B = static_cast<const float *>(seg_rows_b(e));
-        g.n_units = e->n_units; g.K = static_cast<int32_t>(e->Ks);
+        g.n_units = e->n_units;
         if ((st = begin_kernel(e, e->stream))) return st;
         CU_TRY(e, to.launch(false, pick_rowseg_group(e, e->rg_rows), p.rowgroup_grid, kRowSegWarps * 32, 0, g));
         return mark_kernel(e, "sddmm_rowseg_group_kernel", e->stream);

@@ -452,109 +452,101 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, MINB) sddmm_rowseg_bf16_ker
 //   ghdr[u]  .x = CSR position of the segment in the group's first row, .y = first row * 8 + (count - 1),
 //            .z = row length L (row t of the group holds the segment at .x + t * L: equal lengths, consecutive rows),
 //            .w = rows that share the unit (1 for rows outside matching groups, else G)
-// fp32 storage, rows of 32 * CPL elements (zero-padded where K is less), CPL in {1, 2}; NR = G.  The NR rows of A and
-// NR x 8 sums need the registers that the kernel above gives to 256-bit loads and to rolling: here a group is 8 lanes of
-// 16 bytes, 4 units per warp step.  Bound by latency at 16 warps per SM (load/store unit 66 %, issue slots 57 %, 1.25 eligible
-// warps): with every load an L1 hit it still takes 289 of 302 us (36.8 M nonzeros in 3 x 3 blocks, K = 64).  Tried and no faster: the rolling loop with 16-byte parts (322 us)
-// and with 32-byte parts on 4 lanes (329-440 us: 12 to 16 warps do not cover the latency), packed fp32 arithmetic (332 us).
+// fp32 storage, rows of 8 * LPR elements (zero-padded where K is less), LPR in {4, 8, 16, 32}; NR = G.  A unit is taken by a group of LPR
+// lanes, lane t of it holds bytes [32 t, 32 t + 32) of every row: a row of A or B is ONE 256-bit load.  36.8 M nonzeros in
+// 3 x 3 blocks, K = 32 / 64: 165 / 263 us, against 206 / 292 us for rows in pieces of 16 bytes on 8 lanes (twice the load instructions,
+// 64-bit index arithmetic and a shuffle per column index; 3 CTAs per SM at K = 32).
+// What bounds it: the load/store unit, 139 wavefronts of 128 bytes per 32 columns at K = 64 (B rows 64, A rows 24, shuffles of the
+// reduction 21, indices, S and P the rest), and the latency that 16 warps leave.  So kRun units of one row group go to the same
+// lanes, one after the other, and its rows of A stay in registers from one to the next (an A row is a fourth of the traffic):
+// kRun = 1 / 2 / 4, K = 64: 273 / 263 / 274 us, K = 32, where a row is half as long, 165 / 171 / 188; 14 M nonzeros, K = 128:
+// 210 / 198 / 200, 7 M, K = 256 (two partial units of a row weigh more there): 182 / 196 / 199.  The same two by sddmm_rowseg_kernel,
+// which gathers each B row three times: 423 / 409 us.
+// The loads of a unit are issued together, its arithmetic and all shuffles follow.  Slower: rolling loads (a slot's registers refilled
+// as soon as it is multiplied, as above) with the reduction in between 303 to 363 us; 1 / 3 CTAs per SM 344 / 316.
 struct RowSegGroupArgs {
-    const int4 *ghdr;         // n_units (> 0)
-    const int32_t *col_idx;   // nnz
-    const float *s_val;       // nnz
-    float *p_val;             // nnz
-    const float *A;           // M x K
-    const float *B;           // N x K
+    const int4 *ghdr;          // n_units (> 0)
+    const int32_t *unit_cols;  // 8 column indices per unit
+    const float *s_val;        // nnz
+    float *p_val;              // nnz
+    const float *A;            // M x 8 LPR
+    const float *B;            // N x 8 LPR
     int32_t n_units;
-    int32_t K;
 };
 
-// (K = 32: three resident CTAs per SM -- 207 against 273 us on the banded 3x3-block configuration at K = 32; K = 64 needs
-// the registers of two)
-template <int CPL, int NR>
-__global__ void __launch_bounds__(kRowSegWarps * 32, (CPL == 1) ? 3 : 2) sddmm_rowseg_group_kernel(const RowSegGroupArgs args) {
+__host__ __device__ constexpr int group_run(int lpr) { return lpr == 8 || lpr == 16 ? 2 : 1; }
+__host__ __device__ constexpr int group_step_units(int lpr) { return 32 / lpr * group_run(lpr); }   // of a warp step
+template <int LPR, int NR>
+__global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_group_kernel(const RowSegGroupArgs args) {
+    constexpr int kRun = group_run(LPR);         // consecutive units of a group of lanes
+    constexpr int kUnits = group_step_units(LPR);
+    constexpr int H = LPR == 4 ? 2 : 1;          // sums a lane ends up with (LPR > 8: its first 8 lanes)
+    constexpr uint32_t kRowBytes = 32 * LPR;
     const int lane = threadIdx.x & 31;
-    const int gl = lane & 7;
-    const int gbase = lane & 24;
-    const int grp = lane >> 3;
-    constexpr uint32_t row_bytes = 8 * CPL * sizeof(float4);
-
-    const int64_t n_quads = (static_cast<int64_t>(args.n_units) + 3) >> 2;
-    const int64_t n_warps = static_cast<int64_t>(gridDim.x) * kRowSegWarps;
-    int64_t q = static_cast<int64_t>(blockIdx.x) * kRowSegWarps + (threadIdx.x >> 5);
-    if (q >= n_quads) return;
+    const int t = lane % LPR, grp = lane / LPR;
+    const int n_steps = (args.n_units + kUnits - 1) / kUnits;
+    const int n_warps = static_cast<int>(gridDim.x) * kRowSegWarps;
     const int last_unit = args.n_units - 1;
-    const unsigned char *Ab = reinterpret_cast<const unsigned char *>(args.A) + gl * sizeof(float4);
-    const unsigned char *Bb = reinterpret_cast<const unsigned char *>(args.B) + gl * sizeof(float4);
-
-    // every load is unconditional and in range (clamped unit, clamped slot, clamped row of the group); stores are predicated
-    auto load_unit = [&](int64_t qq) -> int4 {
-        const int64_t u = 4 * qq + grp;
-        return __ldcs(args.ghdr + (u < last_unit ? u : last_unit));
+    const unsigned char *At = reinterpret_cast<const unsigned char *>(args.A) + 32 * t;
+    const unsigned char *Bt = reinterpret_cast<const unsigned char *>(args.B) + 32 * t;
+    int b = static_cast<int>(blockIdx.x) * kRowSegWarps + (threadIdx.x >> 5);
+    if (b >= n_steps) return;
+    // unit k of this group in a warp step (k = kRun: the first one of the warp's next step)
+    auto unit_index = [&](int step, int k) -> int {
+        const int u = kUnits * (step + k / kRun * n_warps) + kRun * grp + k % kRun;
+        return u < last_unit ? u : last_unit;
     };
-    auto own_slot = [&](const int4 &u) -> int { return u.x + min(gl, u.y & 7); };
+    auto load_unit = [&](int u) -> int4 { return __ldcs(args.ghdr + u); };
+    auto load_cols = [&](int u) -> Cols8 { return ld_cols(args.unit_cols + 8 * static_cast<int64_t>(u)); };
 
-    int4 u_cur = load_unit(q);
-    int4 u_nxt = load_unit(q + n_warps);
-    int c_own = __ldcs(args.col_idx + own_slot(u_cur));
-
+    int4 un = load_unit(unit_index(b, 0)), un_next = load_unit(unit_index(b, 1));
+    Cols8 cols = load_cols(unit_index(b, 0));
+    Piece a[NR];
+    int have = -1;   // the unit header's row whose group is in `a`
     while (true) {
-        const int row = u_cur.y >> 3;
-        const int rows = u_cur.w;      // 1 .. NR
-        const int L = u_cur.z;
-        const int slot = own_slot(u_cur);
-        const bool valid = (gl <= (u_cur.y & 7)) && (4 * q + grp <= last_unit);
-
-        // S values of this lane's nonzero in every row of the group (used after the dots)
-        float sv[NR];
 #pragma unroll
-        for (int t = 0; t < NR; ++t) sv[t] = __ldcs(args.s_val + slot + min(t, rows - 1) * L);
-        // this lane's chunks of the group's A rows
-        float4 areg[NR][CPL];
+        for (int k = 0; k < kRun; ++k) {
+            if (kRun == 1 || __any_sync(kFullMask, (un.y >> 3) != have)) {
+                have = un.y >> 3;
 #pragma unroll
-        for (int t = 0; t < NR; ++t) {
-            const unsigned char *arow = Ab + static_cast<uint64_t>(static_cast<uint32_t>(row + min(t, rows - 1))) * row_bytes;
-#pragma unroll
-            for (int c = 0; c < CPL; ++c) areg[t][c] = __ldg(reinterpret_cast<const float4 *>(arow) + 8 * c);
-        }
-        const unsigned char *brow[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            brow[i] = Bb + static_cast<uint64_t>(static_cast<uint32_t>(__shfl_sync(kFullMask, c_own, gbase + i))) * row_bytes;
-
-        float acc[NR][8];
-#pragma unroll
-        for (int t = 0; t < NR; ++t)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) acc[t][i] = 0.f;
-
-        // one 128-byte piece of the 8 B rows at a time: gathered once, used by every row of the group
-        float4 bq[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) bq[i] = __ldg(reinterpret_cast<const float4 *>(brow[i]));
-        const int64_t q_next = q + n_warps;
-        const int4 u_nxt2 = load_unit(q_next + n_warps);
-        c_own = __ldcs(args.col_idx + own_slot(u_nxt));
-#pragma unroll
-        for (int c = 0; c < CPL; ++c) {
-#pragma unroll
-            for (int t = 0; t < NR; ++t)
-#pragma unroll
-                for (int i = 0; i < 8; ++i) acc[t][i] = dot4(areg[t][c], bq[i], acc[t][i]);
-            if (c + 1 < CPL) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) bq[i] = __ldg(reinterpret_cast<const float4 *>(brow[i]) + 8 * (c + 1));
+                for (int r = 0; r < NR; ++r) a[r] = ld_piece(row_at(At, have + min(r, un.w - 1), kRowBytes));
             }
-        }
+            Piece bq[8];
 #pragma unroll
-        for (int t = 0; t < NR; ++t) {
-            const float dot = group8_transpose_reduce(acc[t], gl);
-            if (valid && t < rows) __stcs(args.p_val + u_cur.x + gl + t * L, dot * sv[t]);
+            for (int i = 0; i < 8; ++i) bq[i] = ld_piece(row_at(Bt, cols.v[i], kRowBytes));
+            float sv[H][NR];
+#pragma unroll
+            for (int h = 0; h < H; ++h)
+#pragma unroll
+                for (int r = 0; r < NR; ++r) sv[h][r] = __ldcs(args.s_val + un.x + min(t + 4 * h, un.y & 7) + min(r, un.w - 1) * un.z);
+            const int4 un_next2 = load_unit(unit_index(b, k + 2));
+            cols = load_cols(unit_index(b, k + 1));
+            float acc[NR][8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int r = 0; r < NR; ++r) acc[r][i] = dot_piece(a[r], bq[i], 0.f);
+            const int n = kUnits * b + kRun * grp + k <= last_unit ? (un.y & 7) : -1;
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                const bool live = r < un.w;
+                float *p = args.p_val + un.x + t + r * un.z;
+                if constexpr (LPR >= 8) {
+                    float dot = group8_transpose_reduce(acc[r], t);
+#pragma unroll
+                    for (int o = 8; o < LPR; o *= 2) dot += __shfl_xor_sync(kFullMask, dot, o);
+                    if (live && t <= n) __stcs(p, dot * sv[0][r]);
+                } else {
+                    const float2 dot = group4_transpose_reduce(acc[r], t);
+                    if (live && t <= n) __stcs(p, dot.x * sv[0][r]);
+                    if (live && t + 4 <= n) __stcs(p + 4, dot.y * sv[H - 1][r]);
+                }
+            }
+            un = un_next;
+            un_next = un_next2;
         }
-
-        q = q_next;
-        if (q >= n_quads) break;   // warp-uniform
-        u_cur = u_nxt;
-        u_nxt = u_nxt2;
+        b += n_warps;
+        if (b >= n_steps) break;   // warp-uniform
     }
 }
 
