@@ -866,43 +866,43 @@ RowSegGroupFn pick_rowseg_group(const sddmm_b200_engine *e, int rows) {
 
 using RowSegFn = void (*)(const RowSegArgs);
 
-template <bool SPECIALS, bool COPIES>
+template <int TAIL, bool COPIES>   // (ragged rows of one piece always leave the product out)
 RowSegFn pick_rowseg(int pieces) {
     switch (pieces) {
-        case 1: return sddmm_rowseg_kernel<1, SPECIALS, COPIES, kWholeRows>;
-        case 2: return sddmm_rowseg_kernel<2, SPECIALS, COPIES, kWholeRows>;
-        case 3: return sddmm_rowseg_kernel<3, SPECIALS, COPIES, kWholeRows>;
-        case 4: return sddmm_rowseg_kernel<4, SPECIALS, COPIES, kWholeRows>;
-        case 5: return sddmm_rowseg_kernel<5, SPECIALS, COPIES, kWholeRows>;
-        case 6: return sddmm_rowseg_kernel<6, SPECIALS, COPIES, kWholeRows>;
-        case 7: return sddmm_rowseg_kernel<7, SPECIALS, COPIES, kWholeRows>;
-        default: return sddmm_rowseg_kernel<8, SPECIALS, COPIES, kWholeRows>;
+        case 1: return sddmm_rowseg_kernel<1, TAIL == kTail ? kTailSpecials : TAIL, COPIES, kWholeRows>;
+        case 2: return sddmm_rowseg_kernel<2, TAIL, COPIES, kWholeRows>;
+        case 3: return sddmm_rowseg_kernel<3, TAIL, COPIES, kWholeRows>;
+        case 4: return sddmm_rowseg_kernel<4, TAIL, COPIES, kWholeRows>;
+        case 5: return sddmm_rowseg_kernel<5, TAIL, COPIES, kWholeRows>;
+        case 6: return sddmm_rowseg_kernel<6, TAIL, COPIES, kWholeRows>;
+        case 7: return sddmm_rowseg_kernel<7, TAIL, COPIES, kWholeRows>;
+        default: return sddmm_rowseg_kernel<8, TAIL, COPIES, kWholeRows>;
     }
 }
-template <bool SPECIALS>
+template <int TAIL>
 RowSegFn pick_rowseg_wide(int pieces) {   // (nullptr: an odd number of pieces)
     switch (pieces) {
-        case 2: return sddmm_rowseg_wide_kernel<2, SPECIALS, kWholeRows>;
-        case 4: return sddmm_rowseg_wide_kernel<4, SPECIALS, kWholeRows>;
-        case 6: return sddmm_rowseg_wide_kernel<6, SPECIALS, kWholeRows>;
-        case 8: return sddmm_rowseg_wide_kernel<8, SPECIALS, kWholeRows>;
+        case 2: return sddmm_rowseg_wide_kernel<2, TAIL, kWholeRows>;
+        case 4: return sddmm_rowseg_wide_kernel<4, TAIL, kWholeRows>;
+        case 6: return sddmm_rowseg_wide_kernel<6, TAIL, kWholeRows>;
+        case 8: return sddmm_rowseg_wide_kernel<8, TAIL, kWholeRows>;
         default: return nullptr;
     }
 }
-template <bool SPECIALS, bool COPIES>
+template <int TAIL, bool COPIES>
 RowSegFn pick_rowseg_bf16(int64_t Ks) {
-    if (Ks <= 32) return sddmm_rowseg_bf16_kernel<1, 16, 8, 3, SPECIALS, COPIES>;
-    if (Ks <= 64) return sddmm_rowseg_bf16_kernel<1, 32, 8, 2, SPECIALS, COPIES>;
-    if (Ks <= 128) return sddmm_rowseg_bf16_kernel<2, 32, 4, 2, SPECIALS, COPIES>;
-    if (Ks <= 192) return sddmm_rowseg_bf16_kernel<3, 32, 4, 1, SPECIALS, COPIES>;
-    return sddmm_rowseg_bf16_kernel<4, 32, 2, 1, SPECIALS, COPIES>;
+    if (Ks <= 32) return sddmm_rowseg_bf16_kernel<1, 16, 8, 3, TAIL, COPIES>;
+    if (Ks <= 64) return sddmm_rowseg_bf16_kernel<1, 32, 8, 2, TAIL, COPIES>;
+    if (Ks <= 128) return sddmm_rowseg_bf16_kernel<2, 32, 4, 2, TAIL, COPIES>;
+    if (Ks <= 192) return sddmm_rowseg_bf16_kernel<3, 32, 4, 1, TAIL, COPIES>;
+    return sddmm_rowseg_bf16_kernel<4, 32, 2, 1, TAIL, COPIES>;
 }
 // a slice of K: without panels of a B that does not fit L2, the order that DRAM likes
 template <int PIECES, int STEP>
 RowSegFn pick_rowseg_slice(const sddmm_b200_engine *e, bool copies) {
-    if (copies) return sddmm_rowseg_kernel<PIECES, false, true, STEP>;
-    if (static_cast<double>(e->N) * (128.0 * PIECES) > e->l2_bytes) return sddmm_rowseg_wide_kernel<PIECES, false, STEP>;
-    return sddmm_rowseg_kernel<PIECES, false, false, STEP>;
+    if (copies) return sddmm_rowseg_kernel<PIECES, kNoTail, true, STEP>;
+    if (static_cast<double>(e->N) * (128.0 * PIECES) > e->l2_bytes) return sddmm_rowseg_wide_kernel<PIECES, kNoTail, STEP>;
+    return sddmm_rowseg_kernel<PIECES, kNoTail, false, STEP>;
 }
 template <int PIECES>
 RowSegFn pick_rowseg_slice(const sddmm_b200_engine *e, bool copies, SliceStep step) {
@@ -913,19 +913,19 @@ RowSegFn pick_rowseg_slice(const sddmm_b200_engine *e, bool copies, SliceStep st
     return e->slice_cols == 128 ? pick_rowseg_slice<4>(e, copies, step) : pick_rowseg_slice<2>(e, copies, step);
 }
 // The row-segment kernel instantiation for this engine's storage and K (`copies`: S values from the per-unit copies).
-RowSegFn seg_function(const sddmm_b200_engine *e, bool copies) {
-    const bool specials = leave_out_past_end(e);
-    if (e->mode == SDDMM_B200_BF16) {
-        if (specials) return copies ? pick_rowseg_bf16<true, true>(e->Ks) : pick_rowseg_bf16<true, false>(e->Ks);
-        return copies ? pick_rowseg_bf16<false, true>(e->Ks) : pick_rowseg_bf16<false, false>(e->Ks);
-    }
-    if (e->seg_slices > 1) return pick_rowseg_slice(e, copies, kLastSlice);
+template <int TAIL>
+RowSegFn seg_function_tail(const sddmm_b200_engine *e, bool copies) {
+    if (e->mode == SDDMM_B200_BF16) return copies ? pick_rowseg_bf16<TAIL, true>(e->Ks) : pick_rowseg_bf16<TAIL, false>(e->Ks);
     const int pieces = static_cast<int>((e->Ks + 31) / 32);
     // whole rows of a B that does not fit L2, without panels (rows too short for them): the order that DRAM likes
     if (!copies && static_cast<double>(e->N) * e->Ks * 4.0 > e->l2_bytes)
-        if (RowSegFn fn = specials ? pick_rowseg_wide<true>(pieces) : pick_rowseg_wide<false>(pieces)) return fn;
-    if (specials) return copies ? pick_rowseg<true, true>(pieces) : pick_rowseg<true, false>(pieces);
-    return copies ? pick_rowseg<false, true>(pieces) : pick_rowseg<false, false>(pieces);
+        if (RowSegFn fn = pick_rowseg_wide<TAIL>(pieces)) return fn;
+    return copies ? pick_rowseg<TAIL, true>(pieces) : pick_rowseg<TAIL, false>(pieces);
+}
+RowSegFn seg_function(const sddmm_b200_engine *e, bool copies) {
+    if (e->mode != SDDMM_B200_BF16 && e->seg_slices > 1) return pick_rowseg_slice(e, copies, kLastSlice);
+    if (leave_out_past_end(e)) return seg_function_tail<kTailSpecials>(e, copies);
+    return ragged_rows(e) ? seg_function_tail<kTail>(e, copies) : seg_function_tail<kNoTail>(e, copies);
 }
 // persistent grid of a streaming kernel over `n_units` units, `per_step` of them per warp step
 int seg_grid(sddmm_b200_engine *e, const void *fn, int warps, int per_step, int64_t n_units, int32_t *grid) {

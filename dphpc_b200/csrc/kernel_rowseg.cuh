@@ -133,6 +133,10 @@ __device__ __forceinline__ float2 group4_transpose_reduce(const float (&a)[8], i
 // K in slices, one launch each: P.val carries the sum so far, and S comes in once, with the last slice -- a product per slice would
 // make Inf - Inf of a large or infinite S value where the whole sum has a value, and reads S once per slice.  (The earlier slices
 // multiply by args.one all the same: without the instruction the compiler spills in the first slice, K = 128 256 -> 265 us.)
+// Whether some lanes of a row's last piece lie past its end: never (whole pieces: no addresses and registers for them), such lanes
+// multiply zeros, or they leave the product out.  37.5 M nonzeros, bf16 K = 32 / 128 373 -> 344 / 1117 -> 1067 us without the logic, 6 M
+// K = 128 220 -> 215, 3 M K = 256 213 -> 190.
+enum RowTail : int { kNoTail, kTail, kTailSpecials };
 enum SliceStep : int { kWholeRows, kFirstSlice, kNextSlice, kLastSlice };
 __device__ __forceinline__ constexpr bool step_adds(int step) { return step == kNextSlice || step == kLastSlice; }
 __device__ __forceinline__ constexpr bool step_scales(int step) { return step == kWholeRows || step == kLastSlice; }
@@ -157,7 +161,7 @@ __host__ __device__ constexpr int a_prefetch_stages(int pieces) { return pieces 
 // passes would read in turn).  STEP: which part of the dot products this launch adds up.
 // (All index arithmetic of the loop is 32-bit: with 64-bit selects the compiler splits the loop body and the rolling is
 // lost, 488 -> 574 us.  NP is a compile-time number for the same reason.)
-template <int NP, bool SPECIALS, bool COPIES, int STEP>
+template <int NP, int TAIL, bool COPIES, int STEP>
 __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(const RowSegArgs args) {
     const int lane = threadIdx.x & 31;
     const int t = lane & 3;        // 32-byte part of a piece
@@ -167,7 +171,8 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
     int b = static_cast<int>(blockIdx.x) * kRowSegWarps + (threadIdx.x >> 5);
     if (b >= n_steps) return;
     const int last_unit = args.n_units - 1;
-    const bool off = 128 * (NP - 1) + 32 * t >= args.row_bytes;   // this lane's part of the last piece lies past the row
+    constexpr bool SPECIALS = TAIL == kTailSpecials;
+    const bool off = TAIL != kNoTail && 128 * (NP - 1) + 32 * t >= args.row_bytes;   // this lane's part of the last piece lies past the row
     const uint32_t stride = args.row_stride;
     const unsigned char *At = static_cast<const unsigned char *>(args.A) + 32 * t;
     const unsigned char *Bt = static_cast<const unsigned char *>(args.B) + 32 * t;
@@ -239,7 +244,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
 // bound, and it likes few rows open at a time.  The stages go through all pieces of 4 slots, two pieces of 128 bytes at a
 // time, before the other 4: half the rows in flight, twice the bytes of each.  9 M nonzeros in rows of 13, B 358 / 717 MB:
 // K = 128 697 -> 638 us, K = 256 1581 -> 1559; 13 M nonzeros in rows of 9, B 373 MB: K = 64 558 -> 524; with B in L2 the order above is faster (K = 128 385 against 414).
-template <int NP, bool SPECIALS, int STEP>
+template <int NP, int TAIL, int STEP>
 __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_wide_kernel(const RowSegArgs args) {
     const int lane = threadIdx.x & 31;
     const int t = lane & 3;
@@ -249,7 +254,8 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_wide_kernel
     int b = static_cast<int>(blockIdx.x) * kRowSegWarps + (threadIdx.x >> 5);
     if (b >= n_steps) return;
     const int last_unit = args.n_units - 1;
-    const bool off = 128 * (NP - 1) + 32 * t >= args.row_bytes;   // this lane's part of the last piece lies past the row
+    constexpr bool SPECIALS = TAIL == kTailSpecials;
+    const bool off = TAIL != kNoTail && 128 * (NP - 1) + 32 * t >= args.row_bytes;   // this lane's part of the last piece lies past the row
     const uint32_t stride = args.row_stride;
     const unsigned char *At = static_cast<const unsigned char *>(args.A) + 32 * t;
     const unsigned char *Bt = static_cast<const unsigned char *>(args.B) + 32 * t;
@@ -358,7 +364,7 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
 // NP pieces of 4 * LB bytes per row (the last one may be partial), R units' rows in flight per warp.  SPECIALS, as above: the lanes
 // past the end of a row read zeros in place of B as well, since the tensor cores take the products of all lanes (K = 96 / 48 / 16:
 // 260 / 130 / 91 us without, 269 / 138 / 96 with it).
-template <int NP, int LB, int R, int MINB, bool SPECIALS, bool COPIES>
+template <int NP, int LB, int R, int MINB, int TAIL, bool COPIES>
 __global__ void __launch_bounds__(kRowSegWarps * 32, MINB) sddmm_rowseg_bf16_kernel(const RowSegArgs args) {
     const int lane = threadIdx.x & 31;
     const int t = lane & 3;        // LB-byte part of a piece
@@ -368,7 +374,8 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, MINB) sddmm_rowseg_bf16_ker
     int b = static_cast<int>(blockIdx.x) * kRowSegWarps + (threadIdx.x >> 5);
     if (b >= n_steps) return;
     const int last_unit = args.n_units - 1, last_step = n_steps - 1;
-    const bool off = 4 * LB * (NP - 1) + LB * t >= args.row_bytes;   // this lane's part of the last piece lies past the row
+    constexpr bool SPECIALS = TAIL == kTailSpecials;
+    const bool off = TAIL != kNoTail && 4 * LB * (NP - 1) + LB * t >= args.row_bytes;   // this lane's part of the last piece lies past the row
     const uint32_t stride = args.row_stride;
     const unsigned char *At = static_cast<const unsigned char *>(args.A) + LB * t;
     const unsigned char *Bt = static_cast<const unsigned char *>(args.B) + LB * t;
