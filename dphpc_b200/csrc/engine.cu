@@ -193,7 +193,7 @@ struct sddmm_b200_engine {
     // Y goes back to the host in up to kSpmmChunks row ranges, each as soon as its part of the kernel is done
     static constexpr int kSpmmChunks = 8;
     cudaEvent_t ev_chunk[kSpmmChunks] = {};
-    int32_t spmm_cut[kSpmmChunks + 1] = {};   // units before row M * c / kSpmmChunks
+    int32_t spmm_cut[kSpmmChunks + 1] = {};   // units before row range c
 
     // plan
     sddmm_b200_plan_info plan;
@@ -951,7 +951,8 @@ int enqueue_units(sddmm_b200_engine *e, const Runs &runs, int64_t n, bool have_s
     }
     const bool scanned = tiles > kDirectTiles;
     if (scanned) k_scan_sums<<<1, kScanBlock, 0, s>>>(e->d_scan_tiles, tiles, &e->d_pc->units);
-    k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, skip_hint);
+    k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, skip_hint,
+                                                   e->mode != SDDMM_B200_BF16);   // (whose kernel loads a unit at a time)
     CU_TRY(e, cudaGetLastError());
     return SDDMM_B200_OK;
 }
@@ -2076,7 +2077,7 @@ int sddmm_b200_spmm(sddmm_b200_engine *e, int64_t K2, const float *X, float *Y) 
     constexpr int kMost = sddmm_b200_engine::kSpmmChunks;
     const int chunks = ybytes >= (size_t(32) << 20) ? 8 : ybytes >= (size_t(16) << 20) ? 4 : ybytes >= (size_t(8) << 20) ? 2 : 1;
     int64_t row[kMost + 1];
-    for (int c = 0; c <= chunks; ++c) row[c] = e->M * (c * (kMost / chunks)) / kMost;
+    for (int c = 0; c <= chunks; ++c) row[c] = range_start(e->M, c * (kMost / chunks), kMost);
     for (int c = 0; c < chunks; ++c) {
         const int32_t u0 = e->spmm_cut[c * (kMost / chunks)], u1 = e->spmm_cut[(c + 1) * (kMost / chunks)];
         if (u1 > u0) {

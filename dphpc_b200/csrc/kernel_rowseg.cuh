@@ -46,6 +46,7 @@ struct RowSegArgs {
 };
 
 constexpr int kRowSegWarps = 8;
+constexpr int kSlotStep = 2;   // slots that are loaded or left out together (see most_slots)
 
 // ---- 256-bit loads (32-byte aligned) and packed fp32 arithmetic ------------------------------------------------------
 // (volatile: the order in which the loads are written is the order of the rolling loop)
@@ -84,9 +85,10 @@ __device__ __forceinline__ Piece ld_piece_of_two(const unsigned char *p) {
     return r;
 }
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+// (read once: first to leave L2 as well, 37.5 M nonzeros, rows of 26, K = 32 478 -> 465 us)
 __device__ __forceinline__ Cols8 ld_cols(const int32_t *p) {
     Cols8 r;
-    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+    asm volatile("ld.global.nc.L1::no_allocate.L2::evict_first.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
                  : "l"(p));
     return r;
@@ -181,6 +183,11 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
     auto unit_index = [&](int step) -> int { const int u = 8 * step + grp; return u < last_unit ? u : last_unit; };
     auto load_unit = [&](int step) -> int2 { return __ldcs(args.units + unit_index(step)); };
     auto load_cols = [&](int step) -> Cols8 { return ld_cols(args.unit_cols + 8 * static_cast<int64_t>(unit_index(step))); };
+    // The slots that any unit of a step fills.  Short runs lie side by side in the list, by length (unit_plan.cuh), so where rows are
+    // short whole steps have few; the loads of the others are left out (their sums come from old registers and are not stored).
+    // Power-law rows, K = 32: 5 M nonzeros 66 -> 60 us, 36 M 428 -> 402; Poisson rows of 10 48 -> 45.  One slot at a time
+    // 396 us, but K = 128 in L2 100 against 95; loads that depend on their own lane's count serialise the loop.
+    auto most_slots = [&](const int2 &u) -> int { return static_cast<int>(__reduce_max_sync(kFullMask, static_cast<unsigned>(u.y) & 7u)) + 1; };
     auto piece_offset = [&](int p) -> int { return p == NP - 1 ? o_last : 128 * p; };
     auto load_a = [&](int row, int p) -> Piece {
         const unsigned char *q = row_at(At + piece_offset(p), row, stride);
@@ -192,6 +199,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
     Piece a = load_a(un.y >> 3, 0), bq[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) bq[i] = ld_piece(row_at(Bt + piece_offset(0), cols.v[i], stride));
+    int slots = most_slots(un);
     Cols8 cols_next = load_cols(b + n_warps);
 
     while (true) {
@@ -207,6 +215,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
         const int2 un_next2 = load_unit(next + n_warps);
         const Cols8 cols_next2 = load_cols(next + n_warps);
 
+        const int slots_next = most_slots(un_next);
         float acc[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[i] = 0.f;
@@ -222,8 +231,10 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
             for (int i = 0; i < 8; ++i) {
                 const float sum = dot_piece(a, bq[i], acc[i]);
                 acc[i] = SPECIALS && last && off ? acc[i] : sum;
-                const unsigned char *q = row_at(Bt + piece_offset(p_next), last ? cols_next.v[i] : cols.v[i], stride);
-                bq[i] = NP > 1 && p_next % 2 == 0 ? ld_piece_of_two(q) : ld_piece(q);
+                if (i / kSlotStep * kSlotStep < (last ? slots_next : slots)) {   // warp-uniform
+                    const unsigned char *q = row_at(Bt + piece_offset(p_next), last ? cols_next.v[i] : cols.v[i], stride);
+                    bq[i] = NP > 1 && p_next % 2 == 0 ? ld_piece_of_two(q) : ld_piece(q);
+                }
             }
             a = a_next;
         }
@@ -234,6 +245,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
         if (next >= n_steps) break;   // warp-uniform
         b = next;
         un = un_next;
+        slots = slots_next;
         un_next = un_next2;
         cols = cols_next;
         cols_next = cols_next2;

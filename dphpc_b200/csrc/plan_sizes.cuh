@@ -12,6 +12,8 @@ namespace sddmm {
 // several blocks to build (200 000 rows: 113 us in 196 blocks of 1024 entries), larger ones for long lists.
 constexpr int kUnitTileMax = 1024;
 __host__ __device__ __forceinline__ int unit_tile(int64_t n) { return n > (1 << 20) ? kUnitTileMax : n > (1 << 18) ? 256 : 128; }
+// first of `parts` row ranges' rows, on a tile of the list over whole rows
+__host__ __device__ __forceinline__ int64_t range_start(int64_t M, int c, int parts) { return c >= parts ? M : M * c / parts / unit_tile(M) * unit_tile(M); }
 inline int64_t unit_tiles(int64_t n) { return (n + unit_tile(n) - 1) / unit_tile(n); }
 
 // A block of the list's second kernel adds up the sums of all tiles before its own, which is quadratic in their number: fine for a few
