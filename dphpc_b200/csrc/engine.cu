@@ -940,9 +940,8 @@ int seg_grid(sddmm_b200_engine *e, const void *fn, int warps, int per_step, int6
 // Enqueue the list over n entries; *units = how many there are goes to the plan counters.  have_sums: k_row_stats has left the tile
 // sums and the total.
 template <typename Runs, typename HDR>
-int enqueue_units(sddmm_b200_engine *e, const Runs &runs, int64_t n, bool have_sums, int64_t cap, HDR *units, int32_t *unit_cols,
+int enqueue_units(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_t n, bool have_sums, int64_t cap, HDR *units, int32_t *unit_cols,
                   unsigned long long skip_hint = ~0ull) {
-    cudaStream_t s = e->stream;
     const int tiles = static_cast<int>(unit_tiles(n));
     if (int rc = check_tile_sums(e, tiles)) return rc;
     if (!have_sums) {
@@ -1001,7 +1000,7 @@ int build_rowgroup_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
         e->d_rp, e->d_col, M, nnz, best, best_first, 1, e->d_group_ok, &e->d_pc->group_cover[bs], &e->d_pc->group_count[bs]);
     if (units) {
         const RunsOfGroups runs{e->d_rp, e->d_col, M, nnz, best, best_first, e->d_group_ok};
-        if (int rc = enqueue_units(e, runs, e->M, false, e->unit_cap, reinterpret_cast<int4 *>(e->d_units), e->d_unit_cols)) return rc;
+        if (int rc = enqueue_units(e, s, runs, e->M, false, e->unit_cap, reinterpret_cast<int4 *>(e->d_units), e->d_unit_cols)) return rc;
     }
     CU_TRY(e, cudaGetLastError());
     PlanCounters pc;
@@ -1071,19 +1070,18 @@ int build_residual_units(sddmm_b200_engine *e) {
 
 // Enqueue the unit list over the whole matrix with `panels` column panels (1: whole rows, whose tile sums k_row_stats has
 // left when have_sums).
-int enqueue_unit_list(sddmm_b200_engine *e, int32_t panels, bool have_sums, bool unless_tiles = false) {
+int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, int32_t panels, bool have_sums, bool unless_tiles = false) {
     const int32_t M = static_cast<int32_t>(e->M), nnz = static_cast<int32_t>(e->nnz);
-    cudaStream_t s = e->stream;
     const int64_t n = static_cast<int64_t>(panels) * M;
     // (fp32 mode: tiles will most likely be looked for, and found, when the column scan's count is high enough -- no list then)
     const unsigned long long skip = unless_tiles ? (static_cast<unsigned long long>(e->nnz) + kTileHintShare - 1) / kTileHintShare : ~0ull;
     int st;
     if (panels > 1) {
         const RunsOfPanels runs{e->d_rp, e->d_col, M, nnz, panels, e->panel_cols, e->long_rows};
-        st = enqueue_units(e, runs, n, false, e->unit_cap, e->d_units, e->d_unit_cols, skip);
+        st = enqueue_units(e, s, runs, n, false, e->unit_cap, e->d_units, e->d_unit_cols, skip);
     } else {
         const RunsOfRows runs{e->d_rp, e->d_col, M, nnz};
-        st = enqueue_units(e, runs, n, have_sums, e->unit_cap, e->d_units, e->d_unit_cols, skip);
+        st = enqueue_units(e, s, runs, n, have_sums, e->unit_cap, e->d_units, e->d_unit_cols, skip);
     }
     if (st) return st;
     if (e->mode == SDDMM_B200_BF16) k_unit_pad<<<1, 64, 0, s>>>(e->d_units, e->d_unit_cols, e->d_pc, e->unit_cap);
@@ -1132,7 +1130,7 @@ int build_rowseg_plan(sddmm_b200_engine *e, PlanCounters pc, bool built) {
         if (!use_long && panels == 1 && e->slice_cols == 64 && e->nnz < 16 * e->M && gathered_bytes(e, 64) > e->l2_bytes) e->seg_slices = 1;
     }
     if (!built || panels > 1) {
-        if (int rc = enqueue_unit_list(e, panels, false)) return rc;
+        if (int rc = enqueue_unit_list(e, e->stream, panels, false)) return rc;
         if (int rc = read_counters(e, &pc)) return rc;
     }
     e->seg_copies = panels > 1;
@@ -1173,6 +1171,17 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     bool early_list = whole_rows && e->nnz > 0;
     k_row_stats<<<static_cast<int>(unit_tiles(e->M)), kUnitBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, e->d_rowstart,
                                                                                             whole_rows ? e->d_scan_tiles : nullptr, e->d_pc);
+    // The list of whole rows needs the row statistics only: where the operands come from this GPU's memory it is built on the side
+    // stream, behind their copies, while the columns are looked at here (each of the three kernels leaves much of the chip idle: 5.2 M
+    // nonzeros, K = 64, upload and run 272 -> 256 us; 4 M, power law, 266 -> 249).  Not for rows long enough to lie in 64-wide tiles,
+    // where the count of the column scan may make the list unnecessary (18 M in 64 x 64 blocks, upload 489 us, 572 with the list aside).
+    const bool list_aside = early_list && join_copies && e->nnz < 64 * e->M;
+    if (list_aside) {
+        CU_TRY(e, cudaEventRecord(e->ev_fork, s));
+        CU_TRY(e, cudaStreamWaitEvent(e->side_stream, e->ev_fork, 0));
+        if (int rc = enqueue_unit_list(e, e->side_stream, 1, true, e->dense_possible && e->knob_offset_tiles <= 0)) return rc;
+        CU_TRY(e, cudaEventRecord(e->ev_join, e->side_stream));
+    }
     if (e->nnz > 0) {
         const size_t bitmap = (static_cast<size_t>(e->N) + 31) / 32 * 4;
         const int scan_blocks = grid_for(e->nnz, 4 * kColScanThreads, e->sm_count * 2);
@@ -1186,9 +1195,10 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         CU_TRY(e, cudaGetLastError());
         if (group_possible(e))
             if (int rc = enqueue_group_sample(e)) return rc;
-        if (early_list)
-            if (int rc = enqueue_unit_list(e, 1, true, e->dense_possible && e->knob_offset_tiles <= 0)) return rc;
+        if (early_list && !list_aside)
+            if (int rc = enqueue_unit_list(e, s, 1, true, e->dense_possible && e->knob_offset_tiles <= 0)) return rc;
     }
+    if (list_aside) CU_TRY(e, cudaStreamWaitEvent(s, e->ev_join, 0));
     CU_TRY(e, cudaGetLastError());
     if (join_copies && !tiles_first && no_panels && !e->slice_major) {   // (... or whether the copies are made slice by slice)
         CU_TRY(e, cudaStreamWaitEvent(s, e->ev_h2d, 0));
@@ -1704,7 +1714,10 @@ int sddmm_b200_upload_csr_device(sddmm_b200_engine *e, int64_t M, int64_t N, int
     if (M < 1) return fail(e, SDDMM_B200_ERR_ARG, "need M >= 1");
     DeviceGuard g(e->device);
     int32_t last = 0;
-    CU_TRY(e, cudaMemcpy(&last, row_ptr + M, sizeof(int32_t), cudaMemcpyDeviceToHost));
+    // (on the legacy stream, as a plain cudaMemcpy: behind what the caller has enqueued there; into pinned memory, which saves a staged copy)
+    CU_TRY(e, cudaMemcpyAsync(e->h_pc, row_ptr + M, sizeof(int32_t), cudaMemcpyDeviceToHost, cudaStreamLegacy));
+    CU_TRY(e, cudaStreamSynchronize(cudaStreamLegacy));
+    std::memcpy(&last, e->h_pc, sizeof(int32_t));
     const int64_t nnz = last;
     int st = check_dims(e, M, N, K, nnz);
     if (st) return st;
@@ -2033,7 +2046,7 @@ int spmm_prepare(sddmm_b200_engine *e, int64_t K2, bool own_x) {
         const int32_t Mi = static_cast<int32_t>(e->M);
         cudaStream_t s = e->stream;
         const RunsOfRows runs{e->d_rp, e->d_col, Mi, static_cast<int32_t>(e->nnz)};
-        if (int rc = enqueue_units(e, runs, e->M, false, static_cast<int64_t>(cap), e->d_spmm_units, static_cast<int32_t *>(nullptr))) return rc;
+        if (int rc = enqueue_units(e, s, runs, e->M, false, static_cast<int64_t>(cap), e->d_spmm_units, static_cast<int32_t *>(nullptr))) return rc;
         k_unit_cuts<<<1, 32, 0, s>>>(e->d_spmm_units, Mi, sddmm_b200_engine::kSpmmChunks, -1, e->d_pc);
         CU_TRY(e, cudaGetLastError());
         PlanCounters pc;
