@@ -366,6 +366,10 @@ void choose_k_slices(sddmm_b200_engine *e) {
 //     K = 32 480 / 370 us; 36 M, 2.6 M rows, K = 32 561 us without panels, 447 us.
 // Knob "long_rows": 0 = never, T >= 1 = threshold T with the panels that the "panels" knob or the rule gives.
 // (K = 128: where the long rows get panels the rows are taken whole, 565 us against 586 in two slices)
+// What fills L2 in effect: a line that is read by SMs of both dies is kept in both halves of L2, so gathers at random begin to miss in a
+// table of half its size, and from 0.85 times its size on the misses cost more than panels do.
+constexpr double kPanelsFrom = 0.85;
+
 bool long_rows_whole(const sddmm_b200_engine *e) { return e->seg_slices > 1 && e->Ks == 128 && e->knob_k_slices < 0; }
 
 void choose_long_rows(sddmm_b200_engine *e) {
@@ -374,12 +378,15 @@ void choose_long_rows(sddmm_b200_engine *e) {
     if (e->knob_long_rows == 0) return;
     const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20);
     const double b = gathered_bytes(e, e->seg_slices > 1 && !long_rows_whole(e) ? e->slice_cols : e->Ks);
-    if (b <= l2 && !(e->knob_long_rows >= 1 && e->knob_panels >= 2)) return;
-    // B 333 MB, K = 32: 4 panels 458 us, 6 446 us, 8 442-447 us
-    e->panels_long = e->knob_panels >= 1 ? static_cast<int>(std::min(64.0, e->knob_panels)) : static_cast<int>(std::max(2.0, std::min(8.0, std::ceil(b / (0.5 * l2)))));
+    // (see kPanelsFrom.)  Power law, rows of 25 on average, without / with: K = 32, B 94 / 117 / 131 MB 178 / 172, 233 / 214, 270 / 239 us,
+    // rows of 10 93 / 92, 118 / 114, 134 / 127; K = 64, 117 MB 205 / 194; bf16 K = 64, 117 MB 320 / 281.
+    if (b <= kPanelsFrom * l2 && !(e->knob_long_rows >= 1 && e->knob_panels >= 2)) return;
+    // B 333 MB, K = 32: 4 panels 407 us, 6 402 us, 8 401 us; 189 MB, 2 / 3 / 4 / 6: 300 / 287 / 286 / 286
+    e->panels_long = e->knob_panels >= 1 ? static_cast<int>(std::min(64.0, e->knob_panels)) : static_cast<int>(std::max(4.0, std::min(8.0, std::ceil(b / (0.5 * l2)))));
     if (e->panels_long < 2) return;
-    // runs of 16 nonzeros or more on average (powers of two: the histogram's bins)
-    e->long_threshold = e->knob_long_rows >= 1 ? static_cast<int>(e->knob_long_rows) : e->panels_long <= 4 ? 64 : 128;
+    // (a power of two: the histogram's bins.  From 64 nonzeros on instead, 4 panels, K = 64, rows of 10: B 117 MB 106 -> 114 us, 189 MB
+    // 161 -> 166; K = 32 within 1 %)
+    e->long_threshold = e->knob_long_rows >= 1 ? static_cast<int>(e->knob_long_rows) : 128;
 }
 
 int choose_panels(const sddmm_b200_engine *e) {
@@ -392,7 +399,12 @@ int choose_panels(const sddmm_b200_engine *e) {
     // Rows too short on average.  The longer a row of B, the more a gather that misses L2 costs against a half-empty segment.  Poisson
     // rows, without / with 2 panels: K = 32, B 186 MB, mean 11 / 13 / 15: 282 / 290, 324 / 320, 368 / 353 us; K = 64, B 371 MB, mean
     // 9 / 11 / 13 / 15: 524 / 537, 619 / 607, 723 / 685, 839 / 768; K = 96, B 346 MB, mean 10 / 13: 601 / 538, 779 / 655.
-    if (b_bytes <= l2 || mean < (bf ? 16.0 : cols <= 32 ? 13.0 : cols <= 64 ? 11.0 : 9.0)) return 1;
+    // With B between 0.85 and 1 times L2 only longer rows gain, 1 / 2 panels: K = 32, 117 MB, mean 20 / 40: 216 / 221, 403 / 368, 131 MB 258 / 238,
+    // 444 / 377; K = 64, 117 MB, mean 12 / 20 / 40: 134 / 132, 205 / 190, 364 / 326; K = 128 the same; bf16 K = 64 and 128, mean 20 / 40:
+    // 283 / 283, 522 / 481 and 199 / 202, 371 / 337.  (Slices of K, whose P.val is read and written once more for each: not below L2.)
+    if (b_bytes <= (e->seg_slices > 1 ? 1.0 : kPanelsFrom) * l2) return 1;
+    if (b_bytes <= l2) return mean < (bf ? 28.0 : cols <= 32 ? 24.0 : 16.0) ? 1 : 2;
+    if (mean < (bf ? (cols <= 32 ? 26.0 : cols <= 64 ? 20.0 : 13.0) : cols <= 32 ? 13.0 : cols <= 64 ? 11.0 : 9.0)) return 1;
     // Slices of 128 columns: panels that fit L2 one by one, if an average row has 3 nonzeros for each, or none.  Sustained, B 205 MB,
     // mean 10, 1 / 2 panels: 577 / 527 us; 358 MB, 9.6, 1 / 2 / 3: 1158 / 1174 / 1122; 461 MB, 9.5: 1549 / 1659 / 1640, 12, 1 / 2 / 3 / 4:
     // 2006 / 1999 / 1905 / 1859; longer rows, 358 MB, 30, 3 / 4 / 5: 2390 / 2086 / 2084; 512 MB, 20, 4 / 5 / 6: 2836 / 2651 / 2834; 744 MB,
@@ -402,17 +414,18 @@ int choose_panels(const sddmm_b200_engine *e) {
         if (mean < 16.0) return 3.0 * need > mean || need > 4.0 ? 1 : static_cast<int>(need);
         return static_cast<int>(std::min(8.0, std::min(std::ceil(b_bytes / (0.8 * l2)), std::floor(mean / 3.5))));
     }
-    // bf16 storage, measured with 1.45 M rows of B: K = 64 (B 1.5 x L2) 590 / 618 / 634 us with 1 / 2 / 3 panels, K = 128 (3 x L2)
-    // 1809 / 1142 / 1092 / 1096 / 1150 us with 1 .. 5
+    // bf16 storage, 1 / 2 / 3 / 4 panels.  K = 64: B 157 MB, mean 14 308 / 308 / 349 / 417, 26 431 / 404 / 414 / 434, 45 414 / 377 / 372 / 386;
+    // 262 MB, 26 630 / 473 / 484 / 488, 45 633 / 434 / 436 / 436.  K = 128: 157 MB, 14 230 / 215 / 265 / 294, 26 393 / 368 / 358 / 352, 45
+    // 625 / 526 / 498 / 534; 388 MB, 14 908 / 725 / 749 / 831, 26 1175 / 804 / 763 / 739, 45 1521 / 764 / 679 / 652
     if (bf) {
-        if (b_bytes <= 2.0 * l2) return 1;
-        return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(static_cast<int64_t>(std::ceil(b_bytes / l2)), e->nnz / std::max<int64_t>(1, 8 * e->M)), 4)));
+        if (cols <= 64) return static_cast<int>(std::max(2.0, std::min(4.0, std::ceil(b_bytes / (1.25 * l2)))));
+        return static_cast<int>(std::min(std::min(4.0, std::ceil(b_bytes / (0.8 * l2))), std::max(2.0, std::floor(mean / 6.0))));
     }
-    // measured on B200 (126 MB of L2): a run shorter than a segment wastes gather slots, so panels of about 96 MB for rows of one
-    // piece (B 186 MB: 2 / 3 panels 507 / 514 us), 80 MB for longer rows, where a slot's waste weighs less against its row
+    // measured on B200 (126 MB of L2): a run shorter than a segment wastes gather slots, so panels of about 100 MB for rows of one
+    // piece (B 199 MB, mean 26: 2 / 3 panels 344 / 365 us), 80 MB for longer rows, where a slot's waste weighs less against its row
     // (K = 64, B 179 MB: 428 / 414 us, B 372 MB: 3 / 4 panels 1138 / 1116); at most 2, or one per 6 nonzeros of an average row,
     // and never more than 4 (5: 3 % slower)
-    const double panel = e->knob_panel_mb > 0 ? e->knob_panel_mb * (1 << 20) : (cols <= 32 ? 0.75 : 0.6) * l2;
+    const double panel = e->knob_panel_mb > 0 ? e->knob_panel_mb * (1 << 20) : (cols <= 32 ? 0.8 : 0.6) * l2;
     return static_cast<int>(std::min(std::ceil(b_bytes / panel), std::min(4.0, std::max(2.0, std::floor(mean / 6.0)))));
 }
 
@@ -901,7 +914,7 @@ RowSegFn pick_rowseg_bf16(int64_t Ks) {
 template <int PIECES, int STEP>
 RowSegFn pick_rowseg_slice(const sddmm_b200_engine *e, bool copies) {
     if (copies) return sddmm_rowseg_kernel<PIECES, kNoTail, true, STEP>;
-    if (static_cast<double>(e->N) * (128.0 * PIECES) > e->l2_bytes) return sddmm_rowseg_wide_kernel<PIECES, kNoTail, STEP>;
+    if (static_cast<double>(e->N) * (128.0 * PIECES) > e->l2_bytes) return sddmm_rowseg_wide_kernel<PIECES, false, STEP>;
     return sddmm_rowseg_kernel<PIECES, kNoTail, false, STEP>;
 }
 template <int PIECES>
@@ -919,7 +932,7 @@ RowSegFn seg_function_tail(const sddmm_b200_engine *e, bool copies) {
     const int pieces = static_cast<int>((e->Ks + 31) / 32);
     // whole rows of a B that does not fit L2, without panels (rows too short for them): the order that DRAM likes
     if (!copies && static_cast<double>(e->N) * e->Ks * 4.0 > e->l2_bytes)
-        if (RowSegFn fn = pick_rowseg_wide<TAIL>(pieces)) return fn;
+        if (RowSegFn fn = pick_rowseg_wide<TAIL == kTailSpecials>(pieces)) return fn;
     return copies ? pick_rowseg<TAIL, true>(pieces) : pick_rowseg<TAIL, false>(pieces);
 }
 RowSegFn seg_function(const sddmm_b200_engine *e, bool copies) {
