@@ -892,13 +892,13 @@ RowSegFn pick_rowseg(int pieces) {
         default: return sddmm_rowseg_kernel<8, TAIL, COPIES, kWholeRows>;
     }
 }
-template <int TAIL>
+template <bool SPECIALS>
 RowSegFn pick_rowseg_wide(int pieces) {   // (nullptr: an odd number of pieces)
     switch (pieces) {
-        case 2: return sddmm_rowseg_wide_kernel<2, TAIL, kWholeRows>;
-        case 4: return sddmm_rowseg_wide_kernel<4, TAIL, kWholeRows>;
-        case 6: return sddmm_rowseg_wide_kernel<6, TAIL, kWholeRows>;
-        case 8: return sddmm_rowseg_wide_kernel<8, TAIL, kWholeRows>;
+        case 2: return sddmm_rowseg_wide_kernel<2, SPECIALS, kWholeRows>;
+        case 4: return sddmm_rowseg_wide_kernel<4, SPECIALS, kWholeRows>;
+        case 6: return sddmm_rowseg_wide_kernel<6, SPECIALS, kWholeRows>;
+        case 8: return sddmm_rowseg_wide_kernel<8, SPECIALS, kWholeRows>;
         default: return nullptr;
     }
 }
@@ -950,11 +950,19 @@ int seg_grid(sddmm_b200_engine *e, const void *fn, int warps, int per_step, int6
     return SDDMM_B200_OK;
 }
 
+// Short runs side by side (k_unit_build): for the fp32 kernels, which then leave out empty slots (the bf16 kernel loads a unit at a
+// time), where the gathers hit L2 or only long rows are cut into panels.  Poisson rows of 8, B 262 MB, K = 128 265 -> 273 us with the
+// order, K = 256 245 -> 260.
+bool list_by_size(const sddmm_b200_engine *e) {
+    if (e->mode == SDDMM_B200_BF16) return false;
+    return e->long_rows > 0 || e->l2_bytes <= 0 || gathered_bytes(e, e->seg_slices > 1 ? e->slice_cols : e->Ks) <= kPanelsFrom * e->l2_bytes;
+}
+
 // Enqueue the list over n entries; *units = how many there are goes to the plan counters.  have_sums: k_row_stats has left the tile
 // sums and the total.
 template <typename Runs, typename HDR>
 int enqueue_units(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_t n, bool have_sums, int64_t cap, HDR *units, int32_t *unit_cols,
-                  unsigned long long skip_hint = ~0ull) {
+                  unsigned long long skip_hint = ~0ull, bool by_size = false) {
     const int tiles = static_cast<int>(unit_tiles(n));
     if (int rc = check_tile_sums(e, tiles)) return rc;
     if (!have_sums) {
@@ -963,8 +971,7 @@ int enqueue_units(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_
     }
     const bool scanned = tiles > kDirectTiles;
     if (scanned) k_scan_sums<<<1, kScanBlock, 0, s>>>(e->d_scan_tiles, tiles, &e->d_pc->units);
-    k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, skip_hint,
-                                                   e->mode != SDDMM_B200_BF16);   // (whose kernel loads a unit at a time)
+    k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, skip_hint, by_size);
     CU_TRY(e, cudaGetLastError());
     return SDDMM_B200_OK;
 }
@@ -1091,10 +1098,10 @@ int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, int32_t panels, bool
     int st;
     if (panels > 1) {
         const RunsOfPanels runs{e->d_rp, e->d_col, M, nnz, panels, e->panel_cols, e->long_rows};
-        st = enqueue_units(e, s, runs, n, false, e->unit_cap, e->d_units, e->d_unit_cols, skip);
+        st = enqueue_units(e, s, runs, n, false, e->unit_cap, e->d_units, e->d_unit_cols, skip, list_by_size(e));
     } else {
         const RunsOfRows runs{e->d_rp, e->d_col, M, nnz};
-        st = enqueue_units(e, s, runs, n, have_sums, e->unit_cap, e->d_units, e->d_unit_cols, skip);
+        st = enqueue_units(e, s, runs, n, have_sums, e->unit_cap, e->d_units, e->d_unit_cols, skip, list_by_size(e));
     }
     if (st) return st;
     if (e->mode == SDDMM_B200_BF16) k_unit_pad<<<1, 64, 0, s>>>(e->d_units, e->d_unit_cols, e->d_pc, e->unit_cap);

@@ -137,7 +137,7 @@ __device__ __forceinline__ float2 group4_transpose_reduce(const float (&a)[8], i
 // multiply by args.one all the same: without the instruction the compiler spills in the first slice, K = 128 256 -> 265 us.)
 // Whether some lanes of a row's last piece lie past its end: never (whole pieces: no addresses and registers for them), such lanes
 // multiply zeros, or they leave the product out.  37.5 M nonzeros, bf16 K = 32 / 128 373 -> 344 / 1117 -> 1067 us without the logic, 6 M
-// K = 128 220 -> 215, 3 M K = 256 213 -> 190.
+// K = 128 220 -> 215, 3 M K = 256 213 -> 190.  (The kernel for B beyond L2 keeps one form: without the logic its registers spill.)
 enum RowTail : int { kNoTail, kTail, kTailSpecials };
 enum SliceStep : int { kWholeRows, kFirstSlice, kNextSlice, kLastSlice };
 __device__ __forceinline__ constexpr bool step_adds(int step) { return step == kNextSlice || step == kLastSlice; }
@@ -186,7 +186,9 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
     // The slots that any unit of a step fills.  Short runs lie side by side in the list, by length (unit_plan.cuh), so where rows are
     // short whole steps have few; the loads of the others are left out (their sums come from old registers and are not stored).
     // Power-law rows, K = 32: 5 M nonzeros 66 -> 60 us, 36 M 428 -> 402; Poisson rows of 10 48 -> 45.  One slot at a time
-    // 396 us, but K = 128 in L2 100 against 95; loads that depend on their own lane's count serialise the loop.
+    // 396 us, but K = 128 in L2 100 against 95; loads that depend on their own lane's count serialise the loop.  (Panels of rows of an
+    // odd number of pieces, which the compiler does not roll with the branches in: K = 96, 9 M nonzeros 286 -> 349 us.)
+    constexpr bool kLeaveOut = !(COPIES && NP > 1 && NP % 2 == 1);
     auto most_slots = [&](const int2 &u) -> int { return static_cast<int>(__reduce_max_sync(kFullMask, static_cast<unsigned>(u.y) & 7u)) + 1; };
     auto piece_offset = [&](int p) -> int { return p == NP - 1 ? o_last : 128 * p; };
     auto load_a = [&](int row, int p) -> Piece {
@@ -231,7 +233,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
             for (int i = 0; i < 8; ++i) {
                 const float sum = dot_piece(a, bq[i], acc[i]);
                 acc[i] = SPECIALS && last && off ? acc[i] : sum;
-                if (i / kSlotStep * kSlotStep < (last ? slots_next : slots)) {   // warp-uniform
+                if (!kLeaveOut || i / kSlotStep * kSlotStep < (last ? slots_next : slots)) {   // warp-uniform
                     const unsigned char *q = row_at(Bt + piece_offset(p_next), last ? cols_next.v[i] : cols.v[i], stride);
                     bq[i] = NP > 1 && p_next % 2 == 0 ? ld_piece_of_two(q) : ld_piece(q);
                 }
@@ -256,7 +258,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
 // bound, and it likes few rows open at a time.  The stages go through all pieces of 4 slots, two pieces of 128 bytes at a
 // time, before the other 4: half the rows in flight, twice the bytes of each.  9 M nonzeros in rows of 13, B 358 / 717 MB:
 // K = 128 697 -> 638 us, K = 256 1581 -> 1559; 13 M nonzeros in rows of 9, B 373 MB: K = 64 558 -> 524; with B in L2 the order above is faster (K = 128 385 against 414).
-template <int NP, int TAIL, int STEP>
+template <int NP, bool SPECIALS, int STEP>
 __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_wide_kernel(const RowSegArgs args) {
     const int lane = threadIdx.x & 31;
     const int t = lane & 3;
@@ -266,8 +268,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_wide_kernel
     int b = static_cast<int>(blockIdx.x) * kRowSegWarps + (threadIdx.x >> 5);
     if (b >= n_steps) return;
     const int last_unit = args.n_units - 1;
-    constexpr bool SPECIALS = TAIL == kTailSpecials;
-    const bool off = TAIL != kNoTail && 128 * (NP - 1) + 32 * t >= args.row_bytes;   // this lane's part of the last piece lies past the row
+    const bool off = 128 * (NP - 1) + 32 * t >= args.row_bytes;   // this lane's part of the last piece lies past the row
     const uint32_t stride = args.row_stride;
     const unsigned char *At = static_cast<const unsigned char *>(args.A) + 32 * t;
     const unsigned char *Bt = static_cast<const unsigned char *>(args.B) + 32 * t;

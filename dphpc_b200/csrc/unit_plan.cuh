@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs runs, int64_t n, 
 }
 
 // A list is ordered by size (k_unit_build) from one short row in this many on: with fewer the kernel gains nothing and building takes
-// longer (5.2 M nonzeros in rows of 26: upload and run 247 us, 250 with the order).
+// longer (5.2 M nonzeros in rows of 26: upload and run 247 us, 250 with the order).  Not where DRAM is the bound, see list_by_size.
 constexpr unsigned kShortRowShare = 16;
 
 // pass 2: the units of a tile.  HDR = int2 (plain units) or int4 (row groups).  scanned: tile_sums holds the units before each tile.
