@@ -866,8 +866,18 @@ template <int LPR>
 RowSegGroupFn pick_rowseg_group_rows(int rows) {
     return rows == 2 ? sddmm_rowseg_group_kernel<LPR, 2> : rows == 3 ? sddmm_rowseg_group_kernel<LPR, 3> : sddmm_rowseg_group_kernel<LPR, 4>;
 }
-// rows of 32, 64, 128 or 256 elements (nullptr: no instantiation)
+// rows of 32, 64, 128 or 256 elements, bf16 rows of 192 too (nullptr: no instantiation)
 RowSegGroupFn pick_rowseg_group(const sddmm_b200_engine *e, int rows) {
+    if (e->mode == SDDMM_B200_BF16) {
+        switch (e->Ks) {
+            case 32: return sddmm_rowseg_group_bf16_kernel<1, 16, 4>;
+            case 64: return sddmm_rowseg_group_bf16_kernel<1, 32, 2>;
+            case 128: return sddmm_rowseg_group_bf16_kernel<2, 32, 1>;
+            case 192: return sddmm_rowseg_group_bf16_kernel<3, 32, 1>;
+            case 256: return sddmm_rowseg_group_bf16_kernel<4, 32, 1>;
+            default: return nullptr;
+        }
+    }
     switch (e->Ks) {
         case 32: return pick_rowseg_group_rows<4>(rows);
         case 64: return pick_rowseg_group_rows<8>(rows);
@@ -977,8 +987,9 @@ int enqueue_units(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_
 }
 
 bool group_possible(const sddmm_b200_engine *e) {
-    if (e->mode == SDDMM_B200_BF16 || (e->flags & SDDMM_B200_FLAG_NO_ROW_GROUPS) || e->M < 4) return false;
-    return e->knob_group_units != 0 && e->use_seg ? pick_rowseg_group(e, 2) != nullptr : (e->K == 32 || e->K == 64);
+    if ((e->flags & SDDMM_B200_FLAG_NO_ROW_GROUPS) || e->M < 4) return false;
+    if (e->knob_group_units != 0 && e->use_seg) return pick_rowseg_group(e, 2) != nullptr;
+    return e->mode != SDDMM_B200_BF16 && (e->K == 32 || e->K == 64);
 }
 // candidates: G = 2, 3, 4 rows per group, first full group starting at row 0 .. G-1 (counters slot = G(G-1)/2 - 1 + first)
 int group_slot(int G, int first) { return G * (G - 1) / 2 - 1 + first; }
@@ -994,7 +1005,7 @@ int enqueue_group_sample(sddmm_b200_engine *e) {
 }
 
 // Row groups: groups of 2, 3 or 4 consecutive rows with one column list (first full group at row 0 .. G-1) share each gather of B.
-// The path is taken (for the whole matrix) when it removes at least 30 % of the gathers; fp32 storage, K <= 256.
+// The path is taken (for the whole matrix) when it removes at least 30 % of the gathers; K <= 256.
 // base_pc: counters that include enqueue_group_sample's.
 int build_rowgroup_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
     if (!group_possible(e) || base_pc.max_row_nnz > 8192) return SDDMM_B200_OK;
@@ -1031,7 +1042,7 @@ int build_rowgroup_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
         if (pc.units == 0 || pc.units > static_cast<unsigned long long>(std::min<int64_t>(e->unit_cap, kUnitLimit)))
             return fail(e, SDDMM_B200_ERR_CUDA, "row-group plan: %llu units for a list of %lld", pc.units, (long long)e->unit_cap);
         e->n_units = static_cast<int32_t>(pc.units);
-        if (int rc = seg_grid(e, reinterpret_cast<const void *>(pick_rowseg_group(e, best)), kRowSegWarps, group_step_units(static_cast<int>(e->Ks / 8)), e->n_units, &p.rowgroup_grid)) return rc;
+        if (int rc = seg_grid(e, reinterpret_cast<const void *>(pick_rowseg_group(e, best)), kRowSegWarps, e->mode == SDDMM_B200_BF16 ? 8 : group_step_units(static_cast<int>(e->Ks / 8)), e->n_units, &p.rowgroup_grid)) return rc;
         p.rowseg_units = e->n_units;
         p.rowseg_panels = 1;
     } else {

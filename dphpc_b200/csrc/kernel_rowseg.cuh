@@ -570,4 +570,92 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_group_kerne
     }
 }
 
+// The same for bf16 storage, on mma.sync as sddmm_rowseg_bf16_kernel: the 16 rows of the first operand are the gathered B rows of the 8
+// slots of two units, the 8 columns of the second one are the rows of A of their groups, 4 (of which NR count) for each.  Half of the
+// products are used where that kernel uses an eighth, and a B row is gathered once for the group.  Lane (slot g, part t) ends up with
+// slot g of the pair's unit t / 2, rows 2 (t % 2) and 2 (t % 2) + 1 of its group.  NP pieces of 4 * LB bytes per row, whole rows.
+// A step is 8 units, PAIRS pairs of them at a time.  36.8 M nonzeros in 3 x 3 blocks, K = 32 / 64, by sddmm_rowseg_bf16_kernel 243 / 345 us,
+// with PAIRS = 4 149 / 239, 2 188 / 210; 20 M, K = 128 (96 the same), 312, PAIRS = 2 161, 1 150; 12 M, K = 192, 285 -> 122; 10 M, K = 256
+// (192 bytes spilled), 299 -> 172.
+template <int NP, int LB, int PAIRS>
+__global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_group_bf16_kernel(const RowSegGroupArgs args) {
+    constexpr uint32_t kRowBytes = 4 * LB * NP;
+    const int lane = threadIdx.x & 31, t = lane & 3, grp = lane >> 2;
+    const int n_steps = (args.n_units + 7) >> 3, last_unit = args.n_units - 1;
+    const int n_warps = static_cast<int>(gridDim.x) * kRowSegWarps;
+    const unsigned char *At = reinterpret_cast<const unsigned char *>(args.A) + LB * t;
+    const unsigned char *Bt = reinterpret_cast<const unsigned char *>(args.B) + LB * t;
+    int b = static_cast<int>(blockIdx.x) * kRowSegWarps + (threadIdx.x >> 5);
+    if (b >= n_steps) return;
+
+    struct Row {
+        Frag<LB> p[NP];
+    };
+    auto load_row = [&](Row &f, const unsigned char *base, int row) {
+        const unsigned char *q = row_at(base, row, kRowBytes);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) ld_frag(f.p[p], q + 4 * LB * p);
+    };
+    auto load_unit = [&](int step) -> int4 { return __ldcs(args.ghdr + min(8 * step + (lane & 7), last_unit)); };   // unit lane % 8 of a step
+    auto load_cols = [&](int step) -> Cols8 {   // slot grp of the step's 8 units
+        Cols8 c;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) c.v[u] = __ldcs(args.unit_cols + 8 * static_cast<int64_t>(min(8 * step + u, last_unit)) + grp);
+        return c;
+    };
+
+    int4 un = load_unit(b);
+    Cols8 cols = load_cols(b);
+    while (true) {
+        const int next = b + n_warps;
+        const int4 un_next = load_unit(next);
+        const Cols8 cols_next = load_cols(next);
+#pragma unroll
+        for (int g = 0; g < 4; g += PAIRS) {
+            Row a[PAIRS], x[PAIRS], y[PAIRS];
+            float s0[PAIRS], s1[PAIRS];
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) {
+                const int u = 2 * (g + i);
+                const int ua = u + (grp >> 2);
+                const int row = __shfl_sync(kFullMask, un.y, ua) >> 3, rows = __shfl_sync(kFullMask, un.w, ua);
+                load_row(a[i], At, row + min(grp & 3, rows - 1));
+                load_row(x[i], Bt, cols.v[u]);
+                load_row(y[i], Bt, cols.v[u + 1]);
+            }
+            bool on0[PAIRS], on1[PAIRS];
+            int at[PAIRS], step_l[PAIRS];
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) {
+                const int uo = 2 * (g + i) + (t >> 1), r = 2 * (t & 1);
+                const int start = __shfl_sync(kFullMask, un.x, uo), code = __shfl_sync(kFullMask, un.y, uo);
+                const int len = __shfl_sync(kFullMask, un.z, uo), rows = __shfl_sync(kFullMask, un.w, uo);
+                const bool live = grp <= (code & 7) && 8 * b + uo <= last_unit;
+                on0[i] = live && r < rows;
+                on1[i] = live && r + 1 < rows;
+                at[i] = start + grp + r * len;
+                step_l[i] = len;
+                s0[i] = on0[i] ? __ldcs(args.s_val + at[i]) : 0.f;
+                s1[i] = on1[i] ? __ldcs(args.s_val + at[i] + len) : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) {
+                float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int p = 0; p < NP; ++p)
+#pragma unroll
+                    for (int k = 0; k < LB / 4; k += 2)
+                        mma_bf16(c, x[i].p[p].r[k], y[i].p[p].r[k], x[i].p[p].r[k + 1], y[i].p[p].r[k + 1], a[i].p[p].r[k], a[i].p[p].r[k + 1]);
+                const bool second = t >= 2;   // columns 4 .. 7 belong to the second unit, whose slots are rows 8 .. 15
+                if (on0[i]) __stcs(args.p_val + at[i], (second ? c[2] : c[0]) * s0[i]);
+                if (on1[i]) __stcs(args.p_val + at[i] + step_l[i], (second ? c[3] : c[1]) * s1[i]);
+            }
+        }
+        if (next >= n_steps) break;   // warp-uniform
+        b = next;
+        un = un_next;
+        cols = cols_next;
+    }
+}
+
 }  // namespace sddmm
