@@ -1210,7 +1210,8 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     if (list_aside) {
         CU_TRY(e, cudaEventRecord(e->ev_fork, s));
         CU_TRY(e, cudaStreamWaitEvent(e->side_stream, e->ev_fork, 0));
-        if (int rc = enqueue_unit_list(e, e->side_stream, 1, true, e->dense_possible && e->knob_offset_tiles <= 0)) return rc;
+        // (whatever the column scan will have counted: its count grows while the list's blocks would look at it)
+        if (int rc = enqueue_unit_list(e, e->side_stream, 1, true)) return rc;
         CU_TRY(e, cudaEventRecord(e->ev_join, e->side_stream));
     }
     if (e->nnz > 0) {
@@ -1240,7 +1241,8 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     if (int rc = read_counters(e, &pc)) return rc;
     if (pc.bad_coo) return fail(e, SDDMM_B200_ERR_INDEX, "COO row indices must be sorted and inside [0, M)");
     if (pc.bad_row_ptr) return fail(e, SDDMM_B200_ERR_INDEX, "row_ptr must start at 0, end at nnz and be non-decreasing");
-    if (e->dense_possible && e->knob_offset_tiles <= 0 && pc.window_hint * kTileHintShare >= static_cast<unsigned long long>(e->nnz)) early_list = false;   // (it was left out)
+    if (!list_aside && e->dense_possible && e->knob_offset_tiles <= 0 && pc.window_hint * kTileHintShare >= static_cast<unsigned long long>(e->nnz))
+        early_list = false;   // (it was left out)
     if (pc.bad_col) return fail(e, SDDMM_B200_ERR_INDEX, "column index outside [0, N)");
 
     sddmm_b200_plan_info &p = e->plan;
