@@ -401,18 +401,20 @@ int choose_panels(const sddmm_b200_engine *e) {
     // 9 / 11 / 13 / 15: 524 / 537, 619 / 607, 723 / 685, 839 / 768; K = 96, B 346 MB, mean 10 / 13: 601 / 538, 779 / 655.
     // With B between 0.85 and 1 times L2 only longer rows gain, 1 / 2 panels: K = 32, 117 MB, mean 20 / 40: 216 / 221, 403 / 368, 131 MB 258 / 238,
     // 444 / 377; K = 64, 117 MB, mean 12 / 20 / 40: 134 / 132, 205 / 190, 364 / 326; K = 128 the same; bf16 K = 64 and 128, mean 20 / 40:
-    // 283 / 283, 522 / 481 and 199 / 202, 371 / 337.  (Slices of K, whose P.val is read and written once more for each: not below L2.)
-    if (b_bytes <= (e->seg_slices > 1 ? 1.0 : kPanelsFrom) * l2) return 1;
-    if (b_bytes <= l2) return mean < (bf ? 28.0 : cols <= 32 ? 24.0 : 16.0) ? 1 : 2;
-    if (mean < (bf ? (cols <= 32 ? 26.0 : cols <= 64 ? 20.0 : 13.0) : cols <= 32 ? 13.0 : cols <= 64 ? 11.0 : 9.0)) return 1;
+    // 283 / 283, 522 / 481 and 199 / 202, 371 / 337; slices of K, 121 MB each, mean 12 / 24 / 50: K = 128 304 / 279, 548 / 490, 873 / 659, K = 256,
+    // mean 12 / 40, 290 / 268, 790 / 617.
+    if (b_bytes <= kPanelsFrom * l2) return 1;
+    if (b_bytes <= l2) return mean < (e->seg_slices > 1 ? 11.0 : bf ? 28.0 : cols <= 32 ? 24.0 : 16.0) ? 1 : 2;
+    // (K = 32, B 262 / 388 MB, mean 8 / 10 / 12: 347 / 342, 418 / 392, 500 / 438 and 616 / 569, 726 / 654, 719 / 638)
+    if (mean < (bf ? (cols <= 32 ? 26.0 : cols <= 64 ? 20.0 : 13.0) : cols <= 32 ? (b_bytes > 1.8 * l2 ? 10.0 : 13.0) : cols <= 64 ? 11.0 : 9.0)) return 1;
     // Slices of 128 columns: panels that fit L2 one by one, if an average row has 3 nonzeros for each, or none.  Sustained, B 205 MB,
     // mean 10, 1 / 2 panels: 577 / 527 us; 358 MB, 9.6, 1 / 2 / 3: 1158 / 1174 / 1122; 461 MB, 9.5: 1549 / 1659 / 1640, 12, 1 / 2 / 3 / 4:
     // 2006 / 1999 / 1905 / 1859; longer rows, 358 MB, 30, 3 / 4 / 5: 2390 / 2086 / 2084; 512 MB, 20, 4 / 5 / 6: 2836 / 2651 / 2834; 744 MB,
-    // 26, 4 / 5 / 6 / 7: 6027 / 5815 / 5538 / 5347.
+    // 26, 4 / 5 / 6 / 7: 6027 / 5815 / 5538 / 5347; 210 MB, 40, 2 / 4: 828 / 711.
     if (cols == 128 && e->seg_slices > 1 && !bf) {
         const double need = std::ceil(b_bytes / l2);
         if (mean < 16.0) return 3.0 * need > mean || need > 4.0 ? 1 : static_cast<int>(need);
-        return static_cast<int>(std::min(8.0, std::min(std::ceil(b_bytes / (0.8 * l2)), std::floor(mean / 3.5))));
+        return static_cast<int>(std::min(8.0, std::min(std::ceil(b_bytes / (0.6 * l2)), std::floor(mean / 3.5))));
     }
     // bf16 storage, 1 / 2 / 3 / 4 panels.  K = 64: B 157 MB, mean 14 308 / 308 / 349 / 417, 26 431 / 404 / 414 / 434, 45 414 / 377 / 372 / 386;
     // 262 MB, 26 630 / 473 / 484 / 488, 45 633 / 434 / 436 / 436.  K = 128: 157 MB, 14 230 / 215 / 265 / 294, 26 393 / 368 / 358 / 352, 45
