@@ -864,9 +864,15 @@ RowGroupFn pick_rowgroup(int rows, int cpl) {
 }
 
 using RowSegGroupFn = void (*)(const RowSegGroupArgs);
-template <int LPR>
+template <int LPR, int RUN>
 RowSegGroupFn pick_rowseg_group_rows(int rows) {
-    return rows == 2 ? sddmm_rowseg_group_kernel<LPR, 2> : rows == 3 ? sddmm_rowseg_group_kernel<LPR, 3> : sddmm_rowseg_group_kernel<LPR, 4>;
+    return rows == 2 ? sddmm_rowseg_group_kernel<LPR, 2, RUN> : rows == 3 ? sddmm_rowseg_group_kernel<LPR, 3, RUN> : sddmm_rowseg_group_kernel<LPR, 4, RUN>;
+}
+// units that one group of lanes takes one after the other, see the kernel: rows of 64 and 128 elements, where every warp of the chip has
+// two steps or more all the same (70 000 nonzeros in 3 x 3 blocks, K = 64: 11.7 us with one, 12.5 with two)
+int group_run(const sddmm_b200_engine *e) {
+    const int64_t warps = 2 * kRowSegWarps * static_cast<int64_t>(e->sm_count);
+    return (e->Ks == 64 || e->Ks == 128) && e->n_units > 2 * warps * (256 / e->Ks) ? 2 : 1;
 }
 // rows of 32, 64, 128 or 256 elements, bf16 rows of 192 too (nullptr: no instantiation)
 RowSegGroupFn pick_rowseg_group(const sddmm_b200_engine *e, int rows) {
@@ -881,10 +887,10 @@ RowSegGroupFn pick_rowseg_group(const sddmm_b200_engine *e, int rows) {
         }
     }
     switch (e->Ks) {
-        case 32: return pick_rowseg_group_rows<4>(rows);
-        case 64: return pick_rowseg_group_rows<8>(rows);
-        case 128: return pick_rowseg_group_rows<16>(rows);
-        case 256: return pick_rowseg_group_rows<32>(rows);
+        case 32: return pick_rowseg_group_rows<4, 1>(rows);
+        case 64: return group_run(e) == 2 ? pick_rowseg_group_rows<8, 2>(rows) : pick_rowseg_group_rows<8, 1>(rows);
+        case 128: return group_run(e) == 2 ? pick_rowseg_group_rows<16, 2>(rows) : pick_rowseg_group_rows<16, 1>(rows);
+        case 256: return pick_rowseg_group_rows<32, 1>(rows);
         default: return nullptr;
     }
 }
@@ -896,7 +902,7 @@ RowSegFn pick_rowseg(int pieces) {
     switch (pieces) {
         case 1: return sddmm_rowseg_kernel<1, TAIL == kTail ? kTailSpecials : TAIL, COPIES, kWholeRows>;
         case 2: return sddmm_rowseg_kernel<2, TAIL, COPIES, kWholeRows>;
-        case 3: return sddmm_rowseg_kernel<3, TAIL, COPIES, kWholeRows>;
+        case 3: return sddmm_rowseg_kernel<3, TAIL == kNoTail ? kTail : TAIL, COPIES, kWholeRows>;   // (see RowTail)
         case 4: return sddmm_rowseg_kernel<4, TAIL, COPIES, kWholeRows>;
         case 5: return sddmm_rowseg_kernel<5, TAIL, COPIES, kWholeRows>;
         case 6: return sddmm_rowseg_kernel<6, TAIL, COPIES, kWholeRows>;
@@ -917,7 +923,7 @@ RowSegFn pick_rowseg_wide(int pieces) {   // (nullptr: an odd number of pieces)
 template <int TAIL, bool COPIES>
 RowSegFn pick_rowseg_bf16(int64_t Ks) {
     if (Ks <= 32) return sddmm_rowseg_bf16_kernel<1, 16, 8, 3, TAIL, COPIES>;
-    if (Ks <= 64) return sddmm_rowseg_bf16_kernel<1, 32, 8, 2, TAIL, COPIES>;
+    if (Ks <= 64) return sddmm_rowseg_bf16_kernel<1, 32, 8, 2, TAIL == kNoTail ? kTail : TAIL, COPIES>;   // (see RowTail)
     if (Ks <= 128) return sddmm_rowseg_bf16_kernel<2, 32, 4, 2, TAIL, COPIES>;
     if (Ks <= 192) return sddmm_rowseg_bf16_kernel<3, 32, 4, 1, TAIL, COPIES>;
     return sddmm_rowseg_bf16_kernel<4, 32, 2, 1, TAIL, COPIES>;
@@ -966,7 +972,8 @@ int seg_grid(sddmm_b200_engine *e, const void *fn, int warps, int per_step, int6
 // time), where the gathers hit L2 or only long rows are cut into panels.  Poisson rows of 8, B 262 MB, K = 128 265 -> 273 us with the
 // order, K = 256 245 -> 260.
 bool list_by_size(const sddmm_b200_engine *e) {
-    if (e->mode == SDDMM_B200_BF16) return false;
+    const int64_t pieces = e->seg_slices > 1 ? e->slice_cols / 32 : (e->Ks + 31) / 32;
+    if (e->mode == SDDMM_B200_BF16 || pieces == 3 || (e->long_rows > 0 && pieces > 1 && pieces % 2 == 1)) return false;   // (these load all slots)
     return e->long_rows > 0 || e->l2_bytes <= 0 || gathered_bytes(e, e->seg_slices > 1 ? e->slice_cols : e->Ks) <= kPanelsFrom * e->l2_bytes;
 }
 
@@ -1044,7 +1051,7 @@ int build_rowgroup_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
         if (pc.units == 0 || pc.units > static_cast<unsigned long long>(std::min<int64_t>(e->unit_cap, kUnitLimit)))
             return fail(e, SDDMM_B200_ERR_CUDA, "row-group plan: %llu units for a list of %lld", pc.units, (long long)e->unit_cap);
         e->n_units = static_cast<int32_t>(pc.units);
-        if (int rc = seg_grid(e, reinterpret_cast<const void *>(pick_rowseg_group(e, best)), kRowSegWarps, e->mode == SDDMM_B200_BF16 ? 8 : group_step_units(static_cast<int>(e->Ks / 8)), e->n_units, &p.rowgroup_grid)) return rc;
+        if (int rc = seg_grid(e, reinterpret_cast<const void *>(pick_rowseg_group(e, best)), kRowSegWarps, e->mode == SDDMM_B200_BF16 ? 8 : static_cast<int>(256 / e->Ks) * group_run(e), e->n_units, &p.rowgroup_grid)) return rc;
         p.rowseg_units = e->n_units;
         p.rowseg_panels = 1;
     } else {

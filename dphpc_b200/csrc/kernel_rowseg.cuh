@@ -137,7 +137,8 @@ __device__ __forceinline__ float2 group4_transpose_reduce(const float (&a)[8], i
 // multiply by args.one all the same: without the instruction the compiler spills in the first slice, K = 128 256 -> 265 us.)
 // Whether some lanes of a row's last piece lie past its end: never (whole pieces: no addresses and registers for them), such lanes
 // multiply zeros, or they leave the product out.  37.5 M nonzeros, bf16 K = 32 / 128 373 -> 344 / 1117 -> 1067 us without the logic, 6 M
-// K = 128 220 -> 215, 3 M K = 256 213 -> 190.  (The kernel for B beyond L2 keeps one form: without the logic its registers spill.)
+// K = 128 220 -> 215, 3 M K = 256 213 -> 190.  (The kernel for B beyond L2 keeps one form, without the
+// logic its registers spill; so do rows of three pieces, K = 96: 44 against 46 us, and bf16 rows of 64, 10 M K = 64: 109 against 123.)
 enum RowTail : int { kNoTail, kTail, kTailSpecials };
 enum SliceStep : int { kWholeRows, kFirstSlice, kNextSlice, kLastSlice };
 __device__ __forceinline__ constexpr bool step_adds(int step) { return step == kNextSlice || step == kLastSlice; }
@@ -186,9 +187,10 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
     // The slots that any unit of a step fills.  Short runs lie side by side in the list, by length (unit_plan.cuh), so where rows are
     // short whole steps have few; the loads of the others are left out (their sums come from old registers and are not stored).
     // Power-law rows, K = 32: 5 M nonzeros 66 -> 60 us, 36 M 428 -> 402; Poisson rows of 10 48 -> 45.  One slot at a time
-    // 396 us, but K = 128 in L2 100 against 95; loads that depend on their own lane's count serialise the loop.  (Panels of rows of an
-    // odd number of pieces, which the compiler does not roll with the branches in: K = 96, 9 M nonzeros 286 -> 349 us.)
-    constexpr bool kLeaveOut = !(COPIES && NP > 1 && NP % 2 == 1);
+    // 396 us, but K = 128 in L2 100 against 95; loads that depend on their own lane's count serialise the loop.  (Not for rows of
+    // three pieces and panels of rows of an odd number, which the compiler does not roll with the branches in: K = 96, panels, 9 M
+    // nonzeros 286 -> 349 us, 52 000 nonzeros 13 -> 15.)
+    constexpr bool kLeaveOut = NP != 3 && !(COPIES && NP > 1 && NP % 2 == 1);
     auto most_slots = [&](const int2 &u) -> int { return static_cast<int>(__reduce_max_sync(kFullMask, static_cast<unsigned>(u.y) & 7u)) + 1; };
     auto piece_offset = [&](int p) -> int { return p == NP - 1 ? o_last : 128 * p; };
     auto load_a = [&](int row, int p) -> Piece {
@@ -201,7 +203,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
     Piece a = load_a(un.y >> 3, 0), bq[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) bq[i] = ld_piece(row_at(Bt + piece_offset(0), cols.v[i], stride));
-    int slots = most_slots(un);
+    int slots = kLeaveOut ? most_slots(un) : 8;   // of the step
     Cols8 cols_next = load_cols(b + n_warps);
 
     while (true) {
@@ -217,7 +219,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
         const int2 un_next2 = load_unit(next + n_warps);
         const Cols8 cols_next2 = load_cols(next + n_warps);
 
-        const int slots_next = most_slots(un_next);
+        const int slots_next = kLeaveOut ? most_slots(un_next) : 8;
         float acc[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[i] = 0.f;
@@ -477,9 +479,9 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, MINB) sddmm_rowseg_bf16_ker
 // 3 x 3 blocks, K = 32 / 64: 165 / 263 us, against 206 / 292 us for rows in pieces of 16 bytes on 8 lanes (twice the load instructions,
 // 64-bit index arithmetic and a shuffle per column index; 3 CTAs per SM at K = 32).
 // What bounds it: the load/store unit, 139 wavefronts of 128 bytes per 32 columns at K = 64 (B rows 64, A rows 24, shuffles of the
-// reduction 21, indices, S and P the rest), and the latency that 16 warps leave.  So kRun units of one row group go to the same
+// reduction 21, indices, S and P the rest), and the latency that 16 warps leave.  So RUN units of one row group go to the same
 // lanes, one after the other, and its rows of A stay in registers from one to the next (an A row is a fourth of the traffic):
-// kRun = 1 / 2 / 4, K = 64: 273 / 263 / 274 us, K = 32, where a row is half as long, 165 / 171 / 188; 14 M nonzeros, K = 128:
+// RUN = 1 / 2 / 4, K = 64: 273 / 263 / 274 us, K = 32, where a row is half as long, 165 / 171 / 188; 14 M nonzeros, K = 128:
 // 210 / 198 / 200, 7 M, K = 256 (two partial units of a row weigh more there): 182 / 196 / 199.  The same two by sddmm_rowseg_kernel,
 // which gathers each B row three times: 423 / 409 us.
 // The loads of a unit are issued together, its arithmetic and all shuffles follow.  Slower: rolling loads (a slot's registers refilled
@@ -494,12 +496,10 @@ struct RowSegGroupArgs {
     int32_t n_units;
 };
 
-__host__ __device__ constexpr int group_run(int lpr) { return lpr == 8 || lpr == 16 ? 2 : 1; }
-__host__ __device__ constexpr int group_step_units(int lpr) { return 32 / lpr * group_run(lpr); }   // of a warp step
-template <int LPR, int NR>
+template <int LPR, int NR, int RUN>
 __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_group_kernel(const RowSegGroupArgs args) {
-    constexpr int kRun = group_run(LPR);         // consecutive units of a group of lanes
-    constexpr int kUnits = group_step_units(LPR);
+    constexpr int kRun = RUN;                    // consecutive units of a group of lanes
+    constexpr int kUnits = 32 / LPR * kRun;      // per warp step
     constexpr int H = LPR == 4 ? 2 : 1;          // sums a lane ends up with (LPR > 8: its first 8 lanes)
     constexpr uint32_t kRowBytes = 32 * LPR;
     const int lane = threadIdx.x & 31;
