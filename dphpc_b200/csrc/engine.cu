@@ -864,17 +864,19 @@ RowGroupFn pick_rowgroup(int rows, int cpl) {
 }
 
 using RowSegGroupFn = void (*)(const RowSegGroupArgs);
-template <int LPR, int RUN>
+template <int LPR, int RUN, bool WHOLE>
 RowSegGroupFn pick_rowseg_group_rows(int rows) {
-    return rows == 2 ? sddmm_rowseg_group_kernel<LPR, 2, RUN> : rows == 3 ? sddmm_rowseg_group_kernel<LPR, 3, RUN> : sddmm_rowseg_group_kernel<LPR, 4, RUN>;
+    return rows == 2 ? sddmm_rowseg_group_kernel<LPR, 2, RUN, WHOLE> : rows == 3 ? sddmm_rowseg_group_kernel<LPR, 3, RUN, WHOLE> : sddmm_rowseg_group_kernel<LPR, 4, RUN, WHOLE>;
 }
+// lanes per row
+int group_lanes(const sddmm_b200_engine *e) { return e->Ks <= 32 ? 4 : e->Ks <= 64 ? 8 : e->Ks <= 128 ? 16 : 32; }
 // units that one group of lanes takes one after the other, see the kernel: rows of 64 and 128 elements, where every warp of the chip has
 // two steps or more all the same (70 000 nonzeros in 3 x 3 blocks, K = 64: 11.7 us with one, 12.5 with two)
 int group_run(const sddmm_b200_engine *e) {
     const int64_t warps = 2 * kRowSegWarps * static_cast<int64_t>(e->sm_count);
     return (e->Ks == 64 || e->Ks == 128) && e->n_units > 2 * warps * (256 / e->Ks) ? 2 : 1;
 }
-// rows of 32, 64, 128 or 256 elements, bf16 rows of 192 too (nullptr: no instantiation)
+// rows of up to 256 elements, bf16 rows of 32, 64, 128, 192 or 256 (nullptr: no instantiation)
 RowSegGroupFn pick_rowseg_group(const sddmm_b200_engine *e, int rows) {
     if (e->mode == SDDMM_B200_BF16) {
         switch (e->Ks) {
@@ -886,12 +888,13 @@ RowSegGroupFn pick_rowseg_group(const sddmm_b200_engine *e, int rows) {
             default: return nullptr;
         }
     }
-    switch (e->Ks) {
-        case 32: return pick_rowseg_group_rows<4, 1>(rows);
-        case 64: return group_run(e) == 2 ? pick_rowseg_group_rows<8, 2>(rows) : pick_rowseg_group_rows<8, 1>(rows);
-        case 128: return group_run(e) == 2 ? pick_rowseg_group_rows<16, 2>(rows) : pick_rowseg_group_rows<16, 1>(rows);
-        case 256: return pick_rowseg_group_rows<32, 1>(rows);
-        default: return nullptr;
+    if (e->Ks > 256 || e->Ks % 8 != 0) return nullptr;
+    const bool whole = e->Ks == 8 * group_lanes(e);
+    switch (group_lanes(e)) {
+        case 4: return whole ? pick_rowseg_group_rows<4, 1, true>(rows) : pick_rowseg_group_rows<4, 1, false>(rows);
+        case 8: return !whole ? pick_rowseg_group_rows<8, 1, false>(rows) : group_run(e) == 2 ? pick_rowseg_group_rows<8, 2, true>(rows) : pick_rowseg_group_rows<8, 1, true>(rows);
+        case 16: return !whole ? pick_rowseg_group_rows<16, 1, false>(rows) : group_run(e) == 2 ? pick_rowseg_group_rows<16, 2, true>(rows) : pick_rowseg_group_rows<16, 1, true>(rows);
+        default: return whole ? pick_rowseg_group_rows<32, 1, true>(rows) : pick_rowseg_group_rows<32, 1, false>(rows);
     }
 }
 
@@ -1051,7 +1054,7 @@ int build_rowgroup_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
         if (pc.units == 0 || pc.units > static_cast<unsigned long long>(std::min<int64_t>(e->unit_cap, kUnitLimit)))
             return fail(e, SDDMM_B200_ERR_CUDA, "row-group plan: %llu units for a list of %lld", pc.units, (long long)e->unit_cap);
         e->n_units = static_cast<int32_t>(pc.units);
-        if (int rc = seg_grid(e, reinterpret_cast<const void *>(pick_rowseg_group(e, best)), kRowSegWarps, e->mode == SDDMM_B200_BF16 ? 8 : static_cast<int>(256 / e->Ks) * group_run(e), e->n_units, &p.rowgroup_grid)) return rc;
+        if (int rc = seg_grid(e, reinterpret_cast<const void *>(pick_rowseg_group(e, best)), kRowSegWarps, e->mode == SDDMM_B200_BF16 ? 8 : 32 / group_lanes(e) * group_run(e), e->n_units, &p.rowgroup_grid)) return rc;
         p.rowseg_units = e->n_units;
         p.rowseg_panels = 1;
     } else {
@@ -1503,6 +1506,7 @@ int launch_all(sddmm_b200_engine *e, float *p_val, cudaGraph_t graph = nullptr) 
         g.ghdr = reinterpret_cast<const int4 *>(e->d_units); g.unit_cols = e->d_unit_cols; g.s_val = e->d_sval; g.p_val = p_val;
         g.A = static_cast<const float *>(seg_rows_a(e)); g.B = static_cast<const float *>(seg_rows_b(e));
         g.n_units = e->n_units;
+        g.row_bytes = static_cast<uint32_t>(e->Ks * elem_bytes(e));
         if ((st = begin_kernel(e, e->stream))) return st;
         CU_TRY(e, to.launch(false, pick_rowseg_group(e, e->rg_rows), p.rowgroup_grid, kRowSegWarps * 32, 0, g));
         return mark_kernel(e, "sddmm_rowseg_group_kernel", e->stream);

@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, MINB) sddmm_rowseg_bf16_ker
 //   ghdr[u]  .x = CSR position of the segment in the group's first row, .y = first row * 8 + (count - 1),
 //            .z = row length L (row t of the group holds the segment at .x + t * L: equal lengths, consecutive rows),
 //            .w = rows that share the unit (1 for rows outside matching groups, else G)
-// fp32 storage, rows of 8 * LPR elements (zero-padded where K is less), LPR in {4, 8, 16, 32}; NR = G.  A unit is taken by a group of LPR
+// fp32 storage, rows of at most 8 * LPR elements, LPR in {4, 8, 16, 32}; NR = G.  A unit is taken by a group of LPR
 // lanes, lane t of it holds bytes [32 t, 32 t + 32) of every row: a row of A or B is ONE 256-bit load.  36.8 M nonzeros in
 // 3 x 3 blocks, K = 32 / 64: 165 / 263 us, against 206 / 292 us for rows in pieces of 16 bytes on 8 lanes (twice the load instructions,
 // 64-bit index arithmetic and a shuffle per column index; 3 CTAs per SM at K = 32).
@@ -491,24 +491,29 @@ struct RowSegGroupArgs {
     const int32_t *unit_cols;  // 8 column indices per unit
     const float *s_val;        // nnz
     float *p_val;              // nnz
-    const float *A;            // M x 8 LPR
-    const float *B;            // N x 8 LPR
+    const float *A;            // M rows
+    const float *B;            // N rows
     int32_t n_units;
+    uint32_t row_bytes;        // of a row of A or B, a multiple of 32
 };
 
-template <int LPR, int NR, int RUN>
+// WHOLE: a row fills its lanes.  Else (rows of 16 or 96 elements, say) the lanes past its end read its last 32 bytes once more and leave
+// their products out.  20 M nonzeros, K = 8 / 16: 87 / 91 us, by sddmm_rowseg_kernel 175 / 176; 14 M, K = 96 215 (325), 7 M, K = 192 / 224 201 / 203
+// (317 / 361).  Zeros in place of both operands, from a line of their own, cost a wavefront per load: K = 96 253, K = 192 247.
+template <int LPR, int NR, int RUN, bool WHOLE>
 __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_group_kernel(const RowSegGroupArgs args) {
     constexpr int kRun = RUN;                    // consecutive units of a group of lanes
     constexpr int kUnits = 32 / LPR * kRun;      // per warp step
     constexpr int H = LPR == 4 ? 2 : 1;          // sums a lane ends up with (LPR > 8: its first 8 lanes)
-    constexpr uint32_t kRowBytes = 32 * LPR;
     const int lane = threadIdx.x & 31;
     const int t = lane % LPR, grp = lane / LPR;
+    const bool off = !WHOLE && 32u * t >= args.row_bytes;
+    const uint32_t stride = WHOLE ? 32 * LPR : args.row_bytes, part = off ? stride - 32 : 32u * t;
     const int n_steps = (args.n_units + kUnits - 1) / kUnits;
     const int n_warps = static_cast<int>(gridDim.x) * kRowSegWarps;
     const int last_unit = args.n_units - 1;
-    const unsigned char *At = reinterpret_cast<const unsigned char *>(args.A) + 32 * t;
-    const unsigned char *Bt = reinterpret_cast<const unsigned char *>(args.B) + 32 * t;
+    const unsigned char *At = reinterpret_cast<const unsigned char *>(args.A) + part;
+    const unsigned char *Bt = reinterpret_cast<const unsigned char *>(args.B) + part;
     int b = static_cast<int>(blockIdx.x) * kRowSegWarps + (threadIdx.x >> 5);
     if (b >= n_steps) return;
     // unit k of this group in a warp step (k = kRun: the first one of the warp's next step)
@@ -529,11 +534,11 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_group_kerne
             if (kRun == 1 || __any_sync(kFullMask, (un.y >> 3) != have)) {
                 have = un.y >> 3;
 #pragma unroll
-                for (int r = 0; r < NR; ++r) a[r] = ld_piece(row_at(At, have + min(r, un.w - 1), kRowBytes));
+                for (int r = 0; r < NR; ++r) a[r] = ld_piece(row_at(At, have + min(r, un.w - 1), stride));
             }
             Piece bq[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) bq[i] = ld_piece(row_at(Bt, cols.v[i], kRowBytes));
+            for (int i = 0; i < 8; ++i) bq[i] = ld_piece(row_at(Bt, cols.v[i], stride));
             float sv[H][NR];
 #pragma unroll
             for (int h = 0; h < H; ++h)
@@ -545,7 +550,10 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_group_kerne
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int r = 0; r < NR; ++r) acc[r][i] = dot_piece(a[r], bq[i], 0.f);
+                for (int r = 0; r < NR; ++r) {
+                    const float dot = dot_piece(a[r], bq[i], 0.f);
+                    acc[r][i] = off ? 0.f : dot;
+                }
             const int n = kUnits * b + kRun * grp + k <= last_unit ? (un.y & 7) : -1;
 #pragma unroll
             for (int r = 0; r < NR; ++r) {
