@@ -976,6 +976,7 @@ int seg_grid(sddmm_b200_engine *e, const void *fn, int warps, int per_step, int6
 // order, K = 256 245 -> 260.
 bool list_by_size(const sddmm_b200_engine *e) {
     const int64_t pieces = e->seg_slices > 1 ? e->slice_cols / 32 : (e->Ks + 31) / 32;
+    if (e->Ks < 32) return false;
     if (e->mode == SDDMM_B200_BF16 || pieces == 3 || (e->long_rows > 0 && pieces > 1 && pieces % 2 == 1)) return false;   // (these load all slots)
     return e->long_rows > 0 || e->l2_bytes <= 0 || gathered_bytes(e, e->seg_slices > 1 ? e->slice_cols : e->Ks) <= kPanelsFrom * e->l2_bytes;
 }
@@ -998,7 +999,18 @@ int enqueue_units(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_
     return SDDMM_B200_OK;
 }
 
+// Matching the groups and building their list takes 30 to 40 us and 10 us per million nonzeros, which a plan of one run does not get
+// back (190 000 nonzeros, K = 16, uploaded and run: 112 us, 148 with groups; 2 M, K = 128, 190 / 222).  So the gathers that disappear have to be worth
+// something, at the rate of the L2 -> SM fabric (rows of less than a line at a line's): 4 us of a run in bf16, 60 in fp32, but for
+// rows of 32 and 64 elements, which have always been taken.  Knob "group_units" = 1: whatever they are worth.
+bool groups_pay(const sddmm_b200_engine *e, double gathers) {
+    const bool bf = e->mode == SDDMM_B200_BF16;
+    if (!e->use_seg || e->knob_group_units >= 0 || (!bf && (e->Ks == 32 || e->Ks == 64))) return true;
+    return gathers * std::max(128.0, static_cast<double>(e->Ks) * static_cast<double>(elem_bytes(e))) / 18.6e6 >= (bf ? 4.0 : 60.0);
+}
+
 bool group_possible(const sddmm_b200_engine *e) {
+    if (!groups_pay(e, 0.75 * static_cast<double>(e->nnz))) return false;   // (groups of four rows throughout)
     if ((e->flags & SDDMM_B200_FLAG_NO_ROW_GROUPS) || e->M < 4) return false;
     if (e->knob_group_units != 0 && e->use_seg) return pick_rowseg_group(e, 2) != nullptr;
     return e->mode != SDDMM_B200_BF16 && (e->K == 32 || e->K == 64);
@@ -1032,6 +1044,7 @@ int build_rowgroup_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
             if (saved > best_saved) { best_saved = saved; best = G; best_first = first; }
         }
     if (best == 0 || best_saved < 0.3 * static_cast<double>(e->nnz)) return SDDMM_B200_OK;
+    if (!groups_pay(e, best_saved)) return SDDMM_B200_OK;
     const int32_t n_groups = group_count(M, best, best_first);
     const int bs = group_slot(best, best_first);
     const bool units = e->knob_group_units != 0 && e->use_seg;

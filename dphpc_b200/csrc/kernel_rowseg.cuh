@@ -188,9 +188,9 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
     // short whole steps have few; the loads of the others are left out (their sums come from old registers and are not stored).
     // Power-law rows, K = 32: 5 M nonzeros 66 -> 60 us, 36 M 428 -> 402; Poisson rows of 10 48 -> 45.  One slot at a time
     // 396 us, but K = 128 in L2 100 against 95; loads that depend on their own lane's count serialise the loop.  (Not for rows of
-    // three pieces and panels of rows of an odd number, which the compiler does not roll with the branches in: K = 96, panels, 9 M
+    // one ragged piece, 0.5 M nonzeros, K = 16 15.6 against 18 us, nor of three pieces and panels of rows of an odd number, which the compiler does not roll with the branches in: K = 96, panels, 9 M
     // nonzeros 286 -> 349 us, 52 000 nonzeros 13 -> 15.)
-    constexpr bool kLeaveOut = NP != 3 && !(COPIES && NP > 1 && NP % 2 == 1);
+    constexpr bool kLeaveOut = NP != 3 && !(NP == 1 && TAIL == kTailSpecials) && !(COPIES && NP > 1 && NP % 2 == 1);
     auto most_slots = [&](const int2 &u) -> int { return static_cast<int>(__reduce_max_sync(kFullMask, static_cast<unsigned>(u.y) & 7u)) + 1; };
     auto piece_offset = [&](int p) -> int { return p == NP - 1 ? o_last : 128 * p; };
     auto load_a = [&](int row, int p) -> Piece {

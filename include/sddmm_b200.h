@@ -181,7 +181,7 @@ int sddmm_b200_get_plan(sddmm_b200_engine *e, sddmm_b200_plan_info *info);
  *   "panel_mb"      target size of one panel of B in MiB
  *   "rowseg"        0: never take the row-segment kernel, 1: take it whenever it applies
  *   "b_fraction"    accepted and without effect (the share of the gathers of B that carried an L2 eviction hint: it made no difference)
- *   "group_units"   0: rows with identical column lists run the warp-per-group kernel instead of shared segments
+ *   "group_units"   0: rows with identical column lists run the warp-per-group kernel instead of shared segments; 1: shared segments, however little they save
  *   "offset_tiles"  0: dense tiles only on the 64-grid, 1: always also look for half-full 64x64 windows at arbitrary offsets
  *   "k_slices"      fp32 storage: 1 = take K (K >= 128 and a multiple of 64) in slices of 64 columns, 64 = the same,
  *                   copied one after the other where K is 193 to 256, 128 = of 128 columns (K a multiple of 128), one launch each over the same segment list, adding to P.val (default, by K and size, when B is about as
