@@ -164,7 +164,6 @@ struct sddmm_b200_engine {
     int32_t panels_plain = 1;          // column panels when every row is cut
     int32_t panels_long = 1, long_threshold = 0;   // ... when only rows of at least long_threshold (> 0) nonzeros are; the row statistics choose
     int32_t panel_cols = 0;            // columns per panel of the list in use
-    int32_t long_rows = 0;             // > 0: the list in use cuts only rows of at least this many nonzeros, the others follow whole (as one more "panel")
     int32_t n_units = 0;
     bool use_seg = false;
     bool seg_residual = false;         // the row-segment kernel computes what the dense tiles left (units over the uncovered runs)
@@ -366,10 +365,6 @@ void choose_k_slices(sddmm_b200_engine *e) {
 //     K = 32 480 / 370 us; 36 M, 2.6 M rows, K = 32 561 us without panels, 447 us.
 // Knob "long_rows": 0 = never, T >= 1 = threshold T with the panels that the "panels" knob or the rule gives.
 // (K = 128: where the long rows get panels the rows are taken whole, 565 us against 586 in two slices)
-// What fills L2 in effect: a line that is read by SMs of both dies is kept in both halves of L2, so gathers at random begin to miss in a
-// table of half its size, and from 0.85 times its size on the misses cost more than panels do.
-constexpr double kPanelsFrom = 0.85;
-
 bool long_rows_whole(const sddmm_b200_engine *e) { return e->seg_slices > 1 && e->Ks == 128 && e->knob_k_slices < 0; }
 
 void choose_long_rows(sddmm_b200_engine *e) {
@@ -971,14 +966,10 @@ int seg_grid(sddmm_b200_engine *e, const void *fn, int warps, int per_step, int6
     return SDDMM_B200_OK;
 }
 
-// Short runs side by side (k_unit_build): for the fp32 kernels, which then leave out empty slots (the bf16 kernel loads a unit at a
-// time), where the gathers hit L2 or only long rows are cut into panels.  Poisson rows of 8, B 262 MB, K = 128 265 -> 273 us with the
-// order, K = 256 245 -> 260.
-bool list_by_size(const sddmm_b200_engine *e) {
-    const int64_t pieces = e->seg_slices > 1 ? e->slice_cols / 32 : (e->Ks + 31) / 32;
-    if (e->Ks < 32) return false;
-    if (e->mode == SDDMM_B200_BF16 || pieces == 3 || (e->long_rows > 0 && pieces > 1 && pieces % 2 == 1)) return false;   // (these load all slots)
-    return e->long_rows > 0 || e->l2_bytes <= 0 || gathered_bytes(e, e->seg_slices > 1 ? e->slice_cols : e->Ks) <= kPanelsFrom * e->l2_bytes;
+// whether the list is ordered by size (plan_sizes.cuh), for the rows that one launch takes
+bool list_by_size(const sddmm_b200_engine *e, int32_t long_rows) {
+    const int64_t row = e->seg_slices > 1 ? e->slice_cols : e->Ks;
+    return by_size(e->mode == SDDMM_B200_BF16, row, long_rows > 0, gathered_bytes(e, row), e->l2_bytes);
 }
 
 // Enqueue the list over n entries; *units = how many there are goes to the plan counters.  have_sums: k_row_stats has left the tile
@@ -1125,19 +1116,19 @@ int build_residual_units(sddmm_b200_engine *e) {
 }
 
 // Enqueue the unit list over the whole matrix with `panels` column panels (1: whole rows, whose tile sums k_row_stats has
-// left when have_sums).
-int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, int32_t panels, bool have_sums, bool unless_tiles = false) {
+// left when have_sums; long_rows: see RunsOfPanels).
+int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, int32_t panels, int32_t long_rows, bool have_sums, bool unless_tiles = false) {
     const int32_t M = static_cast<int32_t>(e->M), nnz = static_cast<int32_t>(e->nnz);
     const int64_t n = static_cast<int64_t>(panels) * M;
     // (fp32 mode: tiles will most likely be looked for, and found, when the column scan's count is high enough -- no list then)
     const unsigned long long skip = unless_tiles ? (static_cast<unsigned long long>(e->nnz) + kTileHintShare - 1) / kTileHintShare : ~0ull;
     int st;
     if (panels > 1) {
-        const RunsOfPanels runs{e->d_rp, e->d_col, M, nnz, panels, e->panel_cols, e->long_rows};
-        st = enqueue_units(e, s, runs, n, false, e->unit_cap, e->d_units, e->d_unit_cols, skip, list_by_size(e));
+        const RunsOfPanels runs{e->d_rp, e->d_col, M, nnz, panels, e->panel_cols, long_rows};
+        st = enqueue_units(e, s, runs, n, false, e->unit_cap, e->d_units, e->d_unit_cols, skip, list_by_size(e, long_rows));
     } else {
         const RunsOfRows runs{e->d_rp, e->d_col, M, nnz};
-        st = enqueue_units(e, s, runs, n, have_sums, e->unit_cap, e->d_units, e->d_unit_cols, skip, list_by_size(e));
+        st = enqueue_units(e, s, runs, n, have_sums, e->unit_cap, e->d_units, e->d_unit_cols, skip, list_by_size(e, long_rows));
     }
     if (st) return st;
     if (e->mode == SDDMM_B200_BF16) k_unit_pad<<<1, 64, 0, s>>>(e->d_units, e->d_unit_cols, e->d_pc, e->unit_cap);
@@ -1178,7 +1169,6 @@ int build_rowseg_plan(sddmm_b200_engine *e, PlanCounters pc, bool built) {
     }
     const int32_t cut = pc.unsorted_cols ? 1 : use_long ? e->panels_long : plain;
     const int32_t panels = use_long ? cut + 1 : cut;   // (the short rows, whole, are the last entry of the list)
-    e->long_rows = use_long ? e->long_threshold : 0;
     e->panel_cols = static_cast<int32_t>((e->N + cut - 1) / cut);
     if (e->knob_k_slices < 0 && e->K <= 256) {
         if (use_long && long_rows_whole(e)) e->seg_slices = 1;
@@ -1186,7 +1176,7 @@ int build_rowseg_plan(sddmm_b200_engine *e, PlanCounters pc, bool built) {
         if (!use_long && panels == 1 && e->slice_cols == 64 && e->nnz < 16 * e->M && gathered_bytes(e, 64) > e->l2_bytes) e->seg_slices = 1;
     }
     if (!built || panels > 1) {
-        if (int rc = enqueue_unit_list(e, e->stream, panels, false)) return rc;
+        if (int rc = enqueue_unit_list(e, e->stream, panels, use_long ? e->long_threshold : 0, false)) return rc;
         if (int rc = read_counters(e, &pc)) return rc;
     }
     e->seg_copies = panels > 1;
@@ -1236,7 +1226,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         CU_TRY(e, cudaEventRecord(e->ev_fork, s));
         CU_TRY(e, cudaStreamWaitEvent(e->side_stream, e->ev_fork, 0));
         // (whatever the column scan will have counted: its count grows while the list's blocks would look at it)
-        if (int rc = enqueue_unit_list(e, e->side_stream, 1, true)) return rc;
+        if (int rc = enqueue_unit_list(e, e->side_stream, 1, 0, true)) return rc;
         CU_TRY(e, cudaEventRecord(e->ev_join, e->side_stream));
     }
     if (e->nnz > 0) {
@@ -1253,7 +1243,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         if (group_possible(e))
             if (int rc = enqueue_group_sample(e)) return rc;
         if (early_list && !list_aside)
-            if (int rc = enqueue_unit_list(e, s, 1, true, e->dense_possible && e->knob_offset_tiles <= 0)) return rc;
+            if (int rc = enqueue_unit_list(e, s, 1, 0, true, e->dense_possible && e->knob_offset_tiles <= 0)) return rc;
     }
     if (list_aside) CU_TRY(e, cudaStreamWaitEvent(s, e->ev_join, 0));
     CU_TRY(e, cudaGetLastError());

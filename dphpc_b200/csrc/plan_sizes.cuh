@@ -59,4 +59,18 @@ inline int64_t padded_row(bool bf16, int64_t K) {
 // ... and without copies of A and B in that form: fp32 rows as they are, where they are whole 32-byte parts (0: not possible)
 inline int64_t unpadded_row(int64_t K) { return K % 8 == 0 && K <= 256 ? K : 0; }
 
+// What fills L2 in effect: a line that is read by SMs of both dies is kept in both halves of L2, so gathers at random begin to miss in a
+// table of half its size, and from 0.85 times its size on the misses cost more than panels do.
+constexpr double kPanelsFrom = 0.85;
+
+// Whether the short runs of a list lie side by side (k_unit_build): for the fp32 kernels, which then leave out empty slots (the bf16
+// kernel loads a unit at a time; those for rows of three pieces, and for panels of an odd number of them, load all slots), where the
+// gathers hit L2 or only long rows are cut into panels.  Poisson rows of 8, B 262 MB, K = 128 265 -> 273 us with the order, K = 256
+// 245 -> 260.  row: elements of a row of B that one launch takes; gathered: bytes of B it gathers from; l2 <= 0: not known.
+inline bool by_size(bool bf16, int64_t row, bool long_rows, double gathered, double l2) {
+    const int64_t pieces = (row + 31) / 32;
+    if (bf16 || row < 32 || pieces == 3 || (long_rows && pieces > 1 && pieces % 2 == 1)) return false;
+    return long_rows || l2 <= 0 || gathered <= kPanelsFrom * l2;
+}
+
 }  // namespace sddmm

@@ -31,6 +31,22 @@ TEST_CASE(rows_without_copies_are_the_rows_of_the_matrix) {
     }
 }
 
+TEST_CASE(the_order_of_a_list_depends_on_that_list_alone) {
+    // whole rows of an odd number of pieces are ordered, panels for their long rows are not; what the engine held before is no argument
+    const double l2 = 126e6;
+    for (int64_t row : {160, 224}) {
+        CHECK(sddmm::by_size(false, row, false, 50e6, l2));
+        CHECK(!sddmm::by_size(false, row, true, 50e6, l2));
+    }
+    for (int64_t row : {32, 64, 128, 256}) {
+        CHECK(sddmm::by_size(false, row, false, sddmm::kPanelsFrom * l2, l2));
+        CHECK(!sddmm::by_size(false, row, false, 0.86 * l2, l2));   // DRAM is the bound there
+        CHECK(sddmm::by_size(false, row, true, 3 * l2, l2));
+        CHECK(!sddmm::by_size(true, row, false, 50e6, l2));         // bf16
+    }
+    for (int64_t row : {8, 16, 24, 96}) CHECK(!sddmm::by_size(false, row, false, 50e6, l2));
+}
+
 TEST_CASE(building_a_list_loads_a_few_sums_per_tile_whatever_its_length) {
     for (int64_t rows : {int64_t(1) << 18, int64_t(2600000), int64_t(1) << 28})
         for (int64_t panels : {1, 3, 7}) {
