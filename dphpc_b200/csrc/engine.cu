@@ -373,15 +373,20 @@ void choose_long_rows(sddmm_b200_engine *e) {
     if (e->knob_long_rows == 0) return;
     const double l2 = e->l2_bytes > 0 ? e->l2_bytes : 96.0 * (1 << 20);
     const double b = gathered_bytes(e, e->seg_slices > 1 && !long_rows_whole(e) ? e->slice_cols : e->Ks);
+    const bool bf = e->mode == SDDMM_B200_BF16;
     // (see kPanelsFrom.)  Power law, rows of 25 on average, without / with: K = 32, B 94 / 117 / 131 MB 178 / 172, 233 / 214, 270 / 239 us,
     // rows of 10 93 / 92, 118 / 114, 134 / 127; K = 64, 117 MB 205 / 194; bf16 K = 64, 117 MB 320 / 281.
     if (b <= kPanelsFrom * l2 && !(e->knob_long_rows >= 1 && e->knob_panels >= 2)) return;
-    // B 333 MB, K = 32: 4 panels 407 us, 6 402 us, 8 401 us; 189 MB, 2 / 3 / 4 / 6: 300 / 287 / 286 / 286
-    e->panels_long = e->knob_panels >= 1 ? static_cast<int>(std::min(64.0, e->knob_panels)) : static_cast<int>(std::max(4.0, std::min(8.0, std::ceil(b / (0.5 * l2)))));
+    // fp32: B 333 MB, K = 32: 4 panels 407 us, 6 402 us, 8 401 us; 189 MB, 2 / 3 / 4 / 6: 300 / 287 / 286 / 286
+    // bf16, whose lists are not ordered by size and whose kernel loads all slots: a short run costs as much as a full one, so fewer
+    // panels and, with few of them, shorter rows too.  36 M, 2.6 M rows, K = 32, B 166 MB: 3 panels from 64 nonzeros on 358 us, 4
+    // panels from 128 on 363.
+    e->panels_long = e->knob_panels >= 1 ? static_cast<int>(std::min(64.0, e->knob_panels))
+                                         : static_cast<int>(std::max(bf ? 2.0 : 4.0, std::min(8.0, std::ceil(b / (0.5 * l2)))));
     if (e->panels_long < 2) return;
-    // (a power of two: the histogram's bins.  From 64 nonzeros on instead, 4 panels, K = 64, rows of 10: B 117 MB 106 -> 114 us, 189 MB
-    // 161 -> 166; K = 32 within 1 %)
-    e->long_threshold = e->knob_long_rows >= 1 ? static_cast<int>(e->knob_long_rows) : 128;
+    // (a power of two: the histogram's bins.  fp32 from 64 nonzeros on instead, 4 panels, K = 64, rows of 10: B 117 MB 106 -> 114 us,
+    // 189 MB 161 -> 166; K = 32 within 1 %)
+    e->long_threshold = e->knob_long_rows >= 1 ? static_cast<int>(e->knob_long_rows) : bf && e->panels_long <= 4 ? 64 : 128;
 }
 
 int choose_panels(const sddmm_b200_engine *e) {
