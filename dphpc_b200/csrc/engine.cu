@@ -925,7 +925,7 @@ RowSegFn pick_rowseg_wide(int pieces) {   // (nullptr: an odd number of pieces)
 }
 template <int TAIL, bool COPIES>
 RowSegFn pick_rowseg_bf16(int64_t Ks) {
-    if (Ks <= 32) return sddmm_rowseg_bf16_kernel<1, 16, 8, 3, TAIL, COPIES>;
+    if (Ks <= 32) return sddmm_rowseg_bf16_kernel<1, 16, 8, 3, COPIES && TAIL == kNoTail ? kTail : TAIL, COPIES>;   // (see RowTail)
     if (Ks <= 64) return sddmm_rowseg_bf16_kernel<1, 32, 8, 2, TAIL == kNoTail ? kTail : TAIL, COPIES>;   // (see RowTail)
     if (Ks <= 128) return sddmm_rowseg_bf16_kernel<2, 32, 4, 2, TAIL, COPIES>;
     if (Ks <= 192) return sddmm_rowseg_bf16_kernel<3, 32, 4, 1, TAIL, COPIES>;

@@ -135,11 +135,6 @@ __device__ __forceinline__ float2 group4_transpose_reduce(const float (&a)[8], i
 // K in slices, one launch each: P.val carries the sum so far, and S comes in once, with the last slice -- a product per slice would
 // make Inf - Inf of a large or infinite S value where the whole sum has a value, and reads S once per slice.  (The earlier slices
 // multiply by args.one all the same: without the instruction the compiler spills in the first slice, K = 128 256 -> 265 us.)
-// Whether some lanes of a row's last piece lie past its end: never (whole pieces: no addresses and registers for them), such lanes
-// multiply zeros, or they leave the product out.  37.5 M nonzeros, bf16 K = 32 / 128 373 -> 344 / 1117 -> 1067 us without the logic, 6 M
-// K = 128 220 -> 215, 3 M K = 256 213 -> 190.  (The kernel for B beyond L2 keeps one form, without the
-// logic its registers spill; so do rows of three pieces, K = 96: 44 against 46 us, and bf16 rows of 64, 10 M K = 64: 109 against 123.)
-enum RowTail : int { kNoTail, kTail, kTailSpecials };
 enum SliceStep : int { kWholeRows, kFirstSlice, kNextSlice, kLastSlice };
 __device__ __forceinline__ constexpr bool step_adds(int step) { return step == kNextSlice || step == kLastSlice; }
 __device__ __forceinline__ constexpr bool step_scales(int step) { return step == kWholeRows || step == kLastSlice; }
@@ -147,6 +142,13 @@ template <int STEP>
 __device__ __forceinline__ float step_value(float dot, float p, float s) {
     return (step_adds(STEP) ? p + dot : dot) * s;
 }
+
+// Whether some lanes of a row's last piece lie past its end: never (whole pieces: no addresses and registers for them), such lanes
+// multiply zeros, or they leave the product out.  Without the logic: 6 M nonzeros, K = 128 220 -> 215 us, 3 M, K = 256 213 -> 190; bf16,
+// K = 128, 37.5 M 1117 -> 1067, K = 32, 5.2 M 55 -> 44.  It stays where the kernel is slower without: for B beyond L2 (one form, its
+// registers spill), rows of three pieces (K = 96: 44 against 46 us), bf16 rows of 64 (10 M: 109 against 123) and bf16 rows of 32 in
+// panels (power law, 36 M: 349 against 358; Poisson rows of 30, 65 M: 696 against 721).
+enum RowTail : int { kNoTail, kTail, kTailSpecials };
 
 // How many stages before its load a piece of A is asked into L2.  A row of A is used by one or two units and comes from HBM,
 // whose latency under load is longer than a stage: 9 M nonzeros, B in L2, K = 256: 880 us without, 725 with (K = 64 185 -> 168,
