@@ -990,7 +990,12 @@ int enqueue_units(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_
     }
     const bool scanned = tiles > kDirectTiles;
     if (scanned) k_scan_sums<<<1, kScanBlock, 0, s>>>(e->d_scan_tiles, tiles, &e->d_pc->units);
-    k_unit_build<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, skip_hint, by_size);
+    if constexpr (sizeof(HDR) == sizeof(int2)) {
+        if (by_size) k_unit_build<Runs, HDR, true><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, skip_hint);
+        else k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, skip_hint);
+    } else {
+        k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, skip_hint);
+    }
     CU_TRY(e, cudaGetLastError());
     return SDDMM_B200_OK;
 }

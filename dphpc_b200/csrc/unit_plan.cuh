@@ -106,25 +106,25 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs runs, int64_t n, 
 constexpr unsigned kShortRowShare = 16;
 
 // pass 2: the units of a tile.  HDR = int2 (plain units) or int4 (row groups).  scanned: tile_sums holds the units before each tile.
-template <typename Runs, typename HDR>
+// BY_SIZE, plain units, where the row statistics bear it out: the tile's runs of 8 nonzeros or more come first, then the shorter ones, a
+// unit each, from 7 nonzeros down to 1, so that the units of a warp step are of one size and the gather kernel can leave out the slots
+// that none of them fills.  (Longer runs keep their units together: with their last ones sorted too, the units of a row are read by
+// different SMs, and where DRAM is the bound, rows of 26 in two panels, K = 32 takes 540 us instead of 465.  A kernel of its own: with
+// the order as an argument only, power-law panels of 36 M nonzeros take 454 us to build instead of 423.)
+template <typename Runs, typename HDR, bool BY_SIZE>
 __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n, const int32_t *__restrict__ tile_sums, int64_t cap,
                                                            const PlanCounters *__restrict__ pc, HDR *__restrict__ units,
-                                                           int32_t *__restrict__ unit_cols, bool scanned, unsigned long long skip_hint, bool by_size) {
+                                                           int32_t *__restrict__ unit_cols, bool scanned, unsigned long long skip_hint) {
     // enqueued before the host has seen the counters: nothing is written for a pattern that it is about to refuse, or for one
     // that will be computed otherwise
     if (pc->window_hint >= skip_hint) return;
     if (pc->bad_row_ptr || pc->bad_coo || (Runs::kSorted && pc->unsorted_cols)) return;
-    if (by_size) by_size = kShortRowShare * (pc->hist[1] + pc->hist[2] + pc->hist[3]) >= pc->rows_nonempty;   // (rows of 1 .. 7 nonzeros)
+    const bool by_size = BY_SIZE && kShortRowShare * (pc->hist[1] + pc->hist[2] + pc->hist[3]) >= pc->rows_nonempty;   // (rows of 1 .. 7 nonzeros)
     constexpr int kPerThread = kUnitTileMax / kUnitBlock;
     __shared__ int32_t first_unit[kUnitTileMax];   // of the tile's entries, relative to the tile
     __shared__ int32_t start[kUnitTileMax], length[kUnitTileMax];
-    // by_size, plain units (HDR = int2): the tile's runs of 8 nonzeros or more come first, then the shorter ones, a unit each, from 7
-    // nonzeros down to 1, so that the units of a warp step are of one size and the gather kernel can leave out the slots that none of
-    // them fills.  (Longer runs keep their units together: with their last ones sorted too, the units of a row are read by different
-    // SMs, and where DRAM is the bound, rows of 26 in two panels, K = 32 takes 540 us instead of 465.)
-    constexpr bool kBySize = sizeof(HDR) == sizeof(int2);
     __shared__ int32_t of_size[8];                 // short runs of each length; then the first one's place
-    __shared__ int32_t short_run[kBySize ? kUnitTileMax : 1];   // their entries, by place
+    __shared__ int32_t short_run[BY_SIZE ? kUnitTileMax : 1];   // their entries, by place
     const int tile = unit_tile(n);
     int64_t before = 0;
     if (scanned) {
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n,
     const int64_t base = static_cast<int64_t>(blockIdx.x) * tile;
     const int per_thread = (tile + kUnitBlock - 1) / kUnitBlock;
     int32_t cnt[kPerThread], rank[kPerThread], local = 0;
-    if (kBySize && by_size) {
+    if (by_size) {
         if (threadIdx.x < 8) of_size[threadIdx.x] = 0;
         __syncthreads();
     }
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n,
         if (base + i < n) runs.run(base + i, s, e);
         start[i] = s;
         length[i] = e - s;
-        const bool is_short = kBySize && by_size && e > s && e - s < 8;
+        const bool is_short = by_size && e > s && e - s < 8;
         cnt[k] = is_short ? 0 : (e - s + 7) >> 3;
         local += cnt[k];
         if (is_short) rank[k] = atomicAdd(&of_size[e - s], 1);   // (their order has no effect on any result)
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n,
     int32_t total;
     int32_t at = block_inclusive_scan(local, &total) - local;
     const int32_t in_order = total;
-    if (kBySize && by_size) {
+    if (by_size) {
         if (threadIdx.x == 0)
             for (int n = 7; n > 0; --n) {
                 const int32_t c = of_size[n];
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n,
         const int i = threadIdx.x * per_thread + k;
         if (k < per_thread && i < tile) {
             first_unit[i] = at;
-            if (kBySize && by_size && length[i] > 0 && length[i] < 8) short_run[of_size[length[i]] + rank[k] - in_order] = i;
+            if (by_size && length[i] > 0 && length[i] < 8) short_run[of_size[length[i]] + rank[k] - in_order] = i;
         }
         at += cnt[k];
     }
@@ -190,14 +190,14 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n,
             u[k] = min(u0 + k * kGroups, total - 1);
             entry[k] = 0;
         }
-        for (int half = u0 < in_order ? tile >> 1 : 0; half > 0; half >>= 1)   // the entry that holds unit u: the last one that starts at or before it (tile: a power of two)
+        for (int half = !BY_SIZE || u0 < in_order ? tile >> 1 : 0; half > 0; half >>= 1)   // the entry that holds unit u: the last one that starts at or before it (tile: a power of two)
 #pragma unroll
             for (int k = 0; k < kBatch; ++k)
                 if (first_unit[entry[k] + half] <= u[k]) entry[k] += half;
 #pragma unroll
         for (int k = 0; k < kBatch; ++k) {
-            if (kBySize && u[k] >= in_order) entry[k] = short_run[u[k] - in_order];
-            const int32_t skip = kBySize && u[k] >= in_order ? 0 : 8 * (u[k] - first_unit[entry[k]]);
+            if (BY_SIZE && u[k] >= in_order) entry[k] = short_run[u[k] - in_order];
+            const int32_t skip = BY_SIZE && u[k] >= in_order ? 0 : 8 * (u[k] - first_unit[entry[k]]);
             first[k] = start[entry[k]] + skip;
             count[k] = min(8, length[entry[k]] - skip);
             c[k] = runs.col[first[k] + min(slot, count[k] - 1)];
