@@ -981,7 +981,7 @@ bool list_by_size(const sddmm_b200_engine *e, int32_t long_rows) {
 // sums and the total.
 template <typename Runs, typename HDR>
 int enqueue_units(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_t n, bool have_sums, int64_t cap, HDR *units, int32_t *unit_cols,
-                  unsigned long long skip_hint = ~0ull, bool by_size = false) {
+                  const ListGate &gate = ListGate{}, bool by_size = false) {
     const int tiles = static_cast<int>(unit_tiles(n));
     if (int rc = check_tile_sums(e, tiles)) return rc;
     if (!have_sums) {
@@ -991,35 +991,38 @@ int enqueue_units(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_
     const bool scanned = tiles > kDirectTiles;
     if (scanned) k_scan_sums<<<1, kScanBlock, 0, s>>>(e->d_scan_tiles, tiles, &e->d_pc->units);
     if constexpr (sizeof(HDR) == sizeof(int2)) {
-        if (by_size) k_unit_build<Runs, HDR, true><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, skip_hint);
-        else k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, skip_hint);
+        if (by_size) k_unit_build<Runs, HDR, true><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate);
+        else k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate);
     } else {
-        k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, skip_hint);
+        k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate);
     }
     CU_TRY(e, cudaGetLastError());
     return SDDMM_B200_OK;
 }
 
+// Gathers of B that have to disappear before row groups are taken.  They have to be 30 % of all.
 // Matching the groups and building their list takes 30 to 40 us and 10 us per million nonzeros, which a plan of one run does not get
 // back (190 000 nonzeros, K = 16, uploaded and run: 112 us, 148 with groups; 2 M, K = 128, 190 / 222).  So the gathers that disappear have to be worth
 // something, at the rate of the L2 -> SM fabric (rows of less than a line at a line's): 4 us of a run in bf16, 60 in fp32, but for
 // rows of 32 and 64 elements, which have always been taken.  Knob "group_units" = 1: whatever they are worth.
-bool groups_pay(const sddmm_b200_engine *e, double gathers) {
+double groups_from(const sddmm_b200_engine *e) {
     const bool bf = e->mode == SDDMM_B200_BF16;
-    if (!e->use_seg || e->knob_group_units >= 0 || (!bf && (e->Ks == 32 || e->Ks == 64))) return true;
-    return gathers * std::max(128.0, static_cast<double>(e->Ks) * static_cast<double>(elem_bytes(e))) / 18.6e6 >= (bf ? 4.0 : 60.0);
+    const double share = 0.3 * static_cast<double>(e->nnz);
+    if (!e->use_seg || e->knob_group_units >= 0 || (!bf && (e->Ks == 32 || e->Ks == 64))) return share;
+    return std::max(share, (bf ? 4.0 : 60.0) * 18.6e6 / std::max(128.0, static_cast<double>(e->Ks) * static_cast<double>(elem_bytes(e))));
 }
 
 bool group_possible(const sddmm_b200_engine *e) {
-    if (!groups_pay(e, 0.75 * static_cast<double>(e->nnz))) return false;   // (groups of four rows throughout)
+    if (0.75 * static_cast<double>(e->nnz) < groups_from(e)) return false;   // (groups of four rows throughout)
     if ((e->flags & SDDMM_B200_FLAG_NO_ROW_GROUPS) || e->M < 4) return false;
     if (e->knob_group_units != 0 && e->use_seg) return pick_rowseg_group(e, 2) != nullptr;
     return e->mode != SDDMM_B200_BF16 && (e->K == 32 || e->K == 64);
 }
 // candidates: G = 2, 3, 4 rows per group, first full group starting at row 0 .. G-1 (counters slot = G(G-1)/2 - 1 + first)
 int group_slot(int G, int first) { return G * (G - 1) / 2 - 1 + first; }
-// G and `first` are chosen on a sample of the groups (about 8 000 rows' worth, at most 1 in 16 of them); the chosen grouping is then matched exactly
-int group_sample(const sddmm_b200_engine *e) { return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(16, e->M / 8192))); }
+// G and `first` are chosen on a sample of the groups (about 8 000 rows' worth, at most 1 in 64 of them); the chosen grouping is then matched exactly.
+// (At most 1 in 16, every upload of a large matrix pays: 2.6 M rows 51 us, 1 in 64 MEASURE.)
+int group_sample(const sddmm_b200_engine *e) { return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(64, e->M / 8192))); }
 int enqueue_group_sample(sddmm_b200_engine *e) {
     const int every = group_sample(e);
     const dim3 grid(grid_for((e->M / 2 / every + 2) * 32, kBlock, e->sm_count * 2), 9);
@@ -1033,21 +1036,14 @@ int enqueue_group_sample(sddmm_b200_engine *e) {
 // The path is taken (for the whole matrix) when it removes at least 30 % of the gathers; K <= 256.
 // base_pc: counters that include enqueue_group_sample's.
 int build_rowgroup_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
-    if (!group_possible(e) || base_pc.max_row_nnz > 8192) return SDDMM_B200_OK;
+    if (!group_possible(e) || base_pc.max_row_nnz > kGroupRowMax) return SDDMM_B200_OK;
     cudaStream_t s = e->stream;
     const int every = group_sample(e);
     const int32_t M = static_cast<int32_t>(e->M), nnz = static_cast<int32_t>(e->nnz);
-    int best = 0, best_first = 0;
-    double best_saved = 0.0;
-    for (int G = 2; G <= 4; ++G)
-        for (int first = 0; first < G; ++first) {
-            const double saved = static_cast<double>(base_pc.group_cover[group_slot(G, first)]) * every * (1.0 - 1.0 / G);   // gathers of B that disappear (estimate)
-            if (saved > best_saved) { best_saved = saved; best = G; best_first = first; }
-        }
-    if (best == 0 || best_saved < 0.3 * static_cast<double>(e->nnz)) return SDDMM_B200_OK;
-    if (!groups_pay(e, best_saved)) return SDDMM_B200_OK;
+    int bs = 0;
+    if (group_saving(base_pc.group_cover, every, &bs) < groups_from(e)) return SDDMM_B200_OK;
+    const int best = bs < 2 ? 2 : bs < 5 ? 3 : 4, best_first = bs - group_slot(best, 0);
     const int32_t n_groups = group_count(M, best, best_first);
-    const int bs = group_slot(best, best_first);
     const bool units = e->knob_group_units != 0 && e->use_seg;
     e->group_tried = true;
     // exact match of the chosen grouping, and -- speculating that the sample was right -- the unit list over it
@@ -1127,18 +1123,16 @@ int build_residual_units(sddmm_b200_engine *e) {
 
 // Enqueue the unit list over the whole matrix with `panels` column panels (1: whole rows, whose tile sums k_row_stats has
 // left when have_sums; long_rows: see RunsOfPanels).
-int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, int32_t panels, int32_t long_rows, bool have_sums, bool unless_tiles = false) {
+int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, int32_t panels, int32_t long_rows, bool have_sums, const ListGate &gate = ListGate{}) {
     const int32_t M = static_cast<int32_t>(e->M), nnz = static_cast<int32_t>(e->nnz);
     const int64_t n = static_cast<int64_t>(panels) * M;
-    // (fp32 mode: tiles will most likely be looked for, and found, when the column scan's count is high enough -- no list then)
-    const unsigned long long skip = unless_tiles ? (static_cast<unsigned long long>(e->nnz) + kTileHintShare - 1) / kTileHintShare : ~0ull;
     int st;
     if (panels > 1) {
         const RunsOfPanels runs{e->d_rp, e->d_col, M, nnz, panels, e->panel_cols, long_rows};
-        st = enqueue_units(e, s, runs, n, false, e->unit_cap, e->d_units, e->d_unit_cols, skip, list_by_size(e, long_rows));
+        st = enqueue_units(e, s, runs, n, false, e->unit_cap, e->d_units, e->d_unit_cols, gate, list_by_size(e, long_rows));
     } else {
         const RunsOfRows runs{e->d_rp, e->d_col, M, nnz};
-        st = enqueue_units(e, s, runs, n, have_sums, e->unit_cap, e->d_units, e->d_unit_cols, skip, list_by_size(e, long_rows));
+        st = enqueue_units(e, s, runs, n, have_sums, e->unit_cap, e->d_units, e->d_unit_cols, gate, list_by_size(e, long_rows));
     }
     if (st) return st;
     if (e->mode == SDDMM_B200_BF16) k_unit_pad<<<1, 64, 0, s>>>(e->d_units, e->d_unit_cols, e->d_pc, e->unit_cap);
@@ -1224,7 +1218,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     const bool tiles_first = e->dense_possible && e->mode != SDDMM_B200_FP32;   // (fp32 mode: tiles are the exception)
     const bool no_panels = e->panels_plain == 1 && e->long_threshold == 0;   // (else the row statistics decide first)
     const bool whole_rows = e->use_seg && !tiles_first && no_panels;
-    bool early_list = whole_rows && e->nnz > 0;
+    const bool early_list = whole_rows && e->nnz > 0;
     k_row_stats<<<static_cast<int>(unit_tiles(e->M)), kUnitBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, e->d_rowstart,
                                                                                             whole_rows ? e->d_scan_tiles : nullptr, e->d_pc);
     // The list of whole rows needs the row statistics only: where the operands come from this GPU's memory it is built on the side
@@ -1232,11 +1226,17 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     // nonzeros, K = 64, upload and run 272 -> 256 us; 4 M, power law, 266 -> 249).  Not for rows long enough to lie in 64-wide tiles,
     // where the count of the column scan may make the list unnecessary (18 M in 64 x 64 blocks, upload 489 us, 572 with the list aside).
     const bool list_aside = early_list && join_copies && e->nnz < 64 * e->M;
+    ListGate gate;
+    if (e->nnz > 0 && group_possible(e)) {
+        if (int rc = enqueue_group_sample(e)) return rc;
+        gate.groups_from = groups_from(e);
+        gate.every = group_sample(e);
+    }
     if (list_aside) {
         CU_TRY(e, cudaEventRecord(e->ev_fork, s));
         CU_TRY(e, cudaStreamWaitEvent(e->side_stream, e->ev_fork, 0));
-        // (whatever the column scan will have counted: its count grows while the list's blocks would look at it)
-        if (int rc = enqueue_unit_list(e, e->side_stream, 1, 0, true)) return rc;
+        gate.columns_scanned = false;
+        if (int rc = enqueue_unit_list(e, e->side_stream, 1, 0, true, gate)) return rc;
         CU_TRY(e, cudaEventRecord(e->ev_join, e->side_stream));
     }
     if (e->nnz > 0) {
@@ -1250,10 +1250,11 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
             k_col_scan<false><<<scan_blocks, kColScanThreads, 0, s>>>(e->d_col, e->nnz, static_cast<int32_t>(e->N), e->d_rowstart, e->d_touched, e->d_pc);
         }
         CU_TRY(e, cudaGetLastError());
-        if (group_possible(e))
-            if (int rc = enqueue_group_sample(e)) return rc;
-        if (early_list && !list_aside)
-            if (int rc = enqueue_unit_list(e, s, 1, 0, true, e->dense_possible && e->knob_offset_tiles <= 0)) return rc;
+        if (early_list && !list_aside) {
+            // (fp32 mode: tiles will most likely be looked for, and found, when the column scan's count is high enough)
+            if (e->dense_possible && e->knob_offset_tiles <= 0) gate.tile_hint = (static_cast<unsigned long long>(e->nnz) + kTileHintShare - 1) / kTileHintShare;
+            if (int rc = enqueue_unit_list(e, s, 1, 0, true, gate)) return rc;
+        }
     }
     if (list_aside) CU_TRY(e, cudaStreamWaitEvent(s, e->ev_join, 0));
     CU_TRY(e, cudaGetLastError());
@@ -1266,8 +1267,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     if (int rc = read_counters(e, &pc)) return rc;
     if (pc.bad_coo) return fail(e, SDDMM_B200_ERR_INDEX, "COO row indices must be sorted and inside [0, M)");
     if (pc.bad_row_ptr) return fail(e, SDDMM_B200_ERR_INDEX, "row_ptr must start at 0, end at nnz and be non-decreasing");
-    if (!list_aside && e->dense_possible && e->knob_offset_tiles <= 0 && pc.window_hint * kTileHintShare >= static_cast<unsigned long long>(e->nnz))
-        early_list = false;   // (it was left out)
+    const bool list_built = early_list && pc.list_built != 0;
     if (pc.bad_col) return fail(e, SDDMM_B200_ERR_INDEX, "column index outside [0, N)");
 
     sddmm_b200_plan_info &p = e->plan;
@@ -1307,7 +1307,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         if (st) return st;
         if (e->rg_rows) return SDDMM_B200_OK;
         // (a grouping that was tried and dropped has used the list's memory)
-        st = build_rowseg_plan(e, pc, early_list && !e->group_tried);
+        st = build_rowseg_plan(e, pc, list_built && !e->group_tried);
         if (st) return st;
         if (e->use_seg) return SDDMM_B200_OK;
     }

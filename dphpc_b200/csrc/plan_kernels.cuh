@@ -35,6 +35,7 @@ struct PlanCounters {
     unsigned long long window_hint;      // nonzeros (estimate from every fourth one) whose 31st successor lies less than 64 columns ahead
     int block_samples;                   // sampled nonzeros that lie in what looks like a 64x64 block
     int n_anchors;                       // candidate origins of the arbitrary-offset tile detection
+    int list_built;                      // 1: a list that was enqueued early has been written (see ListGate)
 };
 
 __device__ __forceinline__ int len_bin(int len) {

@@ -101,6 +101,31 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs runs, int64_t n, 
     }
 }
 
+// What may show that a list enqueued before the host has seen the counters will not be used (default: nothing).  k_unit_build reads
+// here only what kernels BEFORE it in its stream have finished: threads of one block that saw a count grow would disagree.
+struct ListGate {
+    unsigned long long tile_hint = ~0ull;   // nonzeros that look like 64-wide tiles from which on these will be looked for, and found
+    double groups_from = -1.0;              // gathers saved by row groups from which on these will be taken (< 0: not looked at)
+    int every = 1;                          // of how many groups one is in the sample
+    bool columns_scanned = true;            // false: the column scan runs beside (nothing that it counts is read)
+};
+// Gathers that the best grouping saves, by the sample, and its slot
+__host__ __device__ __forceinline__ double group_saving(const unsigned long long *cover, int every, int *slot) {
+    double best = 0.0;
+    for (int y = 0; y < 9; ++y) {
+        const int G = y < 2 ? 2 : y < 5 ? 3 : 4;
+        const double saved = static_cast<double>(cover[y]) * every * (1.0 - 1.0 / G);
+        if (saved > best) { best = saved; *slot = y; }
+    }
+    return best;
+}
+constexpr int kGroupRowMax = 8192;   // (nonzeros of a row) matrices with longer ones are not grouped
+__device__ __forceinline__ bool list_unused(const ListGate &gate, const PlanCounters *pc) {
+    if (gate.columns_scanned && pc->window_hint >= gate.tile_hint) return true;
+    int slot;
+    return gate.groups_from >= 0.0 && pc->max_row_nnz <= kGroupRowMax && group_saving(pc->group_cover, gate.every, &slot) >= gate.groups_from;
+}
+
 // A list is ordered by size (k_unit_build) from one short row in this many on: with fewer the kernel gains nothing and building takes
 // longer (5.2 M nonzeros in rows of 26: upload and run 247 us, 250 with the order).  Not where DRAM is the bound, see list_by_size.
 constexpr unsigned kShortRowShare = 16;
@@ -113,12 +138,13 @@ constexpr unsigned kShortRowShare = 16;
 // the order as an argument only, power-law panels of 36 M nonzeros take 454 us to build instead of 423.)
 template <typename Runs, typename HDR, bool BY_SIZE>
 __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n, const int32_t *__restrict__ tile_sums, int64_t cap,
-                                                           const PlanCounters *__restrict__ pc, HDR *__restrict__ units,
-                                                           int32_t *__restrict__ unit_cols, bool scanned, unsigned long long skip_hint) {
+                                                           PlanCounters *__restrict__ pc, HDR *__restrict__ units,
+                                                           int32_t *__restrict__ unit_cols, bool scanned, ListGate gate) {
     // enqueued before the host has seen the counters: nothing is written for a pattern that it is about to refuse, or for one
     // that will be computed otherwise
-    if (pc->window_hint >= skip_hint) return;
+    if (list_unused(gate, pc)) return;
     if (pc->bad_row_ptr || pc->bad_coo || (Runs::kSorted && pc->unsorted_cols)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) pc->list_built = 1;
     const bool by_size = BY_SIZE && kShortRowShare * (pc->hist[1] + pc->hist[2] + pc->hist[3]) >= pc->rows_nonempty;   // (rows of 1 .. 7 nonzeros)
     constexpr int kPerThread = kUnitTileMax / kUnitBlock;
     __shared__ int32_t first_unit[kUnitTileMax];   // of the tile's entries, relative to the tile
