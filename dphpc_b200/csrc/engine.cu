@@ -1000,16 +1000,24 @@ int enqueue_units(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_
     return SDDMM_B200_OK;
 }
 
-// Gathers of B that have to disappear before row groups are taken.  They have to be 30 % of all.
-// Matching the groups and building their list takes 30 to 40 us and 10 us per million nonzeros, which a plan of one run does not get
-// back (190 000 nonzeros, K = 16, uploaded and run: 112 us, 148 with groups; 2 M, K = 128, 190 / 222).  So the gathers that disappear have to be worth
-// something, at the rate of the L2 -> SM fabric (rows of less than a line at a line's): 4 us of a run in bf16, 60 in fp32, but for
-// rows of 32 and 64 elements, which have always been taken.  Knob "group_units" = 1: whatever they are worth.
+// Gathers of B that have to disappear before row groups are taken: 30 % of all, and as many as are worth the planning.  What they save
+// of a run is estimated at the rate of the L2 -> SM fabric (rows of less than a line at a line's; rows that leave lanes idle save
+// less, K = 96, 3.7 M nonzeros: 34 us of 51).  What groups cost is a second look at the counters, the match and a list that cannot be
+// built beside the column scan.
+//   fp32: 30 to 50 us, so that a single run pays from about 45 us on.  Upload and run, without / with groups: K = 128, 1 / 2 / 3.7 M
+//     nonzeros (18 / 37 / 67 us) 134 / 167, 178 / 181, 235 / 223 us; K = 256, 1 / 2 M (37 / 73) 167 / 170, 246 / 218; K = 96, 3.7 M (38) 205 / 230.
+//   fp32 rows of 32 and 64: taken whatever they save.  These are what plans that are held and run again have counted on (without /
+//     with, 1 M: K = 32 19.4 / 13.6 us a run, K = 64 25.7 / 16.4), and a single run, 122 / 160 and 124 / 160 us, is not slower than it was.
+//   bf16: 5 to 15 us (no list is built early there, tiles are looked for first), back by the fourth run from 4 us on: K = 64, 1 / 2 /
+//     3.7 M (4.6 / 9.2 / 17 us) 169 / 179, 193 / 202, 225 / 222 us, a held run 18 / 14, 28 / 19, 43 / 29.
+// Knob "group_units" = 1: whatever they are worth.
 double groups_from(const sddmm_b200_engine *e) {
     const bool bf = e->mode == SDDMM_B200_BF16;
     const double share = 0.3 * static_cast<double>(e->nnz);
     if (!e->use_seg || e->knob_group_units >= 0 || (!bf && (e->Ks == 32 || e->Ks == 64))) return share;
-    return std::max(share, (bf ? 4.0 : 60.0) * 18.6e6 / std::max(128.0, static_cast<double>(e->Ks) * static_cast<double>(elem_bytes(e))));
+    const double bytes = std::max(128.0, static_cast<double>(e->Ks) * static_cast<double>(elem_bytes(e)));
+    const double used = bf || e->Ks <= 32 ? 1.0 : static_cast<double>(e->Ks) / (8.0 * group_lanes(e));   // of a row's lanes
+    return std::max(share, (bf ? 4.0 : 45.0) * 18.6e6 / (bytes * used));
 }
 
 bool group_possible(const sddmm_b200_engine *e) {
@@ -1021,7 +1029,7 @@ bool group_possible(const sddmm_b200_engine *e) {
 // candidates: G = 2, 3, 4 rows per group, first full group starting at row 0 .. G-1 (counters slot = G(G-1)/2 - 1 + first)
 int group_slot(int G, int first) { return G * (G - 1) / 2 - 1 + first; }
 // G and `first` are chosen on a sample of the groups (about 8 000 rows' worth, at most 1 in 64 of them); the chosen grouping is then matched exactly.
-// (At most 1 in 16, every upload of a large matrix pays: 2.6 M rows 51 us, 1 in 64 MEASURE.)
+// (At most 1 in 16, every upload of a large matrix pays: 2.6 M rows 51 us, 1 in 64 19.)
 int group_sample(const sddmm_b200_engine *e) { return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(64, e->M / 8192))); }
 int enqueue_group_sample(sddmm_b200_engine *e) {
     const int every = group_sample(e);
