@@ -163,7 +163,6 @@ struct sddmm_b200_engine {
     int64_t unit_cap = 0;
     int32_t panels_plain = 1;          // column panels when every row is cut
     int32_t panels_long = 1, long_threshold = 0;   // ... when only rows of at least long_threshold (> 0) nonzeros are; the row statistics choose
-    int32_t panel_cols = 0;            // columns per panel of the list in use
     int32_t n_units = 0;
     bool use_seg = false;
     bool seg_residual = false;         // the row-segment kernel computes what the dense tiles left (units over the uncovered runs)
@@ -606,6 +605,15 @@ void settle_specials(sddmm_b200_engine *e) {
     e->specials_known = true;
 }
 
+// the units' copies of S.val follow every change of S.val
+int refresh_unit_values(sddmm_b200_engine *e) {
+    if (!e->use_seg || !e->seg_copies || e->n_units == 0) return SDDMM_B200_OK;
+    k_unit_values<<<grid_for(8 * static_cast<int64_t>(e->n_units), kBlock, e->sm_count * 32), kBlock, 0, e->stream>>>(e->d_units, e->n_units, e->d_sval,
+                                                                                                                e->d_unit_sval);
+    CU_TRY(e, cudaGetLastError());
+    return SDDMM_B200_OK;
+}
+
 int convert_storage(sddmm_b200_engine *e) {
     const int cap = e->sm_count * 8;
     e->specials_known = false;
@@ -613,11 +621,7 @@ int convert_storage(sddmm_b200_engine *e) {
     const int32_t last_part = static_cast<int32_t>((seg_row_bytes(e) - seg_part_bytes(e)) / static_cast<int32_t>(elem_bytes(e)));
     *static_cast<volatile int32_t *>(e->h_specials) = 0;
     if (seen) CU_TRY(e, cudaMemsetAsync(seen, 0, sizeof(int32_t), e->stream));
-    if (e->use_seg && e->seg_copies && e->n_units > 0) {   // the units' copies of S.val follow every change of S.val
-        k_unit_values<<<grid_for(8 * static_cast<int64_t>(e->n_units), kBlock, cap * 4), kBlock, 0, e->stream>>>(e->d_units, e->n_units, e->d_sval,
-                                                                                                           e->d_unit_sval);
-        CU_TRY(e, cudaGetLastError());
-    }
+    if (int rc = refresh_unit_values(e)) return rc;
     if (e->d_Ax && e->n_dense > 0) {  // hi/lo-concatenated operands of the fp32-grade tensor-core mode (only when tiles were found)
         k_split_concat_tf32<<<grid_for(e->M * e->K, kBlock, cap), kBlock, 0, e->stream>>>(e->d_A32, e->d_Ax, e->M, static_cast<int32_t>(e->K), 1);
         k_split_concat_tf32<<<grid_for(e->N * e->K, kBlock, cap), kBlock, 0, e->stream>>>(e->d_B32, e->d_Bx, e->N, static_cast<int32_t>(e->K), 0);
@@ -1129,18 +1133,37 @@ int build_residual_units(sddmm_b200_engine *e) {
     return seg_grid(e, reinterpret_cast<const void *>(seg_function(e, false)), kRowSegWarps, 8, e->n_units, &e->plan.rowseg_grid);
 }
 
-// Enqueue the unit list over the whole matrix with `panels` column panels (1: whole rows, whose tile sums k_row_stats has
-// left when have_sums; long_rows: see RunsOfPanels).
-int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, int32_t panels, int32_t long_rows, bool have_sums, const ListGate &gate = ListGate{}) {
+// The forms of the list over the whole matrix
+ListForms list_forms(const sddmm_b200_engine *e) {
+    ListForms f;
+    f.plain = e->panels_plain;
+    f.plain_cols = static_cast<int32_t>((e->N + f.plain - 1) / f.plain);
+    f.plain_for_8 = e->nnz < 16 * e->M && e->knob_panels < 1;
+    f.plain_by_size = list_by_size(e, 0);
+    if (e->long_threshold > 0) {
+        f.longs = e->panels_long;
+        f.long_cols = static_cast<int32_t>((e->N + f.longs - 1) / f.longs);
+        f.long_rows = e->long_threshold;
+        f.long_always = e->knob_long_rows >= 0;
+        f.long_by_size = list_by_size(e, f.long_rows);
+    }
+    return f;
+}
+
+// Enqueue the list over the whole matrix.  have_sums: k_row_stats has left the tile sums of whole rows.
+int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, const ListForms &forms, bool have_sums, const ListGate &gate = ListGate{}) {
     const int32_t M = static_cast<int32_t>(e->M), nnz = static_cast<int32_t>(e->nnz);
-    const int64_t n = static_cast<int64_t>(panels) * M;
     int st;
-    if (panels > 1) {
-        const RunsOfPanels runs{e->d_rp, e->d_col, M, nnz, panels, e->panel_cols, long_rows};
-        st = enqueue_units(e, s, runs, n, false, e->unit_cap, e->d_units, e->d_unit_cols, gate, list_by_size(e, long_rows));
+    if (forms.plain > 1 || forms.long_rows > 0) {
+        const RunsOfForms runs{e->d_rp, e->d_col, M, nnz, forms};
+        // (a grid for either form: the longer list, or the one with more tiles)
+        const int64_t n_plain = e->M * forms.plain, n_long = forms.long_rows > 0 ? e->M * (forms.longs + 1) : 0;
+        const int64_t n = unit_tiles(n_long) > unit_tiles(n_plain) ? n_long : n_plain;
+        const int64_t n_whole = forms.plain_for_8 && unit_tiles(e->M) > unit_tiles(n) ? e->M : n;
+        st = enqueue_units(e, s, runs, n_whole, false, e->unit_cap, e->d_units, e->d_unit_cols, gate, forms.plain_by_size || forms.long_by_size);
     } else {
         const RunsOfRows runs{e->d_rp, e->d_col, M, nnz};
-        st = enqueue_units(e, s, runs, n, have_sums, e->unit_cap, e->d_units, e->d_unit_cols, gate, list_by_size(e, long_rows));
+        st = enqueue_units(e, s, runs, e->M, have_sums, e->unit_cap, e->d_units, e->d_unit_cols, gate, forms.plain_by_size);
     }
     if (st) return st;
     if (e->mode == SDDMM_B200_BF16) k_unit_pad<<<1, 64, 0, s>>>(e->d_units, e->d_unit_cols, e->d_pc, e->unit_cap);
@@ -1148,57 +1171,55 @@ int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, int32_t panels, int3
     return SDDMM_B200_OK;
 }
 
-// Row segments over the whole matrix.  built: panels of the list that is already there (0: none), counted in pc.
-int build_rowseg_plan(sddmm_b200_engine *e, PlanCounters pc, bool built) {
+// Row segments over the whole matrix.  early: the forms of the list that is already there, counted in pc (null: none).
+int build_rowseg_plan(sddmm_b200_engine *e, PlanCounters pc, const ListForms *early) {
     e->seg_copies = false;
     e->n_units = 0;
     if (!e->use_seg) return SDDMM_B200_OK;
-    // (a panel run is a contiguous piece of a row only when its columns are sorted)
-    auto panels_for_long_rows = [&]() -> bool {
-        if (e->long_threshold <= 0 || pc.unsorted_cols) return false;
-        if (e->knob_long_rows >= 0) return true;
-        unsigned long long in_long = 0;   // they only pay when those rows hold a good share of the nonzeros
-        for (int b = 1; b < SDDMM_B200_HIST_BINS; ++b)
-            if ((1ll << (b - 1)) >= e->long_threshold) in_long += pc.hist_nnz[b];
-        return 5 * in_long >= 2 * static_cast<unsigned long long>(e->nnz);   // 40 %
+    auto choose = [&]() -> ListForms::Choice {
+        ListForms f = list_forms(e);
+        if (pc.unsorted_cols) {   // (a panel run is a contiguous piece of a row only when its columns are sorted)
+            f.plain = 1;
+            f.long_rows = 0;
+        }
+        return f.choose(&pc, e->nnz);
     };
-    bool use_long = panels_for_long_rows();
-    if (e->slice_major && e->knob_k_slices < 0 && (use_long || pc.unsorted_cols || e->panels_plain == 1)) {
+    ListForms::Choice c = choose();
+    if (e->slice_major && e->knob_k_slices < 0 && (c.long_rows > 0 || pc.unsorted_cols || e->panels_plain == 1)) {
         e->slice_major = false;   // (slices_apart: the copies pay with plain panels only)
         if (e->Ks == e->K) e->d_Ap = e->d_Bp = nullptr;
         choose_list_forms(e);
-        use_long = panels_for_long_rows();
+        c = choose();
     }
-    int32_t plain = e->panels_plain;
-    if (plain > 1 && e->nnz < 16 * e->M && e->knob_panels < 1) {
-        // a mean that barely pays for panels has to be that of most rows, not of a few long ones: 60 % of them of 8 nonzeros or more
-        unsigned long long rows = 0, of_8 = 0;
-        for (int b = 1; b < SDDMM_B200_HIST_BINS; ++b) {
-            rows += pc.hist[b];
-            if (b >= 4) of_8 += pc.hist[b];
-        }
-        if (10 * of_8 < 6 * rows) plain = 1;
-    }
-    const int32_t cut = pc.unsorted_cols ? 1 : use_long ? e->panels_long : plain;
-    const int32_t panels = use_long ? cut + 1 : cut;   // (the short rows, whole, are the last entry of the list)
-    e->panel_cols = static_cast<int32_t>((e->N + cut - 1) / cut);
     if (e->knob_k_slices < 0 && e->K <= 256) {
-        if (use_long && long_rows_whole(e)) e->seg_slices = 1;
+        if (c.long_rows > 0 && long_rows_whole(e)) e->seg_slices = 1;
         // slices of 64 that do not fit L2 and get no panels either: whole rows
-        if (!use_long && panels == 1 && e->slice_cols == 64 && e->nnz < 16 * e->M && gathered_bytes(e, 64) > e->l2_bytes) e->seg_slices = 1;
+        if (c.panels == 1 && e->slice_cols == 64 && e->nnz < 16 * e->M && gathered_bytes(e, 64) > e->l2_bytes) e->seg_slices = 1;
     }
-    if (!built || panels > 1) {
-        if (int rc = enqueue_unit_list(e, e->stream, panels, use_long ? e->long_threshold : 0, false)) return rc;
+    bool built = false;
+    if (early) {
+        const ListForms::Choice was = early->choose(&pc, e->nnz);
+        built = was.panels == c.panels && was.long_rows == c.long_rows && (c.panels == 1 || was.panel_cols == c.panel_cols);
+    }
+    if (!built) {
+        ListForms f;   // the one form
+        f.plain = c.long_rows > 0 ? 1 : c.panels;
+        f.plain_cols = f.long_cols = c.panel_cols;
+        f.longs = c.panels - 1;
+        f.long_rows = c.long_rows;
+        f.long_always = true;
+        f.plain_by_size = f.long_by_size = list_by_size(e, c.long_rows);
+        if (int rc = enqueue_unit_list(e, e->stream, f, false)) return rc;
         if (int rc = read_counters(e, &pc)) return rc;
     }
-    e->seg_copies = panels > 1;
+    e->seg_copies = c.panels > 1;
     if (pc.units == 0 || pc.units > static_cast<unsigned long long>(std::min<int64_t>(e->unit_cap, kUnitLimit)))
         return fail(e, SDDMM_B200_ERR_CUDA, "row-segment plan: %llu units for a list of %lld", pc.units, (long long)e->unit_cap);
     e->n_units = static_cast<int32_t>(pc.units);
     sddmm_b200_plan_info &p = e->plan;
     p.rowseg_nnz = e->nnz;
     p.rowseg_units = e->n_units;
-    p.rowseg_panels = panels;
+    p.rowseg_panels = c.panels;
     p.rowseg_passes = e->seg_slices;
     p.rowtile_nnz = 0;
     p.rowtile_items = 0;
@@ -1221,19 +1242,22 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     if (e->d_coo_rows)   // (rows out of order or out of range are counted, and every later kernel checks the bounds it gets from row_ptr)
         k_coo_to_row_ptr<<<grid_for(e->nnz + 1, kBlock, cap), kBlock, 0, s>>>(e->d_coo_rows, e->nnz, static_cast<int32_t>(e->M),
                                                                               e->coo_row_base, e->d_rp, e->d_pc);
-    // What will most likely run is enqueued before anything is read back: the plain or panel-major unit list (not where
-    // tiles, or the row statistics, decide first) and the sample that looks for row groups.
+    // What will most likely run is enqueued before anything is read back: the unit list, in the form that the row statistics choose on
+    // the device (not where tiles decide first, or whether the copies of B are made slice by slice), and the sample that looks for row groups.
     const bool tiles_first = e->dense_possible && e->mode != SDDMM_B200_FP32;   // (fp32 mode: tiles are the exception)
-    const bool no_panels = e->panels_plain == 1 && e->long_threshold == 0;   // (else the row statistics decide first)
-    const bool whole_rows = e->use_seg && !tiles_first && no_panels;
-    const bool early_list = whole_rows && e->nnz > 0;
+    const ListForms forms = list_forms(e);
+    const bool whole_rows = forms.plain == 1 && forms.long_rows == 0;
+    const bool early_list = e->use_seg && !tiles_first && (whole_rows || !e->slice_major) && e->nnz > 0;
+    const bool sums_beside = early_list && whole_rows;
     k_row_stats<<<static_cast<int>(unit_tiles(e->M)), kUnitBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, e->d_rowstart,
-                                                                                            whole_rows ? e->d_scan_tiles : nullptr, e->d_pc);
-    // The list of whole rows needs the row statistics only: where the operands come from this GPU's memory it is built on the side
+                                                                                            sums_beside ? e->d_scan_tiles : nullptr, e->d_pc);
+    // The list needs the row statistics only: where the operands come from this GPU's memory it is built on the side
     // stream, behind their copies, while the columns are looked at here (each of the three kernels leaves much of the chip idle: 5.2 M
     // nonzeros, K = 64, upload and run 272 -> 256 us; 4 M, power law, 266 -> 249).  Not for rows long enough to lie in 64-wide tiles,
     // where the count of the column scan may make the list unnecessary (18 M in 64 x 64 blocks, upload 489 us, 572 with the list aside).
-    const bool list_aside = early_list && join_copies && e->nnz < 64 * e->M;
+    // (Panels of columns that turn out not to be sorted are runs that overlap, at most the whole row in each: their sums fit 32 bits.)
+    const int64_t most_units = std::max<int64_t>(forms.plain, forms.longs + 1) * (e->nnz / 8 + e->M);
+    const bool list_aside = early_list && join_copies && e->nnz < 64 * e->M && most_units < (int64_t(1) << 31);
     ListGate gate;
     if (e->nnz > 0 && group_possible(e)) {
         if (int rc = enqueue_group_sample(e)) return rc;
@@ -1244,7 +1268,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         CU_TRY(e, cudaEventRecord(e->ev_fork, s));
         CU_TRY(e, cudaStreamWaitEvent(e->side_stream, e->ev_fork, 0));
         gate.columns_scanned = false;
-        if (int rc = enqueue_unit_list(e, e->side_stream, 1, 0, true, gate)) return rc;
+        if (int rc = enqueue_unit_list(e, e->side_stream, forms, true, gate)) return rc;
         CU_TRY(e, cudaEventRecord(e->ev_join, e->side_stream));
     }
     if (e->nnz > 0) {
@@ -1261,12 +1285,12 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         if (early_list && !list_aside) {
             // (fp32 mode: tiles will most likely be looked for, and found, when the column scan's count is high enough)
             if (e->dense_possible && e->knob_offset_tiles <= 0) gate.tile_hint = (static_cast<unsigned long long>(e->nnz) + kTileHintShare - 1) / kTileHintShare;
-            if (int rc = enqueue_unit_list(e, s, 1, 0, true, gate)) return rc;
+            if (int rc = enqueue_unit_list(e, s, forms, true, gate)) return rc;
         }
     }
     if (list_aside) CU_TRY(e, cudaStreamWaitEvent(s, e->ev_join, 0));
     CU_TRY(e, cudaGetLastError());
-    if (join_copies && !tiles_first && no_panels && !e->slice_major) {   // (... or whether the copies are made slice by slice)
+    if (join_copies && !tiles_first && !e->slice_major) {
         CU_TRY(e, cudaStreamWaitEvent(s, e->ev_h2d, 0));
         if (int rc = convert_storage(e)) return rc;
         e->copies_joined = true;
@@ -1315,7 +1339,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         if (st) return st;
         if (e->rg_rows) return SDDMM_B200_OK;
         // (a grouping that was tried and dropped has used the list's memory)
-        st = build_rowseg_plan(e, pc, list_built && !e->group_tried);
+        st = build_rowseg_plan(e, pc, list_built && !e->group_tried ? &forms : nullptr);
         if (st) return st;
         if (e->use_seg) return SDDMM_B200_OK;
     }
@@ -1423,6 +1447,8 @@ int upload_common(sddmm_b200_engine *e, int64_t M, int64_t N, int64_t K, int64_t
     if (!st && !e->copies_joined) {
         st = cuda_status(e, cudaStreamWaitEvent(s, e->ev_h2d, 0));
         if (!st) st = convert_storage(e);
+    } else if (!st) {
+        st = refresh_unit_values(e);   // (the list was not there yet)
     }
     if (!st) st = cuda_status(e, cudaStreamSynchronize(s));   // the caller's buffers are free again when this returns
     if (st) {   // nothing of a failed upload may still be reading the caller's buffers
@@ -1811,11 +1837,7 @@ int sddmm_b200_update_values(sddmm_b200_engine *e, const float *s_val) {
     if (!s_val && e->nnz) return fail(e, SDDMM_B200_ERR_ARG, "null pointer argument");
     DeviceGuard g(e->device);
     if (e->nnz) CU_TRY(e, e->stager.upload(e->d_sval, s_val, static_cast<size_t>(e->nnz) * 4, e->stream));
-    if (e->use_seg && e->seg_copies && e->n_units > 0) {
-        k_unit_values<<<grid_for(8 * static_cast<int64_t>(e->n_units), kBlock, e->sm_count * 32), kBlock, 0, e->stream>>>(e->d_units, e->n_units,
-                                                                                                                  e->d_sval, e->d_unit_sval);
-        CU_TRY(e, cudaGetLastError());
-    }
+    if (int rc = refresh_unit_values(e)) return rc;
     CU_TRY(e, cudaStreamSynchronize(e->stream));
     return SDDMM_B200_OK;
 }

@@ -13,8 +13,13 @@
 namespace sddmm {
 
 // ---- entries -> runs.  (A row_ptr that has not been validated yet may be anything: runs outside [0, nnz) are empty.) ----
+// settled(pc): the runs themselves, where the row statistics have a say (RunsOfForms); sorted(): whether they need sorted columns;
+// ordered(): whether a list that may be ordered by size is
 struct RunsOfRows {   // one entry per row: the whole row
-    static constexpr bool kSorted = false;   // needs sorted columns
+    static constexpr bool kChosen = false;
+    __device__ __forceinline__ const RunsOfRows &settled(const PlanCounters *) const { return *this; }
+    __device__ __forceinline__ bool sorted() const { return false; }
+    __device__ __forceinline__ bool ordered() const { return true; }
     const int32_t *rp;
     const int32_t *col;
     int32_t M, nnz;
@@ -30,10 +35,14 @@ struct RunsOfRows {   // one entry per row: the whole row
 // columns each); the shorter rows follow whole, as the last "panel" of the list -- a run of one or two nonzeros would
 // leave most of a segment's slots empty.
 struct RunsOfPanels {
-    static constexpr bool kSorted = true;
+    static constexpr bool kChosen = false;
     const int32_t *rp;
     const int32_t *col;
     int32_t M, nnz, panels, panel_cols, long_rows;
+    bool by_size = true;
+    __device__ __forceinline__ const RunsOfPanels &settled(const PlanCounters *) const { return *this; }
+    __device__ __forceinline__ bool sorted() const { return panels > 1; }
+    __device__ __forceinline__ bool ordered() const { return by_size; }
     __device__ __forceinline__ int32_t row(int64_t q) const { return static_cast<int32_t>(q % M); }
     __device__ __forceinline__ void run(int64_t q, int32_t &s, int32_t &e) const {
         const int32_t p = static_cast<int32_t>(q / M), i = static_cast<int32_t>(q - static_cast<int64_t>(p) * M);
@@ -56,13 +65,59 @@ struct RunsOfPanels {
         if (e < s) e = s;                    // (unsorted columns: the list will not be built)
     }
 };
+// The forms that a list over the whole matrix may take, and which one the row statistics choose: on the device for a list that is
+// enqueued before the host has seen them, on the host to know which one that was.
+struct ListForms {
+    int32_t plain = 1, plain_cols = 0;   // column panels for every row (1: whole rows)
+    int32_t longs = 1, long_cols = 0;    // panels for the rows of at least long_rows nonzeros, the others being one more
+    int32_t long_rows = 0;               // (0: no such form)
+    bool long_always = false;            // whatever those rows hold
+    bool plain_for_8 = false;            // plain panels only where most rows have 8 nonzeros or more
+    bool plain_by_size = false, long_by_size = false;
+    struct Choice {
+        int32_t panels, panel_cols, long_rows;
+        bool by_size;
+    };
+    __host__ __device__ __forceinline__ Choice choose(const PlanCounters *pc, int64_t nnz) const {
+        if (long_rows > 0) {
+            unsigned long long in_long = 0;   // they only pay when those rows hold a good share of the nonzeros
+            for (int b = 1; b < SDDMM_B200_HIST_BINS; ++b)
+                if ((1ll << (b - 1)) >= long_rows) in_long += pc->hist_nnz[b];
+            if (long_always || 5 * in_long >= 2 * static_cast<unsigned long long>(nnz)) return Choice{longs + 1, long_cols, long_rows, long_by_size};   // 40 %
+        }
+        if (plain > 1 && plain_for_8) {
+            // a mean that barely pays for panels has to be that of most rows, not of a few long ones: 60 % of them of 8 nonzeros or more
+            unsigned long long rows = 0, of_8 = 0;
+            for (int b = 1; b < SDDMM_B200_HIST_BINS; ++b) {
+                rows += pc->hist[b];
+                if (b >= 4) of_8 += pc->hist[b];
+            }
+            if (10 * of_8 < 6 * rows) return Choice{1, plain_cols, 0, plain_by_size};
+        }
+        return Choice{plain, plain_cols, 0, plain_by_size};
+    }
+};
+struct RunsOfForms {
+    static constexpr bool kChosen = true;
+    const int32_t *rp;
+    const int32_t *col;
+    int32_t M, nnz;
+    ListForms forms;
+    __device__ __forceinline__ RunsOfPanels settled(const PlanCounters *pc) const {
+        const ListForms::Choice c = forms.choose(pc, nnz);
+        return RunsOfPanels{rp, col, M, nnz, c.panels, c.panel_cols, c.long_rows, c.by_size};
+    }
+};
 // rows of group g when groups of G rows start at row `first` (group 0 = the rows before it)
 __device__ __forceinline__ void unit_group_rows(int32_t g, int32_t G, int32_t first, int32_t M, int32_t &r0, int32_t &r1) {
     r0 = g == 0 ? 0 : first + (g - 1) * G;
     r1 = g == 0 ? first : min(r0 + G, M);
 }
 struct RunsOfGroups {   // one entry per row: the leader of a matching group speaks for its whole group
-    static constexpr bool kSorted = false;
+    static constexpr bool kChosen = false;
+    __device__ __forceinline__ const RunsOfGroups &settled(const PlanCounters *) const { return *this; }
+    __device__ __forceinline__ bool sorted() const { return false; }
+    __device__ __forceinline__ bool ordered() const { return false; }
     const int32_t *rp;
     const int32_t *col;
     int32_t M, nnz, G, first;
@@ -84,7 +139,9 @@ struct RunsOfGroups {   // one entry per row: the leader of a matching group spe
 
 // pass 1: units of every tile; the grand total goes to pc->units
 template <typename Runs>
-__global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs runs, int64_t n, int32_t *__restrict__ tile_sums, PlanCounters *__restrict__ pc) {
+__global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs given, int64_t n, int32_t *__restrict__ tile_sums, PlanCounters *__restrict__ pc) {
+    const auto runs = given.settled(pc);
+    if constexpr (Runs::kChosen) n = static_cast<int64_t>(runs.panels) * runs.M;   // (at most the n that the grid was made for)
     const int tile = unit_tile(n);
     const int64_t base = static_cast<int64_t>(blockIdx.x) * tile;
     int32_t local = 0;
@@ -137,15 +194,18 @@ constexpr unsigned kShortRowShare = 16;
 // different SMs, and where DRAM is the bound, rows of 26 in two panels, K = 32 takes 540 us instead of 465.  A kernel of its own: with
 // the order as an argument only, power-law panels of 36 M nonzeros take 454 us to build instead of 423.)
 template <typename Runs, typename HDR, bool BY_SIZE>
-__global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs runs, int64_t n, const int32_t *__restrict__ tile_sums, int64_t cap,
+__global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs given, int64_t n, const int32_t *__restrict__ tile_sums, int64_t cap,
                                                            PlanCounters *__restrict__ pc, HDR *__restrict__ units,
                                                            int32_t *__restrict__ unit_cols, bool scanned, ListGate gate) {
     // enqueued before the host has seen the counters: nothing is written for a pattern that it is about to refuse, or for one
     // that will be computed otherwise
     if (list_unused(gate, pc)) return;
-    if (pc->bad_row_ptr || pc->bad_coo || (Runs::kSorted && pc->unsorted_cols)) return;
+    const auto runs = given.settled(pc);
+    if constexpr (Runs::kChosen) n = static_cast<int64_t>(runs.panels) * runs.M;
+    // (unsorted columns that the column scan has yet to find: the runs overlap, and the list is not used)
+    if (pc->bad_row_ptr || pc->bad_coo || (runs.sorted() && gate.columns_scanned && pc->unsorted_cols)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) pc->list_built = 1;
-    const bool by_size = BY_SIZE && kShortRowShare * (pc->hist[1] + pc->hist[2] + pc->hist[3]) >= pc->rows_nonempty;   // (rows of 1 .. 7 nonzeros)
+    const bool by_size = BY_SIZE && runs.ordered() && kShortRowShare * (pc->hist[1] + pc->hist[2] + pc->hist[3]) >= pc->rows_nonempty;   // (rows of 1 .. 7 nonzeros)
     constexpr int kPerThread = kUnitTileMax / kUnitBlock;
     __shared__ int32_t first_unit[kUnitTileMax];   // of the tile's entries, relative to the tile
     __shared__ int32_t start[kUnitTileMax], length[kUnitTileMax];
