@@ -374,8 +374,10 @@ void choose_long_rows(sddmm_b200_engine *e) {
     const double b = gathered_bytes(e, e->seg_slices > 1 && !long_rows_whole(e) ? e->slice_cols : e->Ks);
     const bool bf = e->mode == SDDMM_B200_BF16;
     // (see kPanelsFrom.)  Power law, rows of 25 on average, without / with: K = 32, B 94 / 117 / 131 MB 178 / 172, 233 / 214, 270 / 239 us,
-    // rows of 10 93 / 92, 118 / 114, 134 / 127; K = 64, 117 MB 205 / 194; bf16 K = 64, 117 MB 320 / 281.
-    if (b <= kPanelsFrom * l2 && !(e->knob_long_rows >= 1 && e->knob_panels >= 2)) return;
+    // rows of 10 93 / 92, 118 / 114, 134 / 127; K = 64, 117 MB 205 / 194.  bf16, where no list is built early: from L2 on, below it a
+    // held run gains less than planning costs a single one (K = 64, 117 MB, rows of 25: 305 / 276, upload and run 1063 / 1250; K = 128
+    // 227 / 216, 861 / 950).
+    if (b <= (bf ? 1.0 : kPanelsFrom) * l2 && !(e->knob_long_rows >= 1 && e->knob_panels >= 2)) return;
     // fp32: B 333 MB, K = 32: 4 panels 407 us, 6 402 us, 8 401 us; 189 MB, 2 / 3 / 4 / 6: 300 / 287 / 286 / 286
     // bf16, whose lists are not ordered by size and whose kernel loads all slots: a short run costs as much as a full one, so fewer
     // panels and, with few of them, shorter rows too.  36 M, 2.6 M rows, K = 32, B 166 MB: 3 panels from 64 nonzeros on 358 us, 4
@@ -399,11 +401,19 @@ int choose_panels(const sddmm_b200_engine *e) {
     // rows, without / with 2 panels: K = 32, B 186 MB, mean 11 / 13 / 15: 282 / 290, 324 / 320, 368 / 353 us; K = 64, B 371 MB, mean
     // 9 / 11 / 13 / 15: 524 / 537, 619 / 607, 723 / 685, 839 / 768; K = 96, B 346 MB, mean 10 / 13: 601 / 538, 779 / 655.
     // With B between 0.85 and 1 times L2 only longer rows gain, 1 / 2 panels: K = 32, 117 MB, mean 20 / 40: 216 / 221, 403 / 368, 131 MB 258 / 238,
-    // 444 / 377; K = 64, 117 MB, mean 12 / 20 / 40: 134 / 132, 205 / 190, 364 / 326; K = 128 the same; bf16 K = 64 and 128, mean 20 / 40:
-    // 283 / 283, 522 / 481 and 199 / 202, 371 / 337; slices of K, 121 MB each, mean 12 / 24 / 50: K = 128 304 / 279, 548 / 490, 873 / 659, K = 256,
-    // mean 12 / 40, 290 / 268, 790 / 617.
+    // 444 / 377; K = 64, 117 MB, mean 12 / 20 / 40: 134 / 132, 205 / 190, 364 / 326; K = 128 the same; bf16 K = 128, mean 20 / 40:
+    // 199 / 202, 371 / 337; slices of K, 121 MB each, mean 12 / 24 / 50: K = 128 304 / 279, 548 / 490, 873 / 659, K = 256,
+    // mean 12 / 40, 290 / 268, 790 / 617.  A single run pays for the planning, so that there has to be something to gain.  Upload and
+    // run, 1 / 2 panels: K = 64, mean 20, 4.0 / 9.1 M nonzeros (1.0 / 2.3 GB of gathers) 289 / 321, 476 / 485, mean 40, 18 M (4.7) 685 / 684; K = 32,
+    // 8.0 / 37 M (1.0 / 4.7) 332 / 355, 918 / 982; slices, K = 128, 5.7 / 11 M 599 / 625, 877 / 818; bf16 K = 64, mean 40, 37 M
+    // 1280 / 1534, a held run 501 / 461.
     if (b_bytes <= kPanelsFrom * l2) return 1;
-    if (b_bytes <= l2) return mean < (e->seg_slices > 1 ? 11.0 : bf ? 28.0 : cols <= 32 ? 24.0 : 16.0) ? 1 : 2;
+    if (b_bytes <= l2) {
+        if (bf) return cols <= 64 || mean < 28.0 ? 1 : 2;
+        if (e->seg_slices > 1) return mean < 11.0 ? 1 : 2;
+        return mean < (cols <= 32 ? 24.0 : 16.0) || static_cast<double>(e->nnz) * static_cast<double>(cols) * 4.0 < 1.4e9 ? 1 : 2;
+    }
+    if (bf && cols > 32 && cols <= 64 && b_bytes <= 1.5 * l2) return 1;
     // (K = 32, B 262 / 388 MB, mean 8 / 10 / 12: 347 / 342, 418 / 392, 500 / 438 and 616 / 569, 726 / 654, 719 / 638)
     if (mean < (bf ? (cols <= 32 ? 26.0 : cols <= 64 ? 20.0 : 13.0) : cols <= 32 ? (b_bytes > 1.8 * l2 ? 10.0 : 13.0) : cols <= 64 ? 11.0 : 9.0)) return 1;
     // Slices of 128 columns: panels that fit L2 one by one, if an average row has 3 nonzeros for each, or none.  Sustained, B 205 MB,
