@@ -157,6 +157,7 @@ struct sddmm_b200_engine {
     int64_t Ks = 0;
     float *d_Ap = nullptr, *d_Bp = nullptr;
     bool d_Ap_wanted = false;
+    bool values_built = false;         // the list came with the units' copies of the S values
     bool slice_major = false;   // ... slice of K after slice of K, each of rows of slice_cols elements
     bool group_tried = false;          // a grouping was matched exactly and then dropped
     bool copies_joined = false;        // the upload's copies and conversions are already ordered before the plan's read-back
@@ -995,20 +996,21 @@ bool list_by_size(const sddmm_b200_engine *e, int32_t long_rows) {
 // sums and the total.
 template <typename Runs, typename HDR>
 int enqueue_units(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_t n, bool have_sums, int64_t cap, HDR *units, int32_t *unit_cols,
-                  const ListGate &gate = ListGate{}, bool by_size = false) {
+                  const ListGate &gate = ListGate{}, bool by_size = false, const UnitValues &values = UnitValues{}) {
     const int tiles = static_cast<int>(unit_tiles(n));
     if (int rc = check_tile_sums(e, tiles)) return rc;
     if (!have_sums) {
-        CU_TRY(e, cudaMemsetAsync(&e->d_pc->units, 0, sizeof(unsigned long long), s));
+        if constexpr (!Runs::kChosen) CU_TRY(e, cudaMemsetAsync(&e->d_pc->units, 0, sizeof(unsigned long long), s));
+        else k_panel_cuts<<<grid_for(e->M, kUnitBlock, e->sm_count * 8), kUnitBlock, 0, s>>>(runs, e->d_pc);
         k_unit_sums<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->d_pc);
     }
     const bool scanned = tiles > kDirectTiles;
     if (scanned) k_scan_sums<<<1, kScanBlock, 0, s>>>(e->d_scan_tiles, tiles, &e->d_pc->units);
     if constexpr (sizeof(HDR) == sizeof(int2)) {
-        if (by_size) k_unit_build<Runs, HDR, true><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate);
-        else k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate);
+        if (by_size) k_unit_build<Runs, HDR, true><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate, values);
+        else k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate, values);
     } else {
-        k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate);
+        k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate, values);
     }
     CU_TRY(e, cudaGetLastError());
     return SDDMM_B200_OK;
@@ -1161,16 +1163,18 @@ ListForms list_forms(const sddmm_b200_engine *e) {
 }
 
 // Enqueue the list over the whole matrix.  have_sums: k_row_stats has left the tile sums of whole rows.
-int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, const ListForms &forms, bool have_sums, const ListGate &gate = ListGate{}) {
+int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, const ListForms &forms, bool have_sums, const ListGate &gate = ListGate{},
+                      const UnitValues &values = UnitValues{}) {
     const int32_t M = static_cast<int32_t>(e->M), nnz = static_cast<int32_t>(e->nnz);
     int st;
     if (forms.plain > 1 || forms.long_rows > 0) {
-        const RunsOfForms runs{e->d_rp, e->d_col, M, nnz, forms};
+        // (the starts of the panels: in the half of the headers' memory that plain units leave)
+        const RunsOfForms runs{e->d_rp, e->d_col, M, nnz, forms, reinterpret_cast<int32_t *>(e->d_units + e->unit_cap + 8), 2 * (e->unit_cap + 8), have_sums};
         // (a grid for either form: the longer list, or the one with more tiles)
         const int64_t n_plain = e->M * forms.plain, n_long = forms.long_rows > 0 ? e->M * (forms.longs + 1) : 0;
         const int64_t n = unit_tiles(n_long) > unit_tiles(n_plain) ? n_long : n_plain;
         const int64_t n_whole = forms.plain_for_8 && unit_tiles(e->M) > unit_tiles(n) ? e->M : n;
-        st = enqueue_units(e, s, runs, n_whole, false, e->unit_cap, e->d_units, e->d_unit_cols, gate, forms.plain_by_size || forms.long_by_size);
+        st = enqueue_units(e, s, runs, n_whole, false, e->unit_cap, e->d_units, e->d_unit_cols, gate, forms.plain_by_size || forms.long_by_size, values);
     } else {
         const RunsOfRows runs{e->d_rp, e->d_col, M, nnz};
         st = enqueue_units(e, s, runs, e->M, have_sums, e->unit_cap, e->d_units, e->d_unit_cols, gate, forms.plain_by_size);
@@ -1181,8 +1185,9 @@ int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, const ListForms &for
     return SDDMM_B200_OK;
 }
 
-// Row segments over the whole matrix.  early: the forms of the list that is already there, counted in pc (null: none).
-int build_rowseg_plan(sddmm_b200_engine *e, PlanCounters pc, const ListForms *early) {
+// Row segments over the whole matrix.  early: the forms of the list that is already there, counted in pc (null: none); early_values:
+// with the copies of the S values.
+int build_rowseg_plan(sddmm_b200_engine *e, PlanCounters pc, const ListForms *early, bool early_values) {
     e->seg_copies = false;
     e->n_units = 0;
     if (!e->use_seg) return SDDMM_B200_OK;
@@ -1207,9 +1212,11 @@ int build_rowseg_plan(sddmm_b200_engine *e, PlanCounters pc, const ListForms *ea
         if (c.panels == 1 && e->slice_cols == 64 && e->nnz < 16 * e->M && gathered_bytes(e, 64) > e->l2_bytes) e->seg_slices = 1;
     }
     bool built = false;
+    e->values_built = false;
     if (early) {
         const ListForms::Choice was = early->choose(&pc, e->nnz);
         built = was.panels == c.panels && was.long_rows == c.long_rows && (c.panels == 1 || was.panel_cols == c.panel_cols);
+        e->values_built = built && early_values;
     }
     if (!built) {
         ListForms f;   // the one form
@@ -1258,14 +1265,14 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     const ListForms forms = list_forms(e);
     const bool whole_rows = forms.plain == 1 && forms.long_rows == 0;
     const bool early_list = e->use_seg && !tiles_first && (whole_rows || !e->slice_major) && e->nnz > 0;
-    const bool sums_beside = early_list && whole_rows;
+    const bool sums_beside = early_list && forms.plain == 1;
     k_row_stats<<<static_cast<int>(unit_tiles(e->M)), kUnitBlock, 0, s>>>(e->d_rp, static_cast<int32_t>(e->M), e->nnz, e->d_rowstart,
                                                                                             sums_beside ? e->d_scan_tiles : nullptr, e->d_pc);
     // The list needs the row statistics only: where the operands come from this GPU's memory it is built on the side
     // stream, behind their copies, while the columns are looked at here (each of the three kernels leaves much of the chip idle: 5.2 M
     // nonzeros, K = 64, upload and run 272 -> 256 us; 4 M, power law, 266 -> 249).  Not for rows long enough to lie in 64-wide tiles,
     // where the count of the column scan may make the list unnecessary (18 M in 64 x 64 blocks, upload 489 us, 572 with the list aside).
-    // (Panels of columns that turn out not to be sorted are runs that overlap, at most the whole row in each: their sums fit 32 bits.)
+    // (Panels of columns that turn out not to be sorted may be runs that overlap, at most the whole row in each: their sums fit 32 bits.)
     const int64_t most_units = std::max<int64_t>(forms.plain, forms.longs + 1) * (e->nnz / 8 + e->M);
     const bool list_aside = early_list && join_copies && e->nnz < 64 * e->M && most_units < (int64_t(1) << 31);
     // The sample of the row groups comes before the list, which may leave its place to theirs, but not before the column scan: between it
@@ -1282,7 +1289,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         if (groups)
             if (int rc = enqueue_group_sample(e, e->side_stream)) return rc;
         gate.columns_scanned = false;
-        if (int rc = enqueue_unit_list(e, e->side_stream, forms, true, gate)) return rc;
+        if (int rc = enqueue_unit_list(e, e->side_stream, forms, sums_beside, gate, UnitValues{e->d_sval, e->d_unit_sval})) return rc;
         CU_TRY(e, cudaEventRecord(e->ev_join, e->side_stream));
     }
     if (e->nnz > 0) {
@@ -1301,7 +1308,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         if (early_list && !list_aside) {
             // (fp32 mode: tiles will most likely be looked for, and found, when the column scan's count is high enough)
             if (e->dense_possible && e->knob_offset_tiles <= 0) gate.tile_hint = (static_cast<unsigned long long>(e->nnz) + kTileHintShare - 1) / kTileHintShare;
-            if (int rc = enqueue_unit_list(e, s, forms, true, gate)) return rc;
+            if (int rc = enqueue_unit_list(e, s, forms, sums_beside, gate)) return rc;
         }
     }
     if (list_aside) CU_TRY(e, cudaStreamWaitEvent(s, e->ev_join, 0));
@@ -1355,7 +1362,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
         if (st) return st;
         if (e->rg_rows) return SDDMM_B200_OK;
         // (a grouping that was tried and dropped has used the list's memory)
-        st = build_rowseg_plan(e, pc, list_built && !e->group_tried ? &forms : nullptr);
+        st = build_rowseg_plan(e, pc, list_built && !e->group_tried ? &forms : nullptr, list_aside);
         if (st) return st;
         if (e->use_seg) return SDDMM_B200_OK;
     }
@@ -1463,7 +1470,7 @@ int upload_common(sddmm_b200_engine *e, int64_t M, int64_t N, int64_t K, int64_t
     if (!st && !e->copies_joined) {
         st = cuda_status(e, cudaStreamWaitEvent(s, e->ev_h2d, 0));
         if (!st) st = convert_storage(e);
-    } else if (!st) {
+    } else if (!st && !e->values_built) {
         st = refresh_unit_values(e);   // (the list was not there yet)
     }
     if (!st) st = cuda_status(e, cudaStreamSynchronize(s));   // the caller's buffers are free again when this returns

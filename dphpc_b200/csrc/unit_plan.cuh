@@ -40,16 +40,38 @@ struct RunsOfPanels {
     const int32_t *col;
     int32_t M, nnz, panels, panel_cols, long_rows;
     bool by_size = true;
+    const int32_t *cuts = nullptr;   // where panel p + 1 starts in row i, at p * M + i (k_panel_cuts; null: it is looked for, in each kernel)
     __device__ __forceinline__ const RunsOfPanels &settled(const PlanCounters *) const { return *this; }
     __device__ __forceinline__ bool sorted() const { return panels > 1; }
     __device__ __forceinline__ bool ordered() const { return by_size; }
-    __device__ __forceinline__ int32_t row(int64_t q) const { return static_cast<int32_t>(q % M); }
+    __device__ __forceinline__ int32_t real_panels() const { return long_rows > 0 ? panels - 1 : panels; }   // (without the short rows)
+    __device__ __forceinline__ void split(int64_t q, int32_t &p, int32_t &i) const {   // (a 64-bit division is several times a 32-bit one)
+        if (panels == 1) {
+            p = 0;
+            i = static_cast<int32_t>(q);
+        } else if ((q >> 32) == 0) {
+            p = static_cast<int32_t>(static_cast<uint32_t>(q) / static_cast<uint32_t>(M));
+            i = static_cast<int32_t>(static_cast<uint32_t>(q) - static_cast<uint32_t>(p) * static_cast<uint32_t>(M));
+        } else {
+            p = static_cast<int32_t>(q / M);
+            i = static_cast<int32_t>(q - static_cast<int64_t>(p) * M);
+        }
+    }
+    __device__ __forceinline__ int32_t row(int64_t q) const {
+        int32_t p, i;
+        split(q, p, i);
+        return i;
+    }
+    __device__ __forceinline__ bool bounds(int32_t i, int32_t &a, int32_t &b) const {
+        a = rp[i];
+        b = rp[i + 1];
+        return a >= 0 && b >= a && b <= nnz;
+    }
     __device__ __forceinline__ void run(int64_t q, int32_t &s, int32_t &e) const {
-        const int32_t p = static_cast<int32_t>(q / M), i = static_cast<int32_t>(q - static_cast<int64_t>(p) * M);
-        const int32_t a = rp[i], b = rp[i + 1];
+        int32_t p, i, a, b;
+        split(q, p, i);
         s = e = 0;
-        if (a < 0 || b < a || b > nnz) return;
-        int32_t cut = panels;
+        if (!bounds(i, a, b)) return;
         if (long_rows > 0) {
             const bool is_long = b - a >= long_rows;
             if (p == panels - 1) {           // the short rows, whole
@@ -58,11 +80,13 @@ struct RunsOfPanels {
                 return;
             }
             if (!is_long) return;
-            cut = panels - 1;                // the real column panels
         }
-        s = p == 0 ? a : lower_col(col, a, b, static_cast<int64_t>(p) * panel_cols);
-        e = p == cut - 1 ? b : lower_col(col, a, b, static_cast<int64_t>(p + 1) * panel_cols);
-        if (e < s) e = s;                    // (unsorted columns: the list will not be built)
+        auto start = [&](int32_t k) -> int32_t {
+            return cuts ? cuts[static_cast<int64_t>(k - 1) * M + i] : lower_col(col, a, b, static_cast<int64_t>(k) * panel_cols);
+        };
+        s = p == 0 ? a : start(p);
+        e = p == real_panels() - 1 ? b : start(p + 1);
+        if (e < s) e = s;                    // (unsorted columns: the list will not be used)
     }
 };
 // The forms that a list over the whole matrix may take, and which one the row statistics choose: on the device for a list that is
@@ -78,23 +102,45 @@ struct ListForms {
         int32_t panels, panel_cols, long_rows;
         bool by_size;
     };
-    __host__ __device__ __forceinline__ Choice choose(const PlanCounters *pc, int64_t nnz) const {
-        if (long_rows > 0) {
-            unsigned long long in_long = 0;   // they only pay when those rows hold a good share of the nonzeros
-            for (int b = 1; b < SDDMM_B200_HIST_BINS; ++b)
-                if ((1ll << (b - 1)) >= long_rows) in_long += pc->hist_nnz[b];
-            if (long_always || 5 * in_long >= 2 * static_cast<unsigned long long>(nnz)) return Choice{longs + 1, long_cols, long_rows, long_by_size};   // 40 %
-        }
-        if (plain > 1 && plain_for_8) {
-            // a mean that barely pays for panels has to be that of most rows, not of a few long ones: 60 % of them of 8 nonzeros or more
-            unsigned long long rows = 0, of_8 = 0;
-            for (int b = 1; b < SDDMM_B200_HIST_BINS; ++b) {
-                rows += pc->hist[b];
-                if (b >= 4) of_8 += pc->hist[b];
-            }
-            if (10 * of_8 < 6 * rows) return Choice{1, plain_cols, 0, plain_by_size};
-        }
+    // what the choice rests on, of the rows of one length bin (hist, hist_nnz: bin 0 holds the empty rows)
+    struct Rows {
+        unsigned long long rows = 0, of_8 = 0, in_long = 0;
+    };
+    __host__ __device__ __forceinline__ Rows of_bin(const PlanCounters *pc, int b) const {
+        Rows r;
+        if (b < 1 || b >= SDDMM_B200_HIST_BINS) return r;
+        r.rows = pc->hist[b];
+        r.of_8 = b >= 4 ? r.rows : 0;
+        r.in_long = (1ll << (b - 1)) >= long_rows ? pc->hist_nnz[b] : 0;
+        return r;
+    }
+    __host__ __device__ __forceinline__ Choice of_rows(const Rows &r, int64_t nnz) const {
+        // panels for the long rows only pay when those hold a good share of the nonzeros, 40 %
+        if (long_rows > 0 && (long_always || 5 * r.in_long >= 2 * static_cast<unsigned long long>(nnz))) return Choice{longs + 1, long_cols, long_rows, long_by_size};
+        // a mean that barely pays for panels has to be that of most rows, not of a few long ones: 60 % of them of 8 nonzeros or more
+        if (plain > 1 && plain_for_8 && 10 * r.of_8 < 6 * r.rows) return Choice{1, plain_cols, 0, plain_by_size};
         return Choice{plain, plain_cols, 0, plain_by_size};
+    }
+    Choice choose(const PlanCounters *pc, int64_t nnz) const {
+        Rows r;
+        for (int b = 1; b < SDDMM_B200_HIST_BINS; ++b) {
+            const Rows bin = of_bin(pc, b);
+            r.rows += bin.rows;
+            r.of_8 += bin.of_8;
+            r.in_long += bin.in_long;
+        }
+        return of_rows(r, nnz);
+    }
+    // (a bin per lane, by whole warps: bin after bin, the loads one after the other, every block of a list takes 4 us longer)
+    __device__ __forceinline__ Choice choose_by_warp(const PlanCounters *pc, int64_t nnz) const {
+        static_assert(SDDMM_B200_HIST_BINS <= 32, "a length bin per lane");
+        Rows r = of_bin(pc, static_cast<int>(threadIdx.x & 31));
+        for (int o = 16; o > 0; o >>= 1) {
+            r.rows += __shfl_xor_sync(kFullMask, r.rows, o);
+            r.of_8 += __shfl_xor_sync(kFullMask, r.of_8, o);
+            r.in_long += __shfl_xor_sync(kFullMask, r.in_long, o);
+        }
+        return of_rows(r, nnz);
     }
 };
 struct RunsOfForms {
@@ -103,11 +149,31 @@ struct RunsOfForms {
     const int32_t *col;
     int32_t M, nnz;
     ListForms forms;
-    __device__ __forceinline__ RunsOfPanels settled(const PlanCounters *pc) const {
-        const ListForms::Choice c = forms.choose(pc, nnz);
-        return RunsOfPanels{rp, col, M, nnz, c.panels, c.panel_cols, c.long_rows, c.by_size};
+    int32_t *cuts;       // room for this many starts of panels
+    int64_t cuts_room;
+    bool have_sums;      // of whole rows
+    __device__ __forceinline__ RunsOfPanels settled(const PlanCounters *pc) const {   // (by whole warps)
+        const ListForms::Choice c = forms.choose_by_warp(pc, nnz);
+        RunsOfPanels r{rp, col, M, nnz, c.panels, c.panel_cols, c.long_rows, c.by_size};
+        if (static_cast<int64_t>(r.real_panels() - 1) * M <= cuts_room) r.cuts = cuts;
+        return r;
     }
 };
+// The starts of the panels, a thread per row: every entry of the list needs two, in both of its kernels, and each is a chain of loads.
+// (Whole rows: nothing to do here, nor in k_unit_sums where k_row_stats has left the sums.)
+__global__ void __launch_bounds__(kUnitBlock) k_panel_cuts(RunsOfForms given, PlanCounters *__restrict__ pc) {
+    const RunsOfPanels runs = given.settled(pc);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !(given.have_sums && runs.panels == 1)) pc->units = 0;
+    if (!runs.cuts || runs.panels == 1) return;
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(kUnitBlock) + threadIdx.x; i < runs.M; i += static_cast<int64_t>(gridDim.x) * kUnitBlock) {
+        int32_t a, b;
+        if (!runs.bounds(static_cast<int32_t>(i), a, b) || b - a < runs.long_rows) continue;   // (not read either)
+        for (int32_t k = 1; k < runs.real_panels(); ++k) {
+            a = lower_col(runs.col, a, b, static_cast<int64_t>(k) * runs.panel_cols);
+            given.cuts[static_cast<int64_t>(k - 1) * runs.M + i] = a;
+        }
+    }
+}
 // rows of group g when groups of G rows start at row `first` (group 0 = the rows before it)
 __device__ __forceinline__ void unit_group_rows(int32_t g, int32_t G, int32_t first, int32_t M, int32_t &r0, int32_t &r1) {
     r0 = g == 0 ? 0 : first + (g - 1) * G;
@@ -141,7 +207,13 @@ struct RunsOfGroups {   // one entry per row: the leader of a matching group spe
 template <typename Runs>
 __global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs given, int64_t n, int32_t *__restrict__ tile_sums, PlanCounters *__restrict__ pc) {
     const auto runs = given.settled(pc);
-    if constexpr (Runs::kChosen) n = static_cast<int64_t>(runs.panels) * runs.M;   // (at most the n that the grid was made for)
+    if constexpr (Runs::kChosen) {
+        if (given.have_sums && runs.panels == 1) {   // (the grid may be a longer list's: no units in the tiles past this one's end)
+            if (threadIdx.x == 0 && blockIdx.x * static_cast<int64_t>(unit_tile(runs.M)) >= runs.M) tile_sums[blockIdx.x] = 0;
+            return;
+        }
+        n = static_cast<int64_t>(runs.panels) * runs.M;   // (at most the n that the grid was made for)
+    }
     const int tile = unit_tile(n);
     const int64_t base = static_cast<int64_t>(blockIdx.x) * tile;
     int32_t local = 0;
@@ -183,6 +255,12 @@ __device__ __forceinline__ bool list_unused(const ListGate &gate, const PlanCoun
     return gate.groups_from >= 0.0 && pc->max_row_nnz <= kGroupRowMax && group_saving(pc->group_cover, gate.every, &slot) >= gate.groups_from;
 }
 
+// The units' copies of the S values, for lists in panels (unit_val null: they are made later, k_unit_values)
+struct UnitValues {
+    const float *s_val = nullptr;
+    float *unit_val = nullptr;
+};
+
 // A list is ordered by size (k_unit_build) from one short row in this many on: with fewer the kernel gains nothing and building takes
 // longer (5.2 M nonzeros in rows of 26: upload and run 247 us, 250 with the order).  Not where DRAM is the bound, see list_by_size.
 constexpr unsigned kShortRowShare = 16;
@@ -196,7 +274,7 @@ constexpr unsigned kShortRowShare = 16;
 template <typename Runs, typename HDR, bool BY_SIZE>
 __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs given, int64_t n, const int32_t *__restrict__ tile_sums, int64_t cap,
                                                            PlanCounters *__restrict__ pc, HDR *__restrict__ units,
-                                                           int32_t *__restrict__ unit_cols, bool scanned, ListGate gate) {
+                                                           int32_t *__restrict__ unit_cols, bool scanned, ListGate gate, UnitValues values) {
     // enqueued before the host has seen the counters: nothing is written for a pattern that it is about to refuse, or for one
     // that will be computed otherwise
     if (list_unused(gate, pc)) return;
@@ -269,8 +347,10 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs given, int64_t n
     // four units at a time: the searches, then the loads, then the stores of all four are in flight together
     constexpr int kBatch = 4, kGroups = kUnitBlock / 8;
     const int slot = threadIdx.x & 7;
+    const bool copy = values.unit_val && runs.sorted();
     for (int32_t u0 = threadIdx.x >> 3; u0 < total; u0 += kBatch * kGroups) {
         int32_t u[kBatch], entry[kBatch], first[kBatch], count[kBatch], c[kBatch];
+        float v[kBatch];
 #pragma unroll
         for (int k = 0; k < kBatch; ++k) {
             u[k] = min(u0 + k * kGroups, total - 1);
@@ -287,11 +367,13 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs given, int64_t n
             first[k] = start[entry[k]] + skip;
             count[k] = min(8, length[entry[k]] - skip);
             c[k] = runs.col[first[k] + min(slot, count[k] - 1)];
+            if (copy) v[k] = values.s_val[first[k] + min(slot, count[k] - 1)];
         }
 #pragma unroll
         for (int k = 0; k < kBatch; ++k) {
             if (u0 + k * kGroups >= total) break;
             if (unit_cols) unit_cols[8 * (before + u[k]) + slot] = c[k];
+            if (copy) values.unit_val[8 * (before + u[k]) + slot] = v[k];
             if (slot == 0) {
                 const int32_t row = runs.row(base + entry[k]);
                 HDR h;
