@@ -1047,10 +1047,10 @@ int group_slot(int G, int first) { return G * (G - 1) / 2 - 1 + first; }
 // G and `first` are chosen on a sample of the groups (about 8 000 rows' worth, at most 1 in 64 of them); the chosen grouping is then matched exactly.
 // (At most 1 in 16, every upload of a large matrix pays: 2.6 M rows 51 us, 1 in 64 19.)
 int group_sample(const sddmm_b200_engine *e) { return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(64, e->M / 8192))); }
-int enqueue_group_sample(sddmm_b200_engine *e, cudaStream_t s) {
+int enqueue_group_sample(sddmm_b200_engine *e) {
     const int every = group_sample(e);
     const dim3 grid(grid_for((e->M / 2 / every + 2) * 32, kBlock, e->sm_count * 2), 9);
-    k_group_match<<<grid, kBlock, 0, s>>>(e->d_rp, e->d_col, static_cast<int32_t>(e->M), static_cast<int32_t>(e->nnz), 0, 0, every, nullptr,
+    k_group_match<<<grid, kBlock, 0, e->stream>>>(e->d_rp, e->d_col, static_cast<int32_t>(e->M), static_cast<int32_t>(e->nnz), 0, 0, every, nullptr,
                                                   e->d_pc->group_cover, e->d_pc->group_count);
     CU_TRY(e, cudaGetLastError());
     return SDDMM_B200_OK;
@@ -1275,19 +1275,14 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     // (Panels of columns that turn out not to be sorted may be runs that overlap, at most the whole row in each: their sums fit 32 bits.)
     const int64_t most_units = std::max<int64_t>(forms.plain, forms.longs + 1) * (e->nnz / 8 + e->M);
     const bool list_aside = early_list && join_copies && e->nnz < 64 * e->M && most_units < (int64_t(1) << 31);
-    // The sample of the row groups comes before the list, which may leave its place to theirs, but not before the column scan: between it
-    // and the row statistics the sample waits for the copies' kernels to end, and the scan with it (18 M nonzeros, bf16: 50 us).
-    ListGate gate;
+    // The sample of the row groups comes behind the column scan: between it and the row statistics the sample waits for the copies'
+    // kernels to end, and the scan with it (18 M nonzeros, bf16: 50 us), and before the list aside it delays that one (5.2 M, K = 64,
+    // upload and run 244 -> 251).  A list behind it leaves its place to the groups' where the sample has found them.
     const bool groups = e->nnz > 0 && group_possible(e);
-    if (groups) {
-        gate.groups_from = groups_from(e);
-        gate.every = group_sample(e);
-    }
+    ListGate gate;
     if (list_aside) {
         CU_TRY(e, cudaEventRecord(e->ev_fork, s));
         CU_TRY(e, cudaStreamWaitEvent(e->side_stream, e->ev_fork, 0));
-        if (groups)
-            if (int rc = enqueue_group_sample(e, e->side_stream)) return rc;
         gate.columns_scanned = false;
         if (int rc = enqueue_unit_list(e, e->side_stream, forms, sums_beside, gate, UnitValues{e->d_sval, e->d_unit_sval})) return rc;
         CU_TRY(e, cudaEventRecord(e->ev_join, e->side_stream));
@@ -1303,9 +1298,13 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
             k_col_scan<false><<<scan_blocks, kColScanThreads, 0, s>>>(e->d_col, e->nnz, static_cast<int32_t>(e->N), e->d_rowstart, e->d_touched, e->d_pc);
         }
         CU_TRY(e, cudaGetLastError());
-        if (groups && !list_aside)
-            if (int rc = enqueue_group_sample(e, s)) return rc;
+        if (groups)
+            if (int rc = enqueue_group_sample(e)) return rc;
         if (early_list && !list_aside) {
+            if (groups) {
+                gate.groups_from = groups_from(e);
+                gate.every = group_sample(e);
+            }
             // (fp32 mode: tiles will most likely be looked for, and found, when the column scan's count is high enough)
             if (e->dense_possible && e->knob_offset_tiles <= 0) gate.tile_hint = (static_cast<unsigned long long>(e->nnz) + kTileHintShare - 1) / kTileHintShare;
             if (int rc = enqueue_unit_list(e, s, forms, sums_beside, gate)) return rc;
