@@ -992,6 +992,21 @@ bool list_by_size(const sddmm_b200_engine *e, int32_t long_rows) {
     return by_size(e->mode == SDDMM_B200_BF16, row, long_rows > 0, gathered_bytes(e, row), e->l2_bytes);
 }
 
+// Enqueue the kernel that writes the list, from tile sums that are there (scanned: as the units before each tile).
+template <typename Runs, typename HDR>
+int enqueue_build(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_t n, bool scanned, int64_t cap, HDR *units, int32_t *unit_cols,
+                  const ListGate &gate, bool by_size, const UnitValues &values) {
+    const int tiles = static_cast<int>(unit_tiles(n));
+    if constexpr (sizeof(HDR) == sizeof(int2)) {
+        if (by_size) k_unit_build<Runs, HDR, true><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate, values);
+        else k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate, values);
+    } else {
+        k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate, values);
+    }
+    CU_TRY(e, cudaGetLastError());
+    return SDDMM_B200_OK;
+}
+
 // Enqueue the list over n entries; *units = how many there are goes to the plan counters.  have_sums: k_row_stats has left the tile
 // sums and the total.
 template <typename Runs, typename HDR>
@@ -1006,14 +1021,7 @@ int enqueue_units(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_
     }
     const bool scanned = tiles > kDirectTiles;
     if (scanned) k_scan_sums<<<1, kScanBlock, 0, s>>>(e->d_scan_tiles, tiles, &e->d_pc->units);
-    if constexpr (sizeof(HDR) == sizeof(int2)) {
-        if (by_size) k_unit_build<Runs, HDR, true><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate, values);
-        else k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate, values);
-    } else {
-        k_unit_build<Runs, HDR, false><<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, cap, e->d_pc, units, unit_cols, scanned, gate, values);
-    }
-    CU_TRY(e, cudaGetLastError());
-    return SDDMM_B200_OK;
+    return enqueue_build(e, s, runs, n, scanned, cap, units, unit_cols, gate, by_size, values);
 }
 
 // Gathers of B that have to disappear before row groups are taken: 30 % of all, and as many as are worth the planning.  What they save
@@ -1169,12 +1177,17 @@ int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, const ListForms &for
     int st;
     if (forms.plain > 1 || forms.long_rows > 0) {
         // (the starts of the panels: in the half of the headers' memory that plain units leave)
-        const RunsOfForms runs{e->d_rp, e->d_col, M, nnz, forms, reinterpret_cast<int32_t *>(e->d_units + e->unit_cap + 8), 2 * (e->unit_cap + 8), have_sums};
+        const RunsOfForms runs{e->d_rp, e->d_col, M, nnz, forms, reinterpret_cast<int32_t *>(e->d_units + e->unit_cap + 8), 2 * (e->unit_cap + 8), have_sums, have_sums};
         // (a grid for either form: the longer list, or the one with more tiles)
         const int64_t n_plain = e->M * forms.plain, n_long = forms.long_rows > 0 ? e->M * (forms.longs + 1) : 0;
         const int64_t n = unit_tiles(n_long) > unit_tiles(n_plain) ? n_long : n_plain;
         const int64_t n_whole = forms.plain_for_8 && unit_tiles(e->M) > unit_tiles(n) ? e->M : n;
-        st = enqueue_units(e, s, runs, n_whole, false, e->unit_cap, e->d_units, e->d_unit_cols, gate, forms.plain_by_size || forms.long_by_size, values);
+        st = enqueue_units(e, s, runs, n_whole, false, e->unit_cap, e->d_units, e->d_unit_cols, gate, (!have_sums && forms.plain_by_size) || forms.long_by_size, values);
+        if (!st && have_sums) {
+            const bool scanned = unit_tiles(n_whole) > kDirectTiles;
+            const WholeRowsOfForms whole{RunsOfRows{e->d_rp, e->d_col, M, nnz}, forms};
+            st = enqueue_build(e, s, whole, e->M, scanned, e->unit_cap, e->d_units, e->d_unit_cols, gate, forms.plain_by_size, UnitValues{});
+        }
     } else {
         const RunsOfRows runs{e->d_rp, e->d_col, M, nnz};
         st = enqueue_units(e, s, runs, e->M, have_sums, e->unit_cap, e->d_units, e->d_unit_cols, gate, forms.plain_by_size);

@@ -13,11 +13,12 @@
 namespace sddmm {
 
 // ---- entries -> runs.  (A row_ptr that has not been validated yet may be anything: runs outside [0, nnz) are empty.) ----
-// settled(pc): the runs themselves, where the row statistics have a say (RunsOfForms); sorted(): whether they need sorted columns;
-// ordered(): whether a list that may be ordered by size is
+// settled(pc): the runs themselves, where the row statistics have a say (RunsOfForms); wanted(): whether k_unit_build is to list them;
+// sorted(): whether they need sorted columns; ordered(): whether a list that may be ordered by size is
 struct RunsOfRows {   // one entry per row: the whole row
     static constexpr bool kChosen = false;
     __device__ __forceinline__ const RunsOfRows &settled(const PlanCounters *) const { return *this; }
+    __device__ __forceinline__ bool wanted(const PlanCounters *) const { return true; }
     __device__ __forceinline__ bool sorted() const { return false; }
     __device__ __forceinline__ bool ordered() const { return true; }
     const int32_t *rp;
@@ -42,6 +43,7 @@ struct RunsOfPanels {
     bool by_size = true;
     const int32_t *cuts = nullptr;   // where panel p + 1 starts in row i, at p * M + i (k_panel_cuts; null: it is looked for, in each kernel)
     __device__ __forceinline__ const RunsOfPanels &settled(const PlanCounters *) const { return *this; }
+    __device__ __forceinline__ bool wanted(const PlanCounters *) const { return true; }
     __device__ __forceinline__ bool sorted() const { return panels > 1; }
     __device__ __forceinline__ bool ordered() const { return by_size; }
     __device__ __forceinline__ int32_t real_panels() const { return long_rows > 0 ? panels - 1 : panels; }   // (without the short rows)
@@ -152,12 +154,22 @@ struct RunsOfForms {
     int32_t *cuts;       // room for this many starts of panels
     int64_t cuts_room;
     bool have_sums;      // of whole rows
+    bool whole_apart;    // whole rows are listed by a kernel of their own (WholeRowsOfForms)
+    __device__ __forceinline__ bool wanted(const PlanCounters *pc) const { return !whole_apart || forms.choose_by_warp(pc, nnz).panels > 1; }
     __device__ __forceinline__ RunsOfPanels settled(const PlanCounters *pc) const {   // (by whole warps)
         const ListForms::Choice c = forms.choose_by_warp(pc, nnz);
         RunsOfPanels r{rp, col, M, nnz, c.panels, c.panel_cols, c.long_rows, c.by_size};
         if (static_cast<int64_t>(r.real_panels() - 1) * M <= cuts_room) r.cuts = cuts;
         return r;
     }
+};
+// ... the whole rows, where these are chosen.  (The kernel for either form takes 111 us for 18 M nonzeros in whole rows, this one 77.)
+struct WholeRowsOfForms {
+    static constexpr bool kChosen = false;
+    RunsOfRows rows;
+    ListForms forms;
+    __device__ __forceinline__ const RunsOfRows &settled(const PlanCounters *) const { return rows; }
+    __device__ __forceinline__ bool wanted(const PlanCounters *pc) const { return forms.choose_by_warp(pc, rows.nnz).panels == 1; }
 };
 // The starts of the panels, a thread per row: every entry of the list needs two, in both of its kernels, and each is a chain of loads.
 // (Whole rows: nothing to do here, nor in k_unit_sums where k_row_stats has left the sums.)
@@ -182,6 +194,7 @@ __device__ __forceinline__ void unit_group_rows(int32_t g, int32_t G, int32_t fi
 struct RunsOfGroups {   // one entry per row: the leader of a matching group speaks for its whole group
     static constexpr bool kChosen = false;
     __device__ __forceinline__ const RunsOfGroups &settled(const PlanCounters *) const { return *this; }
+    __device__ __forceinline__ bool wanted(const PlanCounters *) const { return true; }
     __device__ __forceinline__ bool sorted() const { return false; }
     __device__ __forceinline__ bool ordered() const { return false; }
     const int32_t *rp;
@@ -277,7 +290,7 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs given, int64_t n
                                                            int32_t *__restrict__ unit_cols, bool scanned, ListGate gate, UnitValues values) {
     // enqueued before the host has seen the counters: nothing is written for a pattern that it is about to refuse, or for one
     // that will be computed otherwise
-    if (list_unused(gate, pc)) return;
+    if (list_unused(gate, pc) || !given.wanted(pc)) return;
     const auto runs = given.settled(pc);
     if constexpr (Runs::kChosen) n = static_cast<int64_t>(runs.panels) * runs.M;
     // (unsorted columns that the column scan has yet to find: the runs overlap, and the list is not used)
