@@ -381,8 +381,8 @@ void choose_long_rows(sddmm_b200_engine *e) {
     if (b <= (bf ? 1.0 : kPanelsFrom) * l2 && !(e->knob_long_rows >= 1 && e->knob_panels >= 2)) return;
     // fp32: B 333 MB, K = 32: 4 panels 407 us, 6 402 us, 8 401 us; 189 MB, 2 / 3 / 4 / 6: 300 / 287 / 286 / 286
     // bf16, whose lists are not ordered by size and whose kernel loads all slots: a short run costs as much as a full one, so fewer
-    // panels and, with few of them, shorter rows too.  36 M, 2.6 M rows, K = 32, B 166 MB: 3 panels from 64 nonzeros on 358 us, 4
-    // panels from 128 on 363.
+    // panels and, with few of them, shorter rows too.  36 M, 2.6 M rows, K = 32, B 166 MB: 3 panels from 64 nonzeros on 348 us, 4
+    // panels from 128 on 354.
     e->panels_long = e->knob_panels >= 1 ? static_cast<int>(std::min(64.0, e->knob_panels))
                                          : static_cast<int>(std::max(bf ? 2.0 : 4.0, std::min(8.0, std::ceil(b / (0.5 * l2)))));
     if (e->panels_long < 2) return;
@@ -1016,8 +1016,8 @@ int enqueue_units(sddmm_b200_engine *e, cudaStream_t s, const Runs &runs, int64_
     if (int rc = check_tile_sums(e, tiles)) return rc;
     if (!have_sums) {
         if constexpr (!Runs::kChosen) CU_TRY(e, cudaMemsetAsync(&e->d_pc->units, 0, sizeof(unsigned long long), s));
-        else k_panel_cuts<<<grid_for(e->M, kUnitBlock, e->sm_count * 8), kUnitBlock, 0, s>>>(runs, e->d_pc);
-        k_unit_sums<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->d_pc);
+        else k_panel_cuts<<<grid_for(e->M, kUnitBlock, e->sm_count * 8), kUnitBlock, 0, s>>>(runs, e->d_pc, gate);
+        k_unit_sums<<<tiles, kUnitBlock, 0, s>>>(runs, n, e->d_scan_tiles, e->d_pc, gate);
     }
     const bool scanned = tiles > kDirectTiles;
     if (scanned) k_scan_sums<<<1, kScanBlock, 0, s>>>(e->d_scan_tiles, tiles, &e->d_pc->units);

@@ -171,9 +171,35 @@ struct WholeRowsOfForms {
     __device__ __forceinline__ const RunsOfRows &settled(const PlanCounters *) const { return rows; }
     __device__ __forceinline__ bool wanted(const PlanCounters *pc) const { return forms.choose_by_warp(pc, rows.nnz).panels == 1; }
 };
+// What may show that a list enqueued before the host has seen the counters will not be used (default: nothing).  Its kernels read
+// here only what kernels BEFORE it in its stream have finished: threads of one block that saw a count grow would disagree.
+struct ListGate {
+    unsigned long long tile_hint = ~0ull;   // nonzeros that look like 64-wide tiles from which on these will be looked for, and found
+    double groups_from = -1.0;              // gathers saved by row groups from which on these will be taken (< 0: not looked at)
+    int every = 1;                          // of how many groups one is in the sample
+    bool columns_scanned = true;            // false: the column scan runs beside (nothing that it counts is read)
+};
+// Gathers that the best grouping saves, by the sample, and its slot
+__host__ __device__ __forceinline__ double group_saving(const unsigned long long *cover, int every, int *slot) {
+    double best = 0.0;
+    for (int y = 0; y < 9; ++y) {
+        const int G = y < 2 ? 2 : y < 5 ? 3 : 4;
+        const double saved = static_cast<double>(cover[y]) * every * (1.0 - 1.0 / G);
+        if (saved > best) { best = saved; *slot = y; }
+    }
+    return best;
+}
+constexpr int kGroupRowMax = 8192;   // (nonzeros of a row) matrices with longer ones are not grouped
+__device__ __forceinline__ bool list_unused(const ListGate &gate, const PlanCounters *pc) {
+    if (gate.columns_scanned && pc->window_hint >= gate.tile_hint) return true;
+    int slot;
+    return gate.groups_from >= 0.0 && pc->max_row_nnz <= kGroupRowMax && group_saving(pc->group_cover, gate.every, &slot) >= gate.groups_from;
+}
+
 // The starts of the panels, a thread per row: every entry of the list needs two, in both of its kernels, and each is a chain of loads.
 // (Whole rows: nothing to do here, nor in k_unit_sums where k_row_stats has left the sums.)
-__global__ void __launch_bounds__(kUnitBlock) k_panel_cuts(RunsOfForms given, PlanCounters *__restrict__ pc) {
+__global__ void __launch_bounds__(kUnitBlock) k_panel_cuts(RunsOfForms given, PlanCounters *__restrict__ pc, ListGate gate) {
+    if (list_unused(gate, pc)) return;
     const RunsOfPanels runs = given.settled(pc);
     if (blockIdx.x == 0 && threadIdx.x == 0 && !(given.have_sums && runs.panels == 1)) pc->units = 0;
     if (!runs.cuts || runs.panels == 1) return;
@@ -218,7 +244,8 @@ struct RunsOfGroups {   // one entry per row: the leader of a matching group spe
 
 // pass 1: units of every tile; the grand total goes to pc->units
 template <typename Runs>
-__global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs given, int64_t n, int32_t *__restrict__ tile_sums, PlanCounters *__restrict__ pc) {
+__global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs given, int64_t n, int32_t *__restrict__ tile_sums, PlanCounters *__restrict__ pc, ListGate gate) {
+    if (list_unused(gate, pc)) return;   // (nor will the list be)
     const auto runs = given.settled(pc);
     if constexpr (Runs::kChosen) {
         if (given.have_sums && runs.panels == 1) {   // (the grid may be a longer list's: no units in the tiles past this one's end)
@@ -241,31 +268,6 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs given, int64_t n,
         tile_sums[blockIdx.x] = total;
         if (total) atomicAdd(&pc->units, static_cast<unsigned long long>(total));
     }
-}
-
-// What may show that a list enqueued before the host has seen the counters will not be used (default: nothing).  k_unit_build reads
-// here only what kernels BEFORE it in its stream have finished: threads of one block that saw a count grow would disagree.
-struct ListGate {
-    unsigned long long tile_hint = ~0ull;   // nonzeros that look like 64-wide tiles from which on these will be looked for, and found
-    double groups_from = -1.0;              // gathers saved by row groups from which on these will be taken (< 0: not looked at)
-    int every = 1;                          // of how many groups one is in the sample
-    bool columns_scanned = true;            // false: the column scan runs beside (nothing that it counts is read)
-};
-// Gathers that the best grouping saves, by the sample, and its slot
-__host__ __device__ __forceinline__ double group_saving(const unsigned long long *cover, int every, int *slot) {
-    double best = 0.0;
-    for (int y = 0; y < 9; ++y) {
-        const int G = y < 2 ? 2 : y < 5 ? 3 : 4;
-        const double saved = static_cast<double>(cover[y]) * every * (1.0 - 1.0 / G);
-        if (saved > best) { best = saved; *slot = y; }
-    }
-    return best;
-}
-constexpr int kGroupRowMax = 8192;   // (nonzeros of a row) matrices with longer ones are not grouped
-__device__ __forceinline__ bool list_unused(const ListGate &gate, const PlanCounters *pc) {
-    if (gate.columns_scanned && pc->window_hint >= gate.tile_hint) return true;
-    int slot;
-    return gate.groups_from >= 0.0 && pc->max_row_nnz <= kGroupRowMax && group_saving(pc->group_cover, gate.every, &slot) >= gate.groups_from;
 }
 
 // The units' copies of the S values, for lists in panels (unit_val null: they are made later, k_unit_values)
