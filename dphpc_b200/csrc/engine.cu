@@ -414,7 +414,10 @@ int choose_panels(const sddmm_b200_engine *e) {
         if (e->seg_slices > 1) return mean < 11.0 ? 1 : 2;
         return mean < (cols <= 32 ? 24.0 : 16.0) || static_cast<double>(e->nnz) * static_cast<double>(cols) * 4.0 < 1.4e9 ? 1 : 2;
     }
-    if (bf && cols > 32 && cols <= 64 && b_bytes <= 1.5 * l2) return 1;
+    // (bf16 rows of 33 to 64, where no list is built early: a held run / upload and run, 1 / 2 panels, B 157 MB, mean 26 / 45 499 / 479, 1370 / 1597 and
+    // 574 / 511, 1374 / 1579; 186 MB, mean 26 / 35 / 45 625 / 601, 1628 / 1884, 709 / 567, 1648 / 1736 and 772 / 547, 1632 / 1617; 211 MB, mean
+    // 26 / 35 686 / 621, 1760 / 1971 and 823 / 591, 1837 / 1827)
+    if (bf && cols > 32 && cols <= 64 && b_bytes <= (mean < 32.0 ? 1.5 : 1.3) * l2) return 1;
     // (K = 32, B 262 / 388 MB, mean 8 / 10 / 12: 347 / 342, 418 / 392, 500 / 438 and 616 / 569, 726 / 654, 719 / 638)
     if (mean < (bf ? (cols <= 32 ? 26.0 : cols <= 64 ? 20.0 : 13.0) : cols <= 32 ? (b_bytes > 1.8 * l2 ? 10.0 : 13.0) : cols <= 64 ? 11.0 : 9.0)) return 1;
     // Slices of 128 columns: panels that fit L2 one by one, if an average row has 3 nonzeros for each, or none.  Sustained, B 205 MB,
