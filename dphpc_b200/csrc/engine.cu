@@ -1099,7 +1099,8 @@ int build_rowgroup_plan(sddmm_b200_engine *e, const PlanCounters &base_pc) {
         if (pc.units == 0 || pc.units > static_cast<unsigned long long>(std::min<int64_t>(e->unit_cap, kUnitLimit)))
             return fail(e, SDDMM_B200_ERR_CUDA, "row-group plan: %llu units for a list of %lld", pc.units, (long long)e->unit_cap);
         e->n_units = static_cast<int32_t>(pc.units);
-        if (int rc = seg_grid(e, reinterpret_cast<const void *>(pick_rowseg_group(e, best)), kRowSegWarps, e->mode == SDDMM_B200_BF16 ? 8 : 32 / group_lanes(e) * group_run(e), e->n_units, &p.rowgroup_grid)) return rc;
+        const int per_step = e->mode == SDDMM_B200_BF16 ? 8 : 32 / group_lanes(e) * group_run(e);
+        if (int rc = seg_grid(e, reinterpret_cast<const void *>(pick_rowseg_group(e, best)), kRowSegWarps, per_step, e->n_units, &p.rowgroup_grid)) return rc;
         p.rowseg_units = e->n_units;
         p.rowseg_panels = 1;
     } else {
@@ -1180,16 +1181,16 @@ int enqueue_unit_list(sddmm_b200_engine *e, cudaStream_t s, const ListForms &for
     int st;
     if (forms.plain > 1 || forms.long_rows > 0) {
         // (the starts of the panels: in the half of the headers' memory that plain units leave)
-        const RunsOfForms runs{e->d_rp, e->d_col, M, nnz, forms, reinterpret_cast<int32_t *>(e->d_units + e->unit_cap + 8), 2 * (e->unit_cap + 8), have_sums, have_sums};
-        // (a grid for either form: the longer list, or the one with more tiles)
-        const int64_t n_plain = e->M * forms.plain, n_long = forms.long_rows > 0 ? e->M * (forms.longs + 1) : 0;
-        const int64_t n = unit_tiles(n_long) > unit_tiles(n_plain) ? n_long : n_plain;
-        const int64_t n_whole = forms.plain_for_8 && unit_tiles(e->M) > unit_tiles(n) ? e->M : n;
-        st = enqueue_units(e, s, runs, n_whole, false, e->unit_cap, e->d_units, e->d_unit_cols, gate, (!have_sums && forms.plain_by_size) || forms.long_by_size, values);
+        const RunsOfForms runs{e->d_rp, e->d_col, M, nnz, forms, reinterpret_cast<int32_t *>(e->d_units + e->unit_cap + 8), 2 * (e->unit_cap + 8),
+                               have_sums, have_sums};
+        int64_t most = e->M;   // entries of the form with the most tiles: the grid is made for that one
+        for (const int64_t n : {e->M * forms.plain, forms.long_rows > 0 ? e->M * (forms.longs + 1) : 0})
+            if (unit_tiles(n) > unit_tiles(most)) most = n;
+        st = enqueue_units(e, s, runs, most, false, e->unit_cap, e->d_units, e->d_unit_cols, gate,
+                           (!have_sums && forms.plain_by_size) || forms.long_by_size, values);
         if (!st && have_sums) {
-            const bool scanned = unit_tiles(n_whole) > kDirectTiles;
             const WholeRowsOfForms whole{RunsOfRows{e->d_rp, e->d_col, M, nnz}, forms};
-            st = enqueue_build(e, s, whole, e->M, scanned, e->unit_cap, e->d_units, e->d_unit_cols, gate, forms.plain_by_size, UnitValues{});
+            st = enqueue_build(e, s, whole, e->M, unit_tiles(most) > kDirectTiles, e->unit_cap, e->d_units, e->d_unit_cols, gate, forms.plain_by_size, UnitValues{});
         }
     } else {
         const RunsOfRows runs{e->d_rp, e->d_col, M, nnz};
@@ -1292,7 +1293,7 @@ int build_plan(sddmm_b200_engine *e, int item_nnz, int n_items, bool join_copies
     const int64_t most_units = std::max<int64_t>(forms.plain, forms.longs + 1) * (e->nnz / 8 + e->M);
     const bool list_aside = early_list && join_copies && e->nnz < 64 * e->M && most_units < (int64_t(1) << 31);
     // The sample of the row groups comes behind the column scan: between it and the row statistics the sample waits for the copies'
-    // kernels to end, and the scan with it (18 M nonzeros, bf16: 50 us), and before the list aside it delays that one (5.2 M, K = 64,
+    // kernels to end, and the scan with it (37 M nonzeros, bf16: 90 us), and before the list aside it delays that one (5.2 M, K = 64,
     // upload and run 244 -> 251).  A list behind it leaves its place to the groups' where the sample has found them.
     const bool groups = e->nnz > 0 && group_possible(e);
     ListGate gate;

@@ -58,8 +58,9 @@ constexpr int kRowGroupWarps = 8;
 // G (G - 1) / 2 - 1 + first.  (row_ptr and the columns may not have been validated yet: row bounds are checked here, columns are only compared.)
 // The counts leave a block as one pair of atomics: with a pair per matching group, all on the same two addresses, the exact match of
 // 36.8 M nonzeros in 3 x 3 blocks took 245 us; without 100, and 55 with the next bounds a group ahead.
-__global__ void __launch_bounds__(kPlanBlock) k_group_match(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int32_t M, int32_t nnz, int32_t G, int32_t first,
-                                                            int32_t every, uint8_t *__restrict__ group_ok, unsigned long long *__restrict__ cover, int *__restrict__ groups) {
+__global__ void __launch_bounds__(kPlanBlock) k_group_match(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, int32_t M, int32_t nnz,
+                                                            int32_t G, int32_t first, int32_t every, uint8_t *__restrict__ group_ok,
+                                                            unsigned long long *__restrict__ cover, int *__restrict__ groups) {
     if (G == 0) {
         const int y = static_cast<int>(blockIdx.y);
         G = y < 2 ? 2 : y < 5 ? 3 : 4;

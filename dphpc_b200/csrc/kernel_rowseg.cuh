@@ -9,9 +9,11 @@
 // of a group holds bytes [32t, 32t + 32) of the piece in one 256-bit load, so one load instruction fetches the same piece
 // of 8 B rows (one per unit), and the A piece in registers serves the unit's 8 nonzeros.  The loop is ROLLING: as soon as
 // the B piece of slot i has been multiplied, its registers are given to the piece that slot needs next (the next piece of
-// the same units, or the first one of the next units), so a warp has 8 loads of 1 KB in flight all the time; unit headers
-// and column indices run one to two steps ahead, the A piece one stage ahead.  Every load is unconditional and in range (a
-// slot past a segment's end repeats its last nonzero, a group past the list's end the last unit); stores are predicated.
+// the same units, or the first one of the next units), so a warp has up to 8 loads of 1 KB in flight all the time; unit headers
+// and column indices run one to two steps ahead, the A piece one stage ahead.  Every load is in range (a slot past a segment's
+// end repeats its last nonzero, a group past the list's end the last unit).  Two neighbouring slots that no unit of a step fills
+// are left out by the whole warp (see most_slots): their registers keep what an earlier step or the first one, which loads all
+// slots, has put there, a slot's sum is made of its own registers only, and sums of slots past a unit's count are never stored.
 //
 // What bounds it: per nonzero one B row crosses from L2 to the SM (random 128-byte rows that hit L2: at most 153 G rows/s
 // measured, 64 bytes per clock and SM) and, where B does not fit L2, comes from HBM.  37.5 M nonzeros, K = 32, B in L2:
@@ -158,8 +160,8 @@ __host__ __device__ constexpr int a_prefetch_stages(int pieces) { return pieces 
 
 // fp32 rows of NP pieces.  (From NP = 3 on the 128 registers do not quite hold the loop, a few words of it are spilled; with the
 // registers of one CTA per SM it is 20 % slower.)  The last piece may be partial: the lanes past its end
-// read the row's last 32 bytes once more and multiply them by zero.  SPECIALS: such lanes leave the product out, as a factor of zero does not where B holds an infinity (0 x Inf is
-// NaN).  Rows of one piece always do (K = 16: 335 against 336 us); longer ones only where a conversion of B has seen a non-finite
+// read the row's last 32 bytes once more and multiply them by zero.  SPECIALS: such lanes leave the product out, as a factor of
+// zero does not where B holds an infinity (0 x Inf is NaN).  Rows of one piece always do (K = 16: 335 against 336 us); longer ones only where a conversion of B has seen a non-finite
 // element in the last 32 bytes of a row, since it costs registers that the rolling loop wants (ragged last piece, in L2, K = 33 /
 // 50 / 100: 84 / 46.7 / 110 us without, 89 / 47.8 / 115 with it; zeros read in place of B: 105 / 55 / 114).  COPIES:
 // S values come from per-unit copies in list order (column panels: a run is a short piece of its row, whose sectors two or more panel
@@ -189,9 +191,9 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
     // The slots that any unit of a step fills.  Short runs lie side by side in the list, by length (unit_plan.cuh), so where rows are
     // short whole steps have few; the loads of the others are left out (their sums come from old registers and are not stored).
     // Power-law rows, K = 32: 5 M nonzeros 66 -> 60 us, 36 M 428 -> 402; Poisson rows of 10 48 -> 45.  One slot at a time
-    // 396 us, but K = 128 in L2 100 against 95; loads that depend on their own lane's count serialise the loop.  (Not for rows of
-    // one ragged piece, 0.5 M nonzeros, K = 16 15.6 against 18 us, nor of three pieces and panels of rows of an odd number, which the compiler does not roll with the branches in: K = 96, panels, 9 M
-    // nonzeros 286 -> 349 us, 52 000 nonzeros 13 -> 15.)
+    // 396 us, but K = 128 in L2 100 against 95; loads that depend on their own lane's count serialise the loop.
+    // Not for rows of one ragged piece (0.5 M nonzeros, K = 16 15.6 against 18 us), nor of three pieces and panels of rows of an odd
+    // number, which the compiler does not roll with the branches in (K = 96, panels, 9 M nonzeros 286 -> 349 us, 52 000 13 -> 15).
     constexpr bool kLeaveOut = NP != 3 && !(NP == 1 && TAIL == kTailSpecials) && !(COPIES && NP > 1 && NP % 2 == 1);
     auto most_slots = [&](const int2 &u) -> int { return static_cast<int>(__reduce_max_sync(kFullMask, static_cast<unsigned>(u.y) & 7u)) + 1; };
     auto piece_offset = [&](int p) -> int { return p == NP - 1 ? o_last : 128 * p; };
@@ -261,7 +263,8 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_kernel(cons
 // The same for whole rows (NP even) of a B that does not fit L2 and is gathered without column panels: DRAM is the
 // bound, and it likes few rows open at a time.  The stages go through all pieces of 4 slots, two pieces of 128 bytes at a
 // time, before the other 4: half the rows in flight, twice the bytes of each.  9 M nonzeros in rows of 13, B 358 / 717 MB:
-// K = 128 697 -> 638 us, K = 256 1581 -> 1559; 13 M nonzeros in rows of 9, B 373 MB: K = 64 558 -> 524; with B in L2 the order above is faster (K = 128 385 against 414).
+// K = 128 697 -> 638 us, K = 256 1581 -> 1559; 13 M nonzeros in rows of 9, B 373 MB: K = 64 558 -> 524; with B in L2 the order above is
+// faster (K = 128 385 against 414).
 template <int NP, bool SPECIALS, int STEP>
 __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_wide_kernel(const RowSegArgs args) {
     const int lane = threadIdx.x & 31;
@@ -480,9 +483,10 @@ __global__ void __launch_bounds__(kRowSegWarps * 32, MINB) sddmm_rowseg_bf16_ker
 // lanes, lane t of it holds bytes [32 t, 32 t + 32) of every row: a row of A or B is ONE 256-bit load.  36.8 M nonzeros in
 // 3 x 3 blocks, K = 32 / 64: 165 / 263 us, against 206 / 292 us for rows in pieces of 16 bytes on 8 lanes (twice the load instructions,
 // 64-bit index arithmetic and a shuffle per column index; 3 CTAs per SM at K = 32).
-// What bounds it: the load/store unit, 139 wavefronts of 128 bytes per 32 columns at K = 64 (B rows 64, A rows 24, shuffles of the
-// reduction 21, indices, S and P the rest), and the latency that 16 warps leave.  So RUN units of one row group go to the same
-// lanes, one after the other, and its rows of A stay in registers from one to the next (an A row is a fourth of the traffic):
+// What bounds it: the load/store unit, 139 wavefronts of 128 bytes per 32 columns at K = 64 with RUN = 2 (B rows 64, shuffles of the
+// reduction 22, A rows 12 by the count of the loads, indices, S and P the rest), and the latency that 16 warps leave.  So RUN units of
+// one row group go to the same lanes, one after the other, and its rows of A stay in registers from one to the next (with RUN = 1
+// they are 24 wavefronts):
 // RUN = 1 / 2 / 4, K = 64: 273 / 263 / 274 us, K = 32, where a row is half as long, 165 / 171 / 188; 14 M nonzeros, K = 128:
 // 210 / 198 / 200, 7 M, K = 256 (two partial units of a row weigh more there): 182 / 196 / 199.  The same two by sddmm_rowseg_kernel,
 // which gathers each B row three times: 423 / 409 us.
@@ -499,9 +503,9 @@ struct RowSegGroupArgs {
     uint32_t row_bytes;        // of a row of A or B, a multiple of 32
 };
 
-// WHOLE: a row fills its lanes.  Else (rows of 16 or 96 elements, say) the lanes past its end read its last 32 bytes once more and leave
-// their products out.  20 M nonzeros, K = 8 / 16: 87 / 91 us, by sddmm_rowseg_kernel 175 / 176; 14 M, K = 96 215 (325), 7 M, K = 192 / 224 201 / 203
-// (317 / 361).  Zeros in place of both operands, from a line of their own, cost a wavefront per load: K = 96 253, K = 192 247.
+// WHOLE: a row fills its lanes.  Else (rows of 16 or 96 elements, say) the lanes past its end read its last 32 bytes once more and
+// leave their products out.  20 M nonzeros, K = 8 / 16: 87 / 91 us, by sddmm_rowseg_kernel 175 / 176; 14 M, K = 96 215 (325), 7 M, K = 192 /
+// 224 201 / 203 (317 / 361).  Zeros in place of both operands, from a line of their own, cost a wavefront per load: K = 96 253, K = 192 247.
 template <int LPR, int NR, int RUN, bool WHOLE>
 __global__ void __launch_bounds__(kRowSegWarps * 32, 2) sddmm_rowseg_group_kernel(const RowSegGroupArgs args) {
     constexpr int kRun = RUN;                    // consecutive units of a group of lanes

@@ -118,7 +118,8 @@ struct ListForms {
     }
     __host__ __device__ __forceinline__ Choice of_rows(const Rows &r, int64_t nnz) const {
         // panels for the long rows only pay when those hold a good share of the nonzeros, 40 %
-        if (long_rows > 0 && (long_always || 5 * r.in_long >= 2 * static_cast<unsigned long long>(nnz))) return Choice{longs + 1, long_cols, long_rows, long_by_size};
+        const bool mostly_long = 5 * r.in_long >= 2 * static_cast<unsigned long long>(nnz);
+        if (long_rows > 0 && (long_always || mostly_long)) return Choice{longs + 1, long_cols, long_rows, long_by_size};
         // a mean that barely pays for panels has to be that of most rows, not of a few long ones: 60 % of them of 8 nonzeros or more
         if (plain > 1 && plain_for_8 && 10 * r.of_8 < 6 * r.rows) return Choice{1, plain_cols, 0, plain_by_size};
         return Choice{plain, plain_cols, 0, plain_by_size};
@@ -244,7 +245,8 @@ struct RunsOfGroups {   // one entry per row: the leader of a matching group spe
 
 // pass 1: units of every tile; the grand total goes to pc->units
 template <typename Runs>
-__global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs given, int64_t n, int32_t *__restrict__ tile_sums, PlanCounters *__restrict__ pc, ListGate gate) {
+__global__ void __launch_bounds__(kUnitBlock) k_unit_sums(Runs given, int64_t n, int32_t *__restrict__ tile_sums, PlanCounters *__restrict__ pc,
+                                                          ListGate gate) {
     if (list_unused(gate, pc)) return;   // (nor will the list be)
     const auto runs = given.settled(pc);
     if constexpr (Runs::kChosen) {
@@ -298,7 +300,8 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs given, int64_t n
     // (unsorted columns that the column scan has yet to find: the runs overlap, and the list is not used)
     if (pc->bad_row_ptr || pc->bad_coo || (runs.sorted() && gate.columns_scanned && pc->unsorted_cols)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) pc->list_built = 1;
-    const bool by_size = BY_SIZE && runs.ordered() && kShortRowShare * (pc->hist[1] + pc->hist[2] + pc->hist[3]) >= pc->rows_nonempty;   // (rows of 1 .. 7 nonzeros)
+    // (rows of 1 .. 7 nonzeros)
+    const bool by_size = BY_SIZE && runs.ordered() && kShortRowShare * (pc->hist[1] + pc->hist[2] + pc->hist[3]) >= pc->rows_nonempty;
     constexpr int kPerThread = kUnitTileMax / kUnitBlock;
     __shared__ int32_t first_unit[kUnitTileMax];   // of the tile's entries, relative to the tile
     __shared__ int32_t start[kUnitTileMax], length[kUnitTileMax];
@@ -371,7 +374,8 @@ __global__ void __launch_bounds__(kUnitBlock) k_unit_build(Runs given, int64_t n
             u[k] = min(u0 + k * kGroups, total - 1);
             entry[k] = 0;
         }
-        for (int half = !BY_SIZE || u0 < in_order ? tile >> 1 : 0; half > 0; half >>= 1)   // the entry that holds unit u: the last one that starts at or before it (tile: a power of two)
+        // the entry that holds unit u: the last one that starts at or before it (tile: a power of two)
+        for (int half = !BY_SIZE || u0 < in_order ? tile >> 1 : 0; half > 0; half >>= 1)
 #pragma unroll
             for (int k = 0; k < kBatch; ++k)
                 if (first_unit[entry[k] + half] <= u[k]) entry[k] += half;

@@ -186,9 +186,9 @@ int sddmm_b200_get_plan(sddmm_b200_engine *e, sddmm_b200_plan_info *info);
  *   "k_slices"      fp32 storage: 1 = take K (K >= 128 and a multiple of 64) in slices of 64 columns, 64 = the same,
  *                   copied one after the other where K is 193 to 256, 128 = of 128 columns (K a multiple of 128), one launch each over the same segment list, adding to P.val (default, by K and size, when B is about as
  *                   large as the L2 or larger), 0 = never
- *   "long_rows"     B larger than L2: column panels for the rows of at least this many nonzeros only, the shorter rows follow
- *                   whole (default: 64 or 128, chosen with the number of panels, when such rows hold at least 40 % of the
- *                   nonzeros); 0 = never
+ *   "long_rows"     B of 0.85 times L2 or more (bf16: more than L2): column panels for the rows of at least this many nonzeros only, the
+ *                   shorter rows follow whole (default: 128, in bf16 with up to four panels 64, when such rows hold at least 40 % of
+ *                   the nonzeros); 0 = never
  *   "dense_split3"  fp32-grade mode on dense tiles: 1 = operands through three shared-memory slots and two accumulators in
  *                   tensor memory (default for K >= 64), 0 = one A block + one B block like the other modes */
 int sddmm_b200_set_knob(sddmm_b200_engine *e, const char *name, double value);
